@@ -36,6 +36,7 @@
 // site tensors are not bit-identical to the reference; everything a caller
 // can observe (statevector, probabilities, outcomes) is gauge-invariant and
 // held to a tolerance.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -48,6 +49,8 @@
 #include "dq_gates.hpp"
 #include "dq_handle.cuh"
 #include "dq_rng.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace dq {
 namespace {
@@ -73,7 +76,8 @@ struct MpsView {
   int32_t* cbits;        // batch x ncb
   const dq_cond* conds;
   double2* scratch;      // batch x scratch_elems (global fallback of the SVD work area)
-  int* flags;            // [0] status, [1] first failing instruction, [2] capacity needed
+  int* flags;            // [0] status, [1] first failing instruction, [2] capacity needed,
+                         // [3] first operation of the launch that overflowed it
   unsigned long long* svd_calls;
   const MpsOp* ops;      // the program's operations; a launch runs ops[first + blockIdx.y]
   uint64_t site_elems;   // cap * 2 * cap
@@ -213,6 +217,7 @@ __global__ void __launch_bounds__(1024) k_mps_2q(MpsView v, uint32_t first, uint
   __shared__ double s_part[32];
   __shared__ double s_n2;
   const uint32_t b = blockIdx.x;
+  if (v.flags[3] < (int)first) return;  // an earlier launch overflowed the capacity
   if (!cond_ok(v, op, b)) return;
   uint32_t* dm = v.dims + (uint64_t)b * (v.n + 1);
   const uint32_t q = op.q, cap = v.cap;
@@ -360,6 +365,7 @@ __global__ void __launch_bounds__(1024) k_mps_2q(MpsView v, uint32_t first, uint
     if (keep > cap) {
       atomicMax(&v.flags[2], (int)keep);
       atomicMax(&v.flags[0], MF_CAPACITY);
+      atomicMin(&v.flags[3], (int)first);
     } else {
       atomicAdd(v.svd_calls, 1ull);
     }
@@ -423,6 +429,439 @@ __global__ void __launch_bounds__(1024) k_mps_2q(MpsView v, uint32_t first, uint
   if (tid == 0) dm[q + 1] = keep;
 }
 
+// ---- one step spread over a thread-block cluster ---------------------------------
+//
+// k_mps_2q_cl: the same step for capacities up to kClusterCap with the columns
+// of G spread over the C CTAs of a cluster.  FP64 latency and issue bound (a
+// chain of dependent rounds), so what counts is how few instructions one SM
+// runs per round: a single CTA rotates all cols/2 pairs of a round on one SM,
+// and above capacity 32 it does so out of L2.  Here every CTA keeps two
+// blocks of b <= 8 columns (cols = 2 C b at capacity 64 and C = 8) in shared
+// memory and rotates the pairs that cross them, one warp per pair with its
+// first column in registers; then the blocks move on by the round-robin
+// tournament of blocks (2C - 1 moves make every pair of blocks meet), pulled
+// from the neighbours' shared memory into a second buffer so that one cluster
+// barrier per move is enough.  Pairs inside a block are rotated once a sweep.
+// A sweep rotates every pair of columns exactly once, as the one-CTA form does.
+// A step with few columns uses fewer of the CTAs for its sweeps (16 columns
+// per CTA) and all of them to build theta.
+// One 20-qubit brickwork state at bond 64 (190 steps): 145 ms with one CTA per
+// step and the run repeated at capacities 16, 32 and 64, 16.1 ms here.
+constexpr uint32_t kClWarps = 8;
+constexpr uint32_t kClThreads = 32 * kClWarps;
+constexpr uint32_t kClusterCap = 96;  // two buffers of two blocks stay below 220 KB at C = 8
+
+// rows of a column in shared memory: a whole number of warp widths
+__host__ __device__ inline uint32_t cl_rpl(uint32_t rows) {
+  const uint32_t r = (rows + 31) / 32;
+  return r <= 4 ? r : 6;
+}
+__host__ __device__ inline uint32_t cl_block(uint32_t cols, uint32_t ctas) {
+  return (cols + 2 * ctas - 1) / (2 * ctas);
+}
+// CTAs that hold columns: blocks of at most 8 columns where the cluster allows
+__host__ __device__ inline uint32_t cl_active(uint32_t cols, uint32_t ctas) {
+  uint32_t c = 1;
+  while (c < ctas && 16 * c < cols) c *= 2;
+  return c;
+}
+// double2 elements of one block buffer at capacity cap
+__host__ __device__ inline uint64_t cl_block_elems(uint32_t cap, uint32_t ctas) {
+  const uint32_t b = cl_block(2 * cap, ctas);
+  return (uint64_t)(b < 8 ? 8 : b) * 32 * cl_rpl(2 * cap);
+}
+__host__ __device__ inline uint64_t cl_smem_bytes(uint32_t cap, uint32_t ctas) {
+  return cl_block_elems(cap, ctas) * (ctas > 1 ? 4 : 2) * sizeof(double2);
+}
+
+// Sums of four values over the warp: the first two exchanges halve the values
+// a lane carries (10 shuffled doubles instead of 20).
+__device__ __forceinline__ void warp_sum4(double& a, double& b, double& c, double& d, int lane) {
+  const unsigned full = 0xffffffffu;
+  const bool h = lane & 16, q = lane & 8;
+  double x = h ? c : a, y = h ? d : b;
+  x += __shfl_xor_sync(full, h ? a : c, 16);
+  y += __shfl_xor_sync(full, h ? b : d, 16);
+  double z = q ? y : x;
+  z += __shfl_xor_sync(full, q ? x : y, 8);
+  z += __shfl_xor_sync(full, z, 4);
+  z += __shfl_xor_sync(full, z, 2);
+  z += __shfl_xor_sync(full, z, 1);
+  a = __shfl_sync(full, z, 0);
+  b = __shfl_sync(full, z, 8);
+  c = __shfl_sync(full, z, 16);
+  d = __shfl_sync(full, z, 24);
+}
+
+// The rotation of jacobi_rotation as (c, sigma = s e^{i phi}) with two
+// dependent reciprocal square roots: with d = beta - alpha and r = sqrt(d^2 +
+// 4 |gamma|^2), cos 2x = |d| / r and sin 2x = 2 |gamma| / r give
+// c^2 = (1 + |d| / r) / 2 and sigma = sign(d) gamma / (r c).
+__device__ __forceinline__ bool jacobi_cs(double al, double be, double gr, double gi, double tol2, double neg,
+                                          double& c, double& sr, double& si) {
+  const double g2 = gr * gr + gi * gi;
+  if (!(g2 > tol2 * al * be) || (al <= neg && be <= neg) || !(g2 > 0.0)) return false;
+  const double d = be - al;
+  const double rr = rsqrt(d * d + 4.0 * g2);
+  const double c2 = 0.5 + 0.5 * fabs(d) * rr;
+  const double ic = rsqrt(c2);
+  c = c2 * ic;
+  const double f = copysign(rr * ic, d);
+  sr = f * gr;
+  si = f * gi;
+  return true;
+}
+
+// Rotates the pair (x in registers, column y in shared memory); true if it was.
+template <int RPL>
+__device__ __forceinline__ bool cl_pair(double2 (&x)[RPL], double2* yc, int lane, double tol2, double neg) {
+  double2 y[RPL];
+  double al = 0.0, be = 0.0, gr = 0.0, gi = 0.0;
+#pragma unroll
+  for (int k = 0; k < RPL; ++k) {
+    y[k] = yc[lane + 32 * k];
+    al = fma(x[k].x, x[k].x, fma(x[k].y, x[k].y, al));
+    be = fma(y[k].x, y[k].x, fma(y[k].y, y[k].y, be));
+    gr = fma(x[k].x, y[k].x, fma(x[k].y, y[k].y, gr));
+    gi = fma(x[k].x, y[k].y, fma(-x[k].y, y[k].x, gi));
+  }
+  warp_sum4(al, be, gr, gi, lane);
+  double c, sr, si;
+  if (!jacobi_cs(al, be, gr, gi, tol2, neg, c, sr, si)) return false;
+#pragma unroll
+  for (int k = 0; k < RPL; ++k) {
+    const double2 a = x[k], e = y[k];
+    x[k] = make_double2(fma(c, a.x, -fma(sr, e.x, si * e.y)), fma(c, a.y, -fma(sr, e.y, -si * e.x)));
+    yc[lane + 32 * k] = make_double2(fma(c, e.x, fma(sr, a.x, -si * a.y)), fma(c, e.y, fma(sr, a.y, si * a.x)));
+  }
+  return true;
+}
+
+// The sweeps of one step: every CTA of the cluster calls it (the same number
+// of cluster barriers in each).  Returns the buffer that holds the columns.
+template <int RPL>
+__device__ double2* cl_jacobi(cg::cluster_group& cl, double2* buf0, double2* buf1, uint64_t blk, uint32_t b,
+                              uint32_t act, double tol2, double neg, int (*s_rot)[8]) {
+  const uint32_t rank = cl.block_rank(), nct = cl.num_blocks();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t warp = tid >> 5, ld = 32 * RPL;
+  double2* cur = buf0;
+  double2* nxt = buf1;
+  if (act == 1 && rank != 0) return cur;
+  const bool mine = rank < act;
+  for (int sweep = 0; sweep < kMaxSweeps; ++sweep) {
+    bool rot = false;
+    for (uint32_t mv = 0; mv < 2 * act - 1; ++mv) {
+      if (mine) {
+        double2* X = cur;
+        double2* Y = cur + blk;
+        if (mv == 0) {  // all pairs of this CTA's 2b columns
+          const uint32_t nc = 2 * b;
+          for (uint32_t rd = 0; rd + 1 < nc; ++rd) {
+            for (uint32_t pi = warp; pi < b; pi += kClWarps) {
+              const uint32_t p = pi == 0 ? rd : (rd + pi) % (nc - 1);
+              const uint32_t q = pi == 0 ? nc - 1 : (rd + (nc - 1) - pi) % (nc - 1);
+              double2* xc = p < b ? X + p * ld : Y + (p - b) * ld;
+              double2* yc = q < b ? X + q * ld : Y + (q - b) * ld;
+              double2 x[RPL];
+#pragma unroll
+              for (int k = 0; k < RPL; ++k) x[k] = xc[lane + 32 * k];
+              if (cl_pair<RPL>(x, yc, lane, tol2, neg)) {
+                rot = true;
+#pragma unroll
+                for (int k = 0; k < RPL; ++k) xc[lane + 32 * k] = x[k];
+              }
+            }
+            __syncthreads();
+          }
+        } else {
+          for (uint32_t i0 = 0; i0 < b; i0 += kClWarps) {
+            const uint32_t i = i0 + warp;
+            double2 x[RPL];
+            bool any = false;
+            if (i < b) {
+#pragma unroll
+              for (int k = 0; k < RPL; ++k) x[k] = X[i * ld + lane + 32 * k];
+            }
+            for (uint32_t st = 0; st < b; ++st) {
+              if (i < b) {
+                const uint32_t j = i + st < b ? i + st : i + st - b;
+                any |= cl_pair<RPL>(x, Y + j * ld, lane, tol2, neg);
+              }
+              __syncthreads();
+            }
+            if (any) {
+              rot = true;
+#pragma unroll
+              for (int k = 0; k < RPL; ++k) X[i * ld + lane + 32 * k] = x[k];
+            }
+          }
+        }
+      }
+      if (act == 1) break;
+      const bool last = mv + 2 == 2 * act;
+      if (last) {
+        const int v = __syncthreads_or(rot);
+        if ((uint32_t)tid < nct) cl.map_shared_rank(&s_rot[sweep & 1][0], tid)[rank] = v;
+      }
+      cl.sync();
+      if (mine) {  // blocks move on: T0 stays, B0 -> T1, T_i -> T_{i+1}, T_last -> B_last, B_i -> B_{i-1}
+        const uint32_t xr = rank <= 1 ? 0 : rank - 1;
+        const double2* xs = cl.map_shared_rank(cur, xr) + (rank == 1 ? blk : 0);
+        const double2* ys = rank + 1 < act ? cl.map_shared_rank(cur, rank + 1) + blk : cur;
+        const uint32_t cnt = b * ld;
+        for (uint32_t e = tid; e < cnt; e += kClThreads) {
+          const double2 u = xs[e], w = ys[e];
+          nxt[e] = u;
+          nxt[blk + e] = w;
+        }
+        __syncthreads();
+        double2* t = cur;
+        cur = nxt;
+        nxt = t;
+      }
+    }
+    int v = 0;
+    if (act == 1) {
+      v = __syncthreads_or(rot);
+    } else {
+      for (uint32_t c = 0; c < act; ++c) v |= s_rot[sweep & 1][c];
+    }
+    if (!v) break;
+  }
+  return cur;
+}
+
+__global__ void __launch_bounds__(kClThreads) k_mps_2q_cl(MpsView v, uint32_t first, uint32_t max_keep,
+                                                          double thr) {
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ __align__(16) double2 smem[];
+  __shared__ int s_rot[2][8];
+  __shared__ double s_n2[8];
+  __shared__ double s_part[kClWarps];
+  __shared__ double s_sig[2 * kClusterCap + 64];
+  __shared__ uint32_t s_rank[2 * kClusterCap + 64];
+  __shared__ uint32_t s_own[2 * kClusterCap + 64];
+  __shared__ uint32_t s_keep, s_nown;
+  __shared__ double s_scale;
+  const MpsOp& op = v.ops[first + blockIdx.y];
+  const uint32_t rank = cl.block_rank(), nct = cl.num_blocks();
+  const uint32_t b = blockIdx.x / nct;
+  // an earlier launch overflowed the capacity: the program is run again
+  if (v.flags[3] < (int)first) return;
+  if (!cond_ok(v, op, b)) return;  // the same for every CTA of the cluster
+  uint32_t* dm = v.dims + (uint64_t)b * (v.n + 1);
+  const uint32_t q = op.q, cap = v.cap;
+  const uint32_t L = dm[q], M = dm[q + 1], R = dm[q + 2];
+  const bool tr = R > L;
+  const uint32_t rows = tr ? 2 * R : 2 * L, cols = tr ? 2 * L : 2 * R;
+  const uint32_t tw = 2 * R;   // theta row length
+  double2* TH = v.scratch + ((uint64_t)b * v.slots + blockIdx.y) * v.scratch_elems;
+  double2* A = site(v, q, b);
+  double2* B = site(v, q + 1, b);
+  const double2 zero = make_double2(0.0, 0.0);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t warp = tid >> 5;
+
+  // ---- theta, split over the cluster ---------------------------------------------
+  double n2 = 0.0;  // |theta|_F^2, for the negligible-pair test
+  for (uint32_t t = rank * kClThreads + tid; t < L * R; t += nct * kClThreads) {
+    const uint32_t l = t / R, r = t - (t / R) * R;
+    double2 in[4];
+    for (int i0 = 0; i0 < 2; ++i0)
+      for (int i1 = 0; i1 < 2; ++i1) {
+        double2 acc = zero;
+        const double2* ar = A + (uint64_t)(l * 2 + i0) * cap;
+        for (uint32_t k = 0; k < M; ++k)
+          acc = cadd_x(acc, cmul_x(ar[k], B[(uint64_t)(k * 2 + i1) * cap + r]));
+        in[i0 * 2 + i1] = acc;
+      }
+    for (int o0 = 0; o0 < 2; ++o0)
+      for (int o1 = 0; o1 < 2; ++o1) {
+        const int o = o0 * 2 + o1;
+        double2 acc = zero;
+        for (int i = 0; i < 4; ++i) acc = cadd_x(acc, cmul_x(op.u[o * 4 + i], in[i]));
+        TH[(uint64_t)(l * 2 + o0) * tw + o1 * R + r] = acc;
+        n2 += acc.x * acc.x + acc.y * acc.y;
+      }
+  }
+  n2 = warp_sum(n2);
+  if (lane == 0) s_part[warp] = n2;
+  __syncthreads();
+  if ((uint32_t)tid < nct) {
+    double s = 0.0;
+    for (uint32_t w = 0; w < kClWarps; ++w) s += s_part[w];
+    cl.map_shared_rank(&s_n2[0], tid)[rank] = s;
+  }
+  cl.sync();
+  n2 = 0.0;
+  for (uint32_t c = 0; c < nct; ++c) n2 += s_n2[c];
+
+  // ---- this CTA's columns ----------------------------------------------------------
+  const uint32_t act = cl_active(cols, nct), nb = cl_block(cols, act);
+  const uint32_t rpl = cl_rpl(rows), ld = 32 * rpl;
+  const uint64_t blk = cl_block_elems(cap, nct);
+  double2* buf0 = smem;
+  double2* buf1 = smem + (nct > 1 ? 2 * blk : 0);
+  if (rank < act) {
+    const uint32_t c0 = 2 * rank * nb;
+    // consecutive threads read consecutive addresses of theta in both forms
+    for (uint32_t e = tid; e < 2 * nb * ld; e += kClThreads) {
+      const uint32_t j = tr ? e / ld : e % (2 * nb), row = tr ? e % ld : e / (2 * nb);
+      const uint32_t col = c0 + j;
+      double2 val = zero;
+      if (col < cols && row < rows) {
+        val = tr ? TH[(uint64_t)col * tw + row] : TH[(uint64_t)row * tw + col];
+        if (tr) val.y = -val.y;
+      }
+      buf0[(j < nb ? 0 : blk) + (uint64_t)(j < nb ? j : j - nb) * ld + row] = val;
+    }
+  }
+  __syncthreads();
+  const double tol = (double)rows * DBL_EPSILON;
+  const double neg = tol * tol * n2;
+  double2* G = nullptr;
+  switch (rpl) {
+    case 1: G = cl_jacobi<1>(cl, buf0, buf1, blk, nb, act, tol * tol, neg, s_rot); break;
+    case 2: G = cl_jacobi<2>(cl, buf0, buf1, blk, nb, act, tol * tol, neg, s_rot); break;
+    case 3: G = cl_jacobi<3>(cl, buf0, buf1, blk, nb, act, tol * tol, neg, s_rot); break;
+    case 4: G = cl_jacobi<4>(cl, buf0, buf1, blk, nb, act, tol * tol, neg, s_rot); break;
+    default: G = cl_jacobi<6>(cl, buf0, buf1, blk, nb, act, tol * tol, neg, s_rot); break;
+  }
+  auto column = [&](uint32_t j) { return G + (j < nb ? 0 : blk) + (uint64_t)(j < nb ? j : j - nb) * ld; };
+
+  // ---- singular values to every CTA, ranks in descending order ------------------------
+  const uint32_t ntot = 2 * act * nb, c0 = 2 * rank * nb;  // columns with the zero padding
+  if (rank < act)
+    for (uint32_t j = warp; j < 2 * nb; j += kClWarps) {
+      const double2* g = column(j);
+      double s = 0.0;
+      for (uint32_t i = lane; i < ld; i += 32) s += g[i].x * g[i].x + g[i].y * g[i].y;
+      s = sqrt(warp_sum(s));
+      if ((uint32_t)lane < nct) cl.map_shared_rank(&s_sig[0], lane)[c0 + j] = s;
+    }
+  if (tid == 0) s_nown = 0;
+  cl.sync();
+  for (uint32_t j = tid; j < ntot; j += kClThreads) {
+    uint32_t r = 0;
+    const double sj = s_sig[j];
+    for (uint32_t i = 0; i < ntot; ++i) r += (s_sig[i] > sj || (s_sig[i] == sj && i < j)) ? 1u : 0u;
+    s_rank[j] = r;
+  }
+  __syncthreads();
+  // ---- truncation (simulator.rs:186-218), the same in every CTA -------------------------
+  if (warp == 0) {
+    uint32_t keep = 0;
+    for (uint32_t j = lane; j < ntot; j += 32) keep += (s_rank[j] < cols && s_sig[j] > thr) ? 1u : 0u;
+    for (int o = 16; o > 0; o >>= 1) keep += __shfl_xor_sync(0xffffffffu, keep, o);
+    keep = keep > 1u ? keep : 1u;
+    if (max_keep) keep = keep < max_keep ? keep : max_keep;
+    double kept = 0.0, disc = 0.0;
+    for (uint32_t j = lane; j < ntot; j += 32) {
+      const double s2 = s_sig[j] * s_sig[j];
+      if (s_rank[j] < keep) kept += s2;
+      else disc += s2;
+    }
+    kept = warp_sum(kept);
+    disc = warp_sum(disc);
+    if (lane == 0) {
+      const double total = sqrt(kept + disc);
+      kept = fmax(sqrt(kept), 1e-15);
+      s_scale = disc > 0.0 ? total / kept : 1.0;
+      s_keep = keep;
+      if (rank == 0) {
+        if (keep > cap) {
+          atomicMax(&v.flags[2], (int)keep);
+          atomicMax(&v.flags[0], MF_CAPACITY);
+          atomicMin(&v.flags[3], (int)first);
+        } else {
+          atomicAdd(v.svd_calls, 1ull);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  const uint32_t keep = s_keep;
+  if (keep > cap || rank >= act) return;  // no CTA reads another's shared memory from here on
+  const double scale = s_scale;
+
+  // ---- split: this CTA's kept columns ------------------------------------------------------
+  for (uint32_t j = tid; j < 2 * nb; j += kClThreads)
+    if (s_rank[c0 + j] < keep) s_own[atomicAdd(&s_nown, 1u)] = j;
+  __syncthreads();
+  const uint32_t nown = s_nown;
+  // the factor taken from G itself: U (left) or scale W^H (right)
+  for (uint32_t t = tid; t < nown * rows; t += kClThreads) {
+    const uint32_t o = t / rows, i = t - (t / rows) * rows;
+    const uint32_t j = s_own[o], k = s_rank[c0 + j];
+    const double sj = s_sig[c0 + j];
+    const bool ok = sj > 0.0 && sj * sj > neg;  // a kept column at the rounding level of theta is left zero
+    const double2 g = column(j)[i];
+    if (!tr) {
+      A[(uint64_t)i * cap + k] = ok ? make_double2(g.x / sj, g.y / sj) : zero;
+    } else {
+      const uint32_t s = i / R, r = i - (i / R) * R;
+      B[(uint64_t)(k * 2 + s) * cap + r] = ok ? make_double2(scale * g.x, -scale * g.y) : zero;
+    }
+  }
+  // the factor that multiplies theta, two columns at a time
+  const uint32_t npair = (nown + 1) / 2;
+  if (!tr) {
+    // right: scale / sigma_j * (W_j^H theta)[col]
+    for (uint32_t t = tid; t < npair * tw; t += kClThreads) {
+      const uint32_t o = 2 * (t / tw), col = t - (t / tw) * tw;
+      const uint32_t ja = s_own[o], jb = s_own[o + 1 < nown ? o + 1 : o];
+      const double2* wa = column(ja);
+      const double2* wb = column(jb);
+      double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
+#pragma unroll 4
+      for (uint32_t i = 0; i < rows; ++i) {
+        const double2 x = wa[i], y = wb[i], a = TH[(uint64_t)i * tw + col];
+        ar += x.x * a.x + x.y * a.y;
+        ai += x.x * a.y - x.y * a.x;
+        br += y.x * a.x + y.y * a.y;
+        bi += y.x * a.y - y.y * a.x;
+      }
+      const uint32_t s = col / R, r = col - (col / R) * R;
+      for (uint32_t h = 0; h < 2 && o + h < nown; ++h) {
+        const uint32_t j = h ? jb : ja;
+        const double sj = s_sig[c0 + j];
+        const bool ok = sj > 0.0 && sj * sj > neg;
+        const double f = ok ? scale / sj : 0.0;
+        const double re = h ? br : ar, im = h ? bi : ai;
+        B[(uint64_t)(s_rank[c0 + j] * 2 + s) * cap + r] = ok ? make_double2(f * re, f * im) : zero;
+      }
+    }
+  } else {
+    // left: (theta W_j)[row] / sigma_j^2, one warp per row
+    for (uint32_t row = warp; row < cols; row += kClWarps) {
+      const double2* th = TH + (uint64_t)row * tw;
+      for (uint32_t o = 0; o < nown; o += 2) {
+        const uint32_t ja = s_own[o], jb = s_own[o + 1 < nown ? o + 1 : o];
+        const double2* wa = column(ja);
+        const double2* wb = column(jb);
+        double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
+        for (uint32_t i = lane; i < rows; i += 32) {
+          const double2 a = th[i], x = wa[i], y = wb[i];
+          ar += a.x * x.x - a.y * x.y;
+          ai += a.x * x.y + a.y * x.x;
+          br += a.x * y.x - a.y * y.y;
+          bi += a.x * y.y + a.y * y.x;
+        }
+        warp_sum4(ar, ai, br, bi, lane);
+        if (lane < 2 && o + lane < nown) {
+          const uint32_t j = lane ? jb : ja;
+          const double sj = s_sig[c0 + j], s2 = sj * sj;
+          const bool ok = sj > 0.0 && s2 > neg;
+          A[(uint64_t)row * cap + s_rank[c0 + j]] =
+              ok ? make_double2((lane ? br : ar) / s2, (lane ? bi : ai) / s2) : zero;
+        }
+      }
+    }
+  }
+  if (rank == 0 && tid == 0) dm[q + 1] = keep;
+}
+
 // Batched form of k_mps_2q for capacity <= 16 (theta at most 32 x 32): two
 // warps (64 lanes) per replica, kRepsPer2q replicas per CTA, each replica with
 // its own shared-memory G and its own named barrier (id 1 + slot, 64 threads)
@@ -463,7 +902,8 @@ __global__ void __launch_bounds__(kWarpsPer2q * 32) k_mps_2q_warp(MpsView v, uin
   const uint32_t tl = (uint32_t)(wr * 32 + lane);    // lane within the replica (0..63)
   const int bar = 1 + slot;
   const uint32_t b = blockIdx.x * kRepsPer2q + slot;
-  if (b >= v.batch || !cond_ok(v, op, b)) return;    // the same for both warps of the replica
+  // the same for both warps of the replica (flags[3]: an earlier launch overflowed the capacity)
+  if (b >= v.batch || v.flags[3] < (int)first || !cond_ok(v, op, b)) return;
   const unsigned full = 0xffffffffu;
   const uint32_t cap = v.cap;
   uint32_t* dm = v.dims + (uint64_t)b * (v.n + 1);
@@ -597,6 +1037,7 @@ __global__ void __launch_bounds__(kWarpsPer2q * 32) k_mps_2q_warp(MpsView v, uin
     if (keep > cap) {
       atomicMax(&v.flags[2], (int)keep);
       atomicMax(&v.flags[0], MF_CAPACITY);
+      atomicMin(&v.flags[3], (int)first);
     } else {
       atomicAdd(v.svd_calls, 1ull);
     }
@@ -1127,6 +1568,89 @@ int lower(uint32_t n, const dq_inst* prog, uint64_t ninst, const dq_cond* conds,
   return DQ_OK;
 }
 
+// CTAs per step of k_mps_2q_cl: as many as spread the launch's steps over the
+// chip once (up to 8), at least what the capacity's columns need in shared
+// memory (two buffers of two blocks per CTA).
+uint32_t cluster_ctas(uint32_t cap, uint64_t steps) {
+  uint32_t c = 1;
+  while (c < 8 && (cl_smem_bytes(cap, c) > kMaxSmem || (steps * c * 2 <= 148 && 16 * c < 2 * cap))) c *= 2;
+  return c;
+}
+
+int launch_cluster(dq_mps_s* h, const MpsView& v, uint32_t first, uint32_t count) {
+  const uint32_t c = cluster_ctas(h->cap, (uint64_t)h->batch * count);
+  const size_t smem = cl_smem_bytes(h->cap, c);
+  DQ_CUDA_TRY(cudaFuncSetAttribute(k_mps_2q_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(h->batch * c, count);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = h->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = c;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  DQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_mps_2q_cl, v, first, h->max_bond, h->thr));
+  return DQ_OK;
+}
+
+// An upper bound of the bond dimensions the program can reach from |0...0>: a
+// step multiplies its bond by at most the operator Schmidt rank of its gate,
+// and never past twice either neighbour.  (An underestimate only costs a
+// second run.)
+uint32_t program_bound(uint32_t n, uint32_t max_bond, const std::vector<MpsOp>& ops) {
+  std::vector<uint64_t> d(n + 1, 1);
+  uint64_t top = 1;
+  for (const MpsOp& op : ops) {
+    if (op.kind != M_2Q) continue;
+    // rank of u rearranged to [(o0 i0), (o1 i1)], by elimination with full pivoting
+    hc m[4][4];
+    for (int o0 = 0; o0 < 2; ++o0)
+      for (int o1 = 0; o1 < 2; ++o1)
+        for (int i0 = 0; i0 < 2; ++i0)
+          for (int i1 = 0; i1 < 2; ++i1) {
+            const double2 u = op.u[(o0 * 2 + o1) * 4 + i0 * 2 + i1];
+            m[o0 * 2 + i0][o1 * 2 + i1] = hc{u.x, u.y};
+          }
+    uint32_t rank = 0;
+    for (; rank < 4; ++rank) {
+      int pr = -1, pc = -1;
+      double best = 1e-14;
+      for (int r = rank; r < 4; ++r)
+        for (int c = rank; c < 4; ++c) {
+          const double a = m[r][c].re * m[r][c].re + m[r][c].im * m[r][c].im;
+          if (a > best * best) {
+            best = sqrt(a);
+            pr = r;
+            pc = c;
+          }
+        }
+      if (pr < 0) break;
+      for (int c = 0; c < 4; ++c) std::swap(m[rank][c], m[pr][c]);
+      for (int r = 0; r < 4; ++r) std::swap(m[r][rank], m[r][pc]);
+      const hc p = m[rank][rank];
+      const double pn = p.re * p.re + p.im * p.im;
+      for (int r = rank + 1; r < 4; ++r) {
+        const hc x = m[r][rank];
+        const hc f = hc{(x.re * p.re + x.im * p.im) / pn, (x.im * p.re - x.re * p.im) / pn};
+        for (int c = rank; c < 4; ++c) {
+          m[r][c].re -= f.re * m[rank][c].re - f.im * m[rank][c].im;
+          m[r][c].im -= f.re * m[rank][c].im + f.im * m[rank][c].re;
+        }
+      }
+    }
+    uint64_t& b = d[op.q + 1];
+    b = std::min(b * std::max(rank, 1u), 2 * std::min(d[op.q], d[op.q + 2]));
+    if (max_bond) b = std::min<uint64_t>(b, max_bond);
+    b = std::max<uint64_t>(b, 1);
+    top = std::max(top, b);
+  }
+  return (uint32_t)std::min<uint64_t>(top, 1u << 30);
+}
+
 // Groups consecutive operations into launches: a run of one-qubit gates, or
 // of two-qubit steps (at most `slots`), whose sites are pairwise disjoint
 // commutes exactly, so one launch (blockIdx.y = the operation) runs them all;
@@ -1145,8 +1669,10 @@ int launch_ops(dq_mps_s* h, const std::vector<MpsOp>& ops) {
   const MpsView v = view_of(h);
   const size_t shm = h->smem ? h->work_bytes : 0;
   const int use = h->smem ? 1 : 0;
-  // one SVD per CTA: wide CTAs when few replicas share the GPU (latency), 256
-  // threads and several CTAs per SM otherwise (throughput)
+  // few replicas share the GPU: a cluster per step (16 qubits, bond 32: 100
+  // replicas 18.6 ms, 23.5 ms with one wide CTA per step), wide CTAs above its
+  // capacity.  More replicas fill the chip with one 256-thread CTA per step
+  // (600 replicas at bond 32: 80 ms, 103 ms with clusters).
   const int t2q = h->batch <= 2 * 148 ? 1024 : 256;
   // many replicas of small bonds: one warp per replica
   const bool warp2q = h->batch > 2 * 148 && h->cap <= kWarpCap;
@@ -1173,6 +1699,8 @@ int launch_ops(dq_mps_s* h, const std::vector<MpsOp>& ops) {
         if (warp2q)
           k_mps_2q_warp<<<dim3((h->batch + kRepsPer2q - 1) / kRepsPer2q, count), kWarpsPer2q * 32,
                           kRepsPer2q * warp_work_bytes(h->cap), h->stream>>>(v, first, h->max_bond, h->thr);
+        else if (h->batch <= 2 * 148 && h->cap <= kClusterCap)
+          DQ_TRY(launch_cluster(h, v, first, count));
         else
           k_mps_2q<<<dim3(h->batch, count), t2q, shm, h->stream>>>(v, first, h->max_bond, h->thr, use);
         break;
@@ -1210,6 +1738,15 @@ int run_batch(dq_mps_s* h, const std::vector<MpsOp>& ops, const dq_cond* conds, 
               double* kernel_ms, uint64_t budget = 0, bool* shrink = nullptr) {
   const uint32_t bound = bond_bound(h->n, h->max_bond);
   if (shrink) *shrink = false;
+  // One state: start at the capacity the program can need (up to 64, whose
+  // buffers are small) instead of finding it by overflowing 16 and 32.
+  if (batch == 1 && h->cap < bound) {
+    const uint32_t need = std::min(std::min(program_bound(h->n, h->max_bond, ops), 64u), bound);
+    uint32_t cap = h->cap;
+    while (cap < need) cap *= 2;
+    cap = std::min(cap, bound);
+    if (cap > h->cap) DQ_TRY(alloc_buffers(h, batch, cap, ncb));
+  }
   for (;;) {
     if (h->batch != batch || h->ncb != (ncb ? ncb : 1) || !h->t) DQ_TRY(alloc_buffers(h, batch, h->cap, ncb));
     if (nconds > h->conds_cap) {
@@ -1224,7 +1761,7 @@ int run_batch(dq_mps_s* h, const std::vector<MpsOp>& ops, const dq_cond* conds, 
     for (uint32_t b = 0; b < batch; ++b) seed_key_from_u64(seeds[b], &keys[(size_t)b * 8]);
     DQ_CUDA_TRY(cudaMemcpyAsync(h->key, keys.data(), sizeof(uint32_t) * keys.size(), cudaMemcpyHostToDevice,
                                 h->stream));
-    const int init_flags[4] = {MF_OK, 0x7fffffff, 0, 0};
+    const int init_flags[4] = {MF_OK, 0x7fffffff, 0, 0x7fffffff};
     DQ_CUDA_TRY(cudaMemcpyAsync(h->flags, init_flags, sizeof(init_flags), cudaMemcpyHostToDevice, h->stream));
     DQ_CUDA_TRY(cudaMemsetAsync(h->svd_calls, 0, sizeof(unsigned long long), h->stream));
     cudaEvent_t e0, e1;
@@ -1424,7 +1961,7 @@ int dq_mps_apply_2q(dq_mps_t h, uint32_t a, uint32_t b, const double* u) {
   // Below the bond bound a step may overflow the capacity: run the steps one
   // at a time, and on an overflow (the step wrote nothing) widen and redo it.
   const uint32_t bound = bond_bound(h->n, h->max_bond);
-  const int init_flags[4] = {MF_OK, 0x7fffffff, 0, 0};
+  const int init_flags[4] = {MF_OK, 0x7fffffff, 0, 0x7fffffff};
   if (h->cap >= bound) {
     DQ_CUDA_TRY(cudaMemcpyAsync(h->flags, init_flags, sizeof(init_flags), cudaMemcpyHostToDevice, h->stream));
     DQ_TRY(launch_ops(h, ops));

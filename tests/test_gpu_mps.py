@@ -444,3 +444,25 @@ def test_rank_deficient_thetas_at_rounding_threshold_match_exact_state(thr):
     assert np.max(np.abs(sv - exact)) < 1e-12
     assert abs(np.vdot(sv, sv).real - 1.0) < 1e-12
     assert max(dims) <= 16
+
+
+# the cluster form of the step: one to eight CTAs with columns, a last block with
+# padding, more columns than warps per block, and the largest capacity it takes (96)
+@pytest.mark.parametrize("max_bond", [3, 8, 9, 17, 24, 39, 63, 65, 96, 97])
+def test_cluster_step_matches_oracle(max_bond):
+    c = brickwork_u3_cx(14, 15, seed=max_bond)
+    sv, _, dims, _ = device_run(c, SEED, max_bond=max_bond)
+    ref, _, rdims, _ = _oracle.mps_run(prog_of(c), SEED, max_bond=max_bond)
+    assert dims == rdims and max(dims) == max_bond
+    assert np.max(np.abs(sv - ref)) < 1e-9
+
+
+# batches whose launches take clusters of one, two or four CTAs per step
+@pytest.mark.parametrize("shots,max_bond", [(6, 24), (40, 20), (300, 24), (300, 40), (9, 33)])
+def test_cluster_batches_match_oracle(shots, max_bond):
+    c = trajectory_circuit(11, 9, seed=8)
+    prog = prog_of(c)
+    bits, _ = run_mps_shots(prog, 5, shots, 0, max_bond, 1e-12)
+    for i in sorted({0, 1, shots // 2, shots - 1}):
+        _, rcb, _, _ = _oracle.mps_run(prog, 5 + i, max_bond=max_bond)
+        assert bits[i].tolist() == rcb.tolist(), i
