@@ -11,8 +11,22 @@
 // qubits pair elements across CTAs through distributed shared memory.  A
 // measurement reduces p1 per CTA (fixed order), exchanges the cluster's
 // partials, draws the outcome from the device ChaCha8 stream and collapses
-// in place.  Each cluster loops over trajectories until all shots are done;
-// the state never touches HBM, only the classical registers are written out.
+// in place.
+//
+// Shots share work.  Two shots of one program that have drawn the same
+// outcomes so far hold the same state bit for bit, so a cluster carries a
+// state together with the list of the shots that are in it.  A measurement
+// compares every listed shot's own draw with the state's p1; when both
+// outcomes occur the state is saved (HBM) with one half of the list as a task
+// for any idle cluster and the cluster goes on with the other half.  Each
+// distinct outcome history is computed once instead of once per shot: the
+// bound is the latency of one trajectory while histories are few, and the
+// shared memory and FP64 throughput of one trajectory per shot once every
+// shot is on its own.  4096 shots of 16 qubits with four measure / reset
+// pairs: 205 ms with one trajectory per shot, 0.88 ms here (16 histories); with
+// 16 random outcomes per shot, every shot soon on its own: 132 ms and 96 ms.
+// Clusters take tasks until none is left or running; states otherwise stay in
+// shared memory, and only classical registers are written out.
 //
 // Arithmetic is the exact per-gate arithmetic of dq_engine.cu (num-complex
 // order, no FMA, zero matrix entries skipped), so amplitudes match the
@@ -92,10 +106,22 @@ struct TSweep {          // one fused sweep of an HBM item
   uint32_t ntiles, run_bits;
   uint32_t prog_bytes, pad;
 };
-struct TItem {          // one trajectory: a shot of a program
-  uint32_t prog, pad;
+struct TItem {          // shots [shot, shot + count) of a program
+  uint32_t prog, count;
   uint64_t shot;
 };
+// A state saved at a measurement, to be collapsed to `outcome` and run on for
+// the shots order[src][lo .. hi).  Without a slot (more states than slots) the
+// program is run from the start instead: the listed shots draw the same
+// outcomes again.
+struct alignas(16) TTask {
+  uint32_t prog, oi;      // op index of the measurement
+  uint32_t lo, hi, src;
+  int32_t slot;
+  uint32_t outcome, draws;
+  double p1;
+};
+static_assert(sizeof(TTask) == 48, "TTask is read as three 16-byte words");
 struct TrajParams {
   const TOp* ops;
   const double2* pool;
@@ -103,9 +129,17 @@ struct TrajParams {
   const TProg* progs;
   const TItem* items;
   int32_t* cbits_out;
-  unsigned long long* queue;     // work queue: next item index
+  unsigned long long* queue;     // [0] next item or task, [1] tasks pushed, [2] items and tasks unfinished
   unsigned long long* boundary;  // draws within 1e-12 of p1
   long long* failed;             // lowest (prog << 40 | instruction) that failed
+  // shared shots (nslots and tasks are 0 / null when every item is one shot)
+  uint32_t* order[2];            // shot lists, split from one into the other
+  TTask* tasks;                  // at most one per shot
+  int* ready;                    // task t is complete in memory
+  double2* slots;                // nslots states of 2^n amplitudes
+  int32_t* slot_cbits;           // nslots x ncbits
+  const double* draws;           // draw k of shot s at s * draw_stride + k, or null
+  uint32_t nslots, draw_stride;
   uint64_t nitems;
   const uint8_t* sweep_blob;     // sweep programs of the HBM items (dq_sweep.cuh layout)
   const TSweep* sweeps;
@@ -172,12 +206,59 @@ __device__ double block_sum_all(double v, double* sh) {
   return sh[32];
 }
 
+// The first draws of every shot, one thread per ChaCha8 block of eight.
+__global__ void __launch_bounds__(128) k_traj_draws(const TProg* prog, uint64_t shots, uint32_t blocks,
+                                                    double* out) {
+  const uint64_t i = (uint64_t)blockIdx.x * 128 + threadIdx.x;
+  if (i >= shots * blocks) return;
+  uint32_t key[8], w[16];
+  seed_key_from_u64(prog->base_seed + i / blocks, key);
+  chacha8_stream_block(key, i % blocks, w);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    out[i * 8 + k] = u64_to_f64((uint64_t)w[2 * k] | ((uint64_t)w[2 * k + 1] << 32));
+}
+
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int* p, int v) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// The next item (index below nitems) or task (nitems + t) to run; ~0 when
+// nothing is left.  A cluster that finds none while others still run waits for
+// what they may push, with a limit (seconds): leaving early is safe,
+// the clusters that push also take tasks.
+__device__ unsigned long long next_work(const TrajParams& P) {
+  for (int tries = 0; tries < (1 << 21); ++tries) {
+    unsigned long long h, t;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(h), "=l"(t) : "l"(P.queue) : "memory");
+    if (h < P.nitems || (t > h - P.nitems && ld_acquire(P.ready + (h - P.nitems)))) {
+      if (atomicCAS(P.queue, h, h + 1) == h) return h;
+      continue;
+    }
+    if (!P.tasks || ld_acquire(P.queue + 2) == 0) break;
+    __nanosleep(100);
+  }
+  return ~0ULL;
+}
+
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ double s_bcast[2];
   __shared__ int s_skip[2];  // double-buffered by op parity: one barrier per op suffices
   __shared__ unsigned long long s_item;
+  __shared__ uint32_t s_count[2];   // a split's shots with outcome 0 and 1
+  __shared__ unsigned long long s_task;
 
   cg::cluster_group cl = cg::this_cluster();
   const uint32_t C = cl.num_blocks(), rank = cl.block_rank();
@@ -187,15 +268,35 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
   };
 
   for (;;) {
-    // rank 0 takes the next trajectory from the queue and shares it
-    if (rank == 0 && tid == 0) s_item = atomicAdd(P.queue, 1ULL);
+    // rank 0 takes the next item or task from the queue and shares it
+    if (rank == 0 && tid == 0) s_item = next_work(P);
     sync_all(true);
     const unsigned long long item = (rank == 0) ? s_item : *cl.map_shared_rank(&s_item, 0);
-    if (item >= P.nitems) {
+    if (item == ~0ULL) {
       sync_all(true);  // no CTA leaves while another still reads its shared memory
       break;
     }
-    const TItem it = P.items[item];
+    TItem it;
+    TTask tk{};
+    uint32_t lo = 0, hi = 1, src = 2;  // the shots: order[src][lo .. hi), src 2: it.shot + lo .. hi
+    if (item < P.nitems) {
+      it = P.items[item];
+      hi = it.count;
+      tk.slot = -1;
+    } else {
+      const uint4* rec = reinterpret_cast<const uint4*>(P.tasks + (item - P.nitems));
+      uint4 w[3];
+      for (int i = 0; i < 3; ++i) w[i] = __ldcg(rec + i);
+      memcpy(&tk, w, sizeof(tk));
+      it.prog = tk.prog;
+      it.shot = 0;
+      lo = tk.lo;
+      hi = tk.hi;
+      src = tk.src;
+    }
+    auto shot_at = [&](uint32_t i) -> uint64_t {
+      return src == 2 ? it.shot + i : (uint64_t)__ldcg(P.order[src] + i);
+    };
     const TProg pg = P.progs[it.prog];
     if (pg.hbm) {
       // HBM item: the cluster's CTAs split the tiles of each sweep (tiles
@@ -232,6 +333,7 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
         for (uint32_t i = tid; i < pg.ncbits; i += THREADS)
           P.cbits_out[pg.cbits_off + it.shot * pg.ncbits + i] = -1;
       sync_all(true);
+      if (rank == 0 && tid == 0) atomicAdd(P.queue + 2, ~0ULL);
       continue;
     }
     const uint32_t lb = pg.lb, L = 1u << lb;
@@ -246,14 +348,71 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
       return base + tswz((uint32_t)(g & lmask));
     };
 
-    uint32_t key[8];
-    seed_key_from_u64(pg.base_seed + it.shot, key);
-    uint64_t draws = 0;
-    for (uint32_t i = tid; i < L; i += THREADS) sm[i] = make_double2(0.0, 0.0);
-    for (uint32_t i = tid; i < pg.ncbits; i += THREADS) cb[i] = -1;
-    if (rank == 0 && tid == 0) sm[0] = make_double2(1.0, 0.0);
+    uint64_t draws = tk.draws;
+    if (tk.slot >= 0) {  // slices are saved in their shared-memory layout
+      const double2* s = P.slots + ((uint64_t)tk.slot << pg.n) + gbase;
+#pragma unroll 4
+      for (uint32_t i = tid; i < L; i += THREADS) sm[i] = __ldcg(s + i);
+      for (uint32_t i = tid; i < pg.ncbits; i += THREADS)
+        cb[i] = __ldcg(P.slot_cbits + (uint64_t)tk.slot * pg.ncbits + i);
+    } else {
+      draws = 0;
+      for (uint32_t i = tid; i < L; i += THREADS) sm[i] = make_double2(0.0, 0.0);
+      for (uint32_t i = tid; i < pg.ncbits; i += THREADS) cb[i] = -1;
+      if (rank == 0 && tid == 0) sm[0] = make_double2(1.0, 0.0);
+    }
     bool last_cluster = true;
     sync_all(true);
+
+    // divisor of a collapse (engine.rs:216-235)
+    auto norm_of = [](int o, double p1) {
+      const double q = o == 1 ? p1 : (1.0 - p1 < 0.0 ? 0.0 : 1.0 - p1);
+      const double r = sqrt(q);
+      return r < 1e-15 ? 1e-15 : r;
+    };
+    auto collapse = [&](const TOp& op, int o, double norm) {
+      const uint32_t q = op.t1;
+      const uint64_t qb = 1ULL << q;
+      for (uint32_t i = tid; i < L; i += THREADS) {
+        const bool set = ((gbase | i) & qb) != 0;
+        if (set != (o == 1)) {
+          sm[tswz(i)] = make_double2(0.0, 0.0);
+        } else {
+          const double2 a = sm[tswz(i)];
+          sm[tswz(i)] = make_double2(__ddiv_rn(a.x, norm), __ddiv_rn(a.y, norm));
+        }
+      }
+      if (op.type == T_RESET && o == 1) {
+        // X on q: an exact exchange of the two halves
+        if (C > 1) cl.sync(); else __syncthreads();
+        if (q < lb) {
+          for (uint32_t k = tid; k < L / 2; k += THREADS) {
+            const uint32_t a0 = ins0(k, q), a1 = a0 | (uint32_t)qb;
+            const double2 x = sm[tswz(a0)];
+            sm[tswz(a0)] = sm[tswz(a1)];
+            sm[tswz(a1)] = x;
+          }
+        } else {
+          const uint32_t tbr = 1u << (q - lb);
+          if (!(rank & tbr)) {
+            double2* other = cl.map_shared_rank(sm, rank | tbr);
+            for (uint32_t i = tid; i < L; i += THREADS) {
+              const double2 x = sm[i];
+              sm[i] = other[i];
+              other[i] = x;
+            }
+          }
+        }
+      }
+    };
+    uint32_t oi0 = 0;
+    if (tk.slot >= 0) {  // finish the measurement the state was saved at
+      const TOp op = P.ops[pg.ops_off + tk.oi];
+      collapse(op, (int)tk.outcome, norm_of((int)tk.outcome, tk.p1));
+      if (tid == 0 && op.type == T_MEASURE) cb[op.cbit] = (int)tk.outcome;
+      oi0 = tk.oi + 1;
+      sync_all(true);
+    }
 
     // the next op's descriptor and one-qubit matrix are loaded while the
     // current op runs (global loads, otherwise a round trip before every op)
@@ -264,8 +423,8 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
       if (nxt.type == T_ONEQ)
         for (int i = 0; i < 4; ++i) nu[i] = P.pool[nxt.mat + i];
     };
-    if (pg.nops) fetch(0);
-    for (uint32_t oi = 0; oi < pg.nops; ++oi) {
+    if (oi0 < pg.nops) fetch(oi0);
+    for (uint32_t oi = oi0; oi < pg.nops; ++oi) {
       const TOp op = nxt;
       double2 u[4];
       for (int i = 0; i < 4; ++i) u[i] = nu[i];
@@ -487,58 +646,93 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
               const double* pr = (r == rank) ? red : cl.map_shared_rank(red, r);
               p1 = __dadd_rn(p1, pr[40]);
             }
-            const double rr = chacha8_draw(key, draws);
-            const int o = rr < p1 ? 1 : 0;
-            double norm;
-            if (o == 1) {
-              norm = sqrt(p1);
-              if (norm < 1e-15) norm = 1e-15;
-            } else {
-              double t = 1.0 - p1;
-              if (t < 0.0) t = 0.0;
-              norm = sqrt(t);
-              if (norm < 1e-15) norm = 1e-15;
+            s_bcast[0] = p1;
+            s_count[0] = s_count[1] = 0;
+            if (hi - lo == 1) {
+              const uint64_t shot = shot_at(lo);
+              double rr;
+              if (P.draws && draws < P.draw_stride) {
+                rr = P.draws[shot * P.draw_stride + draws];
+              } else {
+                uint32_t key[8];
+                seed_key_from_u64(pg.base_seed + shot, key);
+                rr = chacha8_draw(key, draws);
+              }
+              if (rank == 0 && draws >= tk.draws && fabs(rr - p1) < 1e-12) atomicAdd(P.boundary, 1ULL);
+              s_count[rr < p1 ? 1 : 0] = 1;
             }
-            if (rank == 0 && fabs(rr - p1) < 1e-12) atomicAdd(P.boundary, 1ULL);
-            s_bcast[0] = (double)o;
-            s_bcast[1] = norm;
-            if (op.type == T_MEASURE) cb[op.cbit] = o;
+          }
+          __syncthreads();
+          const double p1 = s_bcast[0];
+          if (hi - lo > 1) {
+            // each shot's own draw; outcome 0 goes to the front of the other
+            // list, outcome 1 to its back
+            const uint32_t dst = src == 0 ? 1 : 0;
+            if (rank == 0) {
+              for (uint32_t i = lo + tid; i < hi; i += THREADS) {
+                const uint64_t shot = shot_at(i);
+                double rr;
+                if (P.draws && draws < P.draw_stride) {
+                  rr = P.draws[shot * P.draw_stride + draws];
+                } else {
+                  uint32_t key[8];
+                  seed_key_from_u64(pg.base_seed + shot, key);
+                  rr = chacha8_draw(key, draws);
+                }
+                // (a program run again from the start draws what was counted before)
+                if (draws >= tk.draws && fabs(rr - p1) < 1e-12) atomicAdd(P.boundary, 1ULL);
+                if (rr < p1) P.order[dst][hi - 1 - atomicAdd(&s_count[1], 1u)] = (uint32_t)shot;
+                else P.order[dst][lo + atomicAdd(&s_count[0], 1u)] = (uint32_t)shot;
+              }
+              __threadfence();
+            }
+            if (C > 1) cl.sync(); else __syncthreads();
+            if (rank != 0 && tid == 0) {
+              const uint32_t* c0 = cl.map_shared_rank(&s_count[0], 0);
+              s_count[0] = c0[0];
+              s_count[1] = c0[1];
+            }
+            __syncthreads();
+            src = dst;
           }
           ++draws;
-          __syncthreads();
-          const int o = (int)s_bcast[0];
-          const double norm = s_bcast[1];
-          for (uint32_t i = tid; i < L; i += THREADS) {
-            const bool set = ((gbase | i) & qb) != 0;
-            if (set != (o == 1)) {
-              sm[tswz(i)] = make_double2(0.0, 0.0);
-            } else {
-              const double2 a = sm[tswz(i)];
-              sm[tswz(i)] = make_double2(__ddiv_rn(a.x, norm), __ddiv_rn(a.y, norm));
+          const uint32_t n0 = s_count[0], n1 = s_count[1];
+          const int o = n1 > n0 ? 1 : 0;  // go on with the longer list
+          if (n0 && n1) {
+            if (tid == 0 && rank == 0) {
+              atomicAdd(P.queue + 2, 1ULL);
+              s_task = atomicAdd(P.queue + 1, 1ULL);
             }
-          }
-          if (op.type == T_RESET && o == 1) {
-            // X on q: an exact exchange of the two halves
             if (C > 1) cl.sync(); else __syncthreads();
-            if (q < lb) {
-              for (uint32_t k = tid; k < L / 2; k += THREADS) {
-                const uint32_t a0 = ins0(k, q), a1 = a0 | (uint32_t)qb;
-                const double2 x = sm[tswz(a0)];
-                sm[tswz(a0)] = sm[tswz(a1)];
-                sm[tswz(a1)] = x;
-              }
-            } else {
-              const uint32_t tbr = 1u << (q - lb);
-              if (!(rank & tbr)) {
-                double2* other = cl.map_shared_rank(sm, rank | tbr);
-                for (uint32_t i = tid; i < L; i += THREADS) {
-                  const double2 x = sm[i];
-                  sm[i] = other[i];
-                  other[i] = x;
-                }
-              }
+            const unsigned long long t = rank == 0 ? s_task : *cl.map_shared_rank(&s_task, 0);
+            const bool saved = t < P.nslots;
+            if (saved) {
+              double2* d = P.slots + (t << pg.n) + gbase;
+              for (uint32_t i = tid; i < L; i += THREADS) __stcg(d + i, sm[i]);
+              if (rank == 0)
+                for (uint32_t i = tid; i < pg.ncbits; i += THREADS) P.slot_cbits[t * pg.ncbits + i] = cb[i];
+              __threadfence();
             }
+            if (C > 1) cl.sync(); else __syncthreads();
+            if (tid == 0 && rank == 0) {
+              TTask w{};
+              w.prog = it.prog;
+              w.oi = oi;
+              w.lo = o ? lo : lo + n0;
+              w.hi = o ? lo + n0 : hi;
+              w.src = src;
+              w.slot = saved ? (int32_t)t : -1;
+              w.outcome = o ? 0u : 1u;
+              w.draws = (uint32_t)draws;
+              w.p1 = p1;
+              P.tasks[t] = w;
+              st_release(P.ready + t, 1);
+            }
+            if (o) lo += n0; else hi = lo + n0;
           }
+          collapse(op, o, norm_of(o, p1));
+          // read by conditions after this op's closing barrier only
+          if (tid == 0 && op.type == T_MEASURE) cb[op.cbit] = o;
           break;
         }
         case T_RPHASE: {
@@ -610,13 +804,16 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
     // classical bits and (optionally) the final state out; the next
     // trajectory re-initialises after a cluster barrier
     if (rank == 0)
-      for (uint32_t i = tid; i < pg.ncbits; i += THREADS)
-        P.cbits_out[pg.cbits_off + it.shot * pg.ncbits + i] = cb[i];
+      for (uint64_t i = tid; i < (uint64_t)(hi - lo) * pg.ncbits; i += THREADS) {
+        const uint32_t k = (uint32_t)(i / pg.ncbits), c = (uint32_t)(i - (uint64_t)k * pg.ncbits);
+        P.cbits_out[pg.cbits_off + shot_at(lo + k) * pg.ncbits + c] = cb[c];
+      }
     if (pg.state_out) {
       double2* dst = pg.state_out + (it.shot << pg.n) + gbase;
       for (uint32_t i = tid; i < L; i += THREADS) dst[i] = sm[tswz(i)];
     }
     sync_all(true);
+    if (rank == 0 && tid == 0) atomicAdd(P.queue + 2, ~0ULL);
   }
 }
 
@@ -961,6 +1158,18 @@ int add_program(LaunchSet& ls, const dq_inst* prog, uint64_t ninst, const dq_con
   return DQ_OK;
 }
 
+// The shots of the set's only program: one item whose shots share states
+// (shot indices of the lists are 32-bit; more shots than that run one by one).
+void add_shots(LaunchSet& ls, uint64_t shots) {
+  if (shots == 0) return;
+  if (shots < (1ULL << 31)) {
+    ls.items.push_back(TItem{0, (uint32_t)shots, 0});
+    return;
+  }
+  ls.items.resize(shots);
+  for (uint64_t s = 0; s < shots; ++s) ls.items[s] = TItem{0, 1, s};
+}
+
 // Launch geometry of k_traj: opt-in shared memory, cluster dimension and as
 // many clusters as can be resident at once (capped by the item count).
 struct TrajLaunch {
@@ -1028,7 +1237,11 @@ struct LaunchBuffers {
   TItem* items = nullptr;
   uint8_t* blob = nullptr;
   TSweep* sweeps = nullptr;
-  unsigned long long* ctr = nullptr;  // [0] queue, [1] boundary, [2] failed
+  unsigned long long* ctr = nullptr;  // [0..2] queue, [3] boundary, [4] failed
+  void* share = nullptr;              // shot lists, tasks and draws (set_shared)
+  void* slots = nullptr;              // saved states, from the engine's buffer cache
+  size_t slot_bytes = 0;
+  int device = 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaStream_t st = nullptr;
   bool own_st = false;  // destroy st with the buffers
@@ -1042,6 +1255,8 @@ struct LaunchBuffers {
     if (blob) cudaFree(blob);
     if (sweeps) cudaFree(sweeps);
     if (ctr) cudaFree(ctr);
+    if (share) cudaFree(share);
+    if (slots) cache_free(device, slot_bytes, slots);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (own_st && st) cudaStreamDestroy(st);
@@ -1054,6 +1269,68 @@ int upload(T** dst, const std::vector<T>& v, cudaStream_t st) {
   DQ_CUDA_TRY(cudaMalloc((void**)dst, bytes));
   if (!v.empty())
     DQ_CUDA_TRY(cudaMemcpyAsync(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, st));
+  return DQ_OK;
+}
+
+constexpr int kCtrWords = 5;
+constexpr unsigned long long kNotFailed = 0x7fffffffffffffffULL;
+
+uint32_t draws_of(const TOp* ops, size_t n) {
+  uint32_t d = 0;
+  for (size_t i = 0; i < n; ++i) d += ops[i].type == T_MEASURE || ops[i].type == T_RESET;
+  return d;
+}
+
+// Buffers of a launch whose single program is shared by `shots` shots with up
+// to `ndraws` draws each.  Saved states take at most 1 GiB (a split past that
+// runs its program again from the start, as every shot would without sharing),
+// the table of draws at most 64 MiB (draws past it are computed in place).
+int set_shared(LaunchBuffers& b, TrajParams& P, int device, uint32_t n, uint64_t shots, uint32_t ncbits,
+               uint32_t ndraws, cudaStream_t st) {
+  if (shots < 2 || ndraws == 0) return DQ_OK;
+  b.device = device;
+  const size_t state = sizeof(double2) << n;
+  uint64_t slots = std::min<uint64_t>(shots - 1, std::max<uint64_t>((1ULL << 30) / state, 1));
+  while (slots && cache_alloc(device, slots * state, &b.slots) != DQ_OK) {
+    clear_error();
+    b.slots = nullptr;
+    slots /= 2;
+  }
+  b.slot_bytes = slots * state;
+  const uint32_t blocks = (ndraws + 7) / 8;
+  const bool table = shots * blocks * 64 <= (64ULL << 20);
+  size_t off[6], at = 0;
+  const size_t bytes[5] = {4 * shots, 4 * shots, sizeof(TTask) * shots, 4 * (size_t)slots * ncbits,
+                           table ? (size_t)shots * blocks * 64 : 0};
+  for (int i = 0; i < 5; ++i) {
+    off[i] = at;
+    at += (bytes[i] + 15) / 16 * 16;
+  }
+  off[5] = at;  // ready flags
+  DQ_CUDA_TRY(cudaMalloc(&b.share, at + 4 * shots));
+  uint8_t* base = static_cast<uint8_t*>(b.share);
+  P.order[0] = reinterpret_cast<uint32_t*>(base + off[0]);
+  P.order[1] = reinterpret_cast<uint32_t*>(base + off[1]);
+  P.tasks = reinterpret_cast<TTask*>(base + off[2]);
+  P.slot_cbits = reinterpret_cast<int32_t*>(base + off[3]);
+  P.draws = table ? reinterpret_cast<double*>(base + off[4]) : nullptr;
+  P.draw_stride = blocks * 8;
+  P.ready = reinterpret_cast<int*>(base + off[5]);
+  P.slots = static_cast<double2*>(b.slots);
+  P.nslots = (uint32_t)slots;
+  return DQ_OK;
+}
+
+// Work enqueued before every launch of a set_shared program.
+int reset_shared(const TrajParams& P, uint64_t shots, cudaStream_t st) {
+  if (!P.tasks) return DQ_OK;
+  DQ_CUDA_TRY(cudaMemsetAsync(P.ready, 0, 4 * shots, st));
+  if (P.draws) {
+    const uint64_t work = shots * (P.draw_stride / 8);
+    k_traj_draws<<<(unsigned)((work + 127) / 128), 128, 0, st>>>(P.progs, shots, P.draw_stride / 8,
+                                                                  const_cast<double*>(P.draws));
+    DQ_CUDA_TRY(cudaGetLastError());
+  }
   return DQ_OK;
 }
 
@@ -1076,8 +1353,8 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
     DQ_TRY(upload(&b.blob, ls.blob, st));
   }
   DQ_TRY(upload(&b.sweeps, ls.sweeps, st));
-  DQ_CUDA_TRY(cudaMalloc((void**)&b.ctr, 3 * sizeof(unsigned long long)));
-  const unsigned long long init[3] = {0ULL, 0ULL, 0x7fffffffffffffffULL};
+  DQ_CUDA_TRY(cudaMalloc((void**)&b.ctr, kCtrWords * sizeof(unsigned long long)));
+  const unsigned long long init[kCtrWords] = {0ULL, 0ULL, ls.items.size(), 0ULL, kNotFailed};
   DQ_CUDA_TRY(cudaMemcpyAsync(b.ctr, init, sizeof(init), cudaMemcpyHostToDevice, st));
   DQ_CUDA_TRY(cudaEventCreate(&b.e0));
   DQ_CUDA_TRY(cudaEventCreate(&b.e1));
@@ -1089,25 +1366,30 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
   P.items = b.items;
   P.cbits_out = d_cbits;
   P.queue = b.ctr;
-  P.boundary = b.ctr + 1;
-  P.failed = reinterpret_cast<long long*>(b.ctr + 2);
+  P.boundary = b.ctr + 3;
+  P.failed = reinterpret_cast<long long*>(b.ctr + 4);
   P.nitems = ls.items.size();
   P.sweep_blob = b.blob;
   P.sweeps = b.sweeps;
-  (void)device;
+  // several shots of one program share states
+  const uint64_t shots = ls.items.size() == 1 ? ls.items[0].count : 1;
+  const uint32_t ndraws = shots > 1 ? draws_of(ls.enc.ops.data(), ls.enc.ops.size()) : 0;
+  if (shots > 1)
+    DQ_TRY(set_shared(b, P, device, ls.progs[0].n, shots, ls.progs[0].ncbits, ndraws, st));
   TrajLaunch L;
-  DQ_TRY(config_traj(threads, ls.C, traj_smem(ls), P.nitems, &L));
+  DQ_TRY(config_traj(threads, ls.C, traj_smem(ls), P.tasks ? shots : P.nitems, &L));
   const uint32_t clusters = L.clusters;
   DQ_CUDA_TRY(cudaEventRecord(b.e0, st));
+  DQ_TRY(reset_shared(P, shots, st));
   DQ_TRY(launch_traj(L, P, st));
   DQ_CUDA_TRY(cudaEventRecord(b.e1, st));
-  unsigned long long ctr[3];
+  unsigned long long ctr[kCtrWords];
   DQ_CUDA_TRY(cudaMemcpyAsync(ctr, b.ctr, sizeof(ctr), cudaMemcpyDeviceToHost, st));
   DQ_CUDA_TRY(cudaStreamSynchronize(st));
   float ms = 0.f;
   DQ_CUDA_TRY(cudaEventElapsedTime(&ms, b.e0, b.e1));
-  acc->boundary_draws += ctr[1];
-  const long long f = (long long)ctr[2];
+  acc->boundary_draws += ctr[3];
+  const long long f = (long long)ctr[4];
   if (f != 0x7fffffffffffffffLL && (acc->failed_inst < 0 || f < acc->failed_inst))
     acc->failed_inst = f;
   acc->kernel_ms += ms;
@@ -1169,7 +1451,7 @@ struct dq_traj_plan_s {
   int32_t* d_cbits = nullptr;
   int32_t* h_cbits = nullptr;            // pinned
   uint64_t* h_seed = nullptr;            // pinned: base seed of the next replay
-  unsigned long long* h_ctr = nullptr;   // pinned: [0..3) initial, [3..6) results
+  unsigned long long* h_ctr = nullptr;   // pinned: kCtrWords initial, then kCtrWords results
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   dq::TrajLaunch L;
@@ -1213,8 +1495,7 @@ int dq_run_trajectories(int device, uint32_t n, const dq_inst* prog, uint64_t ni
   ls.C = C;
   DQ_TRY(add_program(ls, prog, ninst, conds, nconds, n, lb, base_seed + shot0, 0,
                      (uint32_t)ncbits, nullptr));
-  ls.items.resize(shots);
-  for (uint64_t s = 0; s < shots; ++s) ls.items[s] = TItem{0, 0, s};
+  add_shots(ls, shots);
   acc.prepare_ms = ms_since(t0);
 
   DeviceGuard g(device);
@@ -1463,7 +1744,7 @@ int dq_run_batch(int device, const dq_batch_item* items, uint64_t nitems,
                            o.cbits_off, (uint32_t)it.ncbits,
                            o.state_off == ~0ULL ? nullptr : d_states + o.state_off);
       }
-      ls.items.push_back(TItem{pi, 0, 0});
+      ls.items.push_back(TItem{pi, 1, 0});
     }
     acc.prepare_ms += ms_since(tp);
     mark("encode set");
@@ -1563,8 +1844,7 @@ int dq_traj_plan_create(int device, uint32_t n, const dq_inst* prog, uint64_t ni
   LaunchSet ls;
   ls.C = C;
   DQ_TRY(add_program(ls, prog, ninst, conds, nconds, n, lb, 0, 0, (uint32_t)ncbits, nullptr));
-  ls.items.resize(shots);
-  for (uint64_t s = 0; s < shots; ++s) ls.items[s] = TItem{0, 0, s};
+  add_shots(ls, shots);
   if (ls.enc.pool.empty()) ls.enc.pool.push_back(make_double2(0, 0));
 
   DeviceGuard g(device);
@@ -1595,17 +1875,19 @@ int dq_traj_plan_create(int device, uint32_t n, const dq_inst* prog, uint64_t ni
   if ((rc = upload(&p->buf.conds, ls.conds, st)) != DQ_OK) return bail(rc);
   if ((rc = upload(&p->buf.progs, ls.progs, st)) != DQ_OK) return bail(rc);
   if ((rc = upload(&p->buf.items, ls.items, st)) != DQ_OK) return bail(rc);
-  cu(cudaMalloc((void**)&p->buf.ctr, 3 * sizeof(unsigned long long)), "cudaMalloc(counters)");
+  cu(cudaMalloc((void**)&p->buf.ctr, kCtrWords * sizeof(unsigned long long)), "cudaMalloc(counters)");
   cu(cudaMalloc((void**)&p->d_cbits, std::max<size_t>(out_bytes, 4)), "cudaMalloc(cbits)");
   cu(cudaMallocHost((void**)&p->h_cbits, std::max<size_t>(out_bytes, 4)), "cudaMallocHost(cbits)");
   cu(cudaMallocHost((void**)&p->h_seed, sizeof(uint64_t)), "cudaMallocHost(seed)");
-  cu(cudaMallocHost((void**)&p->h_ctr, 6 * sizeof(unsigned long long)), "cudaMallocHost(counters)");
+  cu(cudaMallocHost((void**)&p->h_ctr, 2 * kCtrWords * sizeof(unsigned long long)), "cudaMallocHost(counters)");
   cu(cudaEventCreate(&p->buf.e0), "cudaEventCreate");
   cu(cudaEventCreate(&p->buf.e1), "cudaEventCreate");
   if (rc != DQ_OK) return bail(rc);
   p->h_ctr[0] = 0;
   p->h_ctr[1] = 0;
-  p->h_ctr[2] = 0x7fffffffffffffffULL;
+  p->h_ctr[2] = ls.items.size();
+  p->h_ctr[3] = 0;
+  p->h_ctr[4] = kNotFailed;
   p->h_seed[0] = 0;
   TrajParams& P = p->P;
   P.ops = p->buf.ops;
@@ -1615,10 +1897,14 @@ int dq_traj_plan_create(int device, uint32_t n, const dq_inst* prog, uint64_t ni
   P.items = p->buf.items;
   P.cbits_out = p->d_cbits;
   P.queue = p->buf.ctr;
-  P.boundary = p->buf.ctr + 1;
-  P.failed = reinterpret_cast<long long*>(p->buf.ctr + 2);
-  P.nitems = shots;
-  if ((rc = config_traj(threads, C, traj_smem(ls), shots, &p->L)) != DQ_OK) return bail(rc);
+  P.boundary = p->buf.ctr + 3;
+  P.failed = reinterpret_cast<long long*>(p->buf.ctr + 4);
+  P.nitems = ls.items.size();
+  if (ls.items.size() == 1 &&
+      (rc = set_shared(p->buf, P, device, n, shots, (uint32_t)ncbits,
+                       draws_of(ls.enc.ops.data(), ls.enc.ops.size()), st)) != DQ_OK)
+    return bail(rc);
+  if ((rc = config_traj(threads, C, traj_smem(ls), P.tasks ? shots : P.nitems, &p->L)) != DQ_OK) return bail(rc);
   cu(cudaStreamSynchronize(st), "cudaStreamSynchronize");
   if (rc != DQ_OK) return bail(rc);
   // capture: seed -> program table, counters reset, launch, results back
@@ -1626,13 +1912,14 @@ int dq_traj_plan_create(int device, uint32_t n, const dq_inst* prog, uint64_t ni
   if (rc != DQ_OK) return bail(rc);
   cu(cudaMemcpyAsync(&p->buf.progs[0].base_seed, p->h_seed, sizeof(uint64_t),
                      cudaMemcpyHostToDevice, st), "capture seed copy");
-  cu(cudaMemcpyAsync(p->buf.ctr, p->h_ctr, 3 * sizeof(unsigned long long), cudaMemcpyHostToDevice,
+  cu(cudaMemcpyAsync(p->buf.ctr, p->h_ctr, kCtrWords * sizeof(unsigned long long), cudaMemcpyHostToDevice,
                      st), "capture counter reset");
+  if (rc == DQ_OK) rc = reset_shared(P, shots, st);
   if (rc == DQ_OK) rc = launch_traj(p->L, P, st);
   if (out_bytes)
     cu(cudaMemcpyAsync(p->h_cbits, p->d_cbits, out_bytes, cudaMemcpyDeviceToHost, st),
        "capture cbits copy");
-  cu(cudaMemcpyAsync(p->h_ctr + 3, p->buf.ctr, 3 * sizeof(unsigned long long),
+  cu(cudaMemcpyAsync(p->h_ctr + kCtrWords, p->buf.ctr, kCtrWords * sizeof(unsigned long long),
                      cudaMemcpyDeviceToHost, st), "capture counter copy");
   cudaGraph_t graph = nullptr;
   const cudaError_t ee = cudaStreamEndCapture(st, &graph);
@@ -1665,8 +1952,8 @@ int dq_traj_plan_run(dq_traj_plan_t p, uint64_t base_seed, int32_t* cbits_out,
   DQ_CUDA_TRY(cudaEventElapsedTime(&ms, p->buf.e0, p->buf.e1));
   if (out_bytes) memcpy(cbits_out, p->h_cbits, out_bytes);
   dq_traj_stats s = p->geom;
-  s.boundary_draws = p->h_ctr[4];
-  const long long f = (long long)p->h_ctr[5];
+  s.boundary_draws = p->h_ctr[kCtrWords + 3];
+  const long long f = (long long)p->h_ctr[kCtrWords + 4];
   s.failed_inst = f == 0x7fffffffffffffffLL ? -1 : (f & ((1LL << 40) - 1));
   s.kernel_ms = ms;
   if (stats) *stats = s;

@@ -210,3 +210,42 @@ def test_graph_plan_replays_match(gpu):
             assert (got == want).all()
         assert st.kernel_ms > 0.0
     plan.release()
+
+
+def measured_circuit(n, rounds, seed, reset=True):
+    """u3 + cx layers with every qubit measured (and some reset) in between: almost every
+    shot has outcomes of its own."""
+    rng = np.random.default_rng(seed)
+    insts, c = [], 0
+    for _ in range(rounds):
+        for q in range(n):
+            insts.append(g("u3", q, *rng.uniform(0, 6, 3).tolist()))
+        insts += [g("cx", q, q + 1) for q in range(n - 1)]
+        for q in range(0, n, 2):
+            insts.append(g("measure", q, c))
+            insts.append(cond(c, 1, 1, g("h", q)))
+            c += 1
+        if reset:
+            insts.append(g("reset", n - 1))
+    return JsonCircuit(n, insts, ncbits=c)
+
+
+# shots that share states: a list that never splits, a chain of splits down to single
+# shots, states of one CTA and of clusters, more splits (n = 16, 1500 shots) than saved states
+@pytest.mark.parametrize("n,rounds,shots,check", [(1, 3, 1, 1), (1, 40, 300, 300), (3, 5, 257, 257),
+                                                  (7, 4, 1000, 200), (13, 2, 130, 12), (14, 2, 130, 12),
+                                                  (16, 2, 1500, 8)])
+def test_shared_shots_match_oracle(gpu, n, rounds, shots, check):
+    prog = prog_of(measured_circuit(n, rounds, 31 + n))
+    got, st = trajectories_resident(prog, 77, shots, 0)
+    want, rc, _ = orc.run_shots(prog, 77, min(check, shots))
+    assert rc == 0 and st.boundary_draws == 0
+    assert np.array_equal(got[:want.shape[0]], want)
+    plan = TrajectoryPlan(prog, shots, 0)
+    for seed in (77, 78, 77):
+        again, st2 = plan.run(seed)
+        if seed == 77:
+            assert np.array_equal(again, got) and st2.boundary_draws == st.boundary_draws
+    plan.release()
+    tail, _ = trajectories_resident(prog, 77, 1, 0, shot0=shots - 1)
+    assert np.array_equal(tail[0], got[-1])
