@@ -466,3 +466,26 @@ def test_cluster_batches_match_oracle(shots, max_bond):
     for i in sorted({0, 1, shots // 2, shots - 1}):
         _, rcb, _, _ = _oracle.mps_run(prog, 5 + i, max_bond=max_bond)
         assert bits[i].tolist() == rcb.tolist(), i
+
+
+# shots that share replicas: one shot, a chain of splits down to a replica per shot, more
+# than 296 replicas at the end (the batched kernels), conditions and resets on the way
+@pytest.mark.parametrize("n,rounds,shots", [(2, 1, 1), (2, 6, 150), (5, 3, 64), (6, 3, 700), (9, 2, 400)])
+def test_shared_shots_match_oracle_per_shot(n, rounds, shots):
+    rng = np.random.default_rng(40 + n)
+    insts, c = [], 0
+    for _ in range(rounds):
+        for q in range(n):
+            insts.append(g("u3", q, *rng.uniform(0, 6, 3).tolist()))
+        insts += [g("cx", q, q + 1) for q in range(n - 1)]
+        for q in range(n):
+            insts += [g("measure", q, c), cond(c, 1, 1, g("h", q))]
+            c += 1
+        insts.append(g("reset", n - 1))
+    prog = prog_of(JsonCircuit(n, insts, ncbits=c))
+    bits, st = run_mps_shots(prog, 9, shots, 0, None, 1e-12)
+    for i in range(0, shots, max(1, shots // 60)):
+        _, rcb, _, calls = _oracle.mps_run(prog, 9 + i)
+        assert bits[i].tolist() == rcb.tolist(), i
+    again, st2 = run_mps_shots(prog, 9, shots, 0, None, 1e-12, batch=97)
+    assert np.array_equal(again, bits) and st2.svd_calls == st.svd_calls
