@@ -770,14 +770,38 @@ int dq_adjoint_batch(int device, uint32_t n, const dq_inst* prog, uint64_t ninst
   for (uint64_t s = 0; s < nsets; ++s)
     if (!plans[s].foffs.empty()) rb = plans[s].rb;
   const uint64_t len = 1ULL << n;
-  // sets resident at a time: psi and lambda of each in about half the free memory
-  size_t freeb = 0, totalb = 0;
-  DQ_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
+  // sets resident at a time: psi and lambda of each in about half the free
+  // memory (asked for when they are large or cannot be had), from the engine's
+  // size-keyed buffer cache: repeated calls (an optimiser loop) do not pay
+  // cudaMalloc/cudaFree
   const uint64_t per_set = 2 * sizeof(double2) * len + 64 * 1024;
-  const uint64_t G = std::max<uint64_t>(1, std::min<uint64_t>(nsets, (freeb / 2) / per_set));
+  uint64_t G = nsets;
+  void* pv = nullptr;
+  void* lv = nullptr;
+  auto take_states = [&]() -> int {
+    int r = cache_alloc(device, sizeof(double2) * len * G, &pv);
+    if (r != DQ_OK) pv = nullptr;
+    else if ((r = cache_alloc(device, sizeof(double2) * len * G, &lv)) != DQ_OK) {
+      cache_free(device, sizeof(double2) * len * G, pv);
+      pv = lv = nullptr;
+    }
+    return r;
+  };
+  int rc = nsets * per_set <= unasked_budget(device) ? take_states() : DQ_ERR_OOM;
+  if (rc == DQ_ERR_OOM) {
+    clear_error();
+    size_t freeb = 0, totalb = 0;
+    DQ_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
+    G = std::max<uint64_t>(1, std::min<uint64_t>(nsets, (freeb / 2) / per_set));
+    rc = take_states();
+  }
   cudaStream_t st = nullptr;
-  DQ_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  int rc = DQ_OK;
+  if (rc == DQ_OK) rc = stream_take(device, &st);
+  if (rc != DQ_OK) {
+    if (pv) cache_free(device, sizeof(double2) * len * G, pv);
+    if (lv) cache_free(device, sizeof(double2) * len * G, lv);
+    return rc;
+  }
   auto cu = [&](cudaError_t e, const char* what) {
     if (e != cudaSuccess && rc == DQ_OK) {
       cudaGetLastError();
@@ -787,7 +811,7 @@ int dq_adjoint_batch(int device, uint32_t n, const dq_inst* prog, uint64_t ninst
   };
   DeviceTerms t;
   rc = upload_terms(terms, nterms, n, st, &t);
-  double2 *psi = nullptr, *lam = nullptr;
+  double2 *psi = (double2*)pv, *lam = (double2*)lv;
   double* slots = nullptr;
   double* part = nullptr;
   unsigned* ctr = nullptr;
@@ -829,14 +853,6 @@ int dq_adjoint_batch(int device, uint32_t n, const dq_inst* prog, uint64_t ninst
   acc.forward_sweeps = kf;
   acc.backward_sweeps = kb;
   if (rc == DQ_OK) {
-    // psi and lambda of the group come from the engine's size-keyed buffer
-    // cache: repeated calls (an optimiser loop) do not pay cudaMalloc/cudaFree
-    void* pv = nullptr;
-    void* lv = nullptr;
-    rc = cache_alloc(device, sizeof(double2) * len * G, &pv);
-    if (rc == DQ_OK) rc = cache_alloc(device, sizeof(double2) * len * G, &lv);
-    psi = (double2*)pv;
-    lam = (double2*)lv;
     // the small buffers also from the cache: an optimiser loop repeats their sizes
     void* p = nullptr;
     if (rc == DQ_OK && (rc = cache_alloc(device, sizeof(double) * sl * G, &p)) == DQ_OK) slots = (double*)p;
@@ -968,7 +984,7 @@ int dq_adjoint_batch(int device, uint32_t n, const dq_inst* prog, uint64_t ninst
   if (ctr) cache_free(device, sizeof(unsigned) * G, ctr);
   if (fblob) cache_free(device, fall_bytes, fblob);
   if (d_jobs) cache_free(device, sizeof(SweepJob) * std::max<size_t>(1, kf * G), d_jobs);
-  cudaStreamDestroy(st);
+  stream_give(device, st);
   mark("gradients+finish");
   acc.batched = 1;
   if (stats) *stats = acc;

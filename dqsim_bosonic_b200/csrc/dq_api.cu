@@ -114,6 +114,53 @@ void cache_free(int device, size_t bytes, void* p) {
   }
 }
 
+uint64_t unasked_budget(int device) {
+  static std::mutex mu;
+  static uint64_t total[64];
+  std::lock_guard<std::mutex> lk(mu);
+  uint64_t& t = total[device & 63];
+  if (!t) {
+    size_t f = 0, all = 0;
+    if (cudaMemGetInfo(&f, &all) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    t = all;
+  }
+  return t / 16;
+}
+
+std::mutex g_stream_mu;
+std::map<int, std::vector<cudaStream_t>> g_streams;
+
+int stream_take(int device, cudaStream_t* out) {
+  {
+    std::lock_guard<std::mutex> lk(g_stream_mu);
+    auto& v = g_streams[device];
+    if (!v.empty()) {
+      *out = v.back();
+      v.pop_back();
+      return DQ_OK;
+    }
+  }
+  *out = nullptr;
+  DQ_CUDA_TRY(cudaStreamCreateWithFlags(out, cudaStreamNonBlocking));
+  return DQ_OK;
+}
+
+void stream_give(int device, cudaStream_t st) {
+  if (!st) return;
+  if (cudaStreamSynchronize(st) == cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_stream_mu);
+    auto& v = g_streams[device];
+    if (v.size() < 8) {
+      v.push_back(st);
+      return;
+    }
+  }
+  cudaStreamDestroy(st);
+}
+
 // Pinned host staging buffers, kept by size class (a power of two of at
 // least 1 MiB) so that repeated large uploads neither page-fault fresh host
 // memory nor pay cudaHostAlloc.

@@ -56,6 +56,15 @@ struct DeviceGuard {
 // Device buffers of state size are recycled through a per-(device, size) cache.
 int cache_alloc(int device, size_t bytes, void** out);
 void cache_free(int device, size_t bytes, void* p);
+// Device memory a call may try to allocate before it asks how much is free (a
+// sixteenth of the device's memory): cudaMemGetInfo takes 0.4 to 4 ms next to
+// live memory pools.  A call whose allocation fails asks after all.
+uint64_t unasked_budget(int device);
+// Non-blocking streams for calls without a handle of their own, kept for the
+// next call (at most 8 per device; creating and destroying one takes 150 us).
+// A stream given back has no work pending.
+int stream_take(int device, cudaStream_t* out);
+void stream_give(int device, cudaStream_t st);
 // Pinned host staging buffers (at least `bytes`), recycled by size class.
 int pinned_alloc(size_t bytes, void** out);
 void pinned_free(size_t bytes, void* p);

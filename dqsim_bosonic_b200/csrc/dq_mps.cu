@@ -1457,7 +1457,7 @@ struct dq_mps_s {
   uint32_t nshots = 0;       // shots of the batch when they share replicas, else 0
   uint64_t base_seed = 0;
   bool broken = false;       // a failed reserve lost the state: every later call fails
-  size_t buf_bytes[9] = {};  // sizes of t, dims, key, ctr, cbits, flags, svd_calls, scratch, share
+  size_t buf_bytes[8] = {};  // sizes of t, dims, key, ctr, cbits, flags, svd_calls, scratch
   bool smem = true;
   uint64_t scratch_elems = 0;
   size_t work_bytes = 0;
@@ -1480,8 +1480,8 @@ uint32_t bond_bound(uint32_t n, uint32_t max_bond) {
 // repeated shot runs and simulations of one shape pay no cudaMalloc / cudaFree
 // (a shot run creates and destroys its handle every call).
 void** mps_buf(dq_mps_s* h, int i) {
-  void** p[9] = {(void**)&h->t, (void**)&h->dims, (void**)&h->key, (void**)&h->ctr, (void**)&h->cbits,
-                 (void**)&h->flags, (void**)&h->svd_calls, (void**)&h->scratch, (void**)&h->share};
+  void** p[8] = {(void**)&h->t, (void**)&h->dims, (void**)&h->key, (void**)&h->ctr,
+                 (void**)&h->cbits, (void**)&h->flags, (void**)&h->svd_calls, (void**)&h->scratch};
   return p[i];
 }
 
@@ -1500,14 +1500,15 @@ int mps_take(dq_mps_s* h, int i, size_t bytes) {
 void free_buffers(dq_mps_s* h) {
   // a cached buffer may be handed out at once: nothing may still use it
   if (h->stream) cudaStreamSynchronize(h->stream);
-  for (int i = 0; i < 9; ++i) {
+  for (int i = 0; i < 8; ++i) {
     void** p = mps_buf(h, i);
     if (*p) cache_free(h->device, h->buf_bytes[i], *p);
     *p = nullptr;
     h->buf_bytes[i] = 0;
   }
-  cudaFree(h->conds);
-  cudaFree(h->ops);
+  if (h->conds) cudaFreeAsync(h->conds, h->stream);
+  if (h->ops) cudaFreeAsync(h->ops, h->stream);
+  if (h->share) cudaFreeAsync(h->share, h->stream);
   h->ops = nullptr;
   h->ops_cap = 0;
   h->t = nullptr; h->dims = nullptr; h->key = nullptr; h->ctr = nullptr; h->cbits = nullptr;
@@ -1781,10 +1782,10 @@ uint32_t program_bound(uint32_t n, uint32_t max_bond, const std::vector<MpsOp>& 
 int launch_ops(dq_mps_s* h, const std::vector<MpsOp>& ops) {
   if (ops.empty()) return DQ_OK;
   if (ops.size() > h->ops_cap) {
-    cudaFree(h->ops);
+    if (h->ops) cudaFreeAsync(h->ops, h->stream);
     h->ops = nullptr;
     h->ops_cap = 0;
-    DQ_CUDA_TRY(cudaMalloc(&h->ops, sizeof(MpsOp) * ops.size()));
+    DQ_CUDA_TRY(pool_malloc_async(&h->ops, sizeof(MpsOp) * ops.size(), h->stream));
     h->ops_cap = ops.size();
   }
   DQ_CUDA_TRY(cudaMemcpyAsync(h->ops, ops.data(), sizeof(MpsOp) * ops.size(), cudaMemcpyHostToDevice,
@@ -1894,9 +1895,10 @@ int run_batch(dq_mps_s* h, const std::vector<MpsOp>& ops, const dq_cond* conds, 
   for (;;) {
     if (h->batch != batch || h->ncb != (ncb ? ncb : 1) || !h->t) DQ_TRY(alloc_buffers(h, batch, h->cap, ncb));
     if (nconds > h->conds_cap) {
-      cudaFree(h->conds);
+      if (h->conds) cudaFreeAsync(h->conds, h->stream);
       h->conds = nullptr;
-      DQ_CUDA_TRY(cudaMalloc((void**)&h->conds, sizeof(dq_cond) * nconds));
+      h->conds_cap = 0;
+      DQ_CUDA_TRY(pool_malloc_async((void**)&h->conds, sizeof(dq_cond) * nconds, h->stream));
       h->conds_cap = nconds;
     }
     if (nconds)
@@ -1910,7 +1912,7 @@ int run_batch(dq_mps_s* h, const std::vector<MpsOp>& ops, const dq_cond* conds, 
       size_t nmeas = 1;
       for (const MpsOp& op : ops) nmeas += op.kind == M_MEAS || op.kind == M_RESET;
       h->count_off = share_bytes(batch, h->ncb);
-      if (!h->share) DQ_TRY(mps_take(h, 8, h->count_off + nmeas * sizeof(uint2)));
+      if (!h->share) DQ_CUDA_TRY(pool_malloc_async(&h->share, h->count_off + nmeas * sizeof(uint2), h->stream));
       DQ_CUDA_TRY(cudaMemsetAsync(static_cast<uint8_t*>(h->share) + h->count_off, 0, nmeas * sizeof(uint2), h->stream));
     }
     std::vector<uint32_t> keys((size_t)h->nrep * 8);
@@ -1986,9 +1988,10 @@ int new_handle(uint32_t n, int device, uint32_t max_bond, double thr, dq_mps_s**
   h->max_bond = max_bond;
   h->thr = thr;
   h->cap = std::min<uint32_t>(bond_bound(n, max_bond), 16u);
-  if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
+  const int rc = stream_take(device, &h->stream);
+  if (rc != DQ_OK) {
     delete h;
-    return fail(DQ_ERR_CUDA, "cudaStreamCreate failed");
+    return rc;
   }
   *out = h;
   return DQ_OK;
@@ -1996,9 +1999,8 @@ int new_handle(uint32_t n, int device, uint32_t max_bond, double thr, dq_mps_s**
 
 void destroy_handle(dq_mps_s* h) {
   DeviceGuard g(h->device);
-  cudaStreamSynchronize(h->stream);
   free_buffers(h);
-  cudaStreamDestroy(h->stream);
+  stream_give(h->device, h->stream);
   h->stream = nullptr;
   delete h;
 }
@@ -2277,14 +2279,21 @@ int dq_mps_run_shots(int device, uint32_t n, uint32_t max_bond, double truncatio
   DQ_TRY(new_handle(n, device, max_bond, truncation_threshold, &h));
   DeviceGuard g(device);
   const uint32_t bmax = batch ? batch : 4096u;
-  // device memory for one batch: at most a quarter of the free memory
-  size_t free_b = 0, total_b = 0;
-  cudaMemGetInfo(&free_b, &total_b);
-  const uint64_t budget = std::max<uint64_t>(free_b / 4, 1ull << 28);
+  // device memory for one batch: at most a quarter of the free memory, which
+  // is only asked for when a batch is large or does not fit
+  bool asked = false;
+  uint64_t budget = unasked_budget(device);
+  auto ask = [&] {
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    budget = std::max<uint64_t>(free_b / 4, 1ull << 28);
+    asked = true;
+  };
   int rc = DQ_OK;
   double total_ms = 0.0;
   unsigned long long calls = 0;
   for (uint64_t s0 = 0; s0 < shots && rc == DQ_OK;) {
+    if (!asked && std::min<uint64_t>(bmax, shots - s0) * replica_bytes(n, h->cap, 1) > budget) ask();
     const uint64_t fit = std::max<uint64_t>(budget / replica_bytes(n, h->cap, 1), 1);
     const uint32_t nb = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(bmax, fit), shots - s0);
     int st = 0, fi = 0;
@@ -2292,6 +2301,13 @@ int dq_mps_run_shots(int device, uint32_t n, uint32_t max_bond, double truncatio
     bool shrink = false;
     rc = run_batch(h, ops, conds, nconds, base_seed + shot0 + s0, nb, (uint32_t)ncbits, &st, &fi, &ms, budget,
                    &shrink, nb > 1);
+    if (rc == DQ_ERR_OOM && !asked) {
+      clear_error();
+      free_buffers(h);
+      ask();
+      rc = DQ_OK;
+      continue;
+    }
     if (rc != DQ_OK) break;
     if (shrink) continue;  // capacity grew: redo this chunk with fewer replicas
     int64_t f64 = -1;

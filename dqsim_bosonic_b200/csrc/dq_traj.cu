@@ -1002,8 +1002,7 @@ struct LaunchSet {
   std::vector<dq_cond> conds;
   std::vector<TProg> progs;
   std::vector<TItem> items;
-  std::vector<uint8_t> blob;     // sweep programs of the HBM items
-  // or, when set, the sweep programs staged in pinned host memory
+  // sweep programs of the HBM items, staged in pinned host memory
   const uint8_t* blob_host = nullptr;
   size_t blob_host_bytes = 0;
   std::vector<TSweep> sweeps;
@@ -1235,25 +1234,28 @@ struct LaunchBuffers {
   dq_cond* conds = nullptr;
   TProg* progs = nullptr;
   TItem* items = nullptr;
-  uint8_t* blob = nullptr;
-  TSweep* sweeps = nullptr;
   unsigned long long* ctr = nullptr;  // [0..2] queue, [3] boundary, [4] failed
-  void* share = nullptr;              // shot lists, tasks and draws (set_shared)
+  void* share = nullptr;              // shot lists, tasks, draws and small states (set_shared)
+  void* pooled_share = nullptr;       // the same for one launch, from the engine's pool
   void* slots = nullptr;              // saved states, from the engine's buffer cache
   size_t slot_bytes = 0;
   int device = 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaStream_t st = nullptr;
   bool own_st = false;  // destroy st with the buffers
+  void* block = nullptr;      // one launch's buffers, from the engine's pool on st
+  void* stage = nullptr;      // their pinned image
+  size_t stage_bytes = 0;
   ~LaunchBuffers() {
     if (st) cudaStreamSynchronize(st);
+    if (block) cudaFreeAsync(block, st);
+    if (pooled_share) cudaFreeAsync(pooled_share, st);
+    pinned_free(stage_bytes, stage);
     if (ops) cudaFree(ops);
     if (pool) cudaFree(pool);
     if (conds) cudaFree(conds);
     if (progs) cudaFree(progs);
     if (items) cudaFree(items);
-    if (blob) cudaFree(blob);
-    if (sweeps) cudaFree(sweeps);
     if (ctr) cudaFree(ctr);
     if (share) cudaFree(share);
     if (slots) cache_free(device, slot_bytes, slots);
@@ -1285,38 +1287,45 @@ uint32_t draws_of(const TOp* ops, size_t n) {
 // to `ndraws` draws each.  Saved states take at most 1 GiB (a split past that
 // runs its program again from the start, as every shot would without sharing),
 // the table of draws at most 64 MiB (draws past it are computed in place).
+// st: buffers from the engine's pool on that stream; null: they outlive a launch.
 int set_shared(LaunchBuffers& b, TrajParams& P, int device, uint32_t n, uint64_t shots, uint32_t ncbits,
                uint32_t ndraws, cudaStream_t st) {
   if (shots < 2 || ndraws == 0) return DQ_OK;
   b.device = device;
   const size_t state = sizeof(double2) << n;
-  uint64_t slots = std::min<uint64_t>(shots - 1, std::max<uint64_t>((1ULL << 30) / state, 1));
-  while (slots && cache_alloc(device, slots * state, &b.slots) != DQ_OK) {
-    clear_error();
-    b.slots = nullptr;
-    slots /= 2;
+  uint64_t slots = shots - 1;
+  const bool inline_slots = slots * state <= (64ULL << 20);
+  if (!inline_slots) {  // powers of two: few sizes in the buffer cache
+    slots = 1;
+    while (slots < shots - 1 && 2 * slots * state <= (1ULL << 30)) slots *= 2;
+    while (slots && cache_alloc(device, slots * state, &b.slots) != DQ_OK) {
+      clear_error();
+      b.slots = nullptr;
+      slots /= 2;
+    }
+    b.slot_bytes = slots * state;
   }
-  b.slot_bytes = slots * state;
   const uint32_t blocks = (ndraws + 7) / 8;
   const bool table = shots * blocks * 64 <= (64ULL << 20);
-  size_t off[6], at = 0;
-  const size_t bytes[5] = {4 * shots, 4 * shots, sizeof(TTask) * shots, 4 * (size_t)slots * ncbits,
-                           table ? (size_t)shots * blocks * 64 : 0};
-  for (int i = 0; i < 5; ++i) {
+  size_t off[7], at = 0;
+  const size_t bytes[6] = {4 * shots, 4 * shots, sizeof(TTask) * shots, 4 * (size_t)slots * ncbits,
+                           table ? (size_t)shots * blocks * 64 : 0, inline_slots ? slots * state : 0};
+  for (int i = 0; i < 6; ++i) {
     off[i] = at;
     at += (bytes[i] + 15) / 16 * 16;
   }
-  off[5] = at;  // ready flags
-  DQ_CUDA_TRY(cudaMalloc(&b.share, at + 4 * shots));
-  uint8_t* base = static_cast<uint8_t*>(b.share);
+  off[6] = at;  // ready flags
+  void** mem = st ? &b.pooled_share : &b.share;
+  DQ_CUDA_TRY(st ? pool_malloc_async(mem, at + 4 * shots, st) : cudaMalloc(mem, at + 4 * shots));
+  uint8_t* base = static_cast<uint8_t*>(*mem);
   P.order[0] = reinterpret_cast<uint32_t*>(base + off[0]);
   P.order[1] = reinterpret_cast<uint32_t*>(base + off[1]);
   P.tasks = reinterpret_cast<TTask*>(base + off[2]);
   P.slot_cbits = reinterpret_cast<int32_t*>(base + off[3]);
   P.draws = table ? reinterpret_cast<double*>(base + off[4]) : nullptr;
   P.draw_stride = blocks * 8;
-  P.ready = reinterpret_cast<int*>(base + off[5]);
-  P.slots = static_cast<double2*>(b.slots);
+  P.ready = reinterpret_cast<int*>(base + off[6]);
+  P.slots = inline_slots ? reinterpret_cast<double2*>(base + off[5]) : static_cast<double2*>(b.slots);
   P.nslots = (uint32_t)slots;
   return DQ_OK;
 }
@@ -1341,36 +1350,47 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
   if (ls.enc.pool.empty()) ls.enc.pool.push_back(make_double2(0, 0));
   LaunchBuffers b;
   b.st = st;
-  DQ_TRY(upload(&b.ops, ls.enc.ops, st));
-  DQ_TRY(upload(&b.pool, ls.enc.pool, st));
-  DQ_TRY(upload(&b.conds, ls.conds, st));
-  DQ_TRY(upload(&b.progs, ls.progs, st));
-  DQ_TRY(upload(&b.items, ls.items, st));
-  if (ls.blob_host) {
-    DQ_CUDA_TRY(cudaMalloc((void**)&b.blob, std::max<size_t>(ls.blob_host_bytes, 16)));
-    DQ_CUDA_TRY(cudaMemcpyAsync(b.blob, ls.blob_host, ls.blob_host_bytes, cudaMemcpyHostToDevice, st));
-  } else {
-    DQ_TRY(upload(&b.blob, ls.blob, st));
-  }
-  DQ_TRY(upload(&b.sweeps, ls.sweeps, st));
-  DQ_CUDA_TRY(cudaMalloc((void**)&b.ctr, kCtrWords * sizeof(unsigned long long)));
+  // one allocation and one copy from pinned memory; the sweep programs of HBM
+  // items are already pinned and follow in a copy of their own
   const unsigned long long init[kCtrWords] = {0ULL, 0ULL, ls.items.size(), 0ULL, kNotFailed};
-  DQ_CUDA_TRY(cudaMemcpyAsync(b.ctr, init, sizeof(init), cudaMemcpyHostToDevice, st));
+  struct { const void* p; size_t bytes, off; } part[7] = {
+      {ls.enc.ops.data(), sizeof(TOp) * ls.enc.ops.size(), 0},
+      {ls.enc.pool.data(), sizeof(double2) * ls.enc.pool.size(), 0},
+      {ls.conds.data(), sizeof(dq_cond) * ls.conds.size(), 0},
+      {ls.progs.data(), sizeof(TProg) * ls.progs.size(), 0},
+      {ls.items.data(), sizeof(TItem) * ls.items.size(), 0},
+      {ls.sweeps.data(), sizeof(TSweep) * ls.sweeps.size(), 0},
+      {init, sizeof(init), 0}};
+  size_t image = 0;
+  for (auto& x : part) {
+    x.off = image;
+    image += (x.bytes + 15) / 16 * 16;
+  }
+  DQ_TRY(pinned_alloc(image, &b.stage));
+  b.stage_bytes = image;
+  for (const auto& x : part)
+    if (x.bytes) memcpy(static_cast<uint8_t*>(b.stage) + x.off, x.p, x.bytes);
+  DQ_CUDA_TRY(pool_malloc_async(&b.block, image + ls.blob_host_bytes, st));
+  uint8_t* dev = static_cast<uint8_t*>(b.block);
+  DQ_CUDA_TRY(cudaMemcpyAsync(dev, b.stage, image, cudaMemcpyHostToDevice, st));
+  if (ls.blob_host_bytes)
+    DQ_CUDA_TRY(cudaMemcpyAsync(dev + image, ls.blob_host, ls.blob_host_bytes, cudaMemcpyHostToDevice, st));
+  unsigned long long* d_ctr = reinterpret_cast<unsigned long long*>(dev + part[6].off);
   DQ_CUDA_TRY(cudaEventCreate(&b.e0));
   DQ_CUDA_TRY(cudaEventCreate(&b.e1));
   TrajParams P{};
-  P.ops = b.ops;
-  P.pool = b.pool;
-  P.conds = b.conds;
-  P.progs = b.progs;
-  P.items = b.items;
+  P.ops = reinterpret_cast<const TOp*>(dev);
+  P.pool = reinterpret_cast<const double2*>(dev + part[1].off);
+  P.conds = reinterpret_cast<const dq_cond*>(dev + part[2].off);
+  P.progs = reinterpret_cast<const TProg*>(dev + part[3].off);
+  P.items = reinterpret_cast<const TItem*>(dev + part[4].off);
+  P.sweeps = reinterpret_cast<const TSweep*>(dev + part[5].off);
+  P.sweep_blob = dev + image;
   P.cbits_out = d_cbits;
-  P.queue = b.ctr;
-  P.boundary = b.ctr + 3;
-  P.failed = reinterpret_cast<long long*>(b.ctr + 4);
+  P.queue = d_ctr;
+  P.boundary = d_ctr + 3;
+  P.failed = reinterpret_cast<long long*>(d_ctr + 4);
   P.nitems = ls.items.size();
-  P.sweep_blob = b.blob;
-  P.sweeps = b.sweeps;
   // several shots of one program share states
   const uint64_t shots = ls.items.size() == 1 ? ls.items[0].count : 1;
   const uint32_t ndraws = shots > 1 ? draws_of(ls.enc.ops.data(), ls.enc.ops.size()) : 0;
@@ -1383,8 +1403,9 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
   DQ_TRY(reset_shared(P, shots, st));
   DQ_TRY(launch_traj(L, P, st));
   DQ_CUDA_TRY(cudaEventRecord(b.e1, st));
-  unsigned long long ctr[kCtrWords];
-  DQ_CUDA_TRY(cudaMemcpyAsync(ctr, b.ctr, sizeof(ctr), cudaMemcpyDeviceToHost, st));
+  // into the pinned image, whose copy has been consumed by then
+  const unsigned long long* ctr = static_cast<const unsigned long long*>(b.stage);
+  DQ_CUDA_TRY(cudaMemcpyAsync(b.stage, d_ctr, sizeof(init), cudaMemcpyDeviceToHost, st));
   DQ_CUDA_TRY(cudaStreamSynchronize(st));
   float ms = 0.f;
   DQ_CUDA_TRY(cudaEventElapsedTime(&ms, b.e0, b.e1));
@@ -1500,11 +1521,11 @@ int dq_run_trajectories(int device, uint32_t n, const dq_inst* prog, uint64_t ni
 
   DeviceGuard g(device);
   cudaStream_t st = nullptr;
-  DQ_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  DQ_TRY(stream_take(device, &st));
   int32_t* d_out = nullptr;
   const size_t out_bytes = sizeof(int32_t) * (size_t)shots * ncbits;
   int rc = DQ_OK;
-  cudaError_t e = cudaMalloc((void**)&d_out, std::max<size_t>(out_bytes, 4));
+  cudaError_t e = pool_malloc_async((void**)&d_out, std::max<size_t>(out_bytes, 4), st);
   if (e != cudaSuccess) rc = fail(DQ_ERR_OOM, std::string("cudaMalloc(cbits): ") + cudaGetErrorString(e));
   if (rc == DQ_OK) rc = run_launch(ls, threads, device, st, d_out, &acc);
   if (rc == DQ_OK && out_bytes) {
@@ -1512,9 +1533,8 @@ int dq_run_trajectories(int device, uint32_t n, const dq_inst* prog, uint64_t ni
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = fail(DQ_ERR_CUDA, std::string("copy cbits: ") + cudaGetErrorString(e));
   }
-  cudaStreamSynchronize(st);
-  if (d_out) cudaFree(d_out);
-  cudaStreamDestroy(st);
+  if (d_out) cudaFreeAsync(d_out, st);
+  stream_give(device, st);
   if (acc.failed_inst >= 0) acc.failed_inst &= (1LL << 40) - 1;
   if (stats) *stats = acc;
   DQ_TRY(rc);
@@ -1712,7 +1732,7 @@ int dq_run_batch(int device, const dq_batch_item* items, uint64_t nitems,
   mark("group+encode");
 
   cudaStream_t st = nullptr;
-  DQ_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  DQ_TRY(stream_take(device, &st));
   int rc = DQ_OK;
   double2* d_hbm = nullptr;
   if (hbm_amps) {
@@ -1726,8 +1746,9 @@ int dq_run_batch(int device, const dq_batch_item* items, uint64_t nitems,
     if (outs[c].empty()) continue;
     double2* d_states = nullptr;
     int32_t* d_cbits = nullptr;
-    cudaError_t e = cudaMalloc((void**)&d_states, sizeof(double2) * std::max<uint64_t>(state_amps[c], 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_cbits, sizeof(int32_t) * std::max<uint64_t>(cbit_words[c], 1));
+    cudaError_t e = pool_malloc_async((void**)&d_states, sizeof(double2) * std::max<uint64_t>(state_amps[c], 1), st);
+    if (e == cudaSuccess)
+      e = pool_malloc_async((void**)&d_cbits, sizeof(int32_t) * std::max<uint64_t>(cbit_words[c], 1), st);
     if (e != cudaSuccess) rc = fail(DQ_ERR_OOM, std::string("cudaMalloc(batch outputs): ") + cudaGetErrorString(e));
     const auto tp = std::chrono::steady_clock::now();
     LaunchSet& ls = sets[c];
@@ -1776,9 +1797,9 @@ int dq_run_batch(int device, const dq_batch_item* items, uint64_t nitems,
                             cudaMemcpyDeviceToHost, st);
       if (e != cudaSuccess) rc = fail(DQ_ERR_CUDA, std::string("copy batch outputs: ") + cudaGetErrorString(e));
     }
+    if (d_states) cudaFreeAsync(d_states, st);
+    if (d_cbits) cudaFreeAsync(d_cbits, st);
     cudaStreamSynchronize(st);
-    if (d_states) cudaFree(d_states);
-    if (d_cbits) cudaFree(d_cbits);
     mark("outputs");
     if (rc == DQ_OK && acc.failed_inst >= 0) {
       // map (program << 40 | instruction) back to the caller's item index
@@ -1821,7 +1842,7 @@ int dq_run_batch(int device, const dq_batch_item* items, uint64_t nitems,
     acc.engine_items += 1;
   }
   if (h) dq_state_destroy(h);
-  cudaStreamDestroy(st);
+  stream_give(device, st);
   mark("engine items");
   if (stats) *stats = acc;
   return rc;
@@ -1902,7 +1923,7 @@ int dq_traj_plan_create(int device, uint32_t n, const dq_inst* prog, uint64_t ni
   P.nitems = ls.items.size();
   if (ls.items.size() == 1 &&
       (rc = set_shared(p->buf, P, device, n, shots, (uint32_t)ncbits,
-                       draws_of(ls.enc.ops.data(), ls.enc.ops.size()), st)) != DQ_OK)
+                       draws_of(ls.enc.ops.data(), ls.enc.ops.size()), nullptr)) != DQ_OK)
     return bail(rc);
   if ((rc = config_traj(threads, C, traj_smem(ls), P.tasks ? shots : P.nitems, &p->L)) != DQ_OK) return bail(rc);
   cu(cudaStreamSynchronize(st), "cudaStreamSynchronize");
