@@ -433,3 +433,29 @@ def format_cbits(bits: np.ndarray, num_cbits: int) -> str:
     if num_cbits == 0:
         return ""
     return "".join("1" if bits[i] > 0 else "0" for i in range(num_cbits - 1, -1, -1))
+
+
+def bit_strings(bits: np.ndarray) -> list[str]:
+    """Each row of a 0/1 matrix (at least one column) as a string of its digits."""
+    chars = bits.astype(np.uint32) + ord("0")
+    return chars.view(f"<U{bits.shape[1]}").reshape(-1).tolist()
+
+
+def count_cbits(rows: np.ndarray, num_cbits: int) -> dict[str, int]:
+    """How often each classical register (``format_cbits`` of a row) occurs, in the
+    order of first occurrence."""
+    if rows.shape[0] == 0:
+        return {}
+    if num_cbits == 0:
+        return {"": rows.shape[0]}
+    bits = rows[:, num_cbits - 1::-1] > 0 if num_cbits < rows.shape[1] else rows[:, ::-1] > 0
+    packed = np.packbits(bits, axis=1)
+    if packed.shape[1] <= 8:  # one big-endian integer per row
+        wide = np.zeros((packed.shape[0], 8), dtype=np.uint8)
+        wide[:, : packed.shape[1]] = packed
+        key = wide.view(">u8").reshape(-1).astype(np.uint64)
+    else:
+        key = np.ascontiguousarray(packed).view(f"V{packed.shape[1]}").reshape(-1)
+    _, first, count = np.unique(key, return_index=True, return_counts=True)
+    order = np.argsort(first)
+    return dict(zip(bit_strings(bits[first[order]]), count[order].tolist()))

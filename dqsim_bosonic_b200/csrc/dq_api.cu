@@ -13,9 +13,12 @@
 
 #include <algorithm>
 #include <chrono>
+#include <condition_variable>
 #include <map>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -204,6 +207,120 @@ void pinned_free(size_t bytes, void* p) {
   } else {
     cudaFreeHost(p);
   }
+}
+
+// Pageable host memory takes a copy of its own either way; here it comes out of
+// pinned memory on several host threads (which also take the page faults of a
+// fresh array) while the next chunks cross PCIe.  64 MiB into a fresh array:
+// 13.7 ms as one pageable cudaMemcpy, 3.6 ms here.
+int copy_to_host(const void* src, size_t bytes, const std::vector<HostPiece>& pieces, cudaStream_t st) {
+  constexpr size_t kChunk = 1 << 20;
+  // The driver's own staging copies one small range as fast (4 MiB into memory
+  // already touched: 246 us, 607 us with threads; 16 MiB: 852 and 693 us).
+  if (bytes && bytes < (16u << 20) && pieces.size() == 1 && pieces[0].dst) {
+    DQ_CUDA_TRY(cudaMemcpyAsync(pieces[0].dst, src, bytes, cudaMemcpyDeviceToHost, st));
+    DQ_CUDA_TRY(cudaStreamSynchronize(st));
+    return DQ_OK;
+  }
+  const uint8_t* from = static_cast<const uint8_t*>(src);
+  // calls f(piece, x, y) for the pieces with a destination that overlap bytes [a, b)
+  auto overlaps = [&](size_t a, size_t b, auto f) {
+    auto it = std::upper_bound(pieces.begin(), pieces.end(), a,
+                               [](size_t v, const HostPiece& p) { return v < p.off; });
+    for (size_t i = (size_t)(it - pieces.begin()) - 1; i < pieces.size() && pieces[i].off < b; ++i) {
+      const size_t end = i + 1 < pieces.size() ? pieces[i + 1].off : bytes;
+      const size_t x = std::max(a, pieces[i].off), y = std::min(b, end);
+      if (pieces[i].dst && y > x) f(pieces[i], x, y);
+    }
+  };
+  std::vector<size_t> chunks;  // byte offsets of the chunks somebody wants
+  if (!pieces.empty())
+    for (size_t a = 0; a < bytes; a += kChunk) {
+      bool want = false;
+      overlaps(a, std::min(bytes, a + kChunk), [&](const HostPiece&, size_t, size_t) { want = true; });
+      if (want) chunks.push_back(a);
+    }
+  if (chunks.empty()) return DQ_OK;
+  const size_t n = chunks.size(), slots = std::min<size_t>(n, 32);
+  const size_t stage_bytes = n == 1 ? std::min(bytes - chunks[0], kChunk) : slots * kChunk;
+  void* stage = nullptr;
+  DQ_TRY(pinned_alloc(stage_bytes, &stage));
+  auto slot = [&](size_t c) { return static_cast<uint8_t*>(stage) + (c % slots) * kChunk; };
+  auto issue = [&](size_t c) {
+    return cudaMemcpyAsync(slot(c), from + chunks[c], std::min(bytes - chunks[c], kChunk),
+                           cudaMemcpyDeviceToHost, st);
+  };
+  auto scatter = [&](size_t c) {
+    const size_t a = chunks[c];
+    overlaps(a, std::min(bytes, a + kChunk), [&](const HostPiece& p, size_t x, size_t y) {
+      memcpy(static_cast<uint8_t*>(p.dst) + (x - p.off), slot(c) + (x - a), y - x);
+    });
+  };
+  cudaError_t err = cudaSuccess;  // guarded by mu while threads run
+  std::mutex mu;
+  std::condition_variable cv;
+  size_t issued = 0, next = 0;
+  std::vector<char> busy(slots, 0);  // the slot holds a chunk not copied out yet
+  std::vector<cudaEvent_t> ev(slots, nullptr);
+  std::vector<std::thread> th;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  auto consume = [&] {
+    cudaSetDevice(dev);
+    std::unique_lock<std::mutex> lk(mu);
+    for (;;) {
+      cv.wait(lk, [&] { return next < issued || next == n || err != cudaSuccess; });
+      if (next == n || err != cudaSuccess) return;
+      const size_t c = next++;
+      lk.unlock();
+      const cudaError_t w = cudaEventSynchronize(ev[c % slots]);
+      if (w == cudaSuccess) scatter(c);
+      lk.lock();
+      if (w != cudaSuccess && err == cudaSuccess) err = w;
+      busy[c % slots] = 0;
+      cv.notify_all();
+    }
+  };
+  const size_t want = std::min<size_t>(std::min(8u, std::max(1u, std::thread::hardware_concurrency())), n);
+  if (want > 1) {
+    for (auto& x : ev)
+      if (err == cudaSuccess) err = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
+    try {
+      for (size_t t = 1; t < want && err == cudaSuccess; ++t) th.emplace_back(consume);
+    } catch (const std::system_error&) {  // the threads there are do the work
+    }
+  }
+  if (th.empty()) {
+    for (size_t c = 0; c < n && err == cudaSuccess; ++c) {
+      err = issue(c);
+      if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+      if (err == cudaSuccess) scatter(c);
+    }
+  } else {
+    std::unique_lock<std::mutex> lk(mu);
+    for (size_t c = 0; c < n && err == cudaSuccess; ++c) {
+      cv.wait(lk, [&] { return !busy[c % slots] || err != cudaSuccess; });
+      if (err != cudaSuccess) break;
+      busy[c % slots] = 1;
+      lk.unlock();
+      cudaError_t w = issue(c);
+      if (w == cudaSuccess) w = cudaEventRecord(ev[c % slots], st);
+      lk.lock();
+      if (w != cudaSuccess) err = w;
+      else issued = c + 1;
+      cv.notify_one();
+    }
+    lk.unlock();
+    cv.notify_all();
+    consume();
+    for (auto& x : th) x.join();
+  }
+  for (auto& x : ev)
+    if (x) cudaEventDestroy(x);
+  cudaStreamSynchronize(st);  // nothing may still write the staging buffer
+  pinned_free(stage_bytes, stage);
+  if (err != cudaSuccess) return fail(DQ_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(err));
+  return DQ_OK;
 }
 
 }  // namespace dq
@@ -711,8 +828,7 @@ int dq_state_download(dq_state_t h, double* amps, uint64_t len) {
   if (!amps || len != h->len) return fail(DQ_ERR_INVALID_ARG, "download length must be 2^n amplitudes");
   DeviceGuard g(h->device);
   DQ_TRY(canonicalize(h));
-  DQ_CUDA_TRY(cudaMemcpyAsync(amps, h->amp, h->bytes, cudaMemcpyDeviceToHost, h->stream));
-  return sync_stream(h);
+  return copy_to_host(h->amp, h->bytes, {HostPiece{0, amps}}, h->stream);
 }
 
 int dq_state_copy(dq_state_t dst, dq_state_t src) {

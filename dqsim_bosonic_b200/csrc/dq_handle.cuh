@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "dq_common.cuh"
 #include "dq_engine.cuh"
 #include "dq_fused.cuh"
@@ -68,6 +70,15 @@ void stream_give(int device, cudaStream_t st);
 // Pinned host staging buffers (at least `bytes`), recycled by size class.
 int pinned_alloc(size_t bytes, void** out);
 void pinned_free(size_t bytes, void* p);
+
+// One device range copied to host memory: piece i covers the bytes from
+// pieces[i].off to the next piece's off (the last one to `bytes`), ascending
+// from 0; a null dst is skipped.  Enqueued after the work on st; complete on return.
+struct HostPiece {
+  size_t off;
+  void* dst;
+};
+int copy_to_host(const void* src, size_t bytes, const std::vector<HostPiece>& pieces, cudaStream_t st);
 
 int check_handle(dq_state_t h);            // validates and materialises a lazy basis state
 int check_handle_lazy(dq_state_t h);       // validates only

@@ -1773,30 +1773,25 @@ int dq_run_batch(int device, const dq_batch_item* items, uint64_t nitems,
     if (rc == DQ_OK) rc = run_launch(ls, threads, device, st, d_cbits, &acc);
     if (timing) fprintf(stderr, "[dq_run_batch] kernel         %8.3f ms\n", acc.kernel_ms - k0);
     mark("launch set");
+    std::vector<HostPiece> sp, cp, hp;
     for (const Out& o : outs[c]) {
       if (rc != DQ_OK) break;
       const dq_batch_item& it = items[o.item];
-      e = cudaSuccess;
-      if (plan_of[o.item] >= 0) {
-        // HBM item: undo its sweeps' qubit relabeling, then copy the state out
+      if (o.state_off != ~0ULL) sp.push_back(HostPiece{sizeof(double2) * o.state_off, it.state_out});
+      cp.push_back(HostPiece{sizeof(int32_t) * o.cbits_off, it.ncbits ? it.cbits_out : nullptr});
+      if (plan_of[o.item] >= 0 && it.state_out) {  // HBM item: undo its sweeps' qubit relabeling
         const uint64_t h = (uint64_t)plan_of[o.item];
-        if (it.state_out) {
-          uint64_t extra = 0;
-          rc = materialize_perm(d_hbm + hbm_off[h], it.n, plans[h].perm, st, &extra);
-          acc.launches += (uint32_t)extra;
-          if (rc != DQ_OK) break;
-          e = cudaMemcpyAsync(it.state_out, d_hbm + hbm_off[h], sizeof(double2) << it.n,
-                              cudaMemcpyDeviceToHost, st);
-        }
-      } else if (it.state_out) {
-        e = cudaMemcpyAsync(it.state_out, d_states + o.state_off, sizeof(double2) << it.n,
-                            cudaMemcpyDeviceToHost, st);
+        uint64_t extra = 0;
+        rc = materialize_perm(d_hbm + hbm_off[h], it.n, plans[h].perm, st, &extra);
+        acc.launches += (uint32_t)extra;
       }
-      if (e == cudaSuccess && it.ncbits)
-        e = cudaMemcpyAsync(it.cbits_out, d_cbits + o.cbits_off, sizeof(int32_t) * it.ncbits,
-                            cudaMemcpyDeviceToHost, st);
-      if (e != cudaSuccess) rc = fail(DQ_ERR_CUDA, std::string("copy batch outputs: ") + cudaGetErrorString(e));
     }
+    if (c == 0)
+      for (uint64_t h = 0; h < hbm_items.size(); ++h)
+        hp.push_back(HostPiece{sizeof(double2) * hbm_off[h], items[hbm_items[h]].state_out});
+    if (rc == DQ_OK) rc = copy_to_host(d_hbm, sizeof(double2) * hbm_amps, hp, st);
+    if (rc == DQ_OK) rc = copy_to_host(d_states, sizeof(double2) * state_amps[c], sp, st);
+    if (rc == DQ_OK) rc = copy_to_host(d_cbits, sizeof(int32_t) * cbit_words[c], cp, st);
     if (d_states) cudaFreeAsync(d_states, st);
     if (d_cbits) cudaFreeAsync(d_cbits, st);
     cudaStreamSynchronize(st);

@@ -17,7 +17,7 @@ from typing import Any
 import numpy as np
 
 from . import _native as nat
-from .circuit import Program, format_cbits
+from .circuit import Program, count_cbits
 
 _U64 = (1 << 64) - 1
 _MULTI = ("MPS simulator only supports one- and two-qubit unitary gates plus measurement, "
@@ -189,9 +189,7 @@ class MpsSimulator:
                 bits, st = run_mps_shots(prog, base_seed, shots, self.device, self._max_bond,
                                          self._threshold)
                 svd_calls, svd_time = int(st.svd_calls), float(st.kernel_ms) / 1e3
-            for row in bits:
-                k = format_cbits(row, prog.num_cbits)
-                counts[k] = counts.get(k, 0) + 1
+            counts = count_cbits(bits, prog.num_cbits)
         shots_total = time.perf_counter() - shots_t0
         if profile:
             write_shots_profile(

@@ -18,7 +18,7 @@ from pathlib import Path
 import numpy as np
 
 from . import _native as nat
-from .circuit import format_cbits
+from .circuit import count_cbits
 
 _U64 = (1 << 64) - 1
 
@@ -47,9 +47,7 @@ def run_shots(sim, circuit, shots: int, profile: bool) -> dict[str, int]:
 
         bits, shot_times, fusion_time = run_trajectories(prog, base_seed, shots, sim.device,
                                                          want_times=profile)
-        keys = [format_cbits(row, prog.num_cbits) for row in bits]
-        for k in keys:
-            counts[k] = counts.get(k, 0) + 1
+        counts = count_cbits(bits, prog.num_cbits)
     shots_total = time.perf_counter() - shots_t0
     if profile:
         write_shots_profile(

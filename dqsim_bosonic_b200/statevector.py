@@ -18,7 +18,7 @@ from typing import Any
 import numpy as np
 
 from . import _native as nat
-from .circuit import CircuitDecodeError, Program, circuit_json, decode_program, format_cbits
+from .circuit import CircuitDecodeError, Program, bit_strings, circuit_json, decode_program
 
 _U64 = (1 << 64) - 1
 
@@ -177,7 +177,10 @@ class SimulationResult:
         if idx.size == 0:
             return {}
         vals, cnt = np.unique(idx, return_counts=True)
-        return {format(int(v), f"0{k}b"): int(c) for v, c in zip(vals, cnt)}
+        if cnt.size <= 32:  # (also k = 0, whose only index is "0")
+            return {format(v, f"0{k}b"): c for v, c in zip(vals.tolist(), cnt.tolist())}
+        shift = np.arange(k - 1, -1, -1, dtype=vals.dtype)
+        return dict(zip(bit_strings((vals[:, None] >> shift) & 1), cnt.tolist()))
 
     def fidelity(self, other) -> float:
         """|<self|other>|^2; 0.0 when the lengths differ (simulator.rs:184-191)."""

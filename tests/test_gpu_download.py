@@ -1,0 +1,35 @@
+"""Copies of device results into host arrays (staged through pinned memory)."""
+import numpy as np
+import pytest
+
+from _circuits import brickwork_u3_cx
+from dqsim_bosonic_b200 import _native as nat
+from dqsim_bosonic_b200.batch import run_batch
+from dqsim_bosonic_b200.circuit import decode_circuit_json, encode
+
+pytestmark = pytest.mark.gpu
+
+
+# below one staging chunk (2^16 amplitudes), one, several, and more than the staging ring holds
+@pytest.mark.parametrize("n", [0, 1, 9, 16, 17, 20, 22])
+def test_download_returns_what_was_uploaded(gpu, n):
+    rng = np.random.default_rng(n)
+    v = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    st = nat.State(n, 0)
+    st.upload(v)
+    assert np.array_equal(st.download(), v)
+
+
+@pytest.mark.parametrize("want", [True, {0}, {1, 4}, {2, 3, 5}, set()])
+def test_batch_states_land_in_their_arrays(gpu, want):
+    # shared-memory and HBM items, with pieces that share and that cross staging chunks
+    progs = [encode(decode_circuit_json(brickwork_u3_cx(n, 3, k).model_dump_json()))
+             for k, n in enumerate((10, 18, 16, 12, 17, 19))]
+    _, all_states, _ = run_batch(progs, range(6), want_states=True)
+    _, states, _ = run_batch(progs, range(6), want_states=want)
+    for k, s in enumerate(states):
+        if want is True or k in want:
+            assert np.array_equal(s, all_states[k])
+            assert abs(np.vdot(s, s).real - 1.0) < 1e-12
+        else:
+            assert s is None

@@ -16,7 +16,7 @@ import pytest
 from _circuits import JsonCircuit, cond, g, gate
 from dqsim_bosonic_b200 import simulate_distributed, simulate_monolithic, simulate_monolithic_shots
 from dqsim_bosonic_b200 import _native as nat
-from dqsim_bosonic_b200.circuit import (CircuitDecodeError, decode_circuit_json, encode,
+from dqsim_bosonic_b200.circuit import (CircuitDecodeError, count_cbits, decode_circuit_json, encode,
                                         format_cbits)
 
 ROOT = Path(__file__).resolve().parents[1]
@@ -239,3 +239,19 @@ def test_mps_entry_points_reject_bad_arguments_without_a_gpu(engine_lib):
     rc = L.dq_mps_run_shots(0, 3, 0, 1e-12, nat.ptr(p.insts), p.ninst, None, 0, 1, 0, 4, None, 0, 0,
                             ctypes.byref(st))
     assert rc == nat.DQ_ERR_UNSUPPORTED and st.failed_inst == 1
+
+
+@pytest.mark.parametrize("num_cbits,space", [(0, 1), (1, 1), (1, 4), (5, 5), (8, 9), (63, 64), (64, 64), (65, 70),
+                                             (200, 200)])
+@pytest.mark.parametrize("shots", [0, 1, 257])
+def test_count_cbits_is_format_cbits_counted(num_cbits, space, shots):
+    rng = np.random.default_rng(num_cbits + shots)
+    rows = rng.integers(-1, 2, size=(shots, space), dtype=np.int32)
+    rows[:, rng.random(space) < 0.9] = 0  # few distinct registers
+    want: dict[str, int] = {}
+    for row in rows:
+        k = format_cbits(row, num_cbits)
+        want[k] = want.get(k, 0) + 1
+    got = count_cbits(rows, num_cbits)
+    assert list(got.items()) == list(want.items())
+    assert all(type(k) is str and type(v) is int for k, v in got.items())
