@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(32 * kPermWarps)
 // =========================================================================
 
 inline hc conj(hc a) { return hc{a.re, -a.im}; }
+inline bool is_one_hc(hc a) { return a.re == 1.0 && a.im == 0.0; }
 inline bool is_unit_phase(hc a) { return fabs(a.re * a.re + a.im * a.im - 1.0) < 1e-12; }
 
 enum PKind { PG_DIAG, PG_U1, PG_U1X, PG_U2 };
@@ -200,38 +201,83 @@ struct PGate {
   uint64_t touched = 0;
 };
 
-struct Poly {
+// Extended-precision complex numbers of the rotation planner: the phases and
+// divided-out cosines of hundreds of gates multiply up on the host, and are
+// rounded to double once, in the tables the kernel reads.
+struct hx {
+  long double re, im;
+};
+inline hx operator*(hx a, hx b) { return hx{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
+inline hx conj(hx a) { return hx{a.re, -a.im}; }
+inline bool is_one_hc(hx a) { return a.re == 1.0L && a.im == 0.0L; }
+inline hc rounded(hx a) { return hc{(double)a.re, (double)a.im}; }
+
+template <class C>
+struct PolyT {
   uint32_t n = 0;
-  std::vector<hc> lin;
+  std::vector<C> lin;
   std::vector<char> hl;
-  std::vector<hc> quad;
+  std::vector<C> quad;
   std::vector<char> hq;
   std::vector<int> cnt;
-  hc cst{1, 0};
+  C cst{1, 0};
   bool has_cst = false;
 
   void init(uint32_t nq) {
     n = nq;
-    lin.assign(n, hc{1, 0});
+    lin.assign(n, C{1, 0});
     hl.assign(n, 0);
-    quad.assign((size_t)n * n, hc{1, 0});
+    quad.assign((size_t)n * n, C{1, 0});
     hq.assign((size_t)n * n, 0);
     cnt.assign(n, 0);
-    cst = hc{1, 0};
+    cst = C{1, 0};
     has_cst = false;
   }
-  void mul_lin(uint32_t q, hc w) {
+  void mul_lin(uint32_t q, C w) {
     if (!hl[q]) { hl[q] = 1; ++cnt[q]; lin[q] = w; } else lin[q] = lin[q] * w;
   }
-  void mul_quad(uint32_t a, uint32_t b, hc w) {
+  void mul_quad(uint32_t a, uint32_t b, C w) {
     const uint32_t lo = std::min(a, b), hi = std::max(a, b);
     const size_t k = (size_t)lo * n + hi;
     if (!hq[k]) { hq[k] = 1; ++cnt[lo]; ++cnt[hi]; quad[k] = w; } else quad[k] = quad[k] * w;
   }
   void add(const PGate& g) {
-    if (!(g.cst.re == 1.0 && g.cst.im == 0.0)) { cst = cst * g.cst; has_cst = true; }
-    for (int i = 0; i < g.nlin; ++i) mul_lin(g.lq[i], g.lw[i]);
-    if (g.quad) mul_quad(g.qa, g.qb, g.qw);
+    auto up = [](hc z) { return C{z.re, z.im}; };
+    if (!(g.cst.re == 1.0 && g.cst.im == 0.0)) { cst = cst * up(g.cst); has_cst = true; }
+    for (int i = 0; i < g.nlin; ++i) mul_lin(g.lq[i], up(g.lw[i]));
+    if (g.quad) mul_quad(g.qa, g.qb, up(g.qw));
+  }
+  bool has_quad(uint32_t a, uint32_t b) const {
+    return hq[(size_t)std::min(a, b) * n + std::max(a, b)] != 0;
+  }
+  // The terms after an X on t: x_t -> 1 - x_t.
+  void through_x(uint32_t t) {
+    if (hl[t]) {
+      cst = cst * lin[t];
+      has_cst = true;
+      lin[t] = conj(lin[t]);
+    }
+    for (uint32_t r = 0; r < n; ++r) {
+      if (r == t || !has_quad(t, r)) continue;
+      C& v = quad[(size_t)std::min(t, r) * n + std::max(t, r)];
+      mul_lin(r, v);
+      v = conj(v);
+    }
+  }
+  // The terms after a CX: x_t -> x_t + x_c - 2 x_t x_c.  Second degree only
+  // when no term pairs t with a third qubit (false: nothing done).
+  bool through_cx(uint32_t c, uint32_t t) {
+    const bool own = has_quad(c, t);
+    if (cnt[t] - (hl[t] ? 1 : 0) - (own ? 1 : 0) > 0) return false;
+    const C w = hl[t] ? lin[t] : C{1, 0};
+    const size_t k = (size_t)std::min(c, t) * n + std::max(c, t);
+    const C v = own ? quad[k] : C{1, 0};
+    if (!hl[t] && !own) return true;
+    mul_lin(c, w * v);
+    const C nq = conj(w) * conj(w) * conj(v);
+    if (own) quad[k] = nq;
+    else mul_quad(c, t, nq);
+    return true;
   }
   bool pending(uint32_t q) const { return cnt[q] > 0; }
   bool empty() const {
@@ -240,9 +286,9 @@ struct Poly {
     return true;
   }
   // remove and return all terms containing q
-  void take(uint32_t q, hc* wlin, std::vector<std::pair<uint32_t, hc>>& partners) {
-    *wlin = hl[q] ? lin[q] : hc{1, 0};
-    if (hl[q]) { hl[q] = 0; --cnt[q]; lin[q] = hc{1, 0}; }
+  void take(uint32_t q, C* wlin, std::vector<std::pair<uint32_t, C>>& partners) {
+    *wlin = hl[q] ? lin[q] : C{1, 0};
+    if (hl[q]) { hl[q] = 0; --cnt[q]; lin[q] = C{1, 0}; }
     partners.clear();
     for (uint32_t r = 0; r < n; ++r) {
       if (r == q) continue;
@@ -251,12 +297,14 @@ struct Poly {
       if (!hq[k]) continue;
       partners.push_back({r, quad[k]});
       hq[k] = 0;
-      quad[k] = hc{1, 0};
+      quad[k] = C{1, 0};
       --cnt[q];
       --cnt[r];
     }
   }
 };
+using Poly = PolyT<hc>;
+using PolyX = PolyT<hx>;
 
 struct POp {
   uint32_t type;
@@ -268,9 +316,29 @@ struct POp {
   std::vector<std::pair<uint64_t, hc>> gterms;     // GPHASE per-tile terms (masks)
 };
 
+// A rotation phase (dq_sweep.cuh) before it is encoded.
+struct MFactor {            // diag(1, w) on q, times pr.second for every set partner qubit
+  uint32_t q = ~0u;         // ~0: a factor of the whole tile (w and terms)
+  hx w{1, 0};
+  std::vector<std::pair<uint32_t, hx>> partners;
+  std::vector<std::pair<uint64_t, hx>> terms;
+};
+struct MPhase {
+  std::vector<uint32_t> regs;      // physical, RB of them; the rotated ones first
+  std::vector<double> t;           // rotations on regs[0..]
+  std::vector<std::pair<uint32_t, uint32_t>> flips;  // (control outside the tile, register qubit)
+  bool table = false;              // product of cst, lin and quad over the register qubits
+  hx cst{1, 0}, lin[4], quad[4][4];
+  std::vector<MFactor> cross;      // of register qubits
+  std::vector<MFactor> fin;        // final flush
+  uint32_t vec[kMaxM];             // address vector of every local bit, and the common offset
+  uint32_t off = 0;
+};
+
 struct PSweep {
   std::vector<uint32_t> local;  // physical, ascending, size m
   std::vector<POp> ops;
+  std::vector<MPhase> micro;    // rotation phases (then ops is empty)
 };
 
 // Blob writer (16-byte aligned sections)
@@ -300,6 +368,7 @@ struct Planner {
   // qubits every tile holds (0..4: 512-byte runs; 0..2: 128-byte runs)
   uint64_t pinned = 0x1FULL;
   bool pin_auto = false;
+  bool micro_ok = false;  // the launches of this geometry have the micro build
 
   // cost in FP64 instructions per amplitude
   double gate_cost(const PGate& g) const {
@@ -448,14 +517,409 @@ struct Planner {
   }
 };
 
+// ---- rotation phases: one-qubit gates as phases and real rotations ----------------------
+//
+// Host arithmetic is in extended precision, so rounding is the kernel's alone:
+// against an 80-bit simulation, 40 layers of 13-qubit brickwork are off by
+// 4.2-4.9e-15 (2-norm; 4.6-6.3e-15 with the gates applied as complex 2x2s).
+
+// The segment is made of one-qubit gates, X / CX and diagonal gates, with at
+// least one gate that is neither diagonal nor real: real and Hadamard-only
+// segments have straight-line builds of their own.
+bool micro_eligible(const std::vector<PGate>& G) {
+  bool general = false;
+  for (const PGate& g : G) {
+    if (g.kind == PG_U2 || (g.kind == PG_U1 && g.ctrl != 0)) return false;
+    if (g.kind == PG_U1X && __builtin_popcountll(g.ctrl) > 1) return false;
+    if (g.kind == PG_U1 && !g.real) general = true;
+  }
+  return general;
+}
+
+// u = cst diag(1, phi) [[c, -s], [s, c]] diag(1, lam) with real c, s >= 0 and
+// unit cst, phi, lam; false when u is not unitary to rounding.
+bool split_unitary(const hc* u, long double* c, long double* s, hx* cst, hx* phi, hx* lam) {
+  auto up = [](hc z) { return hx{z.re, z.im}; };
+  auto mod = [](hx z) { return sqrtl(z.re * z.re + z.im * z.im); };
+  auto unit = [&](hx z) {
+    const long double r = mod(z);
+    return r > 0.0L ? hx{z.re / r, z.im / r} : hx{1, 0};
+  };
+  *c = mod(up(u[0]));
+  *s = mod(up(u[2]));
+  if (!(*c > 0.0L || *s > 0.0L)) return false;
+  // the larger entries give the phases
+  if (*c >= *s) {
+    *cst = unit(up(u[0]));
+    const hx w = unit(up(u[3])) * conj(*cst);  // phi lam
+    *phi = *s > 0.0L ? unit(up(u[2])) * conj(*cst) : hx{1, 0};
+    *lam = w * conj(*phi);
+  } else {
+    const hx a = unit(up(u[2])), b = unit(hx{-u[1].re, -u[1].im});  // cst phi, cst lam
+    *cst = *c > 0.0L ? unit(up(u[0])) : hx{1, 0};
+    *phi = a * conj(*cst);
+    *lam = b * conj(*cst);
+  }
+  auto off = [&](hc z, hx w) { return mod(hx{z.re - w.re, z.im - w.im}); };
+  const hx ms{-*s, 0}, pc{*c, 0}, ps{*s, 0};
+  return fabsl(*c * *c + *s * *s - 1.0L) < 1e-14L && off(u[0], *cst * pc) < 4e-15L &&
+         off(u[1], *cst * *lam * ms) < 4e-15L && off(u[2], *cst * *phi * ps) < 4e-15L &&
+         off(u[3], *cst * *phi * *lam * pc) < 4e-15L;
+}
+
+struct MicroPlanner {
+  const Planner& pl;
+  // Against Planner::budget (96): a sweep takes up to 60 rotations.  28-qubit
+  // brickwork of 20 layers: 105 ms, 108 ms with up to 42, 110 ms with up to 29.
+  double rot_cost = 1.6;
+  uint32_t max_rot = 64;
+  // The segment with general gates split into phase, rotation (|t| <= 1) and
+  // phase: small records, since every sweep and phase scans them.
+  struct MGate {
+    uint64_t touched;
+    PKind kind;                          // PG_DIAG, PG_U1 (a rotation) or PG_U1X
+    uint32_t t0;
+    int ctrl;                            // PG_U1X: control qubit or -1
+    int src;                             // PG_DIAG: the segment's gate, or -1: cst diag(1, w) on t0
+    double t;                            // the rotation [[1, -t], [t, 1]] / sqrt(1 + t^2)
+    hx w, cst;
+  };
+  std::vector<MGate> G;
+  const std::vector<PGate>* in = nullptr;
+  bool ok = true;                        // every gate could be split
+
+  void split(const std::vector<PGate>& gates) {
+    in = &gates;
+    G.reserve(gates.size() * 4);
+    auto diag = [&](uint32_t q, hx w, hx cst) {
+      if (is_one_hc(w) && is_one_hc(cst)) return;
+      G.push_back(MGate{1ULL << q, PG_DIAG, q, -1, -1, 0.0, w, cst});
+    };
+    for (size_t i = 0; i < gates.size(); ++i) {
+      const PGate& g = gates[i];
+      if (g.kind != PG_U1) {
+        G.push_back(MGate{g.touched, g.kind, g.t0, g.ctrl ? __builtin_ctzll(g.ctrl) : -1, (int)i, 0.0, hx{1, 0},
+                          hx{1, 0}});
+        continue;
+      }
+      long double c, s;
+      hx cst, phi, lam;
+      if (!split_unitary(g.u, &c, &s, &cst, &phi, &lam)) {
+        ok = false;
+        return;
+      }
+      if (c < s) {
+        // [[c, -s], [s, c]] = [[s, c], [-c, s]] X Z: the quarter turn costs nothing
+        diag(g.t0, lam * hx{-1, 0}, hx{1, 0});
+        G.push_back(MGate{g.touched, PG_U1X, g.t0, -1, -1, 0.0, hx{1, 0}, hx{1, 0}});
+        const long double x = c;
+        c = s;
+        s = -x;
+      } else {
+        diag(g.t0, lam, hx{1, 0});
+      }
+      const double t = (double)(s / c);
+      if (t != 0.0) G.push_back(MGate{g.touched, PG_U1, g.t0, -1, -1, t, hx{1, 0}, hx{1, 0}});
+      diag(g.t0, phi, cst);
+    }
+  }
+  void add_diag(PolyX& poly, const MGate& g) const {
+    if (g.src >= 0) {
+      poly.add((*in)[g.src]);
+      return;
+    }
+    if (!is_one_hc(g.cst)) {
+      poly.cst = poly.cst * g.cst;
+      poly.has_cst = true;
+    }
+    if (!is_one_hc(g.w)) poly.mul_lin(g.t0, g.w);
+  }
+
+  // Every pending term among the phase's registers, and the constant, as one table.
+  void table(MPhase& ph, PolyX& poly) {
+    ph.cst = ph.cst * (poly.has_cst ? poly.cst : hx{1, 0});
+    ph.table = ph.table || !is_one_hc(ph.cst);
+    poly.cst = hx{1, 0};
+    poly.has_cst = false;
+    for (uint32_t a = 0; a < 4; ++a) {
+      const uint32_t x = ph.regs[a];
+      ph.lin[a] = hx{1, 0};
+      if (poly.hl[x]) {
+        ph.table = true;
+        ph.lin[a] = poly.lin[x];
+        poly.hl[x] = 0;
+        --poly.cnt[x];
+        poly.lin[x] = hx{1, 0};
+      }
+      for (uint32_t b = a + 1; b < 4; ++b) {
+        const uint32_t y = ph.regs[b];
+        ph.quad[a][b] = hx{1, 0};
+        if (!poly.has_quad(x, y)) continue;
+        const size_t k = (size_t)std::min(x, y) * poly.n + std::max(x, y);
+        ph.table = true;
+        ph.quad[a][b] = poly.quad[k];
+        poly.hq[k] = 0;
+        poly.quad[k] = hx{1, 0};
+        --poly.cnt[x];
+        --poly.cnt[y];
+      }
+    }
+  }
+  void take_factor(std::vector<MFactor>& to, PolyX& poly, uint32_t q) {
+    MFactor f;
+    f.q = q;
+    poly.take(q, &f.w, f.partners);
+    to.push_back(std::move(f));
+  }
+
+  struct Tile {            // addresses of the local qubits (of the tile being planned)
+    uint64_t S = 0, all = 0;  // local qubits; qubits its gates touch
+    int lidx[64];
+    uint32_t vec[kMaxM], off = 0;
+  };
+  void seal(MPhase& ph, const Tile& T) {
+    memcpy(ph.vec, T.vec, sizeof(ph.vec));
+    ph.off = T.off;
+  }
+  // Fills the phase's registers with the highest local qubits that are left,
+  // so that qubits 0..2 stay thread bits.
+  void fill(MPhase& ph, const std::vector<uint32_t>& local) {
+    for (size_t k = local.size(); k-- > 0 && ph.regs.size() < 4;)
+      if (std::find(ph.regs.begin(), ph.regs.end(), local[k]) == ph.regs.end()) ph.regs.push_back(local[k]);
+  }
+
+  // The phases of the gates `todo` (program order), whose targets are in the tile.
+  void phases(std::vector<int> todo, PSweep& sw, PolyX& poly) {
+    Tile T;
+    for (int& x : T.lidx) x = -1;
+    for (int gi : todo) T.all |= G[gi].touched;
+    for (uint32_t k = 0; k < sw.local.size(); ++k) {
+      T.S |= 1ULL << sw.local[k];
+      T.lidx[sw.local[k]] = (int)k;
+      T.vec[k] = swz(1u << k);
+    }
+    // Runs f(gate) over the gates in order; those it takes (true) are removed,
+    // a gate behind one that stays on a shared qubit is not offered.
+    auto scan = [&](auto f) {
+      uint64_t blocked = 0;
+      size_t stay = 0;
+      for (size_t i = 0; i < todo.size(); ++i) {
+        const MGate& g = G[todo[i]];
+        if (!(g.touched & blocked) && f(g)) continue;
+        todo[stay++] = todo[i];
+        blocked |= g.touched;
+        if (blocked == T.all) {  // nothing later can be offered
+          for (++i; i < todo.size(); ++i) todo[stay++] = todo[i];
+          break;
+        }
+      }
+      const bool any = stay != todo.size();
+      todo.resize(stay);
+      return any;
+    };
+    auto diagonal = [&](const MGate& g) {
+      if (g.kind != PG_DIAG) return false;
+      add_diag(poly, g);
+      return true;
+    };
+    while (!todo.empty()) {
+      // what executes nothing: diagonal gates, X, and CX inside the tile
+      uint64_t must = 0;  // targets whose pending terms a CX cannot pass
+      while (scan([&](const MGate& g) -> bool {
+        if (diagonal(g)) return true;
+        if (g.kind != PG_U1X) return false;
+        const uint32_t vt = T.vec[T.lidx[g.t0]];
+        if (g.ctrl < 0) {
+          poly.through_x(g.t0);
+          T.off ^= vt;
+          return true;
+        }
+        const uint32_t c = (uint32_t)g.ctrl;
+        if (T.lidx[c] < 0) return false;
+        if (!poly.through_cx(c, g.t0)) {
+          must |= 1ULL << g.t0;
+          return false;
+        }
+        T.vec[T.lidx[c]] ^= vt;
+        return true;
+      })) {
+      }
+      if (todo.empty()) break;
+      // targets that can go into a phase now, in program order
+      std::vector<uint32_t> cand;
+      uint64_t seen = 0, blocked = 0;
+      for (int gi : todo) {
+        const MGate& g = G[gi];
+        if (!(g.touched & blocked) && !((seen >> g.t0) & 1ULL)) {
+          cand.push_back(g.t0);
+          seen |= 1ULL << g.t0;
+        }
+        blocked |= g.touched;
+      }
+      // up to four of them, a target's quadratic partners with it; spare places
+      // to partners that are not targets now (their terms then need no factor
+      // of their own)
+      std::vector<uint32_t> pick;
+      auto has = [](const std::vector<uint32_t>& v, uint32_t q) { return std::find(v.begin(), v.end(), q) != v.end(); };
+      auto add_partners = [&](uint32_t q, bool targets) {
+        for (uint32_t r = 0; r < poly.n && pick.size() < 4; ++r)
+          if (r != q && poly.has_quad(q, r) && (T.S >> r & 1ULL) && !has(pick, r) && (!targets || (seen >> r & 1ULL)))
+            pick.push_back(r);
+      };
+      for (uint32_t q : cand) {
+        if (pick.size() >= 4) break;
+        if (has(pick, q)) continue;
+        pick.push_back(q);
+        add_partners(q, true);
+      }
+      for (size_t i = 0; i < pick.size(); ++i) add_partners(pick[i], false);
+      uint64_t R = 0;
+      for (uint32_t q : pick) R |= 1ULL << q;
+      MPhase ph;
+      // X controlled from outside the tile
+      scan([&](const MGate& g) {
+        if (g.kind != PG_U1X || g.ctrl < 0 || !(R >> g.t0 & 1ULL) || (must >> g.t0 & 1ULL)) return false;
+        const uint32_t c = (uint32_t)g.ctrl;
+        if (T.lidx[c] >= 0 || ph.flips.size() >= 4) return false;
+        if (!poly.through_cx(c, g.t0)) {
+          must |= 1ULL << g.t0;
+          return false;
+        }
+        ph.flips.push_back({c, g.t0});
+        return true;
+      });
+      while (scan(diagonal)) {
+      }
+      // rotations of the picked qubits (not of one whose terms a CX waits for)
+      std::vector<int> rots;
+      scan([&](const MGate& g) {
+        if (g.kind != PG_U1 || !(R >> g.t0 & 1ULL)) return false;
+        for (int x : rots)
+          if (G[x].t0 == g.t0) return false;
+        rots.push_back((int)(&g - G.data()));
+        return true;
+      });
+      for (int x : rots) ph.regs.push_back(G[x].t0);
+      for (uint32_t q : pick)
+        if (!has(ph.regs, q)) ph.regs.push_back(q);
+      fill(ph, sw.local);
+      table(ph, poly);
+      for (uint32_t q : ph.regs)
+        if (poly.pending(q) && (must >> q & 1ULL || std::any_of(rots.begin(), rots.end(), [&](int x) {
+              return G[x].t0 == q;
+            })))
+          take_factor(ph.cross, poly, q);
+      for (int x : rots) {
+        const double t = G[x].t;
+        ph.t.push_back(t);
+        poly.cst = poly.cst * hx{1.0L / sqrtl(1.0L + (long double)t * t), 0};  // of the rounded t
+        poly.has_cst = true;
+      }
+      seal(ph, T);
+      sw.micro.push_back(std::move(ph));
+    }
+    // the last phase writes the state by logical addresses: qubits 0..2 must be
+    // its thread bits, and no address change may follow it
+    const MPhase* last = sw.micro.empty() ? nullptr : &sw.micro.back();
+    bool direct = last && memcmp(last->vec, T.vec, sizeof(uint32_t) * sw.local.size()) == 0 && last->off == T.off;
+    if (direct)
+      for (uint32_t q : last->regs)
+        if (q < 3) direct = false;
+    if (!direct) {
+      MPhase ph;
+      fill(ph, sw.local);
+      for (auto& x : ph.lin) x = hx{1, 0};
+      for (auto& r : ph.quad)
+        for (auto& x : r) x = hx{1, 0};
+      seal(ph, T);
+      sw.micro.push_back(std::move(ph));
+    }
+  }
+
+  void plan(PolyX& poly, std::vector<PSweep>& out) {
+    std::vector<int> rem(G.size());
+    for (size_t i = 0; i < G.size(); ++i) rem[i] = (int)i;
+    const uint64_t low = pl.single_tile ? ((1ULL << pl.n) - 1) : pl.pinned;
+    while (!rem.empty()) {
+      // the gates of this sweep, as in Planner::plan
+      uint64_t S = low, blocked = 0;
+      double cost = 0.0;
+      uint32_t rots = 0;
+      bool any = false;
+      std::vector<int> incl, next;
+      for (int gi : rem) {
+        const MGate& g = G[gi];
+        bool take = !(g.touched & blocked);
+        if (take && g.kind != PG_DIAG) {
+          const uint64_t ns = S | (1ULL << g.t0);
+          const double c = g.kind == PG_U1X ? 0.0 : rot_cost;
+          take = (uint32_t)__builtin_popcountll(ns) <= pl.M && (g.kind == PG_U1X || rots < max_rot) &&
+                 (!any || cost + c <= pl.budget);
+          if (take) {
+            S = ns;
+            cost += c;
+            any = true;
+            rots += g.kind != PG_U1X;
+          }
+        }
+        if (take) {
+          incl.push_back(gi);
+        } else {
+          next.push_back(gi);
+          blocked |= g.touched;
+        }
+      }
+      for (uint32_t q = 0; q < pl.n && (uint32_t)__builtin_popcountll(S) < pl.M; ++q) S |= 1ULL << q;
+      PSweep sw;
+      for (uint32_t q = 0; q < pl.n; ++q)
+        if (S >> q & 1ULL) sw.local.push_back(q);
+      rem.swap(next);
+      if (!any) {
+        for (int gi : incl) add_diag(poly, G[gi]);
+        continue;
+      }
+      phases(std::move(incl), sw, poly);
+      out.push_back(std::move(sw));
+    }
+  }
+
+  // Every pending term, in a last phase of the last sweep.
+  void final_flush(PolyX& poly, std::vector<PSweep>& sweeps) {
+    if (poly.empty() && !poly.has_cst) return;
+    PSweep& last = sweeps.back();
+    MPhase ph;
+    fill(ph, last.local);
+    // after an address change (of an empty last phase, or none) the state's order
+    const MPhase& before = last.micro.back();
+    memcpy(ph.vec, before.vec, sizeof(ph.vec));
+    ph.off = before.off;
+    table(ph, poly);
+    for (uint32_t q : ph.regs)
+      if (poly.pending(q)) take_factor(ph.cross, poly, q);
+    for (uint32_t q : last.local)
+      if (poly.pending(q)) take_factor(ph.fin, poly, q);
+    MFactor tile;
+    for (uint32_t q = 0; q < poly.n; ++q) {
+      if (poly.hl[q]) tile.terms.push_back({1ULL << q, poly.lin[q]});
+      for (uint32_t r = q + 1; r < poly.n; ++r)
+        if (poly.has_quad(q, r)) tile.terms.push_back({(1ULL << q) | (1ULL << r), poly.quad[(size_t)q * poly.n + r]});
+    }
+    if (!tile.terms.empty()) ph.fin.push_back(std::move(tile));
+    poly.init(poly.n);
+    // an empty last phase is replaced
+    if (before.t.empty() && !before.table && before.cross.empty() && before.flips.empty()) last.micro.pop_back();
+    last.micro.push_back(std::move(ph));
+  }
+};
+
 // choose thread-bit order: lanes 0..2 need linearly independent swizzle vectors
-bool order_thread_bits(std::vector<uint32_t>& tb) {
+bool order_thread_bits(std::vector<uint32_t>& tb, const uint32_t* vec) {
   const size_t c = tb.size();
   for (size_t i = 0; i < c; ++i)
     for (size_t j = i + 1; j < c; ++j)
       for (size_t k = j + 1; k < c; ++k) {
-        const uint32_t a = swz_vec(tb[i]), b = swz_vec(tb[j]), d = swz_vec(tb[k]);
-        if (a == b || (a ^ b) == 0 || d == a || d == b || d == (a ^ b)) continue;
+        const uint32_t a = vec[tb[i]] & 7u, b = vec[tb[j]] & 7u, d = vec[tb[k]] & 7u;
+        if (a == 0 || b == 0 || a == b || d == 0 || d == a || d == b || d == (a ^ b)) continue;
         std::vector<uint32_t> o = {tb[i], tb[j], tb[k]};
         for (size_t x = 0; x < c; ++x)
           if (x != i && x != j && x != k) o.push_back(tb[x]);
@@ -465,9 +929,47 @@ bool order_thread_bits(std::vector<uint32_t>& tb) {
   return false;
 }
 
-// Encode a planned sweep into the device blob format.
+// Thread and register layout of a phase whose register bits are the local
+// bits `regs`: address tables, and the places of each local bit.  vec: the
+// address vector of every local bit, off: the address of element 0; keep_low:
+// local bits 0..2 are lanes 0..2 (a direct write of the state).
+struct PhaseLayout {
+  std::vector<uint32_t> tb;        // local bits of the thread bits
+  int rix[kMaxM], tix[kMaxM];      // register / thread bit of a local bit, or -1
+};
+int phase_layout(const std::vector<uint32_t>& regs, uint32_t m, uint32_t TBn, uint32_t RB, const uint32_t* vec,
+                 uint32_t off, bool keep_low, SwPhase& sp, PhaseLayout& pl) {
+  const int kSwTB = (int)TBn;
+  pl.tb.clear();
+  for (uint32_t b = 0; b < m; ++b)
+    if (std::find(regs.begin(), regs.end(), b) == regs.end()) pl.tb.push_back(b);
+  if (pl.tb.size() != (size_t)kSwTB || (!keep_low && !order_thread_bits(pl.tb, vec)))
+    return fail(DQ_ERR_INTERNAL, "no bank-conflict-free thread layout");
+  for (int i = 0; i < kMaxM; ++i) pl.rix[i] = pl.tix[i] = -1;
+  for (uint32_t b = 0; b < RB; ++b) {
+    sp.V[b] = vec[regs[b]];
+    pl.rix[regs[b]] = (int)b;
+  }
+  for (uint32_t b = RB; b < 4; ++b) sp.V[b] = 0;
+  for (int i = 0; i < kSwTB; ++i) pl.tix[pl.tb[i]] = i;
+  for (uint32_t ln = 0; ln < 32; ++ln) {
+    sp.lanesw[ln] = off;
+    for (int i = 0; i < 5; ++i)
+      if ((ln >> i) & 1u) sp.lanesw[ln] ^= vec[pl.tb[i]];
+  }
+  for (uint32_t wp = 0; wp < 8; ++wp) {
+    sp.warpsw[wp] = 0;
+    for (int i = 0; i + 5 < kSwTB; ++i)
+      if ((wp >> i) & 1u) sp.warpsw[wp] ^= vec[pl.tb[5 + i]];
+  }
+  return DQ_OK;
+}
+
+// Encode a planned sweep into the device blob format.  general_ops: rotation
+// phases are also written in the general op set (plan inspection; no kernel
+// needs them).
 int encode_sweep(const PSweep& sw_in, const std::vector<PGate>& G, uint32_t TBn, uint32_t RB,
-                 Blob& blob, size_t* offset) {
+                 Blob& blob, size_t* offset, bool general_ops) {
   const int kSwTB = (int)TBn;
   const uint32_t m = (uint32_t)sw_in.local.size();
   if (m != kSwTB + RB) return fail(DQ_ERR_INTERNAL, "sweep local set size mismatch");
@@ -570,6 +1072,153 @@ int encode_sweep(const PSweep& sw_in, const std::vector<PGate>& G, uint32_t TBn,
 
   uint32_t carry_xload = 0;
   std::vector<uint32_t> last_tb, last_regs;  // thread / register bits of the last phase
+  uint32_t plain_vec[kMaxM];
+  for (uint32_t k = 0; k < (uint32_t)kMaxM; ++k) plain_vec[k] = swz(1u << k);
+  std::vector<SwMPhase> MP;     // rotation phases
+  std::vector<SwFinal> FN;
+  std::vector<double2> DS;      // data of the general ops of such a sweep only (after D)
+  std::vector<char> in_ds;      // per op: data counts from the start of DS
+  for (const MPhase& ph : sw_in.micro) {
+    SwPhase sp{};
+    std::vector<uint32_t> regs;
+    for (uint32_t q : ph.regs) regs.push_back((uint32_t)lidx[q]);
+    PhaseLayout lay;
+    const bool last = &ph == &sw_in.micro.back();
+    DQ_TRY(phase_layout(regs, m, TBn, RB, ph.vec, ph.off, last, sp, lay));
+    SwMPhase mp{};
+    sp.op_begin = (uint32_t)O.size();
+    auto push = [&](const EncOp& e, bool ds) {
+      if (!general_ops) return;
+      O.push_back(e);
+      in_ds.push_back(ds ? 1 : 0);
+    };
+    // the 2x2 m on register bit b, in the general op set
+    auto push_u1 = [&](uint32_t type, uint32_t b, uint32_t creg, const hc* mm) {
+      EncOp e{};
+      e.type = type;
+      e.b0 = b;
+      e.creg = creg;
+      e.data = (uint32_t)DS.size();
+      if (general_ops)
+        for (int i = 0; i < 4; ++i) DS.push_back(d2(mm[i]));
+      push(e, true);
+    };
+    // slot, thread table and (for the final flush) register table of a factor
+    auto factors = [&](const MFactor& f, EncOp& so) {
+      std::vector<std::pair<uint64_t, hc>> nl;
+      for (const auto& x : f.terms) nl.push_back({x.first, rounded(x.second)});
+      hx wthr[kMaxTB], wreg[4];
+      for (auto& x : wthr) x = hx{1, 0};
+      for (auto& x : wreg) x = hx{1, 0};
+      bool thr = false;
+      for (const auto& pr : f.partners) {
+        const int l = lidx[pr.first];
+        if (l < 0) {
+          nl.push_back({1ULL << pr.first, rounded(pr.second)});
+        } else if (lay.rix[l] >= 0) {
+          wreg[lay.rix[l]] = wreg[lay.rix[l]] * pr.second;
+          so.flags |= FL_REG;
+        } else {
+          wthr[lay.tix[l]] = wthr[lay.tix[l]] * pr.second;
+          thr = true;
+        }
+      }
+      so.slot = add_slot(rounded(f.w), nl);
+      so.data = (uint32_t)D.size();
+      if (thr) {
+        so.flags |= FL_THR;
+        for (uint32_t ln = 0; ln < 32; ++ln) {
+          hx w{1, 0};
+          for (int i = 0; i < 5; ++i)
+            if ((ln >> i) & 1u) w = w * wthr[i];
+          D.push_back(d2(rounded(w)));
+        }
+        for (uint32_t wp = 0; wp < 8; ++wp) {
+          hx w{1, 0};
+          for (int i = 0; i + 5 < kSwTB; ++i)
+            if ((wp >> i) & 1u) w = w * wthr[5 + i];
+          D.push_back(d2(rounded(w)));
+        }
+      }
+      if (so.flags & FL_REG)
+        for (uint32_t j = 0; j < (1u << RB); ++j) {
+          hx w{1, 0};
+          for (uint32_t b = 0; b < RB; ++b)
+            if ((j >> b) & 1u) w = w * wreg[b];
+          D.push_back(d2(rounded(w)));
+        }
+    };
+    if (ph.flips.size() > 4 || ph.t.size() > 4) return fail(DQ_ERR_INTERNAL, "rotation phase too large");
+    for (const auto& f : ph.flips) {
+      mp.cmask[mp.ncond] = 1ULL << f.first;
+      mp.cxor[mp.ncond++] = ph.vec[lidx[f.second]];
+      EncOp e{};
+      e.type = OP_U1X;
+      e.b0 = (uint32_t)lay.rix[lidx[f.second]];
+      e.cnl = 1ULL << f.first;
+      e.data = (uint32_t)DS.size();
+      push(e, true);
+    }
+    mp.mul = ~0u;
+    if (ph.table) {
+      mp.mul = (uint32_t)D.size();
+      for (uint32_t j = 0; j < (1u << RB); ++j) {
+        hx f = ph.cst;
+        for (uint32_t x = 0; x < RB; ++x) {
+          if (!((j >> x) & 1u)) continue;
+          f = f * ph.lin[x];
+          for (uint32_t y = x + 1; y < RB; ++y)
+            if ((j >> y) & 1u) f = f * ph.quad[x][y];
+        }
+        D.push_back(d2(rounded(f)));
+      }
+      for (uint32_t x = 0; x < RB; ++x) {
+        const hx one = x == 0 ? ph.cst : hx{1, 0};
+        const hc lin[4] = {rounded(one), hc{0, 0}, hc{0, 0}, rounded(one * ph.lin[x])};
+        push_u1(OP_U1, x, 0, lin);
+        for (uint32_t y = x + 1; y < RB; ++y) {
+          const hc qd[4] = {hc{1, 0}, hc{0, 0}, hc{0, 0}, rounded(ph.quad[x][y])};
+          if (!is_one_hc(ph.quad[x][y])) push_u1(OP_U1, y, 1u << x, qd);
+        }
+      }
+    }
+    for (auto& x : mp.cross) x = ~0u;
+    for (const MFactor& f : ph.cross) {
+      EncOp so{};
+      so.type = OP_FLUSH_R;
+      so.b0 = (uint32_t)lay.rix[lidx[f.q]];
+      factors(f, so);
+      if (so.flags & FL_REG) return fail(DQ_ERR_INTERNAL, "register partner left to a cross factor");
+      push(so, false);
+      mp.cross[so.b0] = so.slot | (so.flags << 16);
+      mp.cdata[so.b0] = so.data;
+      ++mp.ncross;
+    }
+    mp.k = (uint32_t)ph.t.size();
+    for (uint32_t x = 0; x < mp.k; ++x) {
+      mp.t[x] = ph.t[x];
+      const hc r[4] = {hc{1, 0}, hc{-ph.t[x], 0}, hc{ph.t[x], 0}, hc{1, 0}};
+      push_u1(OP_U1R, x, 0, r);
+    }
+    if (!ph.fin.empty() && mp.k) return fail(DQ_ERR_INTERNAL, "final flush in a phase with rotations");
+    mp.fin0 = (uint32_t)FN.size();
+    for (const MFactor& f : ph.fin) {
+      EncOp so{};
+      const bool tile = f.q == ~0u;
+      so.type = tile ? OP_GPHASE : OP_FLUSH_T;
+      so.b0 = tile ? 0u : (uint32_t)lay.tix[lidx[f.q]];
+      factors(f, so);
+      push(so, false);
+      FN.push_back(SwFinal{so.slot, so.flags, tile ? ~0u : so.b0, so.data});
+    }
+    mp.nfin = (uint32_t)FN.size() - mp.fin0;
+    sp.op_end = (uint32_t)O.size();
+    last_tb = lay.tb;
+    last_regs = regs;
+    MP.push_back(mp);
+    P.push_back(sp);
+  }
+  if (!sw_in.micro.empty()) phases.clear();
   for (const PhaseTmp& ph : phases) {
     SwPhase sp{};
     // spare register slots take the highest unused local bits, so that the
@@ -578,28 +1227,11 @@ int encode_sweep(const PSweep& sw_in, const std::vector<PGate>& G, uint32_t TBn,
     std::vector<uint32_t> regs = ph.regs;
     for (uint32_t b = m; b-- > 0 && regs.size() < RB;)
       if (std::find(regs.begin(), regs.end(), b) == regs.end()) regs.push_back(b);
-    std::vector<uint32_t> tb;
-    for (uint32_t b = 0; b < m; ++b)
-      if (std::find(regs.begin(), regs.end(), b) == regs.end()) tb.push_back(b);
-    if (tb.size() != (size_t)kSwTB || !order_thread_bits(tb))
-      return fail(DQ_ERR_INTERNAL, "no bank-conflict-free thread layout");
-    int rix[kMaxM], tix[kMaxM];
-    for (int i = 0; i < kMaxM; ++i) rix[i] = tix[i] = -1;
-    for (uint32_t b = 0; b < RB; ++b) { sp.V[b] = swz(1u << regs[b]); rix[regs[b]] = (int)b; }
-    for (uint32_t b = RB; b < 4; ++b) sp.V[b] = 0;
-    for (int i = 0; i < kSwTB; ++i) tix[tb[i]] = i;
-    for (uint32_t ln = 0; ln < 32; ++ln) {
-      uint32_t e = 0;
-      for (int i = 0; i < 5; ++i)
-        if ((ln >> i) & 1u) e |= 1u << tb[i];
-      sp.lanesw[ln] = swz(e);
-    }
-    for (uint32_t wp = 0; wp < 8; ++wp) {
-      uint32_t e = 0;
-      for (int i = 0; i + 5 < kSwTB; ++i)
-        if ((wp >> i) & 1u) e |= 1u << tb[5 + i];
-      sp.warpsw[wp] = swz(e);
-    }
+    PhaseLayout lay;
+    DQ_TRY(phase_layout(regs, m, TBn, RB, plain_vec, 0, false, sp, lay));
+    const std::vector<uint32_t>& tb = lay.tb;
+    const int (&rix)[kMaxM] = lay.rix;
+    const int (&tix)[kMaxM] = lay.tix;
     sp.op_begin = (uint32_t)O.size();
     // flush of a register target: per-tile slot, thread/register factor tables
     auto encode_flush = [&](const POp& op, EncOp& so) {
@@ -834,7 +1466,8 @@ int encode_sweep(const PSweep& sw_in, const std::vector<PGate>& G, uint32_t TBn,
   for (const EncOp& so : O)
     if (((so.type <= OP_U2 || so.type == OP_U1H || so.type == OP_FLUSH_R) && so.b0 >= RB) ||
         (so.type == OP_FLUSH_T && so.b0 >= (uint32_t)kSwTB) || (so.type == OP_U2 && so.b1 >= RB) ||
-        so.slot >= SL.size() + (SL.empty() ? 1 : 0) || so.data > D.size() || so.slot > 0xffffu ||
+        so.slot >= SL.size() + (SL.empty() ? 1 : 0) || so.data > std::max(D.size(), DS.size()) ||
+        so.slot > 0xffffu ||
         so.creg > 0xffu || so.ctl_thr > 0xffu || so.flags > 0xffu)
       return fail(DQ_ERR_INTERNAL, "op encoding out of range");
   std::vector<SwOp> OP(O.size());
@@ -842,7 +1475,7 @@ int encode_sweep(const PSweep& sw_in, const std::vector<PGate>& G, uint32_t TBn,
     const EncOp& e = O[i];
     OP[i].w0 = e.type | (e.b0 << 8) | (e.b1 << 16) | (e.creg << 24);
     OP[i].w1 = e.ctl_thr | (e.flags << 8) | (e.slot << 16);
-    OP[i].data = e.data;
+    OP[i].data = e.data + (i < in_ds.size() && in_ds[i] ? (uint32_t)D.size() : 0u);
     OP[i].cnl = e.cnl;
   }
   SwHeader h{};
@@ -882,16 +1515,14 @@ int encode_sweep(const PSweep& sw_in, const std::vector<PGate>& G, uint32_t TBn,
     bool uonly = !P.empty() && !marked;
     for (const EncOp& e : O)
       if (!(e.type == OP_U1 || e.type == OP_U1R || e.type == OP_U1X) || (e.flags & FL_PRE)) uonly = false;
-    if (uonly) h.flags |= SWF_UONLY;
+    if (uonly || !MP.empty()) h.flags = SWF_UONLY;
   }
   h.tile_xload = tile_xload;
   for (uint32_t k = 0; k < m; ++k) h.local_pos[k] = sw.local[k];
   const size_t hoff = blob.put(&h, 1);
   const size_t po = blob.put(P.data(), P.size());
-  const size_t oo = OP.empty() ? blob.align16() : blob.put(OP.data(), OP.size());
   const size_t so = SL.empty() ? blob.align16() : blob.put(SL.data(), SL.size());
   const size_t eo = SE.empty() ? blob.align16() : blob.put(SE.data(), SE.size());
-  const size_t dd = D.empty() ? blob.align16() : blob.put(D.data(), D.size());
   const size_t ro = blob.put(runoff.data(), runoff.size());
   const size_t rs = blob.put(runswz.data(), runswz.size());
   // The last phase writes straight to the state when its lanes 0..2 are local
@@ -909,7 +1540,20 @@ int encode_sweep(const PSweep& sw_in, const std::vector<PGate>& G, uint32_t TBn,
     for (uint32_t b = 0; b < RB && b < 4; ++b) g.gV[b] = 1ULL << sw.local[last_regs[b]];
     go = blob.put(&g, 1);
   }
+  if (!MP.empty() && !go) return fail(DQ_ERR_INTERNAL, "the last rotation phase cannot write the state");
+  // what the kernel of rotation phases does not need comes last: the general
+  // ops and their data (DS continues D)
+  const size_t mo = MP.empty() ? 0 : blob.put(MP.data(), MP.size());
+  const size_t fo = FN.empty() ? blob.align16() : blob.put(FN.data(), FN.size());
+  size_t oo = blob.align16();
+  if (MP.empty() && !OP.empty()) oo = blob.put(OP.data(), OP.size());
+  const size_t dd = D.empty() ? blob.align16() : blob.put(D.data(), D.size());
+  const size_t stage = blob.align16() - hoff;
+  if (!DS.empty()) blob.put(DS.data(), DS.size());
+  if (!MP.empty() && !OP.empty()) oo = blob.put(OP.data(), OP.size());
   SwHeader* hp = reinterpret_cast<SwHeader*>(blob.buf.data() + hoff);
+  hp->off_micro = mo ? (uint32_t)(mo - hoff) : 0u;
+  hp->off_final = (uint32_t)(fo - hoff);
   hp->off_runoff = (uint32_t)(ro - hoff);
   hp->off_runswz = (uint32_t)(rs - hoff);
   hp->off_gstore = go ? (uint32_t)(go - hoff) : 0u;
@@ -921,7 +1565,8 @@ int encode_sweep(const PSweep& sw_in, const std::vector<PGate>& G, uint32_t TBn,
   blob.align16();
   hp = reinterpret_cast<SwHeader*>(blob.buf.data() + hoff);
   hp->prog_bytes = (uint32_t)(blob.buf.size() - hoff);
-  if (hp->prog_bytes > (uint32_t)max_prog((int)m)) return fail(DQ_ERR_INTERNAL, "sweep program too large");
+  hp->stage_bytes = mo ? (uint32_t)stage : hp->prog_bytes;
+  if (hp->stage_bytes > (uint32_t)max_prog((int)m)) return fail(DQ_ERR_INTERNAL, "sweep program too large");
   *offset = hoff;
   return DQ_OK;
 }
@@ -1104,18 +1749,26 @@ int launch_sweep_r(double2* amp, uint32_t n, const uint8_t* dblob, uint32_t prog
   return DQ_OK;
 }
 
-template <int TB, int RB>
-int launch_sweep_rb(double2* amp, uint32_t n, const uint8_t* dblob, uint32_t prog_bytes,
-                    cudaStream_t st, long long synth, uint32_t run_bits, uint32_t flags) {
-  // default: single-buffered tiles, three 128-thread CTAs per SM (measured
-  // faster than two double-buffered CTAs: the extra warps hide more of the
-  // per-op latency than the prefetch saves); DQSIM_SWEEP_STAGES=2 selects
-  // double buffering
+// DQSIM_SWEEP_STAGES=2: double-buffered tiles
+int sweep_stages() {
   static const int stages = [] {
     const char* e = getenv("DQSIM_SWEEP_STAGES");
     return e ? atoi(e) : 1;
   }();
-  if (TB == 7 && stages != 2) {
+  return stages;
+}
+
+template <int TB, int RB>
+int launch_sweep_rb(double2* amp, uint32_t n, const uint8_t* dblob, uint32_t prog_bytes,
+                    cudaStream_t st, long long synth, uint32_t run_bits, uint32_t flags, bool micro) {
+  // default: single-buffered tiles, three 128-thread CTAs per SM (measured
+  // faster than two double-buffered CTAs: the extra warps hide more of the
+  // per-op latency than the prefetch saves); DQSIM_SWEEP_STAGES=2 selects
+  // double buffering
+  if (TB == 7 && sweep_stages() != 2) {
+    if (RB == 4 && micro)
+      return run_bits == 3 ? launch_sweep_r<7, 4, 1, 3, FORM_M>(amp, n, dblob, prog_bytes, st, synth)
+                           : launch_sweep_r<7, 4, 1, 5, FORM_M>(amp, n, dblob, prog_bytes, st, synth);
     if (RB == 4 && (flags & SWF_HONLY))
       return run_bits == 3 ? launch_sweep_r<7, 4, 1, 3, FORM_H>(amp, n, dblob, prog_bytes, st, synth)
                            : launch_sweep_r<7, 4, 1, 5, FORM_H>(amp, n, dblob, prog_bytes, st, synth);
@@ -1134,19 +1787,19 @@ int launch_sweep_rb(double2* amp, uint32_t n, const uint8_t* dblob, uint32_t pro
 
 int launch_sweep(double2* amp, uint32_t n, uint32_t TB, uint32_t RB, const uint8_t* dblob,
                  uint32_t prog_bytes, cudaStream_t st, long long synth, uint32_t run_bits,
-                 uint32_t flags) {
+                 uint32_t flags, bool micro) {
   if (TB == 8) {
     switch (RB) {
-      case 2: return launch_sweep_rb<8, 2>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags);
-      case 3: return launch_sweep_rb<8, 3>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags);
-      case 4: return launch_sweep_rb<8, 4>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags);
+      case 2: return launch_sweep_rb<8, 2>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags, micro);
+      case 3: return launch_sweep_rb<8, 3>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags, micro);
+      case 4: return launch_sweep_rb<8, 4>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags, micro);
       default: break;
     }
   } else if (TB == 7) {
     switch (RB) {
-      case 2: return launch_sweep_rb<7, 2>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags);
-      case 3: return launch_sweep_rb<7, 3>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags);
-      case 4: return launch_sweep_rb<7, 4>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags);
+      case 2: return launch_sweep_rb<7, 2>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags, micro);
+      case 3: return launch_sweep_rb<7, 3>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags, micro);
+      case 4: return launch_sweep_rb<7, 4>(amp, n, dblob, prog_bytes, st, synth, run_bits, flags, micro);
       default: break;
     }
   }
@@ -1329,31 +1982,71 @@ int fused_run_segment(double2* amp, uint32_t n, std::vector<PGate>& G, Planner& 
                       FusedWork& fw, cudaStream_t st, bool timing, dq_profile* prof,
                       int64_t* lazy_basis) {
   std::vector<PSweep> sweeps;
-  if (pl.pin_auto && !pl.single_tile) {
-    // plan with qubits 0..4 pinned and with 0..2 pinned; the wider tile
-    // choice wins only when it saves at least a tenth of the sweeps (its
-    // 128-byte runs cost a little more per sweep)
-    Poly poly3 = poly;
-    std::vector<PSweep> sweeps3;
-    pl.pinned = 0x1FULL;
-    pl.plan(G, poly, sweeps);
-    pl.final_flush(poly, sweeps);
-    pl.pinned = 0x7ULL;
-    pl.plan(G, poly3, sweeps3);
-    pl.final_flush(poly3, sweeps3);
-    if (10 * sweeps3.size() <= 9 * sweeps.size()) {
-      sweeps.swap(sweeps3);
-      poly = poly3;
-    }
-  } else {
-    pl.plan(G, poly, sweeps);
-    pl.final_flush(poly, sweeps);
-  }
-  if (sweeps.empty()) return DQ_OK;
   Blob blob;
-  std::vector<size_t> offs(sweeps.size());
-  for (size_t i = 0; i < sweeps.size(); ++i)
-    DQ_TRY(encode_sweep(sweeps[i], G, pl.TB, pl.RB, blob, &offs[i]));
+  std::vector<size_t> offs;
+  auto encode = [&]() -> int {
+    blob.buf.clear();
+    offs.assign(sweeps.size(), 0);
+    for (size_t i = 0; i < sweeps.size(); ++i)
+      DQ_TRY(encode_sweep(sweeps[i], G, pl.TB, pl.RB, blob, &offs[i], fw.plan_out && !fw.plan_tb));
+    return DQ_OK;
+  };
+  // one pass of the planner with the given low qubits pinned
+  const bool micro = pl.micro_ok && poly.empty() && !poly.has_cst && micro_eligible(G);
+  uint32_t max_rot = 64;
+  auto plan_with = [&](uint64_t pinned, Poly& p, std::vector<PSweep>& out) {
+    pl.pinned = pinned;
+    out.clear();
+    if (micro) {
+      MicroPlanner mp{pl};
+      mp.max_rot = max_rot;
+      mp.split(G);
+      PolyX px;  // a segment starts without pending terms
+      px.init(pl.n);
+      if (mp.ok) {
+        mp.plan(px, out);
+        if (!out.empty()) {
+          mp.final_flush(px, out);
+          return;
+        }
+      }
+      pl.plan(G, p, out);
+    } else {
+      pl.plan(G, p, out);
+    }
+    pl.final_flush(p, out);
+  };
+  const Poly poly0 = poly;
+  const uint64_t pin0 = pl.pinned;
+  for (;;) {
+    if (micro) {
+      // rotation phases are cheap enough that the two more tile qubits of
+      // 128-byte runs always save sweeps (28-qubit brickwork: 30 against 45)
+      plan_with(pl.pin_auto ? 0x7ULL : pin0, poly, sweeps);
+    } else if (pl.pin_auto && !pl.single_tile) {
+      // plan with qubits 0..4 pinned and with 0..2 pinned; the wider tile
+      // choice wins only when it saves at least a tenth of the sweeps (its
+      // 128-byte runs cost a little more per sweep)
+      Poly poly3 = poly;
+      std::vector<PSweep> sweeps3;
+      plan_with(0x1FULL, poly, sweeps);
+      plan_with(0x7ULL, poly3, sweeps3);
+      if (10 * sweeps3.size() <= 9 * sweeps.size()) {
+        sweeps.swap(sweeps3);
+        poly = poly3;
+      }
+    } else {
+      plan_with(pin0, poly, sweeps);
+    }
+    if (sweeps.empty()) return DQ_OK;
+    const int rc = encode();
+    if (rc == DQ_OK) break;
+    if (!micro || max_rot <= 8) return rc;
+    // a sweep's micro program outgrew its place in shared memory or its slots
+    clear_error();
+    max_rot /= 2;
+    poly = poly0;
+  }
   blob.align16();
   if (fw.plan_out) {  // plan-only: hand the programs back instead of running them
     const size_t base = fw.plan_out->size();
@@ -1382,8 +2075,8 @@ int fused_run_segment(double2* amp, uint32_t n, std::vector<PGate>& G, Planner& 
     const SwHeader* hh = reinterpret_cast<const SwHeader*>(blob.buf.data() + offs[i]);
     // a pending basis state is consumed by the first sweep (it writes every amplitude)
     const long long synth = (lazy_basis && *lazy_basis >= 0) ? (long long)*lazy_basis : -1;
-    DQ_TRY(launch_sweep(amp, n, pl.TB, pl.RB, fw.d_blob + offs[i], hh->prog_bytes, st, synth,
-                        hh->run_bits, hh->flags));
+    DQ_TRY(launch_sweep(amp, n, pl.TB, pl.RB, fw.d_blob + offs[i], hh->stage_bytes, st, synth,
+                        hh->run_bits, hh->flags, hh->off_micro != 0));
     if (lazy_basis) *lazy_basis = -1;
     if (timing) {
       cudaEventRecord(e1, st);
@@ -1415,6 +2108,8 @@ int fused_run(double2* amp, uint32_t n, const dq_inst* prog, uint64_t ninst, con
   pl.TB = TB;
   pl.RB = M - TB;
   pl.single_tile = (M == n);
+  // the trajectory launch runs 8-thread-bit plans, k_sweep and k_sweep_multi 7-bit ones
+  pl.micro_ok = pl.RB == 4 && (TB == 7 ? sweep_stages() != 2 : fw.plan_tb != 0);
   // Pinned tile qubits: 0..4 (512-byte runs) or 0..2 (128-byte runs, two
   // more tile qubits free); by default each segment of 20+ qubits is planned
   // both ways and keeps the one with clearly fewer sweeps.
@@ -1585,11 +2280,12 @@ uint32_t sweep_run_bits(const uint8_t* prog) {
 }
 
 uint32_t sweep_prog_bytes(const uint8_t* prog) {
-  return reinterpret_cast<const SwHeader*>(prog)->prog_bytes;
+  return reinterpret_cast<const SwHeader*>(prog)->stage_bytes;
 }
 
 uint32_t sweep_flags(const uint8_t* prog) {
-  return reinterpret_cast<const SwHeader*>(prog)->flags;
+  const SwHeader* h = reinterpret_cast<const SwHeader*>(prog);
+  return h->off_micro ? SWF_MICRO : h->flags;
 }
 
 int launch_sweep_multi(const SweepJob* d_jobs, uint32_t njobs, uint32_t n, uint32_t rb,
@@ -1605,6 +2301,9 @@ int launch_sweep_multi(const SweepJob* d_jobs, uint32_t njobs, uint32_t n, uint3
                       : launch_sweep_multi_t<7, 3, 5>(d_jobs, njobs, n, max_bytes, st);
     case 4:
       // every job's program allows a restricted build (the flags of all of them ANDed)
+      if (flags & SWF_MICRO)
+        return r3 ? launch_sweep_multi_t<7, 4, 3, FORM_M>(d_jobs, njobs, n, max_bytes, st)
+                  : launch_sweep_multi_t<7, 4, 5, FORM_M>(d_jobs, njobs, n, max_bytes, st);
       if (flags & SWF_HONLY)
         return r3 ? launch_sweep_multi_t<7, 4, 3, FORM_H>(d_jobs, njobs, n, max_bytes, st)
                   : launch_sweep_multi_t<7, 4, 5, FORM_H>(d_jobs, njobs, n, max_bytes, st);

@@ -68,6 +68,10 @@ struct SwHeader {
   uint32_t off_runswz;         // u32 swizzled shared-memory index of run r's first element
   uint32_t flags;              // SWF_* (host side: kernel choice)
   uint32_t off_gstore;         // SwGStore of the last phase (0: none)
+  uint32_t off_micro;          // SwMPhase per phase (0: none); then the ops at off_op are not executed
+  uint32_t off_final;          // its SwFinal entries
+  uint32_t stage_bytes;        // leading bytes the kernel needs (all of it without off_micro)
+  uint32_t pad;
 };
 // Global offsets for the last phase to write its amplitudes straight to the
 // state (present when the phase's lanes 0..2 are local bits 0..2, i.e. each
@@ -82,16 +86,19 @@ struct SwGStore {
 // kernel built with the H-phase path only
 constexpr uint32_t SWF_HONLY = 1u;
 // every op of the sweep is a one-qubit op without a flush (OP_U1, OP_U1R,
-// OP_U1X; controls allowed): the launch may use the kernel built with that
-// part of the interpreter only
+// OP_U1X; controls allowed) or the sweep has rotation phases (off_micro): the
+// launch may use the kernel built with that part of the interpreter, or with
+// the rotation phases, only
 constexpr uint32_t SWF_UONLY = 2u;
 // every phase of the sweep is a straight-line phase (OP_HPHASE) of real 2x2
 // sub-ops only: the launch may use the build with that path only
 constexpr uint32_t SWF_RONLY = 4u;
+// (sweep_flags only, alone: the program has rotation phases)
+constexpr uint32_t SWF_MICRO = 8u;
 // Builds of the tile loop: the whole op interpreter, Hadamard-pattern
 // straight-line phases only, plain one-qubit ops only, real-2x2 straight-line
-// phases only.
-enum : int { FORM_ALL = 0, FORM_H = 1, FORM_U = 2, FORM_R = 3 };
+// phases only, rotation phases only.
+enum : int { FORM_ALL = 0, FORM_H = 1, FORM_U = 2, FORM_R = 3, FORM_M = 4 };
 struct SwPhase {
   uint32_t lanesw[32];         // swizzled local index of the lane bits (thread bits 0..4)
   uint32_t warpsw[8];          // swizzled local index of the warp bits (thread bits 5..7)
@@ -100,6 +107,42 @@ struct SwPhase {
   uint32_t xload;              // XORed into every load address: X gates folded into the load
   uint32_t pad1;
 };
+// ---- rotation phases ----------------------------------------------------------------
+// One-qubit gates, phases and CX only.  A general gate is a phase, a real
+// rotation and a phase.  The planner keeps phases in its phase polynomial,
+// where they commute with controls and pass through CX targets, and divides
+// the rotation by its cosine (after a quarter turn where the sine is larger):
+// [[1, -t], [t, 1]], |t| <= 1.  X and CX among the tile's qubits are changes
+// of the phases' shared-memory addresses and execute nothing.
+// So a phase is: up to four rotations on register bits 0..k-1, 2 fused
+// multiply-adds per amplitude each instead of 8 for a general gate; before
+// them one table of 16 factors, every pending term among the register qubits
+// and the divided-out cosines; a factor per register bit for terms with other
+// qubits; X gates controlled from outside the tile flip the load address.
+// Bound: shared-memory bandwidth (an exchange of the registers per phase, about
+// 180 wavefronts per warp with the table and the descriptors, 56% of the
+// pipe's rate), then HBM.  Interpreting the same rotations op by op in fewer,
+// longer phases is bound by instruction issue instead (197 ms).
+// 28-qubit brickwork, 20 layers of u3 and cx: 77 sweeps of general 2x2s in
+// 190 ms, 30 sweeps of 196 rotation phases in 105 ms.
+struct SwMPhase {
+  uint32_t k, mul;             // rotations; DATA index of the table (~0: none)
+  uint32_t ncross, ncond;
+  double t[4];
+  uint32_t cross[4];           // bit b's factor: slot | flags << 16 (~0: none)
+  uint32_t cdata[4];           // DATA index of its thread table (FL_THR)
+  uint64_t cmask[4];           // load flips: qubits outside the tile that must be 1,
+  uint32_t cxor[4];            // and the address bits they flip
+  uint32_t fin0, nfin, pad0, pad1;  // entries of the final flush, after the rotations
+};
+// a[j] *= W F[j] for threads with bit `bit` set (every thread: ~0), W =
+// slot's factor with FL_THR times the thread table at data, then with FL_REG
+// a register table F follows
+struct SwFinal {
+  uint32_t slot, flags, bit, data;
+};
+static_assert(sizeof(SwMPhase) == 144 && sizeof(SwFinal) == 16, "layout");
+
 // 32 bytes, read as two 128-bit words: w0 = type | b0 << 8 | b1 << 16 | creg << 24,
 // w1 = ctl_thr | flags << 8 | slot << 16, data = first DATA entry, cnl = non-local controls
 struct SwOp {
@@ -406,6 +449,113 @@ __device__ __forceinline__ void exec_u(const uint4 o0, const uint4 o1, double2 (
   }
 }
 
+template <int RB, int B>
+__device__ __forceinline__ void rot_op(double2 (&a)[1 << RB], double t) {
+#pragma unroll
+  for (int j = 0; j < (1 << RB); ++j) {
+    if (j & (1 << B)) continue;
+    const int k = j | (1 << B);
+    const double2 x = a[j], y = a[k];
+    a[j] = make_double2(fma(-t, y.x, x.x), fma(-t, y.y, x.y));
+    a[k] = make_double2(fma(t, x.x, y.x), fma(t, x.y, y.y));
+  }
+}
+
+// The body of a rotation phase with K rotations, from the load to the store
+// (to the tile, or for the last phase with GS to the state).
+// head: the words k, mul, ncross, ncond of M.
+template <int RB, int K>
+__device__ __forceinline__ void rot_phase(const uint4 head, const SwMPhase& M, const SwFinal* __restrict__ FIN,
+                                          uint32_t pt, const uint4 PV, double2* cur,
+                                          const double2* __restrict__ DATA, const double2* __restrict__ slots,
+                                          uint32_t tid, uint64_t base, const SwGStore* __restrict__ GS,
+                                          double2* __restrict__ state) {
+  constexpr int R = 1 << RB;
+  // byte offsets: one XOR per access
+  uint32_t V[4] = {PV.x << 4, PV.y << 4, PV.z << 4, PV.w << 4};
+  uint32_t ptl = pt;
+  for (uint32_t i = 0; i < head.w; ++i)
+    if ((base & M.cmask[i]) == M.cmask[i]) ptl ^= M.cxor[i];
+  char* const tile = reinterpret_cast<char*>(cur);
+  double2 a[R];
+  {
+    uint32_t x[R];
+    x[0] = ptl << 4;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      if (j) x[j] = x[j & (j - 1)] ^ V[j & 1 ? 0 : j & 2 ? 1 : j & 4 ? 2 : 3];
+      a[j] = *reinterpret_cast<const double2*>(tile + x[j]);
+    }
+  }
+  if (head.y != ~0u) {
+    const double2* T = DATA + head.y;
+#pragma unroll
+    for (int j = 0; j < R; ++j) a[j] = cmul_f(a[j], T[j]);
+  }
+  if (head.z) {
+    const uint4 cr = *reinterpret_cast<const uint4*>(M.cross);
+    auto factor = [&](int b, uint32_t c) {
+      double2 W = slots[c & 0xffffu];
+      if ((c >> 16) & FL_THR) {
+        const double2* T = DATA + M.cdata[b];
+        W = cmul_f(W, cmul_f(T[tid & 31u], T[32 + (tid >> 5)]));
+      }
+      return W;
+    };
+    if (cr.x != ~0u) flush_reg<RB, 0>(a, factor(0, cr.x), nullptr);
+    if (cr.y != ~0u) flush_reg<RB, 1>(a, factor(1, cr.y), nullptr);
+    if (cr.z != ~0u) flush_reg<RB, 2>(a, factor(2, cr.z), nullptr);
+    if (cr.w != ~0u) flush_reg<RB, 3>(a, factor(3, cr.w), nullptr);
+  }
+  const double2* t2 = reinterpret_cast<const double2*>(M.t);
+  if constexpr (K > 0) {
+    const double2 t = t2[0];
+    rot_op<RB, 0>(a, t.x);
+    if constexpr (K > 1) rot_op<RB, 1>(a, t.y);
+  }
+  if constexpr (K > 2) {
+    const double2 t = t2[1];
+    rot_op<RB, 2>(a, t.x);
+    if constexpr (K > 3) rot_op<RB, 3>(a, t.y);
+  }
+  if constexpr (K == 0) {  // the final flush has a phase of its own
+    for (uint32_t i = 0; i < M.nfin; ++i) {
+      const SwFinal f = FIN[M.fin0 + i];
+      if (f.bit != ~0u && !((tid >> f.bit) & 1u)) continue;
+      const double2* T = DATA + f.data;
+      double2 W = slots[f.slot];
+      if (f.flags & FL_THR) {
+        W = cmul_f(W, cmul_f(T[tid & 31u], T[32 + (tid >> 5)]));
+        T += 40;
+      }
+#pragma unroll
+      for (int j = 0; j < R; ++j) a[j] = cmul_f(a[j], (f.flags & FL_REG) ? cmul_f(W, T[j]) : W);
+    }
+  }
+  if (GS) {
+    const uint64_t gt = base + GS->glane[tid & 31u] + GS->gwarp[tid >> 5];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      uint64_t g = gt;
+#pragma unroll
+      for (int b = 0; b < RB; ++b)
+        if ((j >> b) & 1) g += GS->gV[b];
+      state[g] = a[j];
+    }
+    return;
+  }
+  // recomputed instead of kept in registers across the phase
+#pragma unroll
+  for (int b = 0; b < RB; ++b) V[b] = opaque(V[b]);
+  uint32_t x[R];
+  x[0] = opaque(pt) << 4;
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    if (j) x[j] = x[j & (j - 1)] ^ V[j & 1 ? 0 : j & 2 ? 1 : j & 4 ? 2 : 3];
+    *reinterpret_cast<double2*>(tile + x[j]) = a[j];
+  }
+}
+
 template <int RB>
 __device__ __forceinline__ void exec_op(const uint4 o0, const uint4 o1, double2 (&a)[1 << RB],
                                         const double2* __restrict__ DATA,
@@ -480,7 +630,8 @@ __device__ __forceinline__ void exec_op(const uint4 o0, const uint4 o1, double2 
 // program's phases are all H phases (SWF_HONLY), so the generic op
 // interpreter is left out of the build.  FORM: FORM_H for SWF_HONLY programs
 // (no op interpreter), FORM_U for SWF_UONLY programs (the one-qubit part of
-// it), FORM_ALL otherwise.
+// it), FORM_R for SWF_RONLY programs, FORM_M for programs with off_micro,
+// FORM_ALL otherwise.
 template <int TB, int RB, int S, int RUNB, int FORM = FORM_ALL>
 __device__ __forceinline__ void sweep_tiles(double2* __restrict__ state, const uint8_t* prog,
                                             uint32_t ntiles, long long synth, double2* bufs,
@@ -612,6 +763,24 @@ __device__ __forceinline__ void sweep_tiles(double2* __restrict__ state, const u
     for (uint32_t p = 0; p < nph; ++p) {
       const SwPhase& P = PH[p];
       const uint32_t pt = P.lanesw[lane] ^ P.warpsw[warp];
+      if constexpr (FORM == FORM_M) {
+        // ncond flips and ops of other threads' elements: the stores of this
+        // phase may hit what another thread still loads only with a flip
+        const SwMPhase& M = reinterpret_cast<const SwMPhase*>(prog + H->off_micro)[p];
+        const SwFinal* FIN = reinterpret_cast<const SwFinal*>(prog + H->off_final);
+        const SwGStore* G = p + 1 == nph ? GS : nullptr;
+        const uint4 head = *reinterpret_cast<const uint4*>(&M);
+        const uint4 pv = *reinterpret_cast<const uint4*>(P.V);
+        switch (head.x) {
+          case 0: rot_phase<RB, 0>(head, M, FIN, pt, pv, cur, DATA, slots, tid, base, G, state); break;
+          case 1: rot_phase<RB, 1>(head, M, FIN, pt, pv, cur, DATA, slots, tid, base, G, state); break;
+          case 2: rot_phase<RB, 2>(head, M, FIN, pt, pv, cur, DATA, slots, tid, base, G, state); break;
+          case 3: rot_phase<RB, 3>(head, M, FIN, pt, pv, cur, DATA, slots, tid, base, G, state); break;
+          default: rot_phase<RB, 4>(head, M, FIN, pt, pv, cur, DATA, slots, tid, base, G, state); break;
+        }
+        if (!G) __syncthreads();
+        continue;
+      }
       const uint32_t ptl = pt ^ P.xload;
       uint32_t V[RB];
 #pragma unroll

@@ -104,7 +104,7 @@ struct TProg {         // one program of a launch
 struct TSweep {          // one fused sweep of an HBM item
   uint64_t off;          // byte offset of its program in the launch's sweep blob
   uint32_t ntiles, run_bits;
-  uint32_t prog_bytes, pad;
+  uint32_t prog_bytes, micro;  // micro: the program has rotation phases
 };
 struct TItem {          // shots [shot, shot + count) of a program
   uint32_t prog, count;
@@ -321,7 +321,11 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
             *reinterpret_cast<uint4*>(sprog + i) =
                 __ldg(reinterpret_cast<const uint4*>(P.sweep_blob + sw.off + i));
           __syncthreads();
-          if (sw.run_bits == 3)
+          if (sw.micro && sw.run_bits == 3)
+            sweep_tiles<8, kHbmTileBits - 8, 2, 3, FORM_M>(pg.hbm, sprog, sw.ntiles, sy, bufs, slots, rank, C);
+          else if (sw.micro)
+            sweep_tiles<8, kHbmTileBits - 8, 2, 5, FORM_M>(pg.hbm, sprog, sw.ntiles, sy, bufs, slots, rank, C);
+          else if (sw.run_bits == 3)
             sweep_tiles<8, kHbmTileBits - 8, 2, 3>(pg.hbm, sprog, sw.ntiles, sy, bufs, slots, rank, C);
           else
             sweep_tiles<8, kHbmTileBits - 8, 2, 5>(pg.hbm, sprog, sw.ntiles, sy, bufs, slots, rank, C);
@@ -1063,7 +1067,7 @@ void add_hbm_program(LaunchSet& ls, const HbmPlan& pl, uint64_t base, uint32_t n
   for (uint64_t off : pl.offs) {
     const uint32_t pb = sweep_prog_bytes(pl.blob.data() + off);
     ls.sweeps.push_back(TSweep{base + off, 1u << (n - kHbmM), sweep_run_bits(pl.blob.data() + off),
-                               pb, 0});
+                               pb, sweep_flags(pl.blob.data() + off) & SWF_MICRO});
     ls.hbm_smem = std::max<size_t>(ls.hbm_smem, sizeof(double2) * (2 * (1u << kHbmM) + kMaxSlots) + pb);
   }
   ls.progs.push_back(pg);
