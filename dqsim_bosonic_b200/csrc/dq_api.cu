@@ -1022,7 +1022,18 @@ int dq_run(dq_state_t h, const dq_inst* prog, uint64_t ninst, const dq_cond* con
   c.timer.st = h->stream;
   int rc = DQ_OK;
   const bool fused = o.exec == DQ_EXEC_FUSED && !o.profile && h->n >= kFusedMinQubits;
-  if (fused) {
+  // Small states run in one launch: programs the fused sweeps do not take, and
+  // with measurements those they do (every measurement ends a sweep and reads
+  // p1 back).  A handful of gates is launched one by one as fast.
+  uint64_t meas = 0;
+  for (uint64_t i = 0; i < ninst; ++i) meas += prog[i].kind == DQ_MEASURE || prog[i].kind == DQ_RESET;
+  const bool small = !o.profile && h->n >= 1 && h->n <= kSmallQubits && ncbits <= kSmallCbits &&
+                     (fused ? meas > 0 : ninst >= 8 || meas > 0);
+  if (small) {
+    if (h->permuted) rc = canonicalize(h);
+    if (rc == DQ_OK)
+      rc = small_run(h, prog, ninst, conds, nconds, seed, cbits, ncbits, o.semantics, &c.prof);
+  } else if (fused) {
     FusedHooks hooks;
     hooks.measure = [&c, h](uint32_t q, int* out) {
       DQ_TRY(materialize_basis(h));
@@ -1127,6 +1138,20 @@ int dq_sample_key(dq_state_t h, const uint32_t* qubits, uint32_t k, const uint32
   for (auto& q : mq) q = h->perm[q];
   qubits = mq.data();
   const uint64_t nj = 1ULL << k;
+  if (sample_small_ok(h->n, qubits, k, shots, h->device)) {
+    const size_t count_at = (shots + 1) / 2 * 2, bytes = sizeof(uint32_t) * (count_at + 2);
+    DQ_TRY(ensure_query_buffers(h, bytes, bytes));
+    uint32_t* dev = static_cast<uint32_t*>(h->q_dev);
+    const uint32_t* host = static_cast<const uint32_t*>(h->q_host);
+    DQ_TRY(launch_sample_small(h->amp, h->n, qubits, k, key8, shots, dev, h->stream, h->device));
+    DQ_CUDA_TRY(cudaMemcpyAsync(h->q_host, dev, bytes, cudaMemcpyDeviceToHost, h->stream));
+    DQ_TRY(sync_stream(h));
+    if (shots) memcpy(out_idx, host, sizeof(uint32_t) * shots);
+    unsigned long long nb = 0;
+    memcpy(&nb, host + count_at, sizeof(nb));
+    if (n_boundary) *n_boundary = nb;
+    return DQ_OK;
+  }
   // CDF, sampled indices and the reductions' workspace in the handle's device
   // query buffer, each part 256-byte aligned
   auto align256 = [](size_t b) { return (b + 255) / 256 * 256; };

@@ -235,15 +235,20 @@ __device__ __forceinline__ uint64_t deposit_j(uint64_t j, const MargParams& P) {
   return bits;
 }
 
-__global__ void k_marg_thread(const double2* __restrict__ s, uint64_t nj, uint64_t nterms,
-                              MargParams P, double* __restrict__ out) {
-  const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (j >= nj) return;
+// output j in the reference's order of additions
+__device__ __forceinline__ double marginal_term(const double2* __restrict__ s, uint64_t j, uint64_t nterms,
+                                                const MargParams& P) {
   const uint64_t jb = deposit_j(j, P);
   double acc = 0.0;
   for (uint64_t r = 0; r < nterms; ++r)
     acc = __dadd_rn(acc, norm_sqr_x(s[insert_zeros(r, P.rest.p, P.rest.np) | jb]));
-  out[j] = acc;
+  return acc;
+}
+
+__global__ void k_marg_thread(const double2* __restrict__ s, uint64_t nj, uint64_t nterms,
+                              MargParams P, double* __restrict__ out) {
+  const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (j < nj) out[j] = marginal_term(s, j, nterms, P);
 }
 
 // One block sums segment `seg` of output j.  When the lowest marginal qubit
@@ -434,24 +439,60 @@ struct Key8 {
   uint32_t k[8];
 };
 
-// sample_counts inner loop (engine.rs:426-431) with draw s computed from the
-// stream position: idx = partition_point(cdf < r).min(len - 1).
-__global__ void k_sample(const double* __restrict__ cdf, uint64_t len, Key8 key, uint64_t shots,
-                         uint32_t* __restrict__ out, unsigned long long* __restrict__ nboundary) {
-  const uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (s >= shots) return;
-  const double r = chacha8_draw(key.k, s);
+// sample_counts inner loop (engine.rs:426-431): idx = partition_point(cdf <
+// r).min(len - 1); near: r lies within 1e-12 of a boundary of that interval.
+__device__ __forceinline__ uint64_t draw_index(const double* cdf, uint64_t len, double r, bool* near) {
   uint64_t lo = 0, hi = len;
   while (lo < hi) {
     const uint64_t mid = lo + ((hi - lo) >> 1);
     if (cdf[mid] < r) lo = mid + 1; else hi = mid;
   }
   if (lo > len - 1) lo = len - 1;
-  out[s] = (uint32_t)lo;
-  const double up = cdf[lo];
-  bool near = fabs(up - r) <= 1e-12;
-  if (lo > 0) near = near || fabs(r - cdf[lo - 1]) <= 1e-12;
+  *near = fabs(cdf[lo] - r) <= 1e-12 || (lo > 0 && fabs(r - cdf[lo - 1]) <= 1e-12);
+  return lo;
+}
+
+// Draw s computed from the stream position.
+__global__ void k_sample(const double* __restrict__ cdf, uint64_t len, Key8 key, uint64_t shots,
+                         uint32_t* __restrict__ out, unsigned long long* __restrict__ nboundary) {
+  const uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (s >= shots) return;
+  bool near;
+  out[s] = (uint32_t)draw_index(cdf, len, chacha8_draw(key.k, s), &near);
   if (near) atomicAdd(nboundary, 1ULL);
+}
+
+// Marginal, CDF and samples of a small distribution in one block: the values of
+// k_marg_thread, k_scan_* and k_sample (same order of additions) without six
+// launches; out: shots indices, then (8-byte aligned) the boundary count.
+__global__ void __launch_bounds__(kScanThreads) k_sample_small(const double2* __restrict__ s, uint32_t nj,
+                                                               uint64_t nterms, MargParams P, Key8 key,
+                                                               uint64_t shots, uint32_t* __restrict__ out) {
+  __shared__ double cdf[kScanChunk];
+  __shared__ unsigned long long near_count;
+  const uint32_t tid = threadIdx.x;
+  if (tid == 0) near_count = 0;
+  for (uint32_t j = tid; j < nj; j += kScanThreads) cdf[j] = marginal_term(s, j, nterms, P);
+  __syncthreads();
+  const uint64_t b0 = (uint64_t)tid * kScanPer;
+  double tot;
+  const double ex = block_exclusive_scan(thread_segment_sum(cdf, nj, b0), &tot);
+  double run = __dadd_rn(0.0, ex);
+  for (int e = 0; e < kScanPer; ++e)
+    if (b0 + e < nj) {
+      run = __dadd_rn(run, cdf[b0 + e]);
+      cdf[b0 + e] = run;
+    }
+  __syncthreads();
+  if (tid == 0) cdf[nj - 1] = 1.0;
+  __syncthreads();
+  for (uint64_t i = tid; i < shots; i += kScanThreads) {
+    bool near;
+    out[i] = (uint32_t)draw_index(cdf, nj, chacha8_draw(key.k, i), &near);
+    if (near) atomicAdd(&near_count, 1ULL);
+  }
+  __syncthreads();
+  if (tid == 0) *reinterpret_cast<unsigned long long*>(out + (shots + 1) / 2 * 2) = near_count;
 }
 
 }  // namespace
@@ -690,6 +731,20 @@ int launch_sample(const double* cdf, uint64_t len, const uint32_t key[8], uint64
   Key8 K;
   for (int i = 0; i < 8; ++i) K.k[i] = key[i];
   k_sample<<<blocks_for(shots, kThreads), kThreads, 0, st>>>(cdf, len, K, shots, d_idx, d_boundary);
+  DQ_CUDA_TRY(cudaGetLastError());
+  return DQ_OK;
+}
+
+bool sample_small_ok(uint32_t n, const uint32_t* qubits, uint32_t k, uint64_t shots, int device) {
+  return (1ULL << k) <= (uint64_t)kScanChunk && shots <= 16384 && plan_marginal(n, qubits, k, device).kind == 1;
+}
+
+int launch_sample_small(const double2* s, uint32_t n, const uint32_t* qubits, uint32_t k, const uint32_t key[8],
+                        uint64_t shots, uint32_t* d_out, cudaStream_t st, int device) {
+  const MargPlan m = plan_marginal(n, qubits, k, device);
+  Key8 K;
+  for (int i = 0; i < 8; ++i) K.k[i] = key[i];
+  k_sample_small<<<1, kScanThreads, 0, st>>>(s, 1u << k, 1ULL << (n - k), m.P, K, shots, d_out);
   DQ_CUDA_TRY(cudaGetLastError());
   return DQ_OK;
 }

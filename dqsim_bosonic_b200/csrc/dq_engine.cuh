@@ -42,6 +42,12 @@ uint64_t marginal_workspace(uint32_t n, const uint32_t* qubits, uint32_t k, int 
 // marginal_workspace() doubles (nullptr: a stream-ordered temporary is used).
 int launch_marginal(const double2* s, uint32_t n, const uint32_t* qubits, uint32_t k,
                     double* d_out, double* d_work, Scratch& sc, cudaStream_t st, int device);
+// Marginal, CDF and samples in one launch, where the distribution fits one
+// block's scan and every output is summed by one thread: d_out holds the
+// shots' indices, then at entry (shots + 1) / 2 * 2 the 64-bit boundary count.
+bool sample_small_ok(uint32_t n, const uint32_t* qubits, uint32_t k, uint64_t shots, int device);
+int launch_sample_small(const double2* s, uint32_t n, const uint32_t* qubits, uint32_t k, const uint32_t key[8],
+                        uint64_t shots, uint32_t* d_out, cudaStream_t st, int device);
 // Device doubles of workspace launch_cdf needs for len entries.
 uint64_t cdf_workspace(uint64_t len);
 // in-place inclusive prefix sum of d[len] (deterministic order), last = 1.0;

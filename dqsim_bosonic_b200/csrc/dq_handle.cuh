@@ -93,6 +93,13 @@ int read_scalars(dq_state_t h, const double* d_src, int count, double* out);
 // Grow the handle's query buffers to at least dev_bytes (device) and
 // host_bytes (pinned host); the stream is drained before a buffer is replaced.
 int ensure_query_buffers(dq_state_t h, size_t dev_bytes, size_t host_bytes);
+// Runs a program of dq_run on a small state in one launch (exact per-gate
+// arithmetic; the state canonical or a pending basis state; no profile, at
+// most kSmallQubits qubits and kSmallCbits classical bits).
+constexpr uint32_t kSmallQubits = 12;
+constexpr uint64_t kSmallCbits = 1024;
+int small_run(dq_state_t h, const dq_inst* prog, uint64_t ninst, const dq_cond* conds, uint64_t nconds,
+              uint64_t seed, int32_t* cbits, uint64_t ncbits, int semantics, dq_profile* prof);
 int gate_qubit_count(int kind);
 int validate_inst(const dq_inst& in, uint32_t n, uint64_t nconds, uint64_t ncbits,
                   const dq_cond* conds, uint64_t idx);

@@ -79,12 +79,13 @@ struct TOp {
   uint32_t cond_first, cond_count;
   int32_t cbit;     // MEASURE: classical bit; FAIL: unused
   uint32_t mat;     // offset into the matrix pool (double2 units)
-  uint32_t remote;  // touches cluster qubits or needs a cluster reduction
+  uint32_t remote;  // bit 0: touches cluster qubits or needs a cluster reduction; kOpMulti
   uint64_t ctrl;    // control mask (all must be 1)
   uint8_t q[8];     // DIAG / DENSE qubits, q[0] = MSB of the matrix index; RPHASE: register bits
   int64_t inst;     // original instruction index (-1: a fused 2x2)
 };
 static_assert(sizeof(TOp) == 48, "TOp layout");
+constexpr uint32_t kOpMulti = 2u;  // TOp::remote: a gate on two or more qubits (call counts)
 
 struct TProg {         // one program of a launch
   uint32_t ops_off, nops;
@@ -100,6 +101,13 @@ struct TProg {         // one program of a launch
   double2* hbm;
   uint32_t sweep_first, nsweeps;
   long long synth;
+  // A run on a state handle (small_run): the state it starts from (null: the
+  // basis state `basis`), the classical bits it starts with (null: unwritten)
+  // and its gate and measurement counts (one-qubit, wider, measurements)
+  const double2* state_in;
+  const int32_t* cbits_in;
+  unsigned long long* counts;
+  uint64_t basis;
 };
 struct TSweep {          // one fused sweep of an HBM item
   uint64_t off;          // byte offset of its program in the launch's sweep blob
@@ -140,6 +148,10 @@ struct TrajParams {
   int32_t* slot_cbits;           // nslots x ncbits
   const double* draws;           // draw k of shot s at s * draw_stride + k, or null
   uint32_t nslots, draw_stride;
+  // ops, pool and conds as one image of stage_bytes at ops, copied to dynamic
+  // shared memory at stage_at when the launch starts (0: read from memory; a
+  // small program's op after op is otherwise a chain of L2 round trips)
+  uint32_t stage_bytes, stage_at;
   uint64_t nitems;
   const uint8_t* sweep_blob;     // sweep programs of the HBM items (dq_sweep.cuh layout)
   const TSweep* sweeps;
@@ -263,6 +275,18 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
   cg::cluster_group cl = cg::this_cluster();
   const uint32_t C = cl.num_blocks(), rank = cl.block_rank();
   const uint32_t tid = threadIdx.x;
+  const TOp* ops = P.ops;
+  const double2* pool = P.pool;
+  const dq_cond* conds = P.conds;
+  if (P.stage_bytes) {
+    uint8_t* st = smraw + P.stage_at;
+    for (uint32_t i = tid * 16u; i < P.stage_bytes; i += THREADS * 16u)
+      *reinterpret_cast<uint4*>(st + i) = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(P.ops) + i));
+    ops = reinterpret_cast<const TOp*>(st);
+    pool = reinterpret_cast<const double2*>(st + (reinterpret_cast<const uint8_t*>(P.pool) - reinterpret_cast<const uint8_t*>(P.ops)));
+    conds = reinterpret_cast<const dq_cond*>(st + (reinterpret_cast<const uint8_t*>(P.conds) - reinterpret_cast<const uint8_t*>(P.ops)));
+    __syncthreads();
+  }
   auto sync_all = [&](bool cluster) {
     if (cluster && C > 1) cl.sync(); else __syncthreads();
   };
@@ -361,10 +385,11 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
         cb[i] = __ldcg(P.slot_cbits + (uint64_t)tk.slot * pg.ncbits + i);
     } else {
       draws = 0;
-      for (uint32_t i = tid; i < L; i += THREADS) sm[i] = make_double2(0.0, 0.0);
-      for (uint32_t i = tid; i < pg.ncbits; i += THREADS) cb[i] = -1;
-      if (rank == 0 && tid == 0) sm[0] = make_double2(1.0, 0.0);
+      for (uint32_t i = tid; i < L; i += THREADS)
+        sm[tswz(i)] = pg.state_in ? pg.state_in[gbase + i] : make_double2(gbase + i == pg.basis ? 1.0 : 0.0, 0.0);
+      for (uint32_t i = tid; i < pg.ncbits; i += THREADS) cb[i] = pg.cbits_in ? pg.cbits_in[i] : -1;
     }
+    unsigned long long n1q = 0, nnq = 0, nmeas = 0;  // thread 0: executed gates and measurements
     bool last_cluster = true;
     sync_all(true);
 
@@ -411,7 +436,7 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
     };
     uint32_t oi0 = 0;
     if (tk.slot >= 0) {  // finish the measurement the state was saved at
-      const TOp op = P.ops[pg.ops_off + tk.oi];
+      const TOp op = ops[pg.ops_off + tk.oi];
       collapse(op, (int)tk.outcome, norm_of((int)tk.outcome, tk.p1));
       if (tid == 0 && op.type == T_MEASURE) cb[op.cbit] = (int)tk.outcome;
       oi0 = tk.oi + 1;
@@ -423,9 +448,9 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
     TOp nxt{};
     double2 nu[4] = {};
     auto fetch = [&](uint32_t k) {
-      nxt = P.ops[pg.ops_off + k];
+      nxt = ops[pg.ops_off + k];
       if (nxt.type == T_ONEQ)
-        for (int i = 0; i < 4; ++i) nu[i] = P.pool[nxt.mat + i];
+        for (int i = 0; i < 4; ++i) nu[i] = pool[nxt.mat + i];
     };
     if (oi0 < pg.nops) fetch(oi0);
     for (uint32_t oi = oi0; oi < pg.nops; ++oi) {
@@ -438,7 +463,7 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
         if (tid == 0) {
           int ok = 1;
           for (uint32_t c = 0; c < op.cond_count && ok; ++c) {
-            const dq_cond cd = P.conds[op.cond_first + c];
+            const dq_cond cd = conds[op.cond_first + c];
             uint64_t actual = 0;
             for (uint64_t b = 0; b < cd.creg_size; ++b) {
               const uint64_t idx = cd.creg_base + b;
@@ -452,7 +477,9 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
         __syncthreads();
         if (s_skip[oi & 1]) continue;
       }
-      const bool remote = op.remote && C > 1;
+      const bool remote = (op.remote & 1u) && C > 1;
+      if (op.type == T_MEASURE || op.type == T_RESET) ++nmeas;
+      else if (op.type != T_RPHASE && op.type != T_FAIL) (op.remote & kOpMulti ? nnq : n1q) += 1;
       if (remote && !last_cluster) cl.sync();
 
       switch (op.type) {
@@ -532,7 +559,7 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
           const uint64_t need = op.ctrl | (1ULL << op.t1);
           const uint64_t hi = need & ~lmask, lo = need & lmask;
           if ((gbase & hi) != hi) break;
-          const double2 e = P.pool[op.mat];
+          const double2 e = pool[op.mat];
           const int np = __popcll((long long)lo);
           const uint32_t count = L >> np;
           const uint32_t p0 = np > 0 ? (uint32_t)(__ffsll((long long)lo) - 1) : 0u;
@@ -570,7 +597,7 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
             const uint64_t g = gbase | o;
             uint32_t idx = 0;
             for (uint32_t b = 0; b < kq; ++b) idx = (idx << 1) | (uint32_t)((g >> op.q[b]) & 1ULL);
-            const double2 d = P.pool[op.mat + idx];
+            const double2 d = pool[op.mat + idx];
             if (d.x == 1.0 && d.y == 0.0) continue;
             sm[tswz(o)] = cmul_x(d, sm[tswz(o)]);
           }
@@ -622,7 +649,7 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
             for (uint32_t r = 0; r < D; ++r) {
               double2 acc = make_double2(0.0, 0.0);
               for (uint32_t c = 0; c < D; ++c) {
-                const double2 uu = P.pool[op.mat + r * D + c];
+                const double2 uu = pool[op.mat + r * D + c];
                 if (uu.x != 0.0 || uu.y != 0.0) acc = cadd_x(acc, cmul_x(uu, v[c]));
               }
               *ptr[r] = acc;
@@ -734,6 +761,7 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
             }
             if (o) lo += n0; else hi = lo + n0;
           }
+          if (op.type == T_RESET && o == 1) ++n1q;  // the flip
           collapse(op, o, norm_of(o, p1));
           // read by conditions after this op's closing barrier only
           if (tid == 0 && op.type == T_MEASURE) cb[op.cbit] = o;
@@ -759,7 +787,8 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) a[j] = sm[sidx(sb, j)];
             for (uint32_t sidx_op = 0; sidx_op < cnt; ++sidx_op) {
-              const TOp so = P.ops[pg.ops_off + oi + 1 + sidx_op];
+              const TOp so = ops[pg.ops_off + oi + 1 + sidx_op];
+              if (gi == 0) (so.remote & kOpMulti ? nnq : n1q) += 1;
               const uint32_t t = so.t1;
               const uint32_t rt = t == r0 ? 0u : (t == r1 ? 1u : (t == r2 ? 2u : 3u));
               uint32_t creg = 0;
@@ -771,7 +800,7 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
               }
               if (so.type == T_ONEQ) {
                 double2 uu[4];
-                for (int i = 0; i < 4; ++i) uu[i] = P.pool[so.mat + i];
+                for (int i = 0; i < 4; ++i) uu[i] = pool[so.mat + i];
                 switch (rt) {
                   case 0: rphase_1q<0>(a, uu, creg); break;
                   case 1: rphase_1q<1>(a, uu, creg); break;
@@ -815,6 +844,11 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
     if (pg.state_out) {
       double2* dst = pg.state_out + (it.shot << pg.n) + gbase;
       for (uint32_t i = tid; i < L; i += THREADS) dst[i] = sm[tswz(i)];
+    }
+    if (pg.counts && rank == 0 && tid == 0) {
+      pg.counts[0] = n1q;
+      pg.counts[1] = nnq;
+      pg.counts[2] = nmeas;
     }
     sync_all(true);
     if (rank == 0 && tid == 0) atomicAdd(P.queue + 2, ~0ULL);
@@ -895,10 +929,17 @@ void encode_gateop(Encoded& e, const GateOp& g, TOp t) {
   e.ops.push_back(t);
 }
 
-// The fused shot program (fuse_program) as device ops, appended to e.
+// The shot program (fuse_program), or with DQ_SEM_SIMULATE the instructions one
+// by one, as device ops, appended to e.
 int encode_program(const dq_inst* prog, uint64_t ninst, uint32_t n, uint32_t cond_base,
-                   Encoded& e) {
-  const std::vector<FusedEntry> fused = fuse_program(prog, ninst, n);
+                   Encoded& e, int semantics = DQ_SEM_SHOTS) {
+  std::vector<FusedEntry> fused;
+  if (semantics == DQ_SEM_SHOTS) {
+    fused = fuse_program(prog, ninst, n);
+  } else {
+    fused.resize(ninst);
+    for (uint64_t i = 0; i < ninst; ++i) fused[i].inst = (int64_t)i;
+  }
   for (const FusedEntry& f : fused) {
     if (f.inst < 0) {
       GateOp g;
@@ -911,7 +952,11 @@ int encode_program(const dq_inst* prog, uint64_t ninst, uint32_t n, uint32_t con
     t.cond_first += cond_base;
     switch (in.kind) {
       case DQ_ID: case DQ_U0: case DQ_BARRIER: case DQ_CLASSICAL: case DQ_G_NOOP:
+        continue;
       case DQ_G_OPAQUE:  // a no-op in the shot path (run_instruction_par)
+        if (semantics == DQ_SEM_SHOTS) continue;
+        t.type = T_FAIL;
+        e.ops.push_back(t);
         continue;
       case DQ_G_UNSUPPORTED:
         t.type = T_FAIL;
@@ -933,6 +978,7 @@ int encode_program(const dq_inst* prog, uint64_t ninst, uint32_t n, uint32_t con
     }
     GateOp g;
     if (!inst_to_op(in, g)) return fail(DQ_ERR_INTERNAL, "instruction kind without a matrix");
+    if (gate_qubit_count(in.kind) != 1) t.remote = kOpMulti;
     encode_gateop(e, g, t);
   }
   return DQ_OK;
@@ -949,10 +995,10 @@ void mark_remote(TOp* ops, size_t count, uint32_t lb) {
       case T_DENSE:
         for (uint32_t b = 0; b < t.k; ++b) touched |= 1ULL << t.q[b];
         break;
-      case T_MEASURE: case T_RESET: t.remote = 1; continue;
+      case T_MEASURE: case T_RESET: t.remote |= 1u; continue;
       default: break;
     }
-    t.remote = (touched & ~lmask) ? 1u : 0u;
+    t.remote = (t.remote & kOpMulti) | ((touched & ~lmask) ? 1u : 0u);
   }
 }
 
@@ -965,7 +1011,7 @@ std::vector<TOp> group_phases(const std::vector<TOp>& ops, uint32_t lb) {
   const uint64_t lmask = (1ULL << lb) - 1;
   auto bits_of = [](const TOp& t) { return t.ctrl | (1ULL << t.t1); };
   auto eligible = [&](const TOp& t) {
-    return (t.type == T_ONEQ || t.type == T_XPERM) && t.cond_count == 0 && !t.remote &&
+    return (t.type == T_ONEQ || t.type == T_XPERM) && t.cond_count == 0 && !(t.remote & 1u) &&
            (bits_of(t) & ~lmask) == 0;
   };
   size_t i = 0;
@@ -1231,6 +1277,16 @@ size_t traj_smem(const LaunchSet& ls) {
                                            sizeof(int32_t) * std::max<uint32_t>(ls.max_ncbits, 1));
 }
 
+// Dynamic shared memory of a launch whose ops, pool and conds are one image of
+// `image` bytes: with the image, when it is small next to the states.
+size_t stage_tables(const LaunchSet& ls, TrajParams& P, size_t image) {
+  const size_t base = (traj_smem(ls) + 15) / 16 * 16;
+  if (ls.hbm_smem || image > 32 * 1024 || base + image > 220 * 1024) return traj_smem(ls);
+  P.stage_bytes = (uint32_t)image;
+  P.stage_at = (uint32_t)base;
+  return base + image;
+}
+
 // Device buffers of one launch, freed on scope exit.
 struct LaunchBuffers {
   TOp* ops = nullptr;
@@ -1401,7 +1457,7 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
   if (shots > 1)
     DQ_TRY(set_shared(b, P, device, ls.progs[0].n, shots, ls.progs[0].ncbits, ndraws, st));
   TrajLaunch L;
-  DQ_TRY(config_traj(threads, ls.C, traj_smem(ls), P.tasks ? shots : P.nitems, &L));
+  DQ_TRY(config_traj(threads, ls.C, stage_tables(ls, P, part[3].off), P.tasks ? shots : P.nitems, &L));
   const uint32_t clusters = L.clusters;
   DQ_CUDA_TRY(cudaEventRecord(b.e0, st));
   DQ_TRY(reset_shared(P, shots, st));
@@ -1455,6 +1511,18 @@ int geometry(uint32_t n, uint32_t max_span, uint32_t force_lb, uint32_t* lb, uin
   return DQ_OK;
 }
 
+// One program on a handle's state in a single launch of one CTA (k_traj): gates,
+// measurements, resets and conditions with the state in shared memory.  Bound by
+// the latency of one op after another; launching every gate and reading every
+// p1 back costs about 3 us a gate and 20 us a measurement instead.
+template <int THREADS>
+cudaError_t launch_small(size_t smem, const TrajParams& P, cudaStream_t st) {
+  const cudaError_t e = cudaFuncSetAttribute(k_traj<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_traj<THREADS><<<1, THREADS, smem, st>>>(P);
+  return cudaGetLastError();
+}
+
 double ms_since(std::chrono::steady_clock::time_point t0) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
@@ -1465,6 +1533,90 @@ void init_stats(dq_traj_stats* s) {
 }
 
 }  // namespace
+}  // namespace dq
+
+namespace dq {
+
+// See dq_handle.cuh.  The handle's state is canonical or a pending basis state.
+int small_run(dq_state_t h, const dq_inst* prog, uint64_t ninst, const dq_cond* conds, uint64_t nconds,
+              uint64_t seed, int32_t* cbits, uint64_t ncbits, int semantics, dq_profile* prof) {
+  Encoded e;
+  DQ_TRY(encode_program(prog, ninst, h->n, 0, e, semantics));
+  mark_remote(e.ops.data(), e.ops.size(), h->n);
+  const std::vector<TOp> ops = group_phases(e.ops, h->n);
+  TProg pg{};
+  pg.nops = (uint32_t)ops.size();
+  pg.n = pg.lb = h->n;
+  pg.ncbits = (uint32_t)ncbits;
+  pg.base_seed = seed;
+  pg.state_out = h->amp;
+  if (h->lazy_basis >= 0) pg.basis = (uint64_t)h->lazy_basis;
+  else pg.state_in = h->amp;
+  const TItem item{0, 1, 0};
+  // one image up: tables, then the words that come back (counters, counts, bits)
+  constexpr size_t kBack = sizeof(unsigned long long) * (kCtrWords + 3);
+  const uint32_t ndraws = std::min<uint32_t>(draws_of(ops.data(), ops.size()), 4096);  // later ones in the kernel
+  const size_t part[6] = {sizeof(TOp) * ops.size(), sizeof(double2) * e.pool.size(), sizeof(dq_cond) * nconds,
+                          sizeof(TProg), sizeof(TItem), sizeof(double) * ndraws};
+  size_t off[7], at = 0;
+  for (int i = 0; i < 6; ++i) {
+    off[i] = at;
+    at += (part[i] + 15) / 16 * 16;
+  }
+  off[6] = at;
+  const size_t back = kBack + sizeof(int32_t) * ncbits, bytes = at + back;
+  DQ_TRY(ensure_query_buffers(h, bytes, bytes));
+  uint8_t* up = static_cast<uint8_t*>(h->q_host);
+  uint8_t* dev = static_cast<uint8_t*>(h->q_dev);
+  unsigned long long* d_ctr = reinterpret_cast<unsigned long long*>(dev + off[6]);
+  pg.counts = d_ctr + kCtrWords;
+  pg.cbits_in = reinterpret_cast<const int32_t*>(dev + off[6] + kBack);
+  const unsigned long long ctr[kCtrWords + 3] = {0, 0, 1, 0, kNotFailed, 0, 0, 0};
+  const void* src[5] = {ops.data(), e.pool.data(), conds, &pg, &item};
+  for (int i = 0; i < 5; ++i)
+    if (part[i]) memcpy(up + off[i], src[i], part[i]);
+  Chacha8Cursor rng;
+  rng.seed(seed);
+  for (uint32_t i = 0; i < ndraws; ++i) reinterpret_cast<double*>(up + off[5])[i] = rng.draw();
+  memcpy(up + off[6], ctr, kBack);
+  if (ncbits) memcpy(up + off[6] + kBack, cbits, sizeof(int32_t) * ncbits);
+  DQ_CUDA_TRY(cudaMemcpyAsync(dev, up, bytes, cudaMemcpyHostToDevice, h->stream));
+  TrajParams P{};
+  P.ops = reinterpret_cast<const TOp*>(dev);
+  P.pool = reinterpret_cast<const double2*>(dev + off[1]);
+  P.conds = reinterpret_cast<const dq_cond*>(dev + off[2]);
+  P.progs = reinterpret_cast<const TProg*>(dev + off[3]);
+  P.items = reinterpret_cast<const TItem*>(dev + off[4]);
+  P.cbits_out = reinterpret_cast<int32_t*>(dev + off[6] + kBack);
+  P.queue = d_ctr;
+  P.boundary = d_ctr + 3;
+  P.failed = reinterpret_cast<long long*>(d_ctr + 4);
+  P.nitems = 1;
+  P.draws = ndraws ? reinterpret_cast<const double*>(dev + off[5]) : nullptr;
+  P.draw_stride = ndraws;
+  LaunchSet ls;
+  ls.max_lb = h->n;
+  ls.max_ncbits = (uint32_t)ncbits;
+  const size_t smem = stage_tables(ls, P, off[3]);
+  DQ_CUDA_TRY(h->n <= 8 ? launch_small<128>(smem, P, h->stream) : launch_small<256>(smem, P, h->stream));
+  h->lazy_basis = -1;  // the kernel writes the state, also up to a failing gate
+  DQ_CUDA_TRY(cudaMemcpyAsync(up + off[6], dev + off[6], back, cudaMemcpyDeviceToHost, h->stream));
+  DQ_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  unsigned long long got[kCtrWords + 3];
+  memcpy(got, up + off[6], kBack);
+  if (ncbits) memcpy(cbits, up + off[6] + kBack, sizeof(int32_t) * ncbits);
+  prof->kernel_launches += 1;
+  prof->boundary_draws += got[3];
+  prof->apply_one_qubit_calls += got[kCtrWords];
+  prof->apply_n_qubit_calls += got[kCtrWords + 1];
+  prof->measure_qubit_calls += got[kCtrWords + 2];
+  if (got[4] != kNotFailed) {
+    prof->failed_inst = (int64_t)(got[4] & ((1ULL << 40) - 1));
+    return fail(DQ_ERR_UNSUPPORTED, "unsupported generic gate");
+  }
+  return DQ_OK;
+}
+
 }  // namespace dq
 
 // A trajectory batch captured once as a CUDA graph (seed upload, counter

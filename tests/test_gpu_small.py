@@ -1,0 +1,86 @@
+"""Small states: whole programs and sampling in one launch each, against the oracle."""
+import numpy as np
+import pytest
+
+import _oracle
+from _circuits import JsonCircuit, cond, g, gate, random_gate
+from dqsim_bosonic_b200 import _native as nat
+from dqsim_bosonic_b200.circuit import decode_circuit_json, encode
+from dqsim_bosonic_b200.statevector import SimulationResult, run_program
+
+pytestmark = pytest.mark.gpu
+
+
+def prog_of(c):
+    return encode(decode_circuit_json(c.model_dump_json()))
+
+
+def mixed(n, depth, seed):
+    rng = np.random.default_rng(seed)
+    insts = []
+    for k in range(depth):
+        r = rng.random()
+        q = int(rng.integers(n))
+        if r < 0.12:
+            insts.append(g("measure", q, int(rng.integers(6))))
+        elif r < 0.18:
+            insts.append(g("reset", q))
+        elif r < 0.3:
+            insts.append(cond(int(rng.integers(5)), 2, int(rng.integers(4)), random_gate(rng, n)))
+        elif r < 0.34 and n > 1:
+            insts.append(g("swap", q, (q + 1) % n))
+        else:
+            insts.append(random_gate(rng, n))
+    return JsonCircuit(n, insts, ncbits=6)
+
+
+# one amplitude per thread and many, the last size that takes the path and the first that
+# does not, programs of one instruction
+@pytest.mark.parametrize("mode", [nat.EXEC_PER_GATE, nat.EXEC_FUSED])
+@pytest.mark.parametrize("n,depth", [(1, 1), (1, 40), (2, 60), (4, 90), (7, 120), (9, 7), (9, 150), (10, 150), (12, 120),
+                                     (13, 60)])
+def test_program_matches_oracle(gpu, n, depth, mode):
+    prog = prog_of(mixed(n, depth, 50 + n))
+    rng = np.random.default_rng(n)
+    v = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    v /= np.linalg.norm(v)
+    for init in (None, v):
+        want, wcb, rc, _ = _oracle.run(prog, 5, init)
+        assert rc == 0
+        st = nat.State(n, 0)
+        if init is not None:
+            st.upload(init)
+        cb, prof = run_program(st, prog, 5, nat.SEM_SIMULATE, mode)
+        assert prof.boundary_draws == 0 and cb.tolist() == wcb.tolist()
+        assert np.max(np.abs(st.download() - want)) < 1e-12
+        executed = prof.apply_one_qubit_calls + prof.apply_n_qubit_calls + prof.measure_qubit_calls
+        assert executed > 0 or depth == 1 or mode == nat.EXEC_FUSED
+
+
+def test_unsupported_gate_stops_the_program(gpu):
+    insts = [g("x", 0), g("h", 1), g("measure", 0, 0), gate("nope", [0]), g("x", 1)]
+    prog = prog_of(JsonCircuit(3, insts, ncbits=1))
+    st = nat.State(3, 0)
+    with pytest.raises(NotImplementedError, match="nope"):
+        run_program(st, prog, 1, nat.SEM_SIMULATE, nat.EXEC_PER_GATE)
+    want = np.zeros(8, dtype=complex)
+    want[1] = want[3] = 1 / np.sqrt(2)  # what came before it was applied
+    assert np.max(np.abs(st.download() - want)) < 1e-15
+
+
+# one block's scan of 2048 entries, its neighbours, sums of several terms, no shots
+@pytest.mark.parametrize("n,k,shots", [(1, 1, 10), (1, 0, 5), (5, 5, 1000), (11, 11, 5000), (12, 12, 300), (11, 5, 257),
+                                       (8, 3, 0), (6, 6, 16385)])
+def test_samples_match_oracle(gpu, n, k, shots):
+    rng = np.random.default_rng(n * 7 + k)
+    v = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    v[rng.random(1 << n) < 0.3] = 0
+    v[0] += 1
+    v /= np.linalg.norm(v)
+    st = nat.State(n, 0)
+    st.upload(v)
+    qs = rng.permutation(n)[:k].tolist()
+    res = SimulationResult(st, n, {}, None)
+    got = res.sample_indices(shots, qs, seed=3)
+    assert res.last_boundary_draws == 0
+    assert got.tolist() == _oracle.sample(v, qs, 3, shots).tolist()
