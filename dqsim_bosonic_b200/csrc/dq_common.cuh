@@ -55,6 +55,18 @@ __device__ __forceinline__ double norm_sqr_x(double2 a) {
   return __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y));
 }
 
+// a / b correctly rounded, given y = 1 / b correctly rounded: two Newton
+// corrections of a y with exact remainders (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990), 5
+// operations instead of a division's sequence when many numbers are divided by
+// one.  Outside the range where the remainders are exact it divides.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  if (!(fabs(a) > 1e-250 && fabs(a) < 1e250)) return a == 0.0 ? a : __ddiv_rn(a, b);
+  double q = a * y;
+  q = fma(fma(-b, q, a), y, q);
+  return fma(fma(-b, q, a), y, q);
+}
+
 // ---- fused-multiply-add complex arithmetic (device) ------------------------
 __device__ __forceinline__ double2 cmul_f(double2 a, double2 b) {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));

@@ -191,6 +191,8 @@ unsigned red_blocks(uint64_t items, int device) {
 
 // ---- collapse / init ------------------------------------------------------------------
 
+// Memory bound with div_by (22 qubits: 23 us with two divisions per amplitude,
+// 13.8 us here).
 __global__ void k_collapse(double2* __restrict__ s, uint64_t count, uint64_t bit, int outcome,
                            double norm) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -200,7 +202,8 @@ __global__ void k_collapse(double2* __restrict__ s, uint64_t count, uint64_t bit
     s[i] = make_double2(0.0, 0.0);
   } else {
     const double2 a = s[i];
-    s[i] = make_double2(__ddiv_rn(a.x, norm), __ddiv_rn(a.y, norm));
+    const double y = __drcp_rn(norm);
+    s[i] = make_double2(div_by(a.x, norm, y), div_by(a.y, norm, y));
   }
 }
 
@@ -227,9 +230,11 @@ struct MargParams {
   uint32_t q[32];     // marginal qubits, q[0] = MSB of j
   Pos32 rest;         // the marginal qubits, ascending (zero bits inserted there)
   uint32_t k;
+  int shift;  // >= 0: the qubits are shift + k - 1, ..., shift, so j deposits as j << shift
 };
 
 __device__ __forceinline__ uint64_t deposit_j(uint64_t j, const MargParams& P) {
+  if (P.shift >= 0) return j << P.shift;
   uint64_t bits = 0;
   for (uint32_t b = 0; b < P.k; ++b) bits |= ((j >> (P.k - 1 - b)) & 1ULL) << P.q[b];
   return bits;
@@ -239,6 +244,7 @@ __device__ __forceinline__ uint64_t deposit_j(uint64_t j, const MargParams& P) {
 __device__ __forceinline__ double marginal_term(const double2* __restrict__ s, uint64_t j, uint64_t nterms,
                                                 const MargParams& P) {
   const uint64_t jb = deposit_j(j, P);
+  if (nterms == 1) return norm_sqr_x(s[jb]);
   double acc = 0.0;
   for (uint64_t r = 0; r < nterms; ++r)
     acc = __dadd_rn(acc, norm_sqr_x(s[insert_zeros(r, P.rest.p, P.rest.np) | jb]));
@@ -637,6 +643,9 @@ MargPlan plan_marginal(uint32_t n, const uint32_t* qubits, uint32_t k, int devic
     mask |= 1ULL << qubits[b];
   }
   m.P.k = k;
+  m.P.shift = k ? (int)qubits[k - 1] : 0;
+  for (uint32_t b = 0; b < k; ++b)
+    if (qubits[b] != (uint32_t)m.P.shift + k - 1 - b) m.P.shift = -1;
   m.P.rest.np = 0;
   for (uint32_t b = 0; b < 64 && m.P.rest.np < 32; ++b)
     if (mask >> b & 1ULL) m.P.rest.p[m.P.rest.np++] = b;

@@ -402,13 +402,14 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
     auto collapse = [&](const TOp& op, int o, double norm) {
       const uint32_t q = op.t1;
       const uint64_t qb = 1ULL << q;
+      const double y = __drcp_rn(norm);
       for (uint32_t i = tid; i < L; i += THREADS) {
         const bool set = ((gbase | i) & qb) != 0;
         if (set != (o == 1)) {
           sm[tswz(i)] = make_double2(0.0, 0.0);
         } else {
           const double2 a = sm[tswz(i)];
-          sm[tswz(i)] = make_double2(__ddiv_rn(a.x, norm), __ddiv_rn(a.y, norm));
+          sm[tswz(i)] = make_double2(div_by(a.x, norm, y), div_by(a.y, norm, y));
         }
       }
       if (op.type == T_RESET && o == 1) {

@@ -84,3 +84,26 @@ def test_samples_match_oracle(gpu, n, k, shots):
     got = res.sample_indices(shots, qs, seed=3)
     assert res.last_boundary_draws == 0
     assert got.tolist() == _oracle.sample(v, qs, 3, shots).tolist()
+
+
+# the collapse divides by multiplying and correcting: every result equals the division, for
+# zeros, numbers near the ends of the range, and norms that are not representable sums
+@pytest.mark.parametrize("n", [1, 5, 14])
+@pytest.mark.parametrize("p1", [0.5, 1 / 3, 1e-14, 0.9999999, 1.0])
+@pytest.mark.parametrize("outcome", [0, 1])
+def test_collapse_is_a_division(gpu, n, p1, outcome):
+    rng = np.random.default_rng(n)
+    v = (rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)) * 2.0 ** rng.integers(-60, 3, size=1 << n)
+    v.real[rng.random(1 << n) < 0.1] = -0.0
+    v[rng.random(1 << n) < 0.05] = 1e-308 + 5e-324j
+    v[rng.random(1 << n) < 0.05] = 1e-251 - 1e280j
+    st = nat.State(n, 0)
+    st.upload(v)
+    q = n // 2
+    nat.check(nat.lib().dq_collapse(st.handle, q, outcome, p1))
+    norm = max(np.sqrt(p1 if outcome else max(1.0 - p1, 0.0)), 1e-15)
+    keep = ((np.arange(1 << n) >> q) & 1) == outcome
+    want = np.where(keep, v.real / norm, 0.0) + 1j * np.where(keep, v.imag / norm, 0.0)
+    got = st.download()
+    assert got.tobytes() == want.tobytes() or (
+        np.array_equal(got.real, want.real) and np.array_equal(got.imag, want.imag))
