@@ -211,6 +211,14 @@ inline hx operator*(hx a, hx b) { return hx{a.re * b.re - a.im * b.im, a.re * b.
 inline hx conj(hx a) { return hx{a.re, -a.im}; }
 inline bool is_one_hc(hx a) { return a.re == 1.0L && a.im == 0.0L; }
 inline hc rounded(hx a) { return hc{(double)a.re, (double)a.im}; }
+// A diagonal entry (rounded to double) as a factor of a polynomial.  X and CX
+// turn factors into their inverses, taken as conjugates: they have to be of
+// modulus one beyond double (or the 2-norm drifts with every such turn).
+inline void factor_of(hc z, hc* out) { *out = z; }
+inline void factor_of(hc z, hx* out) {
+  const long double a = z.re, b = z.im, r = sqrtl(a * a + b * b);
+  *out = hx{a / r, b / r};
+}
 
 template <class C>
 struct PolyT {
@@ -242,7 +250,11 @@ struct PolyT {
     if (!hq[k]) { hq[k] = 1; ++cnt[lo]; ++cnt[hi]; quad[k] = w; } else quad[k] = quad[k] * w;
   }
   void add(const PGate& g) {
-    auto up = [](hc z) { return C{z.re, z.im}; };
+    auto up = [](hc z) {
+      C w;
+      factor_of(z, &w);
+      return w;
+    };
     if (!(g.cst.re == 1.0 && g.cst.im == 0.0)) { cst = cst * up(g.cst); has_cst = true; }
     for (int i = 0; i < g.nlin; ++i) mul_lin(g.lq[i], up(g.lw[i]));
     if (g.quad) mul_quad(g.qa, g.qb, up(g.qw));

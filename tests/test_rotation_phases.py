@@ -79,3 +79,24 @@ def test_kernel(gpu, n, depth, seed, special, cost):
     st.reset()
     run_program(st, prog, 0, nat.SEM_SIMULATE, nat.EXEC_FUSED, 0, False, False, cost)
     assert np.max(np.abs(st.download() - _oracle.run(prog, 0)[0])) < ATOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [11, 14])
+def test_norm_does_not_drift(gpu, n):
+    # 16 n gates that each round the 2-norm by about eps: independent, they add to
+    # 4 sqrt(n) eps (root mean square over circuits); factors a little off modulus one
+    # that pile up would be several times that
+    drift = []
+    for seed in range(10):
+        rng = np.random.default_rng(seed)
+        insts = []
+        for layer in range(8):
+            insts += [g("rx" if layer % 2 else "ry", q, float(rng.uniform(-math.pi, math.pi))) for q in range(n)]
+            insts += [g("rzz", q, (q + 1) % n, float(rng.uniform(-math.pi, math.pi))) for q in range(n)]
+        prog = encode(decode_circuit_json(JsonCircuit(n, insts).model_dump_json()))
+        st = nat.State(n, 0)
+        run_program(st, prog, 0, nat.SEM_SIMULATE, nat.EXEC_FUSED, 0, False, False, 0)
+        v = np.asarray(st.download()).astype(np.clongdouble)
+        drift.append(float(np.vdot(v, v).real - 1))
+    assert np.sqrt(np.mean(np.square(drift))) < 4 * math.sqrt(n) * np.finfo(float).eps
