@@ -19,21 +19,27 @@
 //           (controlled gates with a non-local control: variant 0 = I).
 //   A_TWO   dense 4x4 on two local qubits (rxx, swap-like, psi+-, phi+).
 //   A_DIAG  diagonal on up to two qubits, local or not, applied elementwise.
-//   A_DRUN  header of a run of 4..64 A_DIAG ops applied in one pass: their
-//           gradients from a Walsh-Hadamard transform of conj(lambda) psi,
-//           their phases as one quadratic phase polynomial (op_drun).
-//   A_PHASE header of 2..16 uncontrolled one-qubit ops on three local bits,
-//           applied to 8 amplitudes held in registers per thread (op_phase).
+//   A_PASS  header of a register pass: a thread holds the 8 amplitudes of psi
+//           and lambda that differ in three local bits, applies a run of
+//           diagonal gates on any qubits (diag_grads, diag_apply), then up to
+//           three rotations of one form on those bits (pass_tan).
+//   A_PHASE header of 1..16 other uncontrolled one-qubit ops on three local
+//           bits, applied to registers in order (op_phase).
+// A sweep that ends with a pass writes its results straight to memory and
+// loads the next tile into the freed buffer meanwhile.
 // Gradient terms: Re sum conj(lambda_k) (D_j psi_{k-1}) with psi_{k-1} = V psi_k,
 // summed per thread, reduced per warp into shared slots [slot][warp], per CTA
 // in warp order, and over CTAs in CTA order by k_adj_slots: deterministic for
 // a fixed grid.
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stddef.h>
 #include <stdint.h>
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -54,14 +60,16 @@ constexpr uint32_t kALoMin = 3;  // qubits 0..2 stay local: 128-byte runs per ti
 constexpr uint32_t kAMaxOps = 192;
 constexpr uint32_t kAMaxSlots = 192;
 
-enum AType : uint8_t { A_ONE = 1, A_TWO = 2, A_DIAG = 3, A_DRUN = 4, A_PHASE = 5 };
+enum AType : uint8_t { A_ONE = 1, A_TWO = 2, A_DIAG = 3, A_PASS = 4, A_PHASE = 5 };
 constexpr uint32_t kAPhaseOps = 16;  // ops of one register phase
 constexpr uint32_t kAPhaseStage = 32;  // phase ops of a sweep staged once per CTA, at most
-constexpr uint32_t kAMaxSweepOps = 2 * kAMaxOps;  // ops of a sweep, run and phase headers included
-constexpr uint32_t kADiagRun = 64;  // diagonal ops applied in one elementwise pass
-constexpr uint32_t kADiagRunMin = 4;  // shorter runs stay single A_DIAG ops
+constexpr uint32_t kAMaxSweepOps = 2 * kAMaxOps;  // ops of a sweep, pass headers included
+// shared memory of a sweep (bytes) up to which two CTAs share an SM; phase
+// tables are staged while it is kept
+constexpr size_t kATwoCtas = 108 * 1024;
+constexpr uint32_t kATabTiles = 8;  // tiles of a state from which tables are staged
 
-struct AOp {
+struct alignas(8) AOp {
   uint8_t type;
   uint8_t np;        // derivative matrices (gradient slots) of the op
   uint8_t lt, lt2;   // A_ONE: local target bit; A_TWO: local bits of the 4x4 MSB / LSB
@@ -69,14 +77,20 @@ struct AOp {
   uint8_t skip0;     // A_ONE with selector: variant 0 is the identity with no derivatives
   uint8_t dq[2];     // A_DIAG: qubit encodings (bit 7: local; low 7 bits: local bit or global position)
   uint8_t ndq;       // A_DIAG: 1 or 2 qubits (dq[0] = MSB of the diagonal index)
-  uint8_t cnt;       // A_DRUN / A_PHASE: number of ops that follow it
+  uint8_t cnt;       // A_PASS, A_PHASE: number of one-qubit ops that follow it; A_ONE in one: 1 + its TanForm
   uint8_t pad[2];
-  uint32_t lctrl;    // A_ONE: local control mask (tile offset bits); A_DIAG: run record (pool offset);
-                     // A_DRUN: how many of its ops touch a local qubit (those come first)
-  uint32_t slot;     // first sweep-local gradient slot
-  uint32_t mat;      // offset of the op's matrices in the pool (double2 units)
+  uint32_t lctrl;    // A_ONE: local control mask (tile offset bits), its TanForm record (pool offset);
+                     // A_PASS, A_PHASE: its first PSub
+  uint32_t slot;     // first sweep-local gradient slot; A_PASS: its diagonal run's record in the blob
+  uint32_t mat;      // offset of the op's matrices in the pool (double2 units); A_PASS, A_PHASE:
+                     // factor of both vectors after its ops (pool offset, kNone: 1)
 };
-static_assert(sizeof(AOp) == 24, "AOp layout");
+// A_PASS, A_PHASE: lt, lt2, dq[0]: its register bits.  A_PASS: np: its diagonal
+// run has gradient terms; ndq: it has a diagonal run; dq[1]: that run's index;
+// pad[0]: its rotations' form (0: none)
+constexpr uint32_t kNone = 0xffffffffu;
+static_assert(sizeof(AOp) == 24 && offsetof(AOp, dq) == 6 && offsetof(AOp, ndq) == 8 && offsetof(AOp, lctrl) == 12,
+              "AOp layout (passes read it as words)");
 
 struct ASweepHdr {
   uint32_t n, m, nops, nslots;
@@ -85,8 +99,10 @@ struct ASweepHdr {
   uint32_t npos_cnt;
   uint32_t npos[64];          // non-local bit positions, ascending
   uint32_t phase_ops;         // > 0: every register phase's op data is staged once per CTA
-                              // (phase header lctrl = its first PSub); 0: staged per tile
-  uint32_t pad;
+                              // (pass header lctrl = its first PSub); 0: staged per tile
+  uint32_t direct;            // the last op is a pass that writes to memory itself
+  uint32_t blob0, nblob;      // diagonal runs' records: pool offset and length (double2 units)
+  uint32_t ndrun, ntab;       // diagonal runs, and how many keep phase tables
 };
 
 // One sweep of one (psi, lambda) pair in a multi-job launch.
@@ -144,11 +160,11 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 
 template <int NP>
 __device__ __forceinline__ void flush_acc(const double (&acc)[4], double* accw, uint32_t slot) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
     const double v = warp_sum_d(acc[j]);
-    if (lane == 0) accw[(slot + j) * kAWarps + w] += v;
+    if (lane == 0) accw[slot + j] += v;
   }
 }
 
@@ -289,209 +305,188 @@ __device__ __noinline__ void op_diag(double2* sp, double2* sl, const AOp& op, co
   flush_acc<NP>(acc, accw, op.slot);
 }
 
-// One diagonal op of a run, staged in shared memory for the current tile.
-// The op's diagonal V over its entry index e = 2 b0 + b1 (b0: the MSB qubit;
-// a one-qubit op has b1 = 0) has modulus one, so it is exp(i theta(b0, b1))
-// with theta = al + be b0 + ga b1 + de b0 b1.  For this tile each qubit bit
-// is a constant (non-local qubit, or absent), a bit of threadIdx.x, or one
-// of the three register bits of the run's element layout (o = tid + 256 i).
-struct DRec {
-  double al, be, ga, de;
-  uint32_t k0, k1;  // 0: constant, 1: thread bit, 2: register bit
-  uint32_t p0, p1;  // constant value / bit of threadIdx.x / register bit
+// ---- runs of diagonal gates ----
+//
+// Every diagonal gate is exp(i theta(b0, b1)), so a run of them is one phase
+// exp(i Theta(x)) with Theta a quadratic polynomial in the index bits.  Each
+// bit is a register bit of the pass, a bit of threadIdx.x or a bit of the
+// tile's base.  Theta splits into
+//   - local linear and quadratic terms: per thread a factor and one factor per
+//     register bit (pair_factors), the same for every tile: kept in a table in
+//     shared memory where there are tiles and room enough;
+//   - terms with base bits: a constant and a factor per coupled local bit,
+//     a dozen numbers a tile, made by one warp while the tile is loaded.
+// An element's phase is a product of these: 4 sincos a thread and tile without
+// the table and none with it, where a sincos per element of a summed angle
+// took 8 (and rounded the sum of all angles).
+//
+// Gradients.  The entries have modulus one, so conj(lambda) psi is the same
+// before every gate of the run, and dU U^dagger = i g with g real: a term is a
+// sum of at most four Walsh coefficients of z = Im(conj(lambda) psi), its g in
+// the Walsh basis of its two bits.  A warp transforms its 256 values over the
+// three register bits and the five lane bits (each lane bit is first exchanged
+// with a register bit: 40 shuffles a thread against 160 for butterflies on the
+// complex product), then lane j adds term j to its warp's slot.
+struct DTerm {
+  double w;
+  uint32_t code;  // source lane : 5, warp bits : 3, register : 3, two base bits : 6 each (63: none),
+                  // registers that its 32 terms use : 8
+  uint32_t slot;  // kNone: padding
 };
+struct DAng {
+  double ang;
+  uint32_t code;
+  uint32_t pad;
+};
+// A run's record in the blob (double2 units): 0: (constant angle, factor of
+// both vectors); 1..3: exp(i H01), exp(i H02), exp(i H12) of the register
+// pairs; 4: counts; 5: masks and table; then its terms and angle lists.
+struct DCount {
+  uint32_t nterm;  // a multiple of 32 but for the last terms of a run
+  uint32_t ends;   // local angles: cumulative ends of the lists of T, G0, G1, G2 (a byte each)
+  uint32_t ncst, nlin;
+};
+struct DMask {
+  uint32_t coupled;  // thread bits 0..7, register bits 8..10 with terms in base bits
+  uint32_t pairs;    // register pairs 01, 02, 12 with a term
+  uint32_t tab, pad;
+};
+constexpr uint32_t kDRunHdr = 6, kDFactors = 12;
 
-__device__ __forceinline__ void drec_stage(DRec& D, const AOp& op, const double2* pool, uint64_t base) {
-  const double2* rec = pool + op.lctrl;
-  D.al = rec[0].x;
-  D.be = rec[0].y;
-  D.ga = rec[1].x;
-  D.de = rec[1].y;
-  uint32_t k[2] = {0, 0}, p[2] = {0, 0};
-  for (uint32_t a = 0; a < op.ndq; ++a) {
-    const uint32_t e = op.dq[a];
-    if (e & 0x80u) {
-      const uint32_t bp = e & 0x7fu;
-      k[a] = bp >= 8 ? 2u : 1u;
-      p[a] = bp >= 8 ? bp - 8 : bp;
-    } else {
-      p[a] = (uint32_t)((base >> (e & 0x7fu)) & 1ULL);
-    }
-  }
-  D.k0 = k[0]; D.k1 = k[1];
-  D.p0 = p[0]; D.p1 = p[1];
+__device__ __forceinline__ double2 expi(double a) {
+  double sn, cs;
+  sincos(a, &sn, &cs);
+  return make_double2(cs, sn);
 }
 
-__device__ __forceinline__ void gadd(double& g0, double& g1, double& g2, uint32_t r, double v) {
-  if (r == 0) g0 += v;
-  else if (r == 1) g1 += v;
-  else g2 += v;
+__device__ __forceinline__ void pair_factors(const double2* B, double2 (&f)[4]) {
+  const DCount& C = *reinterpret_cast<const DCount*>(B + 4);
+  const DAng* L = reinterpret_cast<const DAng*>(B + kDRunHdr + C.nterm);
+  uint32_t j = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t e = (C.ends >> (8 * k)) & 0xffu;
+    double x = 0.0;
+    for (; j < e; ++j)
+      if ((threadIdx.x & L[j].code) == L[j].code) x += L[j].ang;
+    f[k] = expi(x);
+  }
 }
 
-// A run of diagonal ops in one elementwise pass.  Every diagonal entry has
-// modulus one, so z = conj(lambda) psi is the same before every op of the
-// run and op k's gradient term is
-//   Re sum_x z_x w_k[e_k(x)],   w_k = V_k dU_k  (entrywise).
-// Expanding w_k in the Walsh basis of its two index bits,
-//   w_k[2 b0 + b1] = sum_S what_k[S] (-1)^(b0 S0 + b1 S1),
-// turns the sum into four Walsh-Hadamard coefficients of z: a warp takes the
-// transform of its own 256 elements over the 8 bits that vary inside it
-// (3 register bits, 5 lane bits; the 3 warp bits and non-local bits are
-// constants that give a sign), after which each lane serves one op.  The run's
-// total phase is exp(i theta(x)) with theta a quadratic polynomial in the
-// index bits: each thread folds the ops into its constant, the linear terms of
-// its three register bits and their pairwise products, and one sincos per
-// element applies it to psi and lambda.  The host writes per op
-// rec[0] = (al, be), rec[1] = (ga, de), rec[2 + S] = what[S] at pool + lctrl.
-__device__ __noinline__ void op_drun(double2* sp, double2* sl, const AOp& hdr, const AOp* sub,
-                                     const double2* pool, uint32_t m, uint64_t base, double* accw,
-                                     DRec* ds) {
-  const uint32_t cnt = hdr.cnt, nloc = hdr.lctrl;  // ops [nloc, cnt) touch non-local qubits only
-  __shared__ double s_tconst;
-  for (uint32_t j = threadIdx.x; j < cnt; j += kAThreads) drec_stage(ds[j], sub[j], pool, base);
-  __syncthreads();
-  const uint32_t L = 1u << m;
-  const uint32_t tid = threadIdx.x;
-  const int lane = tid & 31, w = tid >> 5;
-  // the tile-constant phase of the ops on non-local qubits: one warp, lanes
-  // over the ops, a fixed-order butterfly (read after the barrier below)
-  if (w == 0) {
-    double t = 0.0;
-    for (uint32_t u = nloc + (uint32_t)lane; u < cnt; u += 32) {
-      const DRec& D = ds[u];
-      t += D.al + (D.p0 ? D.be : 0.0) + (D.p1 ? D.ga : 0.0) + ((D.p0 && D.p1) ? D.de : 0.0);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) s_tconst = t;
+// The factors of a run that depend on the tile: E[0..10] per local bit code,
+// E[11] the constant (one warp).
+__device__ __forceinline__ void tile_factors(const double2* B, uint64_t base, double2* E) {
+  const uint32_t lane = threadIdx.x & 31;
+  const DCount& C = *reinterpret_cast<const DCount*>(B + 4);
+  const DAng* cst = reinterpret_cast<const DAng*>(B + kDRunHdr + C.nterm + (C.ends >> 24));
+  const DAng* lin = cst + C.ncst;
+  double c = 0.0;
+  for (uint32_t j = lane; j < C.ncst; j += 32) {
+    const uint32_t p = cst[j].code & 63u, q = (cst[j].code >> 6) & 63u;
+    if ((base >> p & 1ULL) && (q == 63u || (base >> q & 1ULL))) c += cst[j].ang;
   }
-  if (hdr.np) {
-    double2 z[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const uint32_t o = tid + (uint32_t)i * kAThreads;
-      double2 zz = make_double2(0.0, 0.0);
-      if (o < L) {
-        const uint32_t so = swz(o);
-        const double2 a = sp[so], b = sl[so];
-        zz = make_double2(fma(b.x, a.x, b.y * a.y), fma(b.x, a.y, -b.y * a.x));
-      }
-      z[i] = zz;
-    }
-    // Walsh-Hadamard transform over the register bits, then the lane bits:
-    // afterwards lane l, register r holds sum_x z_x (-1)^popc(x & M) over the
-    // warp's elements, M = l | r << 8
-#pragma unroll
-    for (int s = 1; s < 8; s <<= 1)
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (!(i & s)) {
-          const double2 u = z[i], v = z[i | s];
-          z[i] = make_double2(u.x + v.x, u.y + v.y);
-          z[i | s] = make_double2(u.x - v.x, u.y - v.y);
-        }
-#pragma unroll
-    for (int s = 1; s < 32; s <<= 1) {
-      const bool up = (lane & s) != 0;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const double px = __shfl_xor_sync(0xffffffffu, z[i].x, s);
-        const double py = __shfl_xor_sync(0xffffffffu, z[i].y, s);
-        z[i] = up ? make_double2(px - z[i].x, py - z[i].y) : make_double2(z[i].x + px, z[i].y + py);
-      }
-    }
-    for (uint32_t c0 = 0; c0 < cnt; c0 += 32) {
-      const uint32_t j = c0 + (uint32_t)lane;
-      double contrib = 0.0;
-      uint32_t slot = 0xffffffffu;
-      uint32_t src[4] = {0, 0, 0, 0}, reg[4] = {0, 0, 0, 0};
-      double2 wh[4];
-      if (j < cnt && sub[j].np) {
-        const AOp op = sub[j];
-        const DRec& D = ds[j];
-        slot = op.slot;
-        const double2* rec = pool + op.lctrl;
-        uint32_t lm[2], rm[2], cv[2];
-        const uint32_t kk[2] = {D.k0, D.k1}, pp[2] = {D.p0, D.p1};
-#pragma unroll
-        for (int a = 0; a < 2; ++a) {
-          lm[a] = (kk[a] == 1 && pp[a] < 5) ? 1u << pp[a] : 0u;
-          rm[a] = kk[a] == 2 ? 1u << pp[a] : 0u;
-          cv[a] = kk[a] == 0 ? pp[a] : ((kk[a] == 1 && pp[a] >= 5) ? (tid >> pp[a]) & 1u : 0u);
-        }
-#pragma unroll
-        for (int S = 0; S < 4; ++S) {
-          const uint32_t s0 = (uint32_t)S >> 1, s1 = (uint32_t)S & 1u;
-          double2 v = rec[2 + S];
-          if ((s0 & cv[0]) ^ (s1 & cv[1])) v = make_double2(-v.x, -v.y);
-          wh[S] = v;
-          src[S] = (s0 ? lm[0] : 0u) | (s1 ? lm[1] : 0u);
-          reg[S] = (s0 ? rm[0] : 0u) | (s1 ? rm[1] : 0u);
-        }
-      } else {
-#pragma unroll
-        for (int S = 0; S < 4; ++S) wh[S] = make_double2(0.0, 0.0);
-      }
-#pragma unroll
-      for (int S = 0; S < 4; ++S) {
-        double2 pz = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const double px = __shfl_sync(0xffffffffu, z[r].x, (int)src[S]);
-          const double py = __shfl_sync(0xffffffffu, z[r].y, (int)src[S]);
-          if (reg[S] == (uint32_t)r) pz = make_double2(px, py);
-        }
-        contrib = fma(wh[S].x, pz.x, fma(-wh[S].y, pz.y, contrib));
-      }
-      // every gate of a sweep has slots of its own, so each lane adds its
-      // op's term to the warp's slot directly (one writer per slot and warp)
-      if (slot != 0xffffffffu) accw[slot * kAWarps + w] += contrib;
-    }
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  double x = lane == 11 ? B[0].x + c : 0.0;
+  for (uint32_t j = 0; j < C.nlin; ++j)
+    if ((lin[j].code & 15u) == lane && (base >> (lin[j].code >> 4) & 1ULL)) x += lin[j].ang;
+  if (lane < kDFactors) {
+    double2 e = expi(x);
+    if (lane == 11) e = make_double2(e.x * B[0].y, e.y * B[0].y);
+    E[lane] = e;
   }
-  // the run's phase polynomial for this thread's eight elements (the ops on a
-  // local qubit; the others' constant comes from warp 0)
-  double T = 0.0, G0 = 0.0, G1 = 0.0, G2 = 0.0, H01 = 0.0, H02 = 0.0, H12 = 0.0;
-#pragma unroll 2
-  for (uint32_t u = 0; u < nloc; ++u) {
-    const DRec& D = ds[u];
-    const bool r0 = D.k0 == 2, r1 = D.k1 == 2;
-    const bool c0 = D.k0 == 1 ? ((tid >> D.p0) & 1u) != 0 : D.p0 != 0;
-    const bool c1 = D.k1 == 1 ? ((tid >> D.p1) & 1u) != 0 : D.p1 != 0;
-    if (!r0 && !r1) {
-      T += D.al + (c0 ? D.be : 0.0) + (c1 ? D.ga : 0.0) + ((c0 && c1) ? D.de : 0.0);
-    } else if (r0 && !r1) {
-      T += D.al + (c1 ? D.ga : 0.0);
-      gadd(G0, G1, G2, D.p0, D.be + (c1 ? D.de : 0.0));
-    } else if (!r0 && r1) {
-      T += D.al + (c0 ? D.be : 0.0);
-      gadd(G0, G1, G2, D.p1, D.ga + (c0 ? D.de : 0.0));
-    } else {
-      T += D.al;
-      gadd(G0, G1, G2, D.p0, D.be);
-      gadd(G0, G1, G2, D.p1, D.ga);
-      gadd(H01, H02, H12, D.p0 + D.p1 - 1u, D.de);
-    }
-  }
-  __syncthreads();
-  T += s_tconst;
+}
+
+// Exchanges register bit KB with lane bit LB, then the butterfly on it.
+template <int KB, int LB>
+__device__ __forceinline__ void walsh_lane(double (&z)[8], int lane) {
+  const bool up = (lane >> LB) & 1;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t o = tid + (uint32_t)i * kAThreads;
-    if (o < L) {
-      double ang = T;
-      if (i & 1) ang += G0;
-      if (i & 2) ang += G1;
-      if (i & 4) ang += G2;
-      if ((i & 3) == 3) ang += H01;
-      if ((i & 5) == 5) ang += H02;
-      if ((i & 6) == 6) ang += H12;
-      double sn, cs;
-      sincos(ang, &sn, &cs);
-      const double2 ph = make_double2(cs, sn);
-      const uint32_t so = swz(o);
-      sp[so] = cmul2(ph, sp[so]);
-      sl[so] = cmul2(ph, sl[so]);
+  for (int i = 0; i < 8; ++i)
+    if (!(i >> KB & 1)) {
+      const int k = i | (1 << KB);
+      const double r = __shfl_xor_sync(0xffffffffu, up ? z[i] : z[k], 1 << LB);
+      const double kept = up ? z[k] : z[i], d = kept - r;
+      z[i] = kept + r;
+      z[k] = up ? -d : d;
     }
+}
+
+__device__ __forceinline__ void diag_grads(const double2 (&a)[8], const double2 (&b)[8], const double2* B,
+                                           uint64_t base, bool valid, double* accw) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t w = threadIdx.x >> 5;
+  const uint32_t nterm = reinterpret_cast<const DCount*>(B + 4)->nterm;
+  const DTerm* terms = reinterpret_cast<const DTerm*>(B + kDRunHdr);
+  double z[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) z[i] = valid ? fma(b[i].x, a[i].y, -b[i].y * a[i].x) : 0.0;
+#pragma unroll
+  for (int s = 1; s < 8; s <<= 1)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (!(i & s)) {
+        const double u = z[i], v = z[i | s];
+        z[i] = u + v;
+        z[i | s] = u - v;
+      }
+  walsh_lane<0, 0>(z, lane);
+  walsh_lane<1, 1>(z, lane);
+  walsh_lane<2, 2>(z, lane);
+  walsh_lane<0, 3>(z, lane);
+  walsh_lane<1, 4>(z, lane);
+  // the coefficient of register mask R, lane mask M is now in lane
+  // R | (M & 3) << 3, register M3 | M4 << 1 | M2 << 2
+  for (uint32_t c0 = 0; c0 < nterm; c0 += 32) {
+    const uint32_t j = min(c0 + (uint32_t)lane, nterm - 1u);
+    const DTerm t = terms[j];
+    const uint32_t used = t.code >> 23, reg = (t.code >> 8) & 7u;
+    double v = 0.0;
+#pragma unroll
+    for (uint32_t r = 0; r < 8; ++r)
+      if (used >> r & 1u) {
+        const double x = __shfl_sync(0xffffffffu, z[r], (int)(t.code & 31u));
+        if (reg == r) v = x;
+      }
+    const uint32_t p = (t.code >> 11) & 63u, q = (t.code >> 17) & 63u;
+    const uint32_t neg = __popc((t.code >> 5) & w & 7u) + (p != 63u ? (uint32_t)(base >> p) & 1u : 0u) +
+                         (q != 63u ? (uint32_t)(base >> q) & 1u : 0u);
+    if (c0 + (uint32_t)lane < nterm && t.slot != kNone) accw[t.slot] += (neg & 1u) ? -t.w * v : t.w * v;
+  }
+}
+
+__device__ __forceinline__ void diag_apply(double2 (&a)[8], double2 (&b)[8], const double2* B, const double2* E,
+                                           const double2* tabs) {
+  const DMask M = *reinterpret_cast<const DMask*>(B + 5);
+  double2 f[4];
+  if (M.tab != kNone) {
+    const double2* tb = tabs + (size_t)M.tab * 4 * kAThreads + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) f[k] = tb[k * kAThreads];
+  } else {
+    pair_factors(B, f);
+  }
+  f[0] = cmul2(f[0], E[11]);
+#pragma unroll 1
+  for (uint32_t c = M.coupled & 0xffu; c; c &= c - 1) {
+    const uint32_t r = __ffs(c) - 1;
+    if (threadIdx.x >> r & 1u) f[0] = cmul2(f[0], E[r]);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (M.coupled >> (8 + k) & 1u) f[k + 1] = cmul2(f[k + 1], E[8 + k]);
+  double2 h[4] = {f[0], cmul2(f[0], f[1]), cmul2(f[0], f[2]), make_double2(0.0, 0.0)};
+  h[3] = cmul2(h[1], f[2]);
+  if (M.pairs & 1u) h[3] = cmul2(h[3], B[1]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    a[i] = cmul2(h[i], a[i]);
+    b[i] = cmul2(h[i], b[i]);
+    double2 g = cmul2(h[i], f[3]);
+    if ((i & 1) && (M.pairs & 2u)) g = cmul2(g, B[2]);
+    if ((i & 2) && (M.pairs & 4u)) g = cmul2(g, B[3]);
+    a[i | 4] = cmul2(g, a[i | 4]);
+    b[i | 4] = cmul2(g, b[i | 4]);
   }
 }
 
@@ -500,7 +495,8 @@ struct PSub {
   double2 v[4];      // U^dagger
   double2 d[4][4];   // np derivatives in the form D' = dU U^dagger (applied to psi before V)
   uint32_t pb;       // index of the target among the phase bits
-  uint32_t vk;       // 0: general V; 1: real V; 2: real diagonal, imaginary off-diagonal
+  uint32_t vk;       // 0: general V; 1: real V; 2: real diagonal, imaginary off-diagonal;
+                     // 3 + TanForm: v[0] = (t, gradient weight)
   uint32_t np, slot;
   uint32_t tm[4];    // per derivative: bit 2e / 2e + 1 set if Re / Im of D'[e] is non-zero
 };
@@ -577,50 +573,79 @@ __device__ __forceinline__ void phase_one(double2 (&a)[8], double2 (&b)[8], cons
   }
 }
 
-// One op of a straight-line phase on register bit PB: its gradient term from
-// the amplitudes before it, then V on psi and lambda.
-template <int VK, int PB>
-__device__ __forceinline__ double fast_op(double2 (&a)[8], double2 (&b)[8], const PSub& P) {
-  const double acc = grad_terms<PB>(a, b, P.d[0], P.tm[0]);
+// A rotation about Y or X undone up to its scale: V = cos (I + tan G); the host
+// collects the cosines (one factor a sweep) and weights the gradient term with
+// what was not yet applied.  4 FMA a pair and vector against 8, and 4 for the
+// gradient term sum conj(lambda) G psi of the generator G.
+enum TanForm : uint32_t { TF_Y = 0, TF_X = 1 };
+
+template <int PB, uint32_t TF>
+__device__ __forceinline__ double tan_op(double2 (&a)[8], double2 (&b)[8], double t) {
+  double s[2] = {0.0, 0.0};
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int i = pair_lo<PB>(k), j = i | (1 << PB);
-    apply2<VK>(P.v, a[i], a[j]);
-    apply2<VK>(P.v, b[i], b[j]);
+    const double2 l0 = b[i], l1 = b[j], p0 = a[i], p1 = a[j];
+    double& x = s[k & 1];
+    if (TF == TF_Y) {
+      x = fma(l1.x, p0.x, fma(l1.y, p0.y, fma(-l0.x, p1.x, fma(-l0.y, p1.y, x))));
+      a[i] = make_double2(fma(t, p1.x, p0.x), fma(t, p1.y, p0.y));
+      a[j] = make_double2(fma(-t, p0.x, p1.x), fma(-t, p0.y, p1.y));
+      b[i] = make_double2(fma(t, l1.x, l0.x), fma(t, l1.y, l0.y));
+      b[j] = make_double2(fma(-t, l0.x, l1.x), fma(-t, l0.y, l1.y));
+    } else {
+      x = fma(l0.x, p1.y, fma(-l0.y, p1.x, fma(l1.x, p0.y, fma(-l1.y, p0.x, x))));
+      a[i] = make_double2(fma(-t, p1.y, p0.x), fma(t, p1.x, p0.y));
+      a[j] = make_double2(fma(-t, p0.y, p1.x), fma(t, p0.x, p1.y));
+      b[i] = make_double2(fma(-t, l1.y, l0.x), fma(t, l1.x, l0.y));
+      b[j] = make_double2(fma(-t, l0.y, l1.x), fma(t, l0.x, l1.y));
+    }
   }
-  return acc;
+  return s[0] + s[1];
 }
 
-// A register phase of two or three ops on distinct phase bits PB0 < PB1 (<
-// PB2), each with one derivative and the same V shape VK (the encoder sorts
-// such ops by target: ops on distinct qubits commute), as straight-line code;
-// the ops' warp reductions run after all of them, side by side.
-template <int VK, int PB0, int PB1, int PB2>
-__device__ __forceinline__ void phase_fast(double2 (&a)[8], double2 (&b)[8], const PSub* ps,
-                                           double* accw, int lane, int w) {
-  double g0 = fast_op<VK, PB0>(a, b, ps[0]);
-  double g1 = fast_op<VK, PB1>(a, b, ps[1]);
-  double g2 = 0.0;
-  if constexpr (PB2 >= 0) g2 = fast_op<VK, PB2>(a, b, ps[2]);
-  g0 = warp_sum_d(g0);
-  g1 = warp_sum_d(g1);
-  if constexpr (PB2 >= 0) g2 = warp_sum_d(g2);
-  if (lane == 0) {
-    accw[ps[0].slot * kAWarps + w] += g0;
-    accw[ps[1].slot * kAWarps + w] += g1;
-    if constexpr (PB2 >= 0) accw[ps[2].slot * kAWarps + w] += g2;
+template <int PB>
+__device__ __forceinline__ void general_op(double2 (&a)[8], double2 (&b)[8], const PSub& P, bool valid,
+                                           double* accw) {
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  if (P.vk == 0) phase_one<PB, 0>(a, b, P, acc);
+  else if (P.vk == 1) phase_one<PB, 1>(a, b, P, acc);
+  else phase_one<PB, 2>(a, b, P, acc);
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q) {
+    if (q >= P.np) break;
+    const double v = warp_sum_d(valid ? acc[q] : 0.0);
+    if ((threadIdx.x & 31) == 0) accw[P.slot + q] += v;
   }
 }
 
-template <int VK>
-__device__ __forceinline__ void phase_fast_bits(uint32_t form, double2 (&a)[8], double2 (&b)[8],
-                                                const PSub* ps, double* accw, int lane, int w) {
-  switch (form) {
-    case 0: phase_fast<VK, 0, 1, 2>(a, b, ps, accw, lane, w); break;
-    case 1: phase_fast<VK, 0, 1, -1>(a, b, ps, accw, lane, w); break;
-    case 2: phase_fast<VK, 0, 2, -1>(a, b, ps, accw, lane, w); break;
-    default: phase_fast<VK, 1, 2, -1>(a, b, ps, accw, lane, w); break;
-  }
+// Sums of four values over the warp: lane l < 4 returns the sum of g[l] (12
+// shuffles against 40 for one after the other).
+__device__ __forceinline__ double warp_sum4(const double (&g)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool b0 = lane & 1, b1 = lane & 2;
+  const double x = (b0 ? g[1] : g[0]) + __shfl_xor_sync(0xffffffffu, b0 ? g[0] : g[1], 1);
+  const double y = (b0 ? g[3] : g[2]) + __shfl_xor_sync(0xffffffffu, b0 ? g[2] : g[3], 1);
+  double v = (b1 ? y : x) + __shfl_xor_sync(0xffffffffu, b1 ? x : y, 2);
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// N rotations of one form on register bits 0 .. N - 1 (the passes of layered
+// circuits), without a branch between them.
+template <uint32_t TF, int N>
+__device__ __forceinline__ void pass_tan(double2 (&a)[8], double2 (&b)[8], const PSub* ps, bool valid,
+                                         double* accw) {
+  double g[4] = {0.0, 0.0, 0.0, 0.0};
+  g[0] = tan_op<0, TF>(a, b, ps[0].v[0].x);
+  if constexpr (N > 1) g[1] = tan_op<1, TF>(a, b, ps[1].v[0].x);
+  if constexpr (N > 2) g[2] = tan_op<2, TF>(a, b, ps[2].v[0].x);
+#pragma unroll
+  for (int k = 0; k < N; ++k) g[k] = valid ? g[k] : 0.0;
+  const double v = warp_sum4(g);
+  const uint32_t lane = threadIdx.x & 31;
+  if (lane < N && ps[lane].np) accw[ps[lane].slot] += ps[lane].v[0].y * v;
 }
 
 // The op data of one register phase: threads < cnt fill ps[0 .. cnt).
@@ -635,6 +660,11 @@ __device__ __forceinline__ void stage_phase(const AOp& hdr, const AOp* sub, cons
     P.np = op.np;
     P.slot = op.slot;
     P.pb = op.lt == pbits[0] ? 0u : (op.lt == pbits[1] ? 1u : 2u);
+    if (op.cnt) {
+      P.vk = 2u + op.cnt;
+      P.v[0] = pool[op.lctrl];
+      return;
+    }
     for (int i = 0; i < 4; ++i) P.v[i] = mt[i];
     const bool real = mt[0].y == 0.0 && mt[1].y == 0.0 && mt[2].y == 0.0 && mt[3].y == 0.0;
     const bool rxl = mt[0].y == 0.0 && mt[3].y == 0.0 && mt[1].x == 0.0 && mt[2].x == 0.0;
@@ -653,74 +683,89 @@ __device__ __forceinline__ void stage_phase(const AOp& hdr, const AOp* sub, cons
   }
 }
 
-// A register phase: every thread holds the 8 amplitudes of psi and lambda
-// that differ in the phase's three local bits and applies the phase's
-// uncontrolled one-qubit ops (on those bits) in order.  Each op's gradient
-// terms are reduced per warp right after the op (all lanes take part: the
-// group loop runs the same trip count on every thread).  staged: ps already
-// holds the phase's op data (staged once per CTA).
-__device__ __noinline__ void op_phase(double2* sp, double2* sl, const AOp& hdr, const AOp* sub,
-                                      const double2* pool, uint32_t m, double* accw, PSub* ps,
-                                      bool staged) {
-  const uint32_t cnt = hdr.cnt;
-  const uint32_t pbits[3] = {hdr.lt, hdr.lt2, (uint32_t)hdr.dq[0]};
-  if (!staged) {
-    stage_phase(hdr, sub, pool, ps);
-    __syncthreads();
-  }
-  const uint32_t groups = (1u << m) >> 3;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (uint32_t g0 = 0; g0 < groups; g0 += kAThreads) {
-    const uint32_t g = g0 + threadIdx.x;
-    const bool valid = g < groups;
-    const uint32_t ob = ins0a(ins0a(ins0a(valid ? g : 0u, pbits[0]), pbits[1]), pbits[2]);
-    // swz is linear over XOR and ob has the phase bits clear, so
+// The register layout of a pass or phase on local bits q0, q1, q2: thread g
+// holds the elements ob | bits (in the tile at off(e)).
+struct RegBits {
+  uint32_t ob, sb, s0, s1, s2;
+  __device__ __forceinline__ RegBits(uint32_t q0, uint32_t q1, uint32_t q2, uint32_t groups) {
+    const uint32_t lo = min(q0, min(q1, q2)), hi = max(q0, max(q1, q2)), mid = q0 + q1 + q2 - lo - hi;
+    ob = ins0a(ins0a(ins0a(threadIdx.x & (groups - 1u), lo), mid), hi);
+    // swz is linear over XOR and ob has the three bits clear, so
     // swz(ob | bits) = swz(ob) ^ swz(bits)
-    const uint32_t sb = swz(ob);
-    const uint32_t s0 = swz(1u << pbits[0]), s1 = swz(1u << pbits[1]), s2 = swz(1u << pbits[2]);
-    auto off = [&](int i) {
-      return sb ^ ((i & 1) ? s0 : 0u) ^ ((i & 2) ? s1 : 0u) ^ ((i & 4) ? s2 : 0u);
-    };
-    double2 a[8], b[8];
+    sb = swz(ob);
+    s0 = swz(1u << q0);
+    s1 = swz(1u << q1);
+    s2 = swz(1u << q2);
+  }
+  __device__ __forceinline__ uint32_t off(int e) const {
+    return sb ^ ((e & 1) ? s0 : 0u) ^ ((e & 2) ? s1 : 0u) ^ ((e & 4) ? s2 : 0u);
+  }
+};
+
+__device__ __forceinline__ void scale8(double2 (&a)[8], double f) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      a[i] = valid ? sp[off(i)] : make_double2(0.0, 0.0);
-      b[i] = valid ? sl[off(i)] : make_double2(0.0, 0.0);
+  for (int e = 0; e < 8; ++e) a[e] = make_double2(f * a[e].x, f * a[e].y);
+}
+
+// A register phase of any uncontrolled one-qubit ops, in order.  The gradient
+// sums of up to four rotations are reduced together.
+__device__ __noinline__ void op_phase(double2* sp, double2* sl, const AOp& hdr, const PSub* ps,
+                                      const double2* pool, uint32_t m, double* accw) {
+  const uint32_t lane = threadIdx.x & 31, groups = (1u << m) >> 3;
+  const bool valid = threadIdx.x < groups;
+  const RegBits rb(hdr.lt, hdr.lt2, hdr.dq[0], groups);
+  double2 a[8], b[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    a[e] = sp[rb.off(e)];
+    b[e] = sl[rb.off(e)];
+  }
+  double g[4] = {0.0, 0.0, 0.0, 0.0};
+  uint32_t who = 0, pending = 0;  // the ops of g, a byte each
+  auto flush = [&]() {
+    const double v = warp_sum4(g);
+    if (lane < pending) {
+      const PSub& P = ps[(who >> (8 * lane)) & 0xffu];
+      if (P.np) accw[P.slot] += P.v[0].y * v;
     }
-    // straight-line form (header pad[0] = 1 + VK * 4 + bit form)
-    const uint32_t fast = hdr.pad[0];
-    if (fast) {
-      const uint32_t vk = (fast - 1u) >> 2, form = (fast - 1u) & 3u;
-      if (vk == 1) phase_fast_bits<1>(form, a, b, ps, accw, lane, w);
-      else if (vk == 2) phase_fast_bits<2>(form, a, b, ps, accw, lane, w);
-      else phase_fast_bits<0>(form, a, b, ps, accw, lane, w);
-    }
+    pending = 0;
+  };
 #pragma unroll 1
-    for (uint32_t u = 0; u < (fast ? 0u : cnt); ++u) {
-      const PSub& P = ps[u];
-      double acc[4] = {0.0, 0.0, 0.0, 0.0};
-      switch (P.pb * 3 + P.vk) {
-        case 0: phase_one<0, 0>(a, b, P, acc); break;
-        case 1: phase_one<0, 1>(a, b, P, acc); break;
-        case 2: phase_one<0, 2>(a, b, P, acc); break;
-        case 3: phase_one<1, 0>(a, b, P, acc); break;
-        case 4: phase_one<1, 1>(a, b, P, acc); break;
-        case 5: phase_one<1, 2>(a, b, P, acc); break;
-        case 6: phase_one<2, 0>(a, b, P, acc); break;
-        case 7: phase_one<2, 1>(a, b, P, acc); break;
-        default: phase_one<2, 2>(a, b, P, acc); break;
-      }
-      for (uint32_t q = 0; q < P.np; ++q) {
-        const double v = warp_sum_d(acc[q]);
-        if (lane == 0) accw[(P.slot + q) * kAWarps + w] += v;
-      }
+  for (uint32_t u = 0; u < hdr.cnt; ++u) {
+    const PSub& P = ps[u];
+    const double t = P.v[0].x;
+    double v = 0.0;
+    switch (P.pb * 8 + P.vk) {
+      case 3: v = tan_op<0, TF_Y>(a, b, t); break;
+      case 4: v = tan_op<0, TF_X>(a, b, t); break;
+      case 11: v = tan_op<1, TF_Y>(a, b, t); break;
+      case 12: v = tan_op<1, TF_X>(a, b, t); break;
+      case 19: v = tan_op<2, TF_Y>(a, b, t); break;
+      case 20: v = tan_op<2, TF_X>(a, b, t); break;
+      default:
+        if (P.pb == 0) general_op<0>(a, b, P, valid, accw);
+        else if (P.pb == 1) general_op<1>(a, b, P, valid, accw);
+        else general_op<2>(a, b, P, valid, accw);
+        continue;
     }
-    if (valid) {
+    if (pending == 4) flush();
+    g[3] = g[2];
+    g[2] = g[1];
+    g[1] = g[0];
+    g[0] = valid ? v : 0.0;
+    who = who << 8 | u;
+    ++pending;
+  }
+  if (pending) flush();
+  if (hdr.mat != kNone) {
+    scale8(a, pool[hdr.mat].x);
+    scale8(b, pool[hdr.mat].x);
+  }
+  if (valid) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        sp[off(i)] = a[i];
-        sl[off(i)] = b[i];
-      }
+    for (int e = 0; e < 8; ++e) {
+      sp[rb.off(e)] = a[e];
+      sl[rb.off(e)] = b[e];
     }
   }
 }
@@ -728,6 +773,16 @@ __device__ __noinline__ void op_phase(double2* sp, double2* sl, const AOp& hdr, 
 // One backward sweep over tiles t0, t0 + step, ... (< t1) of psi and lambda;
 // the CTA's gradient sums go to partial[slot * nparts + part].  Every thread
 // of the CTA calls it; the caller separates consecutive calls by a barrier.
+// The pass that ends a sweep holds the whole tile in registers: the next
+// tile's copies start before its arithmetic, and its results go to memory from
+// the registers (each eight threads 128 consecutive bytes).
+// 24 qubits, 16 layers of ry, rz and rzz: 42 sweeps in 14.1 ms, of which 8.6 are
+// the tiles' loads and stores alone (1.07 GB a sweep at 5.2 TB/s), 2.0 the passes
+// through shared memory and 3.6 arithmetic that does not hide behind them; 24.3 ms
+// with separate passes for runs and rotations, general 2x2s, a warp sum a rotation
+// and loads that began after the stores.  128 such sets of 20 qubits and 8
+// layers: 53 ms, 93 before.  Prefetching the next tile into L2 at the start of
+// this one gains nothing.
 __device__ __forceinline__ void adj_sweep_body(double2* __restrict__ psi, double2* __restrict__ lam,
                                                const ASweepHdr* __restrict__ hp,
                                                const AOp* __restrict__ ops,
@@ -737,28 +792,24 @@ __device__ __forceinline__ void adj_sweep_body(double2* __restrict__ psi, double
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ ASweepHdr H;
   __shared__ uint64_t hi_tab[1u << (kAMaxLocal - kALoMin)];
-  __shared__ DRec drec[kADiagRun];
-  __shared__ PSub psub[kAPhaseOps];
   if (threadIdx.x == 0) H = *hp;
   __syncthreads();
   const uint32_t m = H.m, L = 1u << m;
+  const uint32_t w = threadIdx.x >> 5;
   double2* sp = reinterpret_cast<double2*>(smraw);
   double2* sl = sp + L;
-  double* accw = reinterpret_cast<double*>(sl + L);
-  // the sweep's ops, and (phase_ops > 0) every register phase's op data, in
-  // shared memory for the whole launch
-  AOp* sops = reinterpret_cast<AOp*>(accw + ((H.nslots ? H.nslots : 1u) * kAWarps + 1u) / 2u * 2u);
+  double2* tabs = sl + L;
+  double2* blob = tabs + (size_t)H.ntab * 4 * kAThreads;
+  double2* fact = blob + H.nblob;  // [tile parity][run][kDFactors]
+  double* acc0 = reinterpret_cast<double*>(fact + 2 * kDFactors * H.ndrun);
+  double* accw = acc0 + w * H.nslots;
+  // the sweep's ops, and (phase_ops > 0) every pass's op data, in shared
+  // memory for the whole launch
+  AOp* sops = reinterpret_cast<AOp*>(acc0 + (H.nslots ? H.nslots : 1u) * kAWarps);
   PSub* psall = reinterpret_cast<PSub*>(sops + (H.nops + 1u) / 2u * 2u);
-  for (uint32_t i = threadIdx.x; i < H.nslots * kAWarps; i += kAThreads) accw[i] = 0.0;
+  for (uint32_t i = threadIdx.x; i < H.nslots * kAWarps; i += kAThreads) acc0[i] = 0.0;
   for (uint32_t i = threadIdx.x; i < H.nops; i += kAThreads) sops[i] = ops[i];
-  __syncthreads();
-  if (H.phase_ops) {
-    for (uint32_t i = 0; i < H.nops; ++i) {
-      const AOp op = sops[i];
-      if (op.type == A_PHASE) stage_phase(op, sops + i + 1, pool, psall + op.lctrl);
-      if (op.type == A_PHASE || op.type == A_DRUN) i += op.cnt;
-    }
-  }
+  for (uint32_t i = threadIdx.x; i < H.nblob; i += kAThreads) blob[i] = pool[H.blob0 + i];
   // offset bits above the 5 contiguous ones -> global bits
   // local bits 0 .. lo_bits-1 are qubits 0 .. lo_bits-1: runs of 2^lo_bits
   // consecutive amplitudes (at least 128 B)
@@ -772,37 +823,155 @@ __device__ __forceinline__ void adj_sweep_body(double2* __restrict__ psi, double
     hi_tab[hv] = g;
   }
   __syncthreads();
+  for (uint32_t i = 0; i < H.nops; ++i) {
+    const AOp op = sops[i];
+    if (op.type != A_PASS && op.type != A_PHASE) continue;
+    if (H.phase_ops) stage_phase(op, sops + i + 1, pool, psall + op.lctrl);
+    if (op.type == A_PASS && op.ndq) {
+      const double2* B = blob + op.slot;
+      const uint32_t tab = reinterpret_cast<const DMask*>(B + 5)->tab;
+      if (tab != kNone) {
+        double2 f[4];
+        pair_factors(B, f);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tabs[((size_t)tab * 4 + k) * kAThreads + threadIdx.x] = f[k];
+      }
+    }
+    i += op.cnt;
+  }
   const uint32_t lo_mask = (1u << lo_bits) - 1u;
-
-  for (uint64_t t = t0; t < t1 && t < H.ntiles; t += step) {
+  // tile index -> its base (the index's bits on the non-local qubits), and the
+  // base of a tile `step` further on: with ones in the local bits a carry
+  // passes over them
+  auto deposit = [&](uint64_t t) {
     uint64_t base = 0;
     for (uint32_t b = 0; b < H.npos_cnt; ++b)
       if (t >> b & 1ULL) base |= 1ULL << H.npos[b];
-    // all of the tile's copies in flight at once (cp.async straight into the
-    // swizzled layout), then one wait
-    for (uint32_t o = threadIdx.x; o < L; o += kAThreads) {
-      const uint64_t g = base | (o & lo_mask) | hi_tab[o >> lo_bits];
-      cp_async16a(sp + swz(o), psi + g);
-      cp_async16a(sl + swz(o), lam + g);
+    return base;
+  };
+  uint64_t local = 0;
+  for (uint32_t b = 0; b < m; ++b) local |= 1ULL << H.lpos[b];
+  const uint64_t advance = deposit(step);
+  // all of a tile's copies in flight at once (cp.async straight into the
+  // swizzled layout)
+  const uint32_t my_s = swz(threadIdx.x & (L - 1u));
+  const uint64_t my_g = (threadIdx.x & lo_mask) | hi_tab[(threadIdx.x & (L - 1u)) >> lo_bits];
+  auto load_tile = [&](uint64_t base) {
+    if (m == kAMaxLocal) {
+      const uint64_t h0 = 1ULL << H.lpos[8], h1 = 1ULL << H.lpos[9], h2 = 1ULL << H.lpos[10];
+      const double2 *gp = psi + (base | my_g), *gl = lam + (base | my_g);
+#pragma unroll
+      for (uint32_t j = 0; j < 8; ++j) {
+        const uint64_t g = ((j & 1u) ? h0 : 0ULL) + ((j & 2u) ? h1 : 0ULL) + ((j & 4u) ? h2 : 0ULL);
+        const uint32_t o = my_s ^ swz(j * kAThreads);
+        cp_async16a(sp + o, gp + g);
+        cp_async16a(sl + o, gl + g);
+      }
+    } else {
+      for (uint32_t o = threadIdx.x; o < L; o += kAThreads) {
+        const uint64_t g = base | (o & lo_mask) | hi_tab[o >> lo_bits];
+        cp_async16a(sp + swz(o), psi + g);
+        cp_async16a(sl + swz(o), lam + g);
+      }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+
+  bool loaded = false;
+  uint32_t parity = 0;
+  uint64_t base = deposit(t0), next = 0;
+  const uint64_t tend = t1 < H.ntiles ? t1 : H.ntiles;
+  for (uint64_t t = t0; t < tend; t += step, parity ^= 1u, base = next) {
+    next = ((base | local) + advance) & ~local;
+    if (!loaded) load_tile(base);
+    loaded = false;
+    // (the other parity's factors may still be in use)
+    double2* E = fact + parity * kDFactors * H.ndrun;
+    {
+      const uint32_t* off = reinterpret_cast<const uint32_t*>(blob);
+      for (uint32_t d = w; d < H.ndrun; d += kAWarps) tile_factors(blob + off[d], base, E + kDFactors * d);
+    }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
     for (uint32_t i = 0; i < H.nops; ++i) {
+      const uint2* ow = reinterpret_cast<const uint2*>(sops + i);
+      const uint2 w0 = ow[0];
+      if ((w0.x & 0xffu) >= A_PASS) {
+        const uint2 w1 = ow[1], w2 = ow[2];
+        const uint32_t cnt = (w1.x >> 8) & 0xffu;
+        const PSub* ps = psall + (H.phase_ops ? w1.y : 0u);
+        if (!H.phase_ops && cnt) {
+          stage_phase(sops[i], sops + i + 1, pool, psall);
+          __syncthreads();
+        }
+        if ((w0.x & 0xffu) == A_PHASE) {
+          op_phase(sp, sl, sops[i], ps, pool, m, accw);
+          i += cnt;
+          __syncthreads();
+          continue;
+        }
+        const uint32_t q0 = (w0.x >> 16) & 0xffu, q1 = w0.x >> 24, q2 = (w0.y >> 16) & 0xffu;
+        const bool valid = threadIdx.x < (L >> 3);
+        const RegBits rb(q0, q1, q2, L >> 3);
+        double2 a[8], b[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          a[e] = sp[rb.off(e)];
+          b[e] = sl[rb.off(e)];
+        }
+        i += cnt;
+        const bool direct = H.direct && i + 1 == H.nops;
+        if (direct) {
+          __syncthreads();
+          if (t + step < tend) {
+            load_tile(next);
+            loaded = true;
+          }
+        }
+        if (w1.x & 0xffu) {
+          const double2* B = blob + w2.x;
+          if (w0.x & 0xff00u) diag_grads(a, b, B, base, valid, accw);
+          diag_apply(a, b, B, E + kDFactors * (w0.y >> 24), tabs);
+        }
+        switch ((w1.x >> 16) & 0xffu) {  // AOp::pad[0]: 1 + TanForm + 2 (count - 1)
+          case 1: pass_tan<TF_Y, 1>(a, b, ps, valid, accw); break;
+          case 2: pass_tan<TF_X, 1>(a, b, ps, valid, accw); break;
+          case 3: pass_tan<TF_Y, 2>(a, b, ps, valid, accw); break;
+          case 4: pass_tan<TF_X, 2>(a, b, ps, valid, accw); break;
+          case 5: pass_tan<TF_Y, 3>(a, b, ps, valid, accw); break;
+          case 6: pass_tan<TF_X, 3>(a, b, ps, valid, accw); break;
+          default: break;
+        }
+        if (w2.y != kNone) {
+          const double f = __ldg(&pool[w2.y].x);
+          scale8(a, f);
+          scale8(b, f);
+        }
+        if (direct) {
+          const uint64_t gb = base | (rb.ob & lo_mask) | hi_tab[rb.ob >> lo_bits];
+          const uint64_t g0 = 1ULL << H.lpos[q0], g1 = 1ULL << H.lpos[q1], g2 = 1ULL << H.lpos[q2];
+          if (valid) {
+            double2 *gp = psi + gb, *gl = lam + gb;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const uint64_t g = ((e & 1) ? g0 : 0ULL) + ((e & 2) ? g1 : 0ULL) + ((e & 4) ? g2 : 0ULL);
+              gp[g] = a[e];
+              gl[g] = b[e];
+            }
+          }
+          break;
+        }
+        if (valid) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            sp[rb.off(e)] = a[e];
+            sl[rb.off(e)] = b[e];
+          }
+        }
+        __syncthreads();
+        continue;
+      }
       const AOp op = sops[i];
-      if (op.type == A_DRUN) {
-        op_drun(sp, sl, op, sops + i + 1, pool, m, base, accw, drec);
-        i += op.cnt;
-        __syncthreads();
-        continue;
-      }
-      if (op.type == A_PHASE) {
-        op_phase(sp, sl, op, sops + i + 1, pool, m, accw, H.phase_ops ? psall + op.lctrl : psub,
-                 H.phase_ops != 0);
-        i += op.cnt;
-        __syncthreads();
-        continue;
-      }
       switch (op.type) {
         case A_ONE:
           switch (op.np) {
@@ -824,17 +993,20 @@ __device__ __forceinline__ void adj_sweep_body(double2* __restrict__ psi, double
       }
       __syncthreads();
     }
-    for (uint32_t o = threadIdx.x; o < L; o += kAThreads) {
-      const uint64_t g = base | (o & lo_mask) | hi_tab[o >> lo_bits];
-      psi[g] = sp[swz(o)];
-      lam[g] = sl[swz(o)];
+    if (!H.direct) {
+      for (uint32_t o = threadIdx.x; o < L; o += kAThreads) {
+        const uint64_t g = base | (o & lo_mask) | hi_tab[o >> lo_bits];
+        psi[g] = sp[swz(o)];
+        lam[g] = sl[swz(o)];
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
+  __syncthreads();
   for (uint32_t s = threadIdx.x; s < H.nslots; s += kAThreads) {
-    double a = 0.0;
-    for (int w = 0; w < kAWarps; ++w) a += accw[s * kAWarps + w];
-    partial[(size_t)s * nparts + part] = a;
+    double x = 0.0;
+    for (int v = 0; v < kAWarps; ++v) x += acc0[v * H.nslots + s];
+    partial[(size_t)s * nparts + part] = x;
   }
 }
 
@@ -872,14 +1044,16 @@ __global__ void k_adj_slots_multi(const AJob* __restrict__ jobs, uint32_t nchunk
   J.out[J.map[s]] = a;
 }
 
-// out[map[s]] = sum over CTAs (in order) of partial[s][cta]
+// out[map[s]] = sum over CTAs of partial[s][cta], a warp per slot (one thread
+// per slot took 14 us a sweep for 296 CTAs)
 __global__ void k_adj_slots(const double* partial, uint32_t nslots, uint32_t ctas,
                             const uint32_t* map, double* out) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= nslots) return;
   double a = 0.0;
-  for (uint32_t c = 0; c < ctas; ++c) a += partial[(size_t)s * ctas + c];
-  out[map[s]] = a;
+  for (uint32_t c = lane; c < ctas; c += 32) a += partial[(size_t)s * ctas + c];
+  a = warp_sum_d(a);
+  if (lane == 0) out[map[s]] = a;
 }
 
 // ---- host planner ----------------------------------------------------------------------------
@@ -1064,31 +1238,185 @@ void push_dprime(std::vector<double2>& pool, const hc du[4], const hc v[4]) {
   push_mats(pool, d, 4);
 }
 
-// The record op_drun reads for a diagonal op: the angle polynomial of its
-// entries V[2 b0 + b1] = exp(i (al + be b0 + ga b1 + de b0 b1)) and the Walsh
-// coefficients what[2 S0 + S1] = 1/4 sum_e V[e] dU[e] (-1)^(b0 S0 + b1 S1).
-// A one-qubit diagonal (entry index b0) is the same with b1 = 0: its
-// coefficients with S1 = 1 vanish.
-void push_drun_record(std::vector<double2>& pool, const hc v[4], const hc dd[4], uint32_t nq) {
+// A diagonal gate's angle polynomial and Walsh weights: its entries are
+// V[2 b0 + b1] = exp(i (al + be b0 + ga b1 + de b0 b1)), and a gradient term is
+// sum_S w[S] (Walsh coefficient of Im(conj(lambda) psi) on the bits in S).
+// A one-qubit diagonal (entry index b0) is the same with b1 = 0: its weights
+// with S1 = 1 vanish.
+struct DiagPoly {
+  double al, be, ga, de;
+  double w[4];
+  bool ok;  // dU U^dagger is imaginary (all supported kinds)
+};
+DiagPoly diag_poly(const AGate& g) {
+  DiagPoly r{};
   double th[4];
-  hc w[4];
+  hc x[4];
+  const uint32_t D = 1u << g.nq;
+  for (uint32_t e = 0; e < 4; ++e) {
+    const uint32_t src = D == 4 ? e : (e >> 1);
+    const hc v = cjh(g.dg[src]), d = g.np ? g.ddg[0][src] : hc{0, 0};
+    th[e] = std::atan2(v.im, v.re);
+    x[e] = v * d;
+  }
+  r.al = th[0];
+  r.be = th[2] - th[0];
+  r.ga = th[1] - th[0];
+  r.de = th[3] - th[2] - th[1] + th[0];
+  double mx = 0.0, re = 0.0;
   for (int e = 0; e < 4; ++e) {
-    const int src = nq == 2 ? e : (e >> 1);
-    th[e] = std::atan2(v[src].im, v[src].re);
-    w[e] = hc{v[src].re * dd[src].re - v[src].im * dd[src].im, v[src].re * dd[src].im + v[src].im * dd[src].re};
+    mx = std::max(mx, std::fabs(x[e].im));
+    re = std::max(re, std::fabs(x[e].re));
   }
-  pool.push_back(make_double2(th[0], th[2] - th[0]));
-  pool.push_back(make_double2(th[1] - th[0], th[3] - th[2] - th[1] + th[0]));
+  r.ok = !(re > 1e-13);
   for (int S = 0; S < 4; ++S) {
-    double re = 0.0, im = 0.0;
-    for (int e = 0; e < 4; ++e) {
-      const bool neg = (((e >> 1) & (S >> 1)) ^ (e & S & 1)) != 0;
-      re += neg ? -w[e].re : w[e].re;
-      im += neg ? -w[e].im : w[e].im;
-    }
-    pool.push_back(make_double2(0.25 * re, 0.25 * im));
+    double im = 0.0;
+    for (int e = 0; e < 4; ++e) im += (((e >> 1) & (S >> 1)) ^ (e & S & 1)) ? -x[e].im : x[e].im;
+    // parts below 1e-14 of the largest entry are rounding residue of zeros
+    r.w[S] = std::fabs(0.25 * im) <= 1e-14 * mx ? 0.0 : -0.25 * im;
   }
+  return r;
 }
+
+// Where a qubit's bit is during a pass: register bit (8 + k), bit of
+// threadIdx.x (0..7), or bit of the tile's base (64 + qubit).
+struct PassBits {
+  uint32_t code[64];
+};
+
+// Appends the record of a run of diagonal gates; sigma: what both vectors
+// carry at that point; pre: the factor the run applies.
+void push_drun(std::vector<double2>& blob, const std::vector<AGate>& gates, const std::vector<uint32_t>& run,
+               const std::vector<uint32_t>& slot, const PassBits& pb, long double sigma, long double pre,
+               uint32_t tab) {
+  const long double kTwoPi = 2.0L * 3.14159265358979323846264338327950288L;
+  long double c0 = 0.0L, H[3] = {0.0L, 0.0L, 0.0L};
+  std::map<uint32_t, long double> loc[4], cst, lin;
+  auto single = [&](uint32_t c, double x) {
+    if (c >= 64) cst[(c - 64) | 63u << 6] += x;
+    else if (c >= 8) loc[c - 7][0] += x;
+    else loc[0][1u << c] += x;
+  };
+  auto pair = [&](uint32_t c, uint32_t d, double x) {
+    if (c > d) std::swap(c, d);
+    if (c >= 64) cst[(c - 64) | (d - 64) << 6] += x;
+    else if (d >= 64) lin[c | (d - 64) << 4] += x;
+    else if (c >= 8) H[c + d - 17] += x;
+    else if (d >= 8) loc[d - 7][1u << c] += x;
+    else loc[0][1u << c | 1u << d] += x;
+  };
+  std::vector<DTerm> layer[4];
+  const double wt = (double)(1.0L / (sigma * sigma));
+  for (uint32_t i : run) {
+    const AGate& g = gates[i];
+    const DiagPoly p = diag_poly(g);
+    const uint32_t ca = pb.code[g.qa], cb = g.nq == 2 ? pb.code[g.qb] : 0;
+    c0 += p.al;
+    if (p.be != 0.0) single(ca, p.be);
+    if (g.nq == 2 && p.ga != 0.0) single(cb, p.ga);
+    if (g.nq == 2 && p.de != 0.0) pair(ca, cb, p.de);
+    if (!g.np) continue;
+    uint32_t nt = 0;
+    for (uint32_t S = 0; S < 4; ++S) {
+      if (p.w[S] == 0.0) continue;
+      uint32_t R = 0, T = 0, nb = 0, base[2] = {63u, 63u};
+      for (uint32_t a = 0; a < 2; ++a) {
+        if (!(S >> (1 - a) & 1u)) continue;
+        const uint32_t c = a ? cb : ca;
+        if (c >= 64) base[nb++] = c - 64;
+        else if (c >= 8) R ^= 1u << (c - 8);
+        else T ^= 1u << c;
+      }
+      DTerm d{};
+      d.w = p.w[S] * wt;
+      const uint32_t reg = (T >> 3 & 1u) | (T >> 4 & 1u) << 1 | (T >> 2 & 1u) << 2;
+      d.code = (R | (T & 3u) << 3) | (T >> 5) << 5 | reg << 8 | base[0] << 11 | base[1] << 17;
+      d.slot = slot[i];
+      layer[nt++].push_back(d);
+    }
+  }
+  // at most one term of a gate among 32 consecutive ones (a lane each)
+  std::vector<DTerm> terms;
+  for (auto& l : layer) {
+    if (l.empty()) continue;
+    while (terms.size() % 32) terms.push_back(DTerm{0.0, 0, kNone});
+    std::stable_sort(l.begin(), l.end(), [](const DTerm& x, const DTerm& y) { return (x.code >> 8 & 7u) < (y.code >> 8 & 7u); });
+    terms.insert(terms.end(), l.begin(), l.end());
+  }
+  for (size_t j = 0; j < terms.size(); j += 32) {
+    uint32_t used = 0;
+    const size_t e = std::min(terms.size(), j + 32);
+    for (size_t k = j; k < e; ++k)
+      if (terms[k].slot != kNone) used |= 1u << (terms[k].code >> 8 & 7u);
+    for (size_t k = j; k < e; ++k) terms[k].code |= used << 23;
+  }
+  auto put = [&](double x, double y) { blob.push_back(make_double2(x, y)); };
+  auto put4 = [&](uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    const uint32_t v[4] = {a, b, c, d};
+    double2 x;
+    memcpy(&x, v, sizeof(x));
+    blob.push_back(x);
+  };
+  auto angs = [&](const std::map<uint32_t, long double>& l) {
+    for (auto& kv : l) {
+      const DAng a{(double)remainderl(kv.second, kTwoPi), kv.first, 0};
+      double2 x;
+      memcpy(&x, &a, sizeof(x));
+      blob.push_back(x);
+    }
+  };
+  uint32_t ends = 0, n = 0, coupled = 0, pairs = 0;
+  for (int k = 0; k < 4; ++k) {
+    n += (uint32_t)loc[k].size();
+    ends |= n << (8 * k);
+  }
+  for (auto& kv : lin) coupled |= 1u << (kv.first & 15u);
+  for (int k = 0; k < 3; ++k)
+    if (H[k] != 0.0L) pairs |= 1u << k;
+  put((double)remainderl(c0, kTwoPi), (double)pre);
+  for (int k = 0; k < 3; ++k) put((double)cosl(H[k]), (double)sinl(H[k]));
+  put4((uint32_t)terms.size(), ends, (uint32_t)cst.size(), (uint32_t)lin.size());
+  put4(coupled, pairs, tab, 0);
+  for (const DTerm& d : terms) {
+    double2 x;
+    memcpy(&x, &d, sizeof(x));
+    blob.push_back(x);
+  }
+  for (int k = 0; k < 4; ++k) angs(loc[k]);
+  angs(cst);
+  angs(lin);
+}
+
+// A rotation about Y or X (V = U^dagger, its derivative along the generator or
+// none): its TanForm, tangent, scale and gradient weight.
+bool tan_form(const AGate& g, uint32_t* form, double* t, long double* scale, double* kappa) {
+  if (g.kind != 0 || g.np > 1) return false;
+  const hc v[4] = {cjh(g.u[0]), cjh(g.u[2]), cjh(g.u[1]), cjh(g.u[3])};
+  const bool y = v[0].im == 0.0 && v[1].im == 0.0 && v[2].im == 0.0 && v[3].im == 0.0 && v[0].re == v[3].re &&
+                 v[1].re == -v[2].re;
+  const bool x = !y && v[0].im == 0.0 && v[3].im == 0.0 && v[1].re == 0.0 && v[2].re == 0.0 &&
+                 v[0].re == v[3].re && v[1].im == v[2].im;
+  if (!y && !x) return false;
+  *kappa = 0.0;
+  if (g.np) {
+    std::vector<double2> d;
+    push_dprime(d, g.du[0], v);
+    for (int e : {0, 3})
+      if (d[e].x != 0.0 || d[e].y != 0.0) return false;
+    const double lo = y ? d[1].x : d[1].y, hi = y ? -d[2].x : d[2].y;
+    if ((y ? d[1].y : d[1].x) != 0.0 || (y ? d[2].y : d[2].x) != 0.0) return false;
+    if (!(std::fabs(lo - hi) <= 1e-14 * std::fabs(hi))) return false;
+    *kappa = y ? d[2].x : -d[2].y;
+  }
+  const long double c = v[0].re, s = y ? v[1].re : v[1].im;
+  *t = (double)(s / c);
+  const long double r = 1.0L / sqrtl(1.0L + (long double)*t * (long double)*t);
+  *scale = c < 0.0L ? -r : r;
+  *form = y ? TF_Y : TF_X;
+  return r > 0x1p-20L;  // a rotation by almost pi is a general op (and a NaN one)
+}
+
+size_t asweep_smem(const ASweepHdr& h);
 
 // Encodes one sweep's ops given its final local set.
 int encode_asweep(const ASweepPlan& sp, uint32_t n, ASweepHdr& hdr, std::vector<AOp>& ops,
@@ -1107,233 +1435,318 @@ int encode_asweep(const ASweepPlan& sp, uint32_t n, ASweepHdr& hdr, std::vector<
   }
   hdr.m = m;
   hdr.ntiles = 1ULL << (n - m);
-  uint32_t slot = 0;
-  for (const AGate& g : sp.gates) {
+  const std::vector<AGate>& gates = sp.gates;
+  std::vector<uint32_t> slot(gates.size());
+  uint32_t nslots = 0;
+  for (size_t i = 0; i < gates.size(); ++i) {
+    slot[i] = nslots;
+    for (int a = 0; a < gates[i].np; ++a) slot_map.push_back(gates[i].slot0 + (uint32_t)a);
+    nslots += (uint32_t)gates[i].np;
+  }
+  // Items: a pass (diagonal run and / or one-qubit group), or a single op
+  struct Item {
+    std::vector<uint32_t> diag, ones;
+    int64_t single = -1;
+    long double pre = 1.0L, post = 1.0L;
+  };
+  std::vector<Item> items;
+  bool general = false;  // an op outside the passes has a derivative
+  for (size_t i = 0; i < gates.size();) {
+    if (m >= 3 && gates[i].kind == 2 && diag_poly(gates[i]).ok) {
+      Item it;
+      for (; i < gates.size() && gates[i].kind == 2 && diag_poly(gates[i]).ok; ++i) it.diag.push_back((uint32_t)i);
+      const bool ones = i < gates.size() && gates[i].kind == 0;
+      if (it.diag.size() == 1 && !ones) {
+        it.single = it.diag[0];
+        general = general || gates[it.diag[0]].np;
+        it.diag.clear();
+      }
+      items.push_back(it);
+      continue;
+    }
+    if (m >= 3 && gates[i].kind == 0) {
+      std::vector<uint32_t> run;
+      uint64_t seen = 0;
+      bool distinct = true;
+      for (; i < gates.size() && gates[i].kind == 0; ++i) {
+        distinct = distinct && !(seen >> gates[i].t & 1ULL);
+        seen |= 1ULL << gates[i].t;
+        run.push_back((uint32_t)i);
+      }
+      // ops on distinct qubits commute: the low local bits first, so that the
+      // last pass can write to memory in whole 128-byte runs
+      if (distinct)
+        std::sort(run.begin(), run.end(), [&](uint32_t x, uint32_t y) { return lidx[gates[x].t] < lidx[gates[y].t]; });
+      for (size_t k = 0; k < run.size();) {
+        std::vector<uint32_t> grp;
+        uint64_t bits = 0;
+        for (; k < run.size() && grp.size() < kAPhaseOps; ++k) {
+          const uint64_t b = bits | 1ULL << gates[run[k]].t;
+          if (__builtin_popcountll(b) > 3) break;
+          bits = b;
+          grp.push_back(run[k]);
+        }
+        if (items.empty() || items.back().single >= 0 || !items.back().ones.empty()) items.push_back(Item());
+        items.back().ones = grp;
+      }
+      continue;
+    }
+    Item it;
+    it.single = (int64_t)i;
+    general = general || gates[i].np;
+    items.push_back(it);
+    ++i;
+  }
+  // The rotations' scales: one factor for the sweep, applied by its first
+  // diagonal run or else after its last rotation; with derivatives outside
+  // the passes each pass applies its own.
+  long double total = 1.0L;
+  int first_diag = -1, last_tan = -1;
+  std::vector<long double> own(items.size(), 1.0L);
+  std::vector<uint8_t> tan(gates.size(), 0);
+  for (size_t k = 0; k < items.size(); ++k) {
+    if (!items[k].diag.empty() && first_diag < 0) first_diag = (int)k;
+    for (uint32_t i : items[k].ones) {
+      uint32_t f;
+      double t, kp;
+      long double c;
+      if (!tan_form(gates[i], &f, &t, &c, &kp) || fabsl(total * c) < 0x1p-300L) continue;
+      tan[i] = 1;
+      own[k] *= c;
+      total *= c;
+      last_tan = (int)k;
+    }
+  }
+  if (general) {
+    for (size_t k = 0; k < items.size(); ++k) (items[k].diag.empty() ? items[k].post : items[k].pre) = own[k];
+  } else if (last_tan >= 0) {
+    if (first_diag >= 0) items[(size_t)first_diag].pre = total;
+    else items[(size_t)last_tan].post = total;
+  }
+  for (const Item& it : items)
+    if (!it.diag.empty()) ++hdr.ndrun;
+  std::vector<double2> blob((hdr.ndrun + 3) / 4, make_double2(0.0, 0.0));
+  std::vector<uint32_t> doff;
+  long double sigma = 1.0L;  // both vectors' factor at this point
+  uint32_t pops = 0, min_last = 0;
+  bool last_pass = false;
+  auto push_one = [&](uint32_t i) {
+    const AGate& g = gates[i];
     AOp op{};
     op.np = (uint8_t)g.np;
-    op.slot = slot;
+    op.slot = slot[i];
     op.sel = -1;
     op.mat = (uint32_t)pool.size();
-    for (int a = 0; a < g.np; ++a) slot_map.push_back(g.slot0 + (uint32_t)a);
-    slot += (uint32_t)g.np;
-    if (g.kind == 0 || g.kind == 1) {
-      op.type = A_ONE;
-      op.lt = (uint8_t)lidx[g.t];
-      const hc v[4] = {cjh(g.u[0]), cjh(g.u[2]), cjh(g.u[1]), cjh(g.u[3])};
-      if (g.kind == 1 && !(sp.Lmask >> g.c & 1ULL)) {
-        // non-local control: variant 0 (control 0) is the identity
-        op.sel = (int8_t)g.c;
-        op.skip0 = 1;
-        const hc id[4] = {R(1), R(0), R(0), R(1)};
-        push_mats(pool, id, 4);
-        for (int a = 0; a < g.np; ++a) {
-          const hc z[4] = {R(0), R(0), R(0), R(0)};
-          push_mats(pool, z, 4);
-        }
-      } else if (g.kind == 1) {
-        op.lctrl = 1u << lidx[g.c];
+    op.type = A_ONE;
+    op.lt = (uint8_t)lidx[g.t];
+    const hc v[4] = {cjh(g.u[0]), cjh(g.u[2]), cjh(g.u[1]), cjh(g.u[3])};
+    if (g.kind == 1 && !(sp.Lmask >> g.c & 1ULL)) {
+      // non-local control: variant 0 (control 0) is the identity
+      op.sel = (int8_t)g.c;
+      op.skip0 = 1;
+      const hc id[4] = {R(1), R(0), R(0), R(1)};
+      push_mats(pool, id, 4);
+      for (int a = 0; a < g.np; ++a) {
+        const hc z[4] = {R(0), R(0), R(0), R(0)};
+        push_mats(pool, z, 4);
       }
-      push_mats(pool, v, 4);
-      for (int a = 0; a < g.np; ++a) push_mats(pool, g.du[a], 4);
-      if (g.kind == 0)
-        for (int a = 0; a < g.np; ++a) push_dprime(pool, g.du[a], v);
-    } else if (g.kind == 3) {
-      op.type = A_TWO;
-      op.lt = (uint8_t)lidx[g.qa];
-      op.lt2 = (uint8_t)lidx[g.qb];
-      hc v[16];
-      for (int r = 0; r < 4; ++r)
-        for (int c = 0; c < 4; ++c) v[r * 4 + c] = cjh(g.m4[c * 4 + r]);
-      push_mats(pool, v, 16);
-      if (g.np) push_mats(pool, g.dm4, 16);
-    } else {
-      op.type = A_DIAG;
-      op.ndq = (uint8_t)g.nq;
-      const uint32_t qs[2] = {g.qa, g.qb};
-      for (uint32_t a = 0; a < g.nq; ++a)
-        op.dq[a] = (sp.Lmask >> qs[a] & 1ULL) ? (uint8_t)(0x80u | lidx[qs[a]]) : (uint8_t)qs[a];
-      hc v[4] = {R(1), R(1), R(1), R(1)};
-      const uint32_t D = 1u << g.nq;
-      for (uint32_t i = 0; i < D; ++i) v[i] = cjh(g.dg[i]);
-      push_mats(pool, v, 4);
-      hc dd[4] = {R(0), R(0), R(0), R(0)};
-      if (g.np > 1) return fail(DQ_ERR_INTERNAL, "diagonal op with more than one derivative");
-      if (g.np) {
-        for (uint32_t i = 0; i < D; ++i) dd[i] = g.ddg[0][i];
-        push_mats(pool, dd, 4);
-      }
-      op.lctrl = (uint32_t)pool.size();
-      push_drun_record(pool, v, dd, g.nq);
+    } else if (g.kind == 1) {
+      op.lctrl = 1u << lidx[g.c];
     }
+    push_mats(pool, v, 4);
+    for (int a = 0; a < g.np; ++a) push_mats(pool, g.du[a], 4);
+    if (g.kind == 0)
+      for (int a = 0; a < g.np; ++a) push_dprime(pool, g.du[a], v);
     ops.push_back(op);
-  }
-  // register phases: maximal runs (two or more) of uncontrolled one-qubit ops
-  // whose targets fit three local bits; diagonal ops end a phase and go to
-  // the diagonal runs, which apply them far more cheaply
-  if (m >= 3) {
-    std::vector<AOp> phased;
-    size_t i = 0;
-    while (i < ops.size()) {
-      const AOp& o = ops[i];
-      const bool one = o.type == A_ONE && o.lctrl == 0 && o.sel < 0;
-      if (!one) {
-        phased.push_back(ops[i++]);
+  };
+  for (const Item& it : items) {
+    last_pass = false;
+    if (it.single >= 0) {
+      const uint32_t i = (uint32_t)it.single;
+      const AGate& g = gates[i];
+      if (g.kind == 0 || g.kind == 1) {
+        push_one(i);
         continue;
       }
-      uint32_t bits[3];
-      uint32_t nb = 0;
-      size_t j = i;
-      uint32_t nones = 0;
-      while (j < ops.size() && j - i < kAPhaseOps) {
-        const AOp& q = ops[j];
-        if (!(q.type == A_ONE && q.lctrl == 0 && q.sel < 0)) break;
-        bool have = false;
-        for (uint32_t b = 0; b < nb; ++b) have = have || bits[b] == q.lt;
-        if (!have) {
-          if (nb == 3) break;
-          bits[nb++] = q.lt;
+      AOp op{};
+      op.np = (uint8_t)g.np;
+      op.slot = slot[i];
+      op.sel = -1;
+      op.mat = (uint32_t)pool.size();
+      if (g.kind == 3) {
+        op.type = A_TWO;
+        op.lt = (uint8_t)lidx[g.qa];
+        op.lt2 = (uint8_t)lidx[g.qb];
+        hc v[16];
+        for (int r = 0; r < 4; ++r)
+          for (int c = 0; c < 4; ++c) v[r * 4 + c] = cjh(g.m4[c * 4 + r]);
+        push_mats(pool, v, 16);
+        if (g.np) push_mats(pool, g.dm4, 16);
+      } else {
+        if (g.np > 1) return fail(DQ_ERR_INTERNAL, "diagonal op with more than one derivative");
+        op.type = A_DIAG;
+        op.ndq = (uint8_t)g.nq;
+        const uint32_t qs[2] = {g.qa, g.qb};
+        for (uint32_t a = 0; a < g.nq; ++a)
+          op.dq[a] = (sp.Lmask >> qs[a] & 1ULL) ? (uint8_t)(0x80u | lidx[qs[a]]) : (uint8_t)qs[a];
+        hc v[4] = {R(1), R(1), R(1), R(1)}, dd[4] = {R(0), R(0), R(0), R(0)};
+        for (uint32_t e = 0; e < (1u << g.nq); ++e) {
+          v[e] = cjh(g.dg[e]);
+          if (g.np) dd[e] = g.ddg[0][e];
         }
-        ++nones;
-        ++j;
+        push_mats(pool, v, 4);
+        if (g.np) push_mats(pool, dd, 4);
       }
-      if (nones < 2) {  // a single op: the plain one-qubit pass
-        for (size_t k = i; k < j; ++k) phased.push_back(ops[k]);
-        i = j;
-        continue;
+      ops.push_back(op);
+      continue;
+    }
+    AOp h{};
+    h.type = A_PASS;
+    h.cnt = (uint8_t)it.ones.size();
+    h.mat = kNone;
+    // register bits: the targets, then the highest other local bits
+    std::vector<uint32_t> bits;
+    auto add_bit = [&](uint32_t b) {
+      if (std::find(bits.begin(), bits.end(), b) == bits.end()) bits.push_back(b);
+    };
+    for (uint32_t i : it.ones) add_bit(lidx[gates[i].t]);
+    for (uint32_t b = m; b-- > 0 && bits.size() < 3;) add_bit(b);
+    h.lt = (uint8_t)bits[0];
+    h.lt2 = (uint8_t)bits[1];
+    h.dq[0] = (uint8_t)bits[2];
+    last_pass = true;
+    min_last = *std::min_element(bits.begin(), bits.end());
+    if (!it.diag.empty()) {
+      PassBits pb;
+      uint32_t rank = 0;
+      for (uint32_t q = 0; q < n; ++q) {
+        if (!(sp.Lmask >> q & 1ULL)) {
+          pb.code[q] = 64 + q;
+          continue;
+        }
+        const size_t k = (size_t)(std::find(bits.begin(), bits.end(), lidx[q]) - bits.begin());
+        pb.code[q] = k < 3 ? 8u + (uint32_t)k : rank++;
       }
-      // three distinct phase bits: fill with other local bits
-      for (uint32_t b = 0; nb < 3 && b < m; ++b) {
-        bool have = false;
-        for (uint32_t c = 0; c < nb; ++c) have = have || bits[c] == b;
-        if (!have) bits[nb++] = b;
+      h.ndq = 1;
+      h.dq[1] = (uint8_t)doff.size();
+      h.slot = (uint32_t)blob.size();
+      for (uint32_t i : it.diag) h.np = (uint8_t)(h.np | (gates[i].np ? 1 : 0));
+      doff.push_back((uint32_t)blob.size());
+      push_drun(blob, gates, it.diag, slot, pb, sigma, it.pre, kNone);
+      sigma *= it.pre;
+    }
+    // up to three rotations of one form on distinct qubits join the pass (the
+    // register bits are their targets in order); other ops are a phase
+    uint32_t form = 0;
+    bool fast = it.ones.size() <= 3;
+    for (size_t k = 0; k < it.ones.size(); ++k) {
+      const AGate& g = gates[it.ones[k]];
+      uint32_t f = 0;
+      double t, kp;
+      long double c;
+      fast = fast && tan[it.ones[k]] && lidx[g.t] == bits[k] && tan_form(g, &f, &t, &c, &kp) && (k == 0 || f == form);
+      form = f;
+    }
+    size_t hi = ops.size();
+    if (fast) {
+      if (!it.ones.empty()) h.pad[0] = (uint8_t)(1 + form + 2 * (it.ones.size() - 1));
+      ops.push_back(h);
+    } else {
+      if (h.ndq) {
+        AOp d = h;
+        d.cnt = 0;
+        ops.push_back(d);
+        h.ndq = h.np = h.dq[1] = 0;
+        h.slot = 0;
+        ++hi;
       }
-      std::sort(bits, bits + 3);
-      AOp h{};
       h.type = A_PHASE;
-      h.cnt = (uint8_t)(j - i);
-      h.lt = (uint8_t)bits[0];
-      h.lt2 = (uint8_t)bits[1];
-      h.dq[0] = (uint8_t)bits[2];
-      std::vector<AOp> run(ops.begin() + (ptrdiff_t)i, ops.begin() + (ptrdiff_t)j);
-      // Straight-line form: two or three ops on distinct qubits, one derivative
-      // each, one V shape.  Such ops commute, so they are sorted by target bit
-      // and the kernel runs them with compile-time register bits.
-      {
-        auto vk_of = [&](const AOp& q) -> int {
-          const double2* mt = pool.data() + q.mat;
-          const bool real = mt[0].y == 0.0 && mt[1].y == 0.0 && mt[2].y == 0.0 && mt[3].y == 0.0;
-          const bool rxl = mt[0].y == 0.0 && mt[3].y == 0.0 && mt[1].x == 0.0 && mt[2].x == 0.0;
-          return real ? 1 : (rxl ? 2 : 0);
-        };
-        bool fast = (run.size() == 2 || run.size() == 3) && nones == run.size();
-        uint32_t distinct = 0;
-        for (size_t a = 0; a < run.size(); ++a) {
-          bool dup = false;
-          for (size_t b2 = 0; b2 < a; ++b2) dup = dup || run[b2].lt == run[a].lt;
-          if (!dup) ++distinct;
-          fast = fast && run[a].np == 1 && vk_of(run[a]) == vk_of(run[0]);
-        }
-        fast = fast && distinct == run.size();
-        if (fast) {
-          std::sort(run.begin(), run.end(), [](const AOp& x, const AOp& y) { return x.lt < y.lt; });
-          uint32_t pb[3] = {0, 0, 0};
-          for (size_t a = 0; a < run.size(); ++a)
-            for (uint32_t b2 = 0; b2 < 3; ++b2)
-              if (bits[b2] == run[a].lt) pb[a] = b2;
-          int form = -1;
-          if (run.size() == 3) form = 0;
-          else if (pb[0] == 0 && pb[1] == 1) form = 1;
-          else if (pb[0] == 0 && pb[1] == 2) form = 2;
-          else if (pb[0] == 1 && pb[1] == 2) form = 3;
-          if (form >= 0) h.pad[0] = (uint8_t)(1 + vk_of(run[0]) * 4 + form);
-        }
+      ops.push_back(h);
+      last_pass = false;
+    }
+    for (uint32_t i : it.ones) {
+      push_one(i);
+      uint32_t f;
+      double t, kp;
+      long double c;
+      if (tan[i] && tan_form(gates[i], &f, &t, &c, &kp)) {
+        AOp& op = ops.back();
+        op.cnt = (uint8_t)(1 + f);
+        op.lctrl = (uint32_t)pool.size();
+        pool.push_back(make_double2(t, (double)((long double)kp / (sigma * sigma))));
+        sigma /= c;
+      } else {  // the derivatives of a general op carry the weight (D', the last entries pushed)
+        const double wt = (double)(1.0L / (sigma * sigma));
+        for (size_t e = pool.size() - 4 * (size_t)gates[i].np; e < pool.size(); ++e)
+          pool[e] = make_double2(wt * pool[e].x, wt * pool[e].y);
       }
-      phased.push_back(h);
-      for (const AOp& q : run) phased.push_back(q);
-      i = j;
     }
-    ops.swap(phased);
+    if (it.post != 1.0L) {
+      ops[hi].mat = (uint32_t)pool.size();
+      pool.push_back(make_double2((double)it.post, 0.0));
+      sigma *= it.post;
+    }
+    pops += (uint32_t)it.ones.size();
   }
-  // runs of consecutive diagonal ops become one A_DRUN header + the ops
-  std::vector<AOp> grouped;
-  for (size_t i = 0; i < ops.size();) {
-    if (ops[i].type == A_PHASE) {
-      const size_t e = i + 1 + ops[i].cnt;
-      for (; i < e; ++i) grouped.push_back(ops[i]);
-      continue;
-    }
-    if (ops[i].type != A_DIAG) {
-      grouped.push_back(ops[i++]);
-      continue;
-    }
-    size_t j = i;
-    while (j < ops.size() && ops[j].type == A_DIAG && j - i < kADiagRun) ++j;
-    if (j - i >= kADiagRunMin) {
-      AOp h{};
-      h.type = A_DRUN;
-      h.cnt = (uint8_t)(j - i);
-      for (size_t k = i; k < j; ++k) h.np = (uint8_t)(h.np | (ops[k].np ? 1 : 0));
-      // ops on a local qubit first, ops on non-local qubits only (a constant
-      // phase over a tile) last; diagonal ops commute.  lctrl = how many
-      // touch a local qubit.
-      auto local = [](const AOp& o) {
-        bool l = false;
-        for (uint32_t a = 0; a < o.ndq; ++a) l = l || (o.dq[a] & 0x80u) != 0;
-        return l;
-      };
-      std::stable_partition(ops.begin() + (ptrdiff_t)i, ops.begin() + (ptrdiff_t)j, local);
-      uint32_t nloc = 0;
-      for (size_t k = i; k < j; ++k) nloc += local(ops[k]) ? 1u : 0u;
-      h.lctrl = nloc;
-      grouped.push_back(h);
-    }
-    for (size_t k = i; k < j; ++k) grouped.push_back(ops[k]);
-    i = j;
-  }
-  ops.swap(grouped);
-  // register phases' op data staged once per CTA when it fits
-  uint32_t pops = 0;
-  for (size_t i = 0; i < ops.size(); ++i)
-    if (ops[i].type == A_PHASE) pops += ops[i].cnt;
+  for (size_t k = 0; k < doff.size(); ++k) memcpy(reinterpret_cast<uint32_t*>(blob.data()) + k, &doff[k], 4);
+  hdr.direct = last_pass && min_last >= kALoMin;
+  // passes' op data staged once per CTA when it fits
   if (pops <= kAPhaseStage) {
     uint32_t b = 0;
-    for (size_t i = 0; i < ops.size(); ++i)
-      if (ops[i].type == A_PHASE) {
-        ops[i].lctrl = b;
-        b += ops[i].cnt;
+    for (AOp& o : ops)
+      if (o.type == A_PASS || o.type == A_PHASE) {
+        o.lctrl = b;
+        b += o.cnt;
       }
     hdr.phase_ops = pops;
   }
   hdr.nops = (uint32_t)ops.size();
-  hdr.nslots = slot;
+  hdr.nslots = nslots;
+  hdr.nblob = (uint32_t)blob.size();
+  hdr.blob0 = (uint32_t)pool.size();
   if (hdr.nops > kAMaxSweepOps) return fail(DQ_ERR_INTERNAL, "too many ops in an adjoint sweep");
+  for (uint32_t off : doff) {
+    ++hdr.ntab;
+    if (hdr.ntiles < kATabTiles || asweep_smem(hdr) > kATwoCtas) {
+      --hdr.ntab;
+      break;
+    }
+    reinterpret_cast<uint32_t*>(blob.data() + off + 5)[2] = hdr.ntab - 1;
+  }
+  pool.insert(pool.end(), blob.begin(), blob.end());
   return DQ_OK;
 }
 
-// Dynamic shared memory of a sweep: psi and lambda tiles, per-warp gradient
-// slots, the op list and the staged phase data (layout as in k_adj_sweep).
-size_t asweep_smem(uint32_t m, uint32_t nslots, uint32_t nops, uint32_t phase_ops) {
-  const size_t slots = ((size_t)(nslots ? nslots : 1) * kAWarps + 1) / 2 * 2;
-  const size_t nops2 = ((size_t)nops + 1) / 2 * 2;
-  return sizeof(double2) * 2 * (1u << m) + sizeof(double) * slots + sizeof(AOp) * nops2 +
-         sizeof(PSub) * phase_ops;
+// Dynamic shared memory of a sweep: psi and lambda tiles, phase tables, the
+// diagonal runs' records and factors, per-warp gradient slots, the op list and
+// the staged op data (layout as in adj_sweep_body).
+size_t asweep_smem(const ASweepHdr& h) {
+  const size_t nops2 = ((size_t)h.nops + 1) / 2 * 2;
+  return sizeof(double2) * (2 * (size_t)(1u << h.m) + (size_t)h.ntab * 4 * kAThreads + h.nblob +
+                            2 * kDFactors * (size_t)h.ndrun) +
+         sizeof(double) * (h.nslots ? h.nslots : 1) * kAWarps + sizeof(AOp) * nops2 +
+         sizeof(PSub) * (h.phase_ops ? h.phase_ops : kAPhaseOps);
 }
 
+// CTAs of a launch: two per SM.  Also lets the sweep kernels use all of an
+// SM's shared memory (sweeps of many different ops need more than half).
 int sweep_ctas(int device) {
   static std::mutex mu;
-  static int per_sm[64];
+  static int ctas[64];
   std::lock_guard<std::mutex> lk(mu);
-  if (per_sm[device & 63] == 0) {
-    const size_t smem_max = asweep_smem(kAMaxLocal, kAMaxSlots, kAMaxSweepOps, kAPhaseStage);
-    DQ_CUDA_TRY(cudaFuncSetAttribute(k_adj_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_max));
-    int b = 1;
-    DQ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_adj_sweep, kAThreads, smem_max));
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    per_sm[device & 63] = std::max(1, b) * sms;
+  if (ctas[device & 63] == 0) {
+    int sms = 148, most = 0;
+    DQ_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    DQ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    for (const void* k : {(const void*)k_adj_sweep, (const void*)k_adj_sweep_multi}) {
+      cudaFuncAttributes fa{};
+      DQ_CUDA_TRY(cudaFuncGetAttributes(&fa, k));
+      DQ_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       most - (int)fa.sharedSizeBytes));
+    }
+    ctas[device & 63] = 2 * sms;
   }
-  return per_sm[device & 63];
+  return ctas[device & 63];
 }
 
 // Segments of the backward pass in backward order: fused sweeps and the
@@ -1487,12 +1900,12 @@ int adjoint_backward_fused(double2* psi, double2* lam, uint32_t n, const dq_inst
     }
     const SweepRef& ref = refs[si++];
     const ASweepHdr& hdr = hdrs[ref.hdr];
-    const size_t smem = asweep_smem(hdr.m, hdr.nslots, hdr.nops, hdr.phase_ops);
+    const size_t smem = asweep_smem(hdr);
     k_adj_sweep<<<ref.grid, kAThreads, smem, st>>>(psi, lam, d_hdr + ref.hdr, d_ops + ref.op0, d_pool,
                                                     d_part);
     cu(cudaGetLastError(), "k_adj_sweep");
     if (ref.nslots && rc == DQ_OK) {
-      k_adj_slots<<<(ref.nslots + 127) / 128, 128, 0, st>>>(d_part, ref.nslots, ref.grid,
+      k_adj_slots<<<(ref.nslots + 3) / 4, 128, 0, st>>>(d_part, ref.nslots, ref.grid,
                                                             d_map + ref.slot0, d_slots);
       cu(cudaGetLastError(), "k_adj_slots");
     }
@@ -1599,7 +2012,7 @@ int adjoint_backward_batch(double2* const* psi, double2* const* lam, const std::
       job_ops.push_back(bo[b] + s.op0[k]);
       job_pool.push_back(bp[b]);
       job_map.push_back(bm[b] + s.slot0[k]);
-      smem[k] = std::max(smem[k], asweep_smem(h.m, h.nslots, h.nops, h.phase_ops));
+      smem[k] = std::max(smem[k], asweep_smem(h));
       maxsl[k] = std::max(maxsl[k], h.nslots);
     }
   }
@@ -1655,17 +2068,6 @@ int adjoint_backward_batch(double2* const* psi, double2* const* lam, const std::
     cu(cudaMemcpyAsync(d_pool, pool.data(), sizeof(double2) * pool.size(), cudaMemcpyHostToDevice, st), "copy");
     cu(cudaMemcpyAsync(d_map, map.data(), sizeof(uint32_t) * map.size(), cudaMemcpyHostToDevice, st), "copy");
     cu(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(AJob) * jobs.size(), cudaMemcpyHostToDevice, st), "copy");
-  }
-  {
-    static std::mutex mu;
-    static uint64_t attr_done = 0;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!((attr_done >> (device & 63)) & 1ULL)) {
-      const size_t smem_max = asweep_smem(kAMaxLocal, kAMaxSlots, kAMaxSweepOps, kAPhaseStage);
-      cu(cudaFuncSetAttribute(k_adj_sweep_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem_max), "cudaFuncSetAttribute");
-      attr_done |= 1ULL << (device & 63);
-    }
   }
   for (size_t k = 0; k < kmax && rc == DQ_OK; ++k) {
     const uint32_t nj = (uint32_t)(job0[k + 1] - job0[k]);

@@ -387,3 +387,56 @@ def test_straight_line_phases_match_per_gate(gpu, n, seed):
     e2, g2 = adjoint_gradient(c, theta, H, exec="per_gate")
     assert abs(e1 - e2) < 1e-12
     assert np.max(np.abs(g1 - g2)) < 1e-11, np.max(np.abs(g1 - g2))
+
+
+def layered_passes(n, layers, seed):
+    """Layers that become register passes and phases of every form: one, two or three
+    rotations about Y or X on a pass, fixed and trainable ones, two on a qubit, diagonal
+    runs before, between and alone, rotations by almost pi, cp (four Walsh terms), single
+    diagonal gates between controlled ones, and (seed odd) more one-qubit ops than are
+    staged once."""
+    rng = np.random.default_rng(seed)
+    c = ParamCircuit(n)
+    th = []
+
+    def p(x):
+        th.append(float(x))
+        return Param(len(th) - 1)
+
+    ang = lambda: rng.choice([rng.uniform(-3.2, 3.2), np.pi - 1e-5, np.pi + 1e-8, 0.0, 1e-9], p=[0.8, 0.05, 0.05, 0.05, 0.05])
+    for layer in range(layers):
+        for q in range(n):
+            if rng.random() < 0.85:
+                fixed = rng.random() < 0.2
+                getattr(c, "rx" if layer % 2 else "ry")(q, float(ang()) if fixed else p(ang()))
+            if layer % 3 == 2 and rng.random() < 0.4:
+                c.u3(q, p(ang()), p(ang()), p(ang()))
+            if layer % 4 == 3 or seed % 2:
+                c.rx(q, p(ang()))
+                c.ry(q, p(ang()))
+        for q in range(n):
+            k = rng.integers(4)
+            if k == 0:
+                c.rz(q, p(ang()))
+            elif k == 1:
+                c.rzz(q, (q + 1) % n, p(ang()))
+            elif k == 2:
+                c.cp(q, (q + 2) % n, p(ang()))
+        if layer == 1:
+            c.crx(0, n - 1, p(ang()))
+            c.rz(1, p(ang()))
+            c.cx(n - 1, 1)
+    return c, np.asarray(th)
+
+
+# tile of fewer bits than a warp's, of 4 to 11 bits, several tiles, phase tables (from 14 qubits)
+@pytest.mark.parametrize("n,layers,seed", [(3, 4, 0), (4, 5, 1), (6, 4, 2), (9, 4, 3), (11, 4, 4), (12, 4, 5), (14, 4, 6),
+                                           (14, 2, 7), (17, 4, 8)])
+def test_register_passes_match_per_gate(gpu, n, layers, seed):
+    # rounding of at most some 500 gates on both vectors, observable of norm below 20: 1e-11
+    c, theta = layered_passes(n, layers, seed)
+    H = random_observable(n, 8, seed=seed)
+    e1, g1 = adjoint_gradient(c, theta, H, exec="fused")
+    e2, g2 = adjoint_gradient(c, theta, H, exec="per_gate")
+    assert abs(e1 - e2) < 1e-12
+    assert np.max(np.abs(g1 - g2)) < 1e-11
