@@ -640,6 +640,16 @@ int do_gate_op(RunCtx& c, const GateOp& op, int cls) {
   return DQ_OK;
 }
 
+// The kernel class of a gate instruction (false: not a gate, or an unsupported one).
+bool gate_op_of(const dq_inst& in, GateOp& op) {
+  switch (in.kind) {
+    case DQ_ID: case DQ_U0: case DQ_BARRIER: case DQ_CLASSICAL: case DQ_G_NOOP: case DQ_G_OPAQUE:
+    case DQ_G_UNSUPPORTED: case DQ_MEASURE: case DQ_RESET:
+      return false;
+    default: return inst_to_op(in, op);
+  }
+}
+
 // One instruction whose conditions hold.
 int exec_inst(RunCtx& c, const dq_inst& in) {
   switch (in.kind) {
@@ -1070,15 +1080,45 @@ int dq_run(dq_state_t h, const dq_inst* prog, uint64_t ninst, const dq_cond* con
       }
     }
   } else {
-    for (uint64_t i = 0; i < ninst; ++i) {
-      const dq_inst& in = prog[i];
-      if (!cond_holds(in, conds, cbits, ncbits)) continue;
-      rc = exec_inst(c, in);
-      if (rc != DQ_OK) {
-        c.prof.failed_inst = (int64_t)i;
-        break;
+    // runs of gates go through memory together (a profiled run times each gate)
+    GateGroup group;
+    std::vector<uint64_t> grouped;
+    auto flush = [&]() -> int {
+      int r = DQ_OK;
+      if (group_worth(group, h->n)) {
+        r = launch_group(h->amp, h->n, group, h->stream, &c.prof.kernel_launches);
+        for (uint64_t k : grouped) ++(gate_qubit_count(prog[k].kind) == 1 ? c.prof.apply_one_qubit_calls
+                                                                           : c.prof.apply_n_qubit_calls);
+      } else {
+        for (uint64_t k : grouped)
+          if (r == DQ_OK) r = exec_inst(c, prog[k]);
       }
+      group.clear();
+      grouped.clear();
+      return r;
+    };
+    for (uint64_t i = 0; i < ninst && rc == DQ_OK; ++i) {
+      const dq_inst& in = prog[i];
+      GateOp op;
+      if (!c.timer.on && in.kind != DQ_MEASURE && in.kind != DQ_RESET && gate_op_of(in, op)) {
+        if (!cond_holds(in, conds, cbits, ncbits)) continue;
+        if (group_add(group, op)) {
+          grouped.push_back(i);
+          continue;
+        }
+        rc = flush();
+        if (rc == DQ_OK && group_add(group, op)) {
+          grouped.push_back(i);
+          continue;
+        }
+      } else {
+        rc = flush();
+        if (!cond_holds(in, conds, cbits, ncbits)) continue;
+      }
+      if (rc == DQ_OK) rc = exec_inst(c, in);
+      if (rc != DQ_OK) c.prof.failed_inst = (int64_t)i;
     }
+    if (rc == DQ_OK) rc = flush();
   }
   if (rc == DQ_OK) rc = sync_stream(h);
   const auto t1 = std::chrono::steady_clock::now();

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "dq_common.cuh"
 #include "dq_gates.hpp"
 
@@ -42,6 +44,31 @@ uint64_t marginal_workspace(uint32_t n, const uint32_t* qubits, uint32_t k, int 
 // marginal_workspace() doubles (nullptr: a stream-ordered temporary is used).
 int launch_marginal(const double2* s, uint32_t n, const uint32_t* qubits, uint32_t k,
                     double* d_out, double* d_work, Scratch& sc, cudaStream_t st, int device);
+// Consecutive gates applied in one pass (k_group).  group_add takes a gate if it
+// fits the group (at most four target qubits); a group that is not worth a
+// pass is launched gate by gate instead.
+constexpr int kGroupOps = 12;
+struct GateGroup {
+  struct Op {
+    GateClass cls;
+    uint32_t t0, t1;      // targets (GC_DIAG: its qubits, 64: none)
+    uint64_t ctrl;        // GC_PHASE: with the target
+    uint32_t mat;
+  };
+  std::vector<Op> ops;
+  std::vector<hc> mats;
+  uint64_t regs = 0;
+  double saved = 0.0;     // single launches less the gates' share of a pass (gate_costs)
+  void clear() {
+    ops.clear();
+    mats.clear();
+    regs = 0;
+    saved = 0.0;
+  }
+};
+bool group_add(GateGroup& g, const GateOp& op);
+bool group_worth(const GateGroup& g, uint32_t n);
+int launch_group(double2* s, uint32_t n, const GateGroup& g, cudaStream_t st, uint64_t* launches);
 // Marginal, CDF and samples in one launch, where the distribution fits one
 // block's scan and every output is summed by one thread: d_out holds the
 // shots' indices, then at entry (shots + 1) / 2 * 2 the 64-bit boundary count.
