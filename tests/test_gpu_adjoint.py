@@ -440,3 +440,25 @@ def test_register_passes_match_per_gate(gpu, n, layers, seed):
     e2, g2 = adjoint_gradient(c, theta, H, exec="per_gate")
     assert abs(e1 - e2) < 1e-12
     assert np.max(np.abs(g1 - g2)) < 1e-11
+
+
+@pytest.mark.parametrize("n", [1, 2, 8, 9, 10, 12, 13])
+def test_pauli_tiles(gpu, n):
+    # states of less than a thread's, a block's and a tile's amplitudes and of several tiles;
+    # groups of one and many terms with masks inside and outside the tile, real and imaginary
+    # coefficients.  1e-12: the tolerance of observables above (about 60 terms of order one)
+    rng = np.random.default_rng(n)
+    v = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    v /= np.linalg.norm(v)
+    terms = []
+    for x in [0, 1, (1 << n) - 1, 1 << (n - 1)] + [int(k) for k in rng.integers(1 << n, size=4)]:
+        zs = rng.integers(1 << n, size=int(rng.choice([1, 2, 9])))
+        terms += [(float(rng.normal()), x, int(z)) for z in zs]
+    arr = np.zeros(len(terms), dtype=nat.PAULI_DTYPE)
+    for k, t in enumerate(terms):
+        arr["coeff"][k], arr["xmask"][k], arr["zmask"][k] = t
+    st = nat.State(n, 0)
+    st.upload(v)
+    out = ctypes.c_double()
+    nat.check(nat.lib().dq_expval_pauli(st.handle, nat.ptr(arr), len(terms), ctypes.byref(out)))
+    assert abs(out.value - orc.expval_pauli(v, arr)) < 1e-12
