@@ -28,9 +28,9 @@
 // A sweep that ends with a pass writes its results straight to memory and
 // loads the next tile into the freed buffer meanwhile.
 // Gradient terms: Re sum conj(lambda_k) (D_j psi_{k-1}) with psi_{k-1} = V psi_k,
-// summed per thread, reduced per warp into shared slots [slot][warp], per CTA
-// in warp order, and over CTAs in CTA order by k_adj_slots: deterministic for
-// a fixed grid.
+// summed per thread, reduced per warp into shared slots [warp][slot], per CTA
+// in warp order, and over CTAs in a fixed order by k_adj_slots: deterministic
+// for a fixed grid.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stddef.h>
@@ -331,7 +331,7 @@ struct DTerm {
   double w;
   uint32_t code;  // source lane : 5, warp bits : 3, register : 3, two base bits : 6 each (63: none),
                   // registers that its 32 terms use : 8
-  uint32_t slot;  // kNone: padding
+  uint32_t slot;
 };
 struct DAng {
   double ang;
@@ -342,14 +342,15 @@ struct DAng {
 // both vectors); 1..3: exp(i H01), exp(i H02), exp(i H12) of the register
 // pairs; 4: counts; 5: masks and table; then its terms and angle lists.
 struct DCount {
-  uint32_t nterm;  // a multiple of 32 but for the last terms of a run
+  uint32_t nterm;
   uint32_t ends;   // local angles: cumulative ends of the lists of T, G0, G1, G2 (a byte each)
   uint32_t ncst, nlin;
 };
 struct DMask {
   uint32_t coupled;  // thread bits 0..7, register bits 8..10 with terms in base bits
   uint32_t pairs;    // register pairs 01, 02, 12 with a term
-  uint32_t tab, pad;
+  uint32_t tab;
+  uint32_t layers;   // its terms in up to four lists (a byte each) with one term of a gate each
 };
 constexpr uint32_t kDRunHdr = 6, kDFactors = 12;
 
@@ -416,7 +417,7 @@ __device__ __forceinline__ void diag_grads(const double2 (&a)[8], const double2 
                                            uint64_t base, bool valid, double* accw) {
   const int lane = threadIdx.x & 31;
   const uint32_t w = threadIdx.x >> 5;
-  const uint32_t nterm = reinterpret_cast<const DCount*>(B + 4)->nterm;
+  const uint32_t layers = reinterpret_cast<const DMask*>(B + 5)->layers;
   const DTerm* terms = reinterpret_cast<const DTerm*>(B + kDRunHdr);
   double z[8];
 #pragma unroll
@@ -437,21 +438,24 @@ __device__ __forceinline__ void diag_grads(const double2 (&a)[8], const double2 
   walsh_lane<1, 4>(z, lane);
   // the coefficient of register mask R, lane mask M is now in lane
   // R | (M & 3) << 3, register M3 | M4 << 1 | M2 << 2
-  for (uint32_t c0 = 0; c0 < nterm; c0 += 32) {
-    const uint32_t j = min(c0 + (uint32_t)lane, nterm - 1u);
-    const DTerm t = terms[j];
-    const uint32_t used = t.code >> 23, reg = (t.code >> 8) & 7u;
-    double v = 0.0;
+  for (uint32_t left = layers; left; left >>= 8) {
+    const uint32_t cnt = left & 0xffu;
+    for (uint32_t c0 = 0; c0 < cnt; c0 += 32) {
+      const DTerm t = terms[min(c0 + (uint32_t)lane, cnt - 1u)];
+      const uint32_t used = t.code >> 23, reg = (t.code >> 8) & 7u;
+      double v = 0.0;
 #pragma unroll
-    for (uint32_t r = 0; r < 8; ++r)
-      if (used >> r & 1u) {
-        const double x = __shfl_sync(0xffffffffu, z[r], (int)(t.code & 31u));
-        if (reg == r) v = x;
-      }
-    const uint32_t p = (t.code >> 11) & 63u, q = (t.code >> 17) & 63u;
-    const uint32_t neg = __popc((t.code >> 5) & w & 7u) + (p != 63u ? (uint32_t)(base >> p) & 1u : 0u) +
-                         (q != 63u ? (uint32_t)(base >> q) & 1u : 0u);
-    if (c0 + (uint32_t)lane < nterm && t.slot != kNone) accw[t.slot] += (neg & 1u) ? -t.w * v : t.w * v;
+      for (uint32_t r = 0; r < 8; ++r)
+        if (used >> r & 1u) {
+          const double x = __shfl_sync(0xffffffffu, z[r], (int)(t.code & 31u));
+          if (reg == r) v = x;
+        }
+      const uint32_t p = (t.code >> 11) & 63u, q = (t.code >> 17) & 63u;
+      const uint32_t neg = __popc((t.code >> 5) & w & 7u) + (p != 63u ? (uint32_t)(base >> p) & 1u : 0u) +
+                           (q != 63u ? (uint32_t)(base >> q) & 1u : 0u);
+      if (c0 + (uint32_t)lane < cnt) accw[t.slot] += (neg & 1u) ? -t.w * v : t.w * v;
+    }
+    terms += cnt;
   }
 }
 
@@ -1335,20 +1339,20 @@ void push_drun(std::vector<double2>& blob, const std::vector<AGate>& gates, cons
       layer[nt++].push_back(d);
     }
   }
-  // at most one term of a gate among 32 consecutive ones (a lane each)
+  // one term of a gate in a list (32 lanes take 32 terms and their slots at once)
   std::vector<DTerm> terms;
-  for (auto& l : layer) {
-    if (l.empty()) continue;
-    while (terms.size() % 32) terms.push_back(DTerm{0.0, 0, kNone});
+  uint32_t layers = 0;
+  for (int k = 0; k < 4; ++k) {
+    std::vector<DTerm>& l = layer[k];
+    layers |= (uint32_t)l.size() << (8 * k);
     std::stable_sort(l.begin(), l.end(), [](const DTerm& x, const DTerm& y) { return (x.code >> 8 & 7u) < (y.code >> 8 & 7u); });
+    for (size_t j = 0; j < l.size(); j += 32) {
+      uint32_t used = 0;
+      const size_t e = std::min(l.size(), j + 32);
+      for (size_t x = j; x < e; ++x) used |= 1u << (l[x].code >> 8 & 7u);
+      for (size_t x = j; x < e; ++x) l[x].code |= used << 23;
+    }
     terms.insert(terms.end(), l.begin(), l.end());
-  }
-  for (size_t j = 0; j < terms.size(); j += 32) {
-    uint32_t used = 0;
-    const size_t e = std::min(terms.size(), j + 32);
-    for (size_t k = j; k < e; ++k)
-      if (terms[k].slot != kNone) used |= 1u << (terms[k].code >> 8 & 7u);
-    for (size_t k = j; k < e; ++k) terms[k].code |= used << 23;
   }
   auto put = [&](double x, double y) { blob.push_back(make_double2(x, y)); };
   auto put4 = [&](uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -1376,7 +1380,7 @@ void push_drun(std::vector<double2>& blob, const std::vector<AGate>& gates, cons
   put((double)remainderl(c0, kTwoPi), (double)pre);
   for (int k = 0; k < 3; ++k) put((double)cosl(H[k]), (double)sinl(H[k]));
   put4((uint32_t)terms.size(), ends, (uint32_t)cst.size(), (uint32_t)lin.size());
-  put4(coupled, pairs, tab, 0);
+  put4(coupled, pairs, tab, layers);
   for (const DTerm& d : terms) {
     double2 x;
     memcpy(&x, &d, sizeof(x));
@@ -1711,7 +1715,7 @@ int encode_asweep(const ASweepPlan& sp, uint32_t n, ASweepHdr& hdr, std::vector<
       --hdr.ntab;
       break;
     }
-    reinterpret_cast<uint32_t*>(blob.data() + off + 5)[2] = hdr.ntab - 1;
+    reinterpret_cast<uint32_t*>(blob.data() + off + 5)[2] = hdr.ntab - 1;  // DMask::tab
   }
   pool.insert(pool.end(), blob.begin(), blob.end());
   return DQ_OK;
@@ -1719,7 +1723,9 @@ int encode_asweep(const ASweepPlan& sp, uint32_t n, ASweepHdr& hdr, std::vector<
 
 // Dynamic shared memory of a sweep: psi and lambda tiles, phase tables, the
 // diagonal runs' records and factors, per-warp gradient slots, the op list and
-// the staged op data (layout as in adj_sweep_body).
+// the staged op data (layout as in adj_sweep_body).  At most 160 KB: 64 of tiles,
+// 22 of records (4 terms and 3 angles a gate, 192 gates), 37 of factors (96 runs),
+// 12 of slots, 21 of ops; tables are added up to kATwoCtas only.
 size_t asweep_smem(const ASweepHdr& h) {
   const size_t nops2 = ((size_t)h.nops + 1) / 2 * 2;
   return sizeof(double2) * (2 * (size_t)(1u << h.m) + (size_t)h.ntab * 4 * kAThreads + h.nblob +

@@ -23,7 +23,7 @@
 // bound is the latency of one trajectory while histories are few, and the
 // shared memory and FP64 throughput of one trajectory per shot once every
 // shot is on its own.  4096 shots of 16 qubits with four measure / reset
-// pairs: 205 ms with one trajectory per shot, 0.88 ms here (16 histories); with
+// pairs: 205 ms with one trajectory per shot, 0.80 ms here (16 histories); with
 // 16 random outcomes per shot, every shot soon on its own: 132 ms and 96 ms.
 // Clusters take tasks until none is left or running; states otherwise stay in
 // shared memory, and only classical registers are written out.

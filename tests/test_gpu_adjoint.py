@@ -462,3 +462,21 @@ def test_pauli_tiles(gpu, n):
     out = ctypes.c_double()
     nat.check(nat.lib().dq_expval_pauli(st.handle, nat.ptr(arr), len(terms), ctypes.byref(out)))
     assert abs(out.value - orc.expval_pauli(v, arr)) < 1e-12
+
+
+@pytest.mark.parametrize("n,pairs", [(2, 20), (3, 96), (11, 96), (13, 40)])
+def test_many_diagonal_runs_of_one_sweep(gpu, n, pairs):
+    # as many runs as a sweep can have, each of a gate with four Walsh terms: the largest
+    # records and factors in shared memory (tolerances as above)
+    rng = np.random.default_rng(pairs)
+    c = ParamCircuit(n)
+    theta = rng.uniform(-np.pi, np.pi, size=2 * pairs)
+    for k in range(pairs):
+        a, b = rng.permutation(n)[:2].tolist()
+        c.cp(int(a), int(b), Param(2 * k))
+        c.ry(int(rng.integers(min(n, 8))), Param(2 * k + 1))
+    H = random_observable(n, 8, seed=n)
+    e1, g1 = adjoint_gradient(c, theta, H, exec="fused")
+    e2, g2 = adjoint_gradient(c, theta, H, exec="per_gate")
+    assert abs(e1 - e2) < 1e-12
+    assert np.max(np.abs(g1 - g2)) < 1e-11
