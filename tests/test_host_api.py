@@ -16,7 +16,7 @@ import pytest
 from _circuits import JsonCircuit, cond, g, gate
 from dqsim_bosonic_b200 import simulate_distributed, simulate_monolithic, simulate_monolithic_shots
 from dqsim_bosonic_b200 import _native as nat
-from dqsim_bosonic_b200.circuit import (CircuitDecodeError, count_cbits, decode_circuit_json, encode,
+from dqsim_bosonic_b200.circuit import (CircuitDecodeError, decode_circuit_json, encode,
                                         format_cbits)
 
 ROOT = Path(__file__).resolve().parents[1]
@@ -245,6 +245,8 @@ def test_mps_entry_points_reject_bad_arguments_without_a_gpu(engine_lib):
                                              (200, 200)])
 @pytest.mark.parametrize("shots", [0, 1, 257])
 def test_count_cbits_is_format_cbits_counted(num_cbits, space, shots):
+    from dqsim_bosonic_b200.circuit import count_cbits
+
     rng = np.random.default_rng(num_cbits + shots)
     rows = rng.integers(-1, 2, size=(shots, space), dtype=np.int32)
     rows[:, rng.random(space) < 0.9] = 0  # few distinct registers
