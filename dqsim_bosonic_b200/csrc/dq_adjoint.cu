@@ -960,18 +960,21 @@ int dq_adjoint_batch(int device, uint32_t n, const dq_inst* prog, uint64_t ninst
   for (uint64_t g0 = 0; g0 < nsets && rc == DQ_OK; g0 += G) {
     const uint64_t g1 = std::min(nsets, g0 + G), ng = g1 - g0;
     ++acc.groups;
-    // forward: sweep k of every set of the group in one launch per run width
+    // forward: sweep k of every set of the group in one launch per run width and
+    // kind of program (whether a set's sweep is rotation phases depends on its
+    // angles, and no kernel build runs both kinds)
     struct Range { size_t begin, end; uint32_t run_bits, max_bytes, flags; };
     std::vector<SweepJob> jobs;
     std::vector<Range> ranges;
     for (size_t k = 0; k < kf; ++k)
-      for (uint32_t rbits : {5u, 3u}) {
+      for (uint32_t kind = 0; kind < 4; ++kind) {
+        const uint32_t rbits = kind & 1 ? 3u : 5u, micro = kind & 2 ? SWF_MICRO : 0u;
         const size_t b0 = jobs.size();
         uint32_t mb = 0, fl = ~0u;
         for (uint64_t s = g0; s < g1; ++s) {
           if (k >= plans[s].foffs.size()) continue;
           const uint8_t* hp = plans[s].fblob.data() + plans[s].foffs[k];
-          if (sweep_run_bits(hp) != rbits) continue;
+          if (sweep_run_bits(hp) != rbits || (sweep_flags(hp) & SWF_MICRO) != micro) continue;
           const uint32_t pb = sweep_prog_bytes(hp);
           mb = std::max(mb, pb);
           fl &= sweep_flags(hp);

@@ -2329,7 +2329,7 @@ uint32_t sweep_prog_bytes(const uint8_t* prog) {
 
 uint32_t sweep_flags(const uint8_t* prog) {
   const SwHeader* h = reinterpret_cast<const SwHeader*>(prog);
-  return h->off_micro ? SWF_MICRO : h->flags;
+  return h->off_micro ? SWF_MICRO : h->flags | SWF_OPS;
 }
 
 int launch_sweep_multi(const SweepJob* d_jobs, uint32_t njobs, uint32_t n, uint32_t rb,
@@ -2337,6 +2337,7 @@ int launch_sweep_multi(const SweepJob* d_jobs, uint32_t njobs, uint32_t n, uint3
   if (!njobs) return DQ_OK;
   if (n < 7 + rb) return fail(DQ_ERR_INVALID_ARG, "state smaller than a tile");
   if (max_bytes > (uint32_t)max_prog(7 + (int)rb)) return fail(DQ_ERR_INTERNAL, "sweep program too large");
+  if (!(flags & (SWF_MICRO | SWF_OPS))) return fail(DQ_ERR_INTERNAL, "rotation phases and ops in one launch");
   const bool r3 = run_bits == 3;
   switch (rb) {
     case 2: return r3 ? launch_sweep_multi_t<7, 2, 3>(d_jobs, njobs, n, max_bytes, st)

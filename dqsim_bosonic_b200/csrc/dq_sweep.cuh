@@ -93,8 +93,6 @@ constexpr uint32_t SWF_UONLY = 2u;
 // every phase of the sweep is a straight-line phase (OP_HPHASE) of real 2x2
 // sub-ops only: the launch may use the build with that path only
 constexpr uint32_t SWF_RONLY = 4u;
-// (sweep_flags only, alone: the program has rotation phases)
-constexpr uint32_t SWF_MICRO = 8u;
 // Builds of the tile loop: the whole op interpreter, Hadamard-pattern
 // straight-line phases only, plain one-qubit ops only, real-2x2 straight-line
 // phases only, rotation phases only.

@@ -7,6 +7,7 @@ central finite differences with h = 1e-6: 1e-7 (truncation ~h^2, rounding
 ~1e-16/h).
 """
 import ctypes
+import math
 
 import numpy as np
 import pytest
@@ -480,3 +481,54 @@ def test_many_diagonal_runs_of_one_sweep(gpu, n, pairs):
     e2, g2 = adjoint_gradient(c, theta, H, exec="per_gate")
     assert abs(e1 - e2) < 1e-12
     assert np.max(np.abs(g1 - g2)) < 1e-11
+
+
+def qaoa(n, layers):
+    c = ParamCircuit(n)
+    for q in range(n):
+        c.h(q)
+    for k in range(layers):
+        for q in range(n):
+            c.rzz(q, (q + 1) % n, Param(2 * k, 2.0))
+        for q in range(n):
+            c.rx(q, Param(2 * k + 1, 2.0))
+    return c
+
+
+def u3_layers(n):
+    c = ParamCircuit(n)
+    for q in range(n):
+        c.u3(q, Param(0), Param(1), Param(2))
+    for q in range(0, n - 1, 2):
+        c.cx(q, q + 1)
+    for q in range(n):
+        c.u3(q, Param(3), Param(1), Param(2))
+    return c
+
+
+# sets whose sweeps are rotation phases beside sets whose sweeps are ops: mixing angle 0 or
+# pi / 2 (rx(2 beta) is diagonal or X) and phases 0 (u3 is real) among random ones
+@pytest.mark.parametrize("n,kind", [(11, "qaoa"), (12, "qaoa"), (12, "u3"), (20, "qaoa"), (20, "u3")])
+def test_batched_sets_with_plans_of_different_kinds(gpu, n, kind):
+    # single sets: as above; gate by gate: rounding of at most 160 gates, observable of norm
+    # below 20
+    from dqsim_bosonic_b200.adjoint import adjoint_gradient_batch
+
+    rng = np.random.default_rng(n)
+    c = qaoa(n, 2) if kind == "qaoa" else u3_layers(n)
+    thetas = rng.uniform(0.1, 1.4, size=(6, c.num_params))
+    if kind == "qaoa":
+        thetas[0, 1::2] = 0.0
+        thetas[2, 1::2] = math.pi / 2
+        thetas[4, 1] = 0.0
+    else:
+        thetas[1, 1:3] = 0.0
+        thetas[3, [0, 3]] = 0.0
+        thetas[4, 1:3] = 0.0
+    H = random_observable(n, 8, seed=n)
+    es, gs = adjoint_gradient_batch(c, thetas, H)
+    for b in range(len(thetas)):
+        for mode in ("fused", "per_gate"):
+            e1, g1 = adjoint_gradient(c, thetas[b], H, exec=mode)
+            assert abs(es[b] - e1) < 1e-11
+            assert np.max(np.abs(gs[b] - g1)) < 1e-11
