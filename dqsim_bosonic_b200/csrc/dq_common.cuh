@@ -55,12 +55,16 @@ __device__ __forceinline__ double norm_sqr_x(double2 a) {
   return __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y));
 }
 
-// a / b correctly rounded, given y = 1 / b correctly rounded: two Newton
-// corrections of a y with exact remainders (Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", 1990), 5
-// operations instead of a division's sequence when many numbers are divided by
-// one.  Outside the range where the remainders are exact it divides.
+// a / b correctly rounded, given y = divisor(b): two Newton corrections of a y
+// with exact remainders (Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", 1990), 5 operations instead of a division's
+// sequence when many numbers are divided by one.  Outside the range where the
+// quotient is normal and the remainders are exact it divides.
+__device__ __forceinline__ double divisor(double b) {  // 1 / b correctly rounded, 0: divide
+  return b > 1e-50 && b < 1e50 ? __drcp_rn(b) : 0.0;
+}
 __device__ __forceinline__ double div_by(double a, double b, double y) {
+  if (y == 0.0) return __ddiv_rn(a, b);
   if (!(fabs(a) > 1e-250 && fabs(a) < 1e250)) return a == 0.0 ? a : __ddiv_rn(a, b);
   double q = a * y;
   q = fma(fma(-b, q, a), y, q);

@@ -366,7 +366,7 @@ __global__ void k_collapse(double2* __restrict__ s, uint64_t count, uint64_t bit
     s[i] = make_double2(0.0, 0.0);
   } else {
     const double2 a = s[i];
-    const double y = __drcp_rn(norm);
+    const double y = divisor(norm);
     s[i] = make_double2(div_by(a.x, norm, y), div_by(a.y, norm, y));
   }
 }

@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(THREADS) k_traj(const TrajParams P) {
     auto collapse = [&](const TOp& op, int o, double norm) {
       const uint32_t q = op.t1;
       const uint64_t qb = 1ULL << q;
-      const double y = __drcp_rn(norm);
+      const double y = divisor(norm);
       for (uint32_t i = tid; i < L; i += THREADS) {
         const bool set = ((gbase | i) & qb) != 0;
         if (set != (o == 1)) {

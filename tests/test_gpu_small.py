@@ -107,3 +107,37 @@ def test_collapse_is_a_division(gpu, n, p1, outcome):
     got = st.download()
     assert got.tobytes() == want.tobytes() or (
         np.array_equal(got.real, want.real) and np.array_equal(got.imag, want.imag))
+
+
+# norms of unnormalised states: infinite and undefined ones, and ones so large that quotients
+# are denormal
+@pytest.mark.parametrize("n", [1, 5, 14])
+@pytest.mark.parametrize("p1", [np.inf, np.nan, 1e302, 1e140, 1e100])
+def test_collapse_by_extreme_norms(gpu, n, p1):
+    rng = np.random.default_rng(n)
+    v = (rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)) * 2.0 ** rng.integers(-820, 500, size=1 << n)
+    v.real[rng.random(1 << n) < 0.1] = -0.0
+    st = nat.State(n, 0)
+    st.upload(v)
+    q = n // 2
+    nat.check(nat.lib().dq_collapse(st.handle, q, 1, p1))
+    norm = max(np.sqrt(p1), 1e-15) if p1 == p1 else p1
+    keep = ((np.arange(1 << n) >> q) & 1) == 1
+    got = st.download()
+    assert np.array_equal(got.real, np.where(keep, v.real / norm, 0.0), equal_nan=True)
+    assert np.array_equal(got.imag, np.where(keep, v.imag / norm, 0.0), equal_nan=True)
+
+
+@pytest.mark.parametrize("n", [3, 12, 14])
+@pytest.mark.parametrize("mode", [nat.EXEC_PER_GATE, nat.EXEC_FUSED])
+def test_measurement_of_an_infinite_norm(gpu, n, mode):
+    # p1 overflows: outcome 1, and every finite amplitude over infinity is zero
+    prog = prog_of(JsonCircuit(n, [g("measure", 0, 0)], ncbits=1))
+    v = np.full(1 << n, 1e160 + 1e-3j)
+    want, wcb, rc, _ = _oracle.run(prog, 3, v)
+    assert rc == 0
+    st = nat.State(n, 0)
+    st.upload(v)
+    cb, _ = run_program(st, prog, 3, nat.SEM_SIMULATE, mode)
+    assert cb.tolist() == wcb.tolist() == [1]
+    assert np.array_equal(st.download(), want)
