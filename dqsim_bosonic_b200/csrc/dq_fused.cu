@@ -611,6 +611,21 @@ bool split_unitary(const hc* u, long double* c, long double* s, hx* cst, hx* phi
          off(u[2], *cst * *phi * ps) < 4e-15L && off(u[3], *cst * *phi * *lam * pc) < 4e-15L;
 }
 
+// The banks (of 16 bytes) that sums of address vectors reach.
+struct BankSpan {
+  uint32_t have = 1;  // bit v: the bank offset v is a sum of the vectors added
+  bool add(uint32_t vec) {
+    const uint32_t v = vec & 7u;
+    if (have >> v & 1u) return false;
+    uint32_t more = have;
+    for (uint32_t u = 0; u < 8; ++u)
+      if (have >> u & 1u) more |= 1u << (u ^ v);
+    have = more;
+    return true;
+  }
+  bool all() const { return have == 0xffu; }
+};
+
 struct MicroPlanner {
   const Planner& pl;
   // Against Planner::budget (96): a sweep takes up to 60 rotations.  28-qubit
@@ -725,11 +740,21 @@ struct MicroPlanner {
     memcpy(ph.vec, T.vec, sizeof(ph.vec));
     ph.off = T.off;
   }
-  // Fills the phase's registers with the highest local qubits that are left,
-  // so that qubits 0..2 stay thread bits.
-  void fill(MPhase& ph, const std::vector<uint32_t>& local) {
+  // Fills the phase's registers with the highest local qubits that are left, so
+  // that qubits 0..2 stay thread bits.  vec (null for a phase that writes the
+  // state, whose thread order is fixed): those first that leave thread bits
+  // reaching every bank.
+  void fill(MPhase& ph, const std::vector<uint32_t>& local, const uint32_t* vec) {
+    auto has = [&](uint32_t q) { return std::find(ph.regs.begin(), ph.regs.end(), q) != ph.regs.end(); };
+    for (size_t k = local.size(); vec && k-- > 0 && ph.regs.size() < 4;) {
+      if (has(local[k])) continue;
+      BankSpan left;
+      for (size_t i = 0; i < local.size(); ++i)
+        if (i != k && !has(local[i])) left.add(vec[i]);
+      if (left.all()) ph.regs.push_back(local[k]);
+    }
     for (size_t k = local.size(); k-- > 0 && ph.regs.size() < 4;)
-      if (std::find(ph.regs.begin(), ph.regs.end(), local[k]) == ph.regs.end()) ph.regs.push_back(local[k]);
+      if (!has(local[k])) ph.regs.push_back(local[k]);
   }
 
   // The phases of the gates `todo` (program order), whose targets are in the tile.
@@ -846,7 +871,7 @@ struct MicroPlanner {
       for (int x : rots) ph.regs.push_back(G[x].t0);
       for (uint32_t q : pick)
         if (!has(ph.regs, q)) ph.regs.push_back(q);
-      fill(ph, sw.local);
+      fill(ph, sw.local, T.vec);
       table(ph, poly);
       for (uint32_t q : ph.regs)
         if (poly.pending(q) && (must >> q & 1ULL || std::any_of(rots.begin(), rots.end(), [&](int x) {
@@ -871,7 +896,7 @@ struct MicroPlanner {
         if (q < 3) direct = false;
     if (!direct) {
       MPhase ph;
-      fill(ph, sw.local);
+      fill(ph, sw.local, nullptr);
       for (auto& x : ph.lin) x = hx{1, 0};
       for (auto& r : ph.quad)
         for (auto& x : r) x = hx{1, 0};
@@ -932,7 +957,7 @@ struct MicroPlanner {
     if (poly.empty() && !poly.has_cst) return;
     PSweep& last = sweeps.back();
     MPhase ph;
-    fill(ph, last.local);
+    fill(ph, last.local, nullptr);
     // after an address change (of an empty last phase, or none) the state's order
     const MPhase& before = last.micro.back();
     memcpy(ph.vec, before.vec, sizeof(ph.vec));
@@ -956,21 +981,17 @@ struct MicroPlanner {
   }
 };
 
-// choose thread-bit order: lanes 0..2 need linearly independent swizzle vectors
-bool order_thread_bits(std::vector<uint32_t>& tb, const uint32_t* vec) {
-  const size_t c = tb.size();
-  for (size_t i = 0; i < c; ++i)
-    for (size_t j = i + 1; j < c; ++j)
-      for (size_t k = j + 1; k < c; ++k) {
-        const uint32_t a = vec[tb[i]] & 7u, b = vec[tb[j]] & 7u, d = vec[tb[k]] & 7u;
-        if (a == 0 || b == 0 || a == b || d == 0 || d == a || d == b || d == (a ^ b)) continue;
-        std::vector<uint32_t> o = {tb[i], tb[j], tb[k]};
-        for (size_t x = 0; x < c; ++x)
-          if (x != i && x != j && x != k) o.push_back(tb[x]);
-        tb = o;
-        return true;
-      }
-  return false;
+// Thread-bit order: lanes 0..2 take bits with linearly independent swizzle
+// vectors, the first ones there are.  With three of them eight lanes reach all
+// banks.  CX gates folded into the address vectors can leave fewer, where a
+// phase's own qubits need the rest in registers: its accesses then take two to
+// eight times as long, at the right addresses all the same.
+void order_thread_bits(std::vector<uint32_t>& tb, const uint32_t* vec) {
+  std::vector<uint32_t> lead, rest;
+  BankSpan span;
+  for (uint32_t b : tb) (span.add(vec[b]) ? lead : rest).push_back(b);
+  lead.insert(lead.end(), rest.begin(), rest.end());
+  tb = lead;
 }
 
 // Thread and register layout of a phase whose register bits are the local
@@ -987,8 +1008,8 @@ int phase_layout(const std::vector<uint32_t>& regs, uint32_t m, uint32_t TBn, ui
   pl.tb.clear();
   for (uint32_t b = 0; b < m; ++b)
     if (std::find(regs.begin(), regs.end(), b) == regs.end()) pl.tb.push_back(b);
-  if (pl.tb.size() != (size_t)kSwTB || (!keep_low && !order_thread_bits(pl.tb, vec)))
-    return fail(DQ_ERR_INTERNAL, "no bank-conflict-free thread layout");
+  if (pl.tb.size() != (size_t)kSwTB) return fail(DQ_ERR_INTERNAL, "phase without its register bits");
+  if (!keep_low) order_thread_bits(pl.tb, vec);
   for (int i = 0; i < kMaxM; ++i) pl.rix[i] = pl.tix[i] = -1;
   for (uint32_t b = 0; b < RB; ++b) {
     sp.V[b] = vec[regs[b]];
