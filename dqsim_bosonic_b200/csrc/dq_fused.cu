@@ -362,6 +362,8 @@ struct PSweep {
   std::vector<uint32_t> local;  // physical, ascending, size m
   std::vector<POp> ops;
   std::vector<MPhase> micro;    // rotation phases (then ops is empty)
+  size_t bytes = 0;             // what their program takes at most, and its slots
+  uint32_t slots = 0;
 };
 
 // Blob writer (16-byte aligned sections)
@@ -630,8 +632,10 @@ struct MicroPlanner {
   const Planner& pl;
   // Against Planner::budget (96): a sweep takes up to 60 rotations.  28-qubit
   // brickwork of 20 layers: 105 ms, 108 ms with up to 42, 110 ms with up to 29.
-  double rot_cost = 1.6;
-  uint32_t max_rot = 64;
+  // X and CX cost nothing here; where they need phases, the program's size ends
+  // the sweep (full).
+  static constexpr double rot_cost = 1.6;
+  static constexpr uint32_t max_rot = 64;
   // The segment with general gates split into phase, rotation (|t| <= 1) and
   // phase: small records, since every sweep and phase scans them.
   struct MGate {
@@ -731,6 +735,32 @@ struct MicroPlanner {
     to.push_back(std::move(f));
   }
 
+  // What the encoded program takes: without phases, of a phase without factors
+  // (with its table), of a factor (its slot, a term per qubit or pair outside the
+  // tile, its tables).
+  size_t frame_bytes() const {
+    return sizeof(SwHeader) + sizeof(SwGStore) + ((sizeof(uint64_t) + sizeof(uint32_t)) << (pl.M - kMinRunBits)) +
+           16 * 16;  // sections start at multiples of 16
+  }
+  static size_t factor_bytes(size_t terms, bool tables) {
+    return sizeof(SwSlot) + sizeof(SwFinal) + sizeof(SwSlotEnt) * terms + (tables ? sizeof(double2) * (32 + 8 + 16) : 0);
+  }
+  static constexpr size_t table_bytes = sizeof(double2) * 16;
+  static constexpr size_t phase_bytes = sizeof(SwPhase) + sizeof(SwMPhase) + table_bytes;
+  void count(PSweep& sw, const MPhase& ph) const {
+    sw.bytes += phase_bytes - (ph.table ? 0 : table_bytes);
+    for (const auto* fs : {&ph.cross, &ph.fin})
+      for (const MFactor& f : *fs) {
+        sw.bytes += factor_bytes(f.terms.size() + f.partners.size(), !f.partners.empty());
+        ++sw.slots;
+      }
+  }
+  // No room for a phase with four factors and the phase that may close the sweep.
+  bool full(const PSweep& sw) const {
+    return sw.bytes + 2 * phase_bytes + 4 * factor_bytes(pl.n, true) > (size_t)max_prog((int)pl.M) ||
+           sw.slots + 4 > (uint32_t)kMaxSlots;
+  }
+
   struct Tile {            // addresses of the local qubits (of the tile being planned)
     uint64_t S = 0, all = 0;  // local qubits; qubits its gates touch
     int lidx[64];
@@ -757,9 +787,11 @@ struct MicroPlanner {
       if (!has(local[k])) ph.regs.push_back(local[k]);
   }
 
-  // The phases of the gates `todo` (program order), whose targets are in the tile.
-  void phases(std::vector<int> todo, PSweep& sw, PolyX& poly) {
+  // The phases of the gates `todo` (program order), whose targets are in the
+  // tile.  Returns those that a full sweep has no room for.
+  std::vector<int> phases(std::vector<int> todo, PSweep& sw, PolyX& poly) {
     Tile T;
+    sw.bytes = frame_bytes();
     for (int& x : T.lidx) x = -1;
     for (int gi : todo) T.all |= G[gi].touched;
     for (uint32_t k = 0; k < sw.local.size(); ++k) {
@@ -813,7 +845,7 @@ struct MicroPlanner {
         return true;
       })) {
       }
-      if (todo.empty()) break;
+      if (todo.empty() || full(sw)) break;
       // targets that can go into a phase now, in program order
       std::vector<uint32_t> cand;
       uint64_t seen = 0, blocked = 0;
@@ -885,6 +917,7 @@ struct MicroPlanner {
         poly.has_cst = true;
       }
       seal(ph, T);
+      count(sw, ph);
       sw.micro.push_back(std::move(ph));
     }
     // the last phase writes the state by logical addresses: qubits 0..2 must be
@@ -901,13 +934,17 @@ struct MicroPlanner {
       for (auto& r : ph.quad)
         for (auto& x : r) x = hx{1, 0};
       seal(ph, T);
+      count(sw, ph);
       sw.micro.push_back(std::move(ph));
     }
+    return todo;
   }
 
   void plan(PolyX& poly, std::vector<PSweep>& out) {
     std::vector<int> rem(G.size());
     for (size_t i = 0; i < G.size(); ++i) rem[i] = (int)i;
+    uint64_t all = 0;
+    for (const MGate& g : G) all |= g.touched;
     const uint64_t low = pl.single_tile ? ((1ULL << pl.n) - 1) : pl.pinned;
     while (!rem.empty()) {
       // the gates of this sweep, as in Planner::plan
@@ -916,8 +953,13 @@ struct MicroPlanner {
       uint32_t rots = 0;
       bool any = false;
       std::vector<int> incl, next;
-      for (int gi : rem) {
+      for (size_t i = 0; i < rem.size(); ++i) {
+        const int gi = rem[i];
         const MGate& g = G[gi];
+        if (blocked == all) {  // nothing later can be taken
+          next.insert(next.end(), rem.begin() + (ptrdiff_t)i, rem.end());
+          break;
+        }
         bool take = !(g.touched & blocked);
         if (take && g.kind != PG_DIAG) {
           const uint64_t ns = S | (1ULL << g.t0);
@@ -947,21 +989,23 @@ struct MicroPlanner {
         for (int gi : incl) add_diag(poly, G[gi]);
         continue;
       }
-      phases(std::move(incl), sw, poly);
+      const std::vector<int> left = phases(std::move(incl), sw, poly);
       out.push_back(std::move(sw));
+      if (left.empty()) continue;
+      next.clear();
+      std::merge(rem.begin(), rem.end(), left.begin(), left.end(), std::back_inserter(next));
+      rem.swap(next);
     }
   }
 
-  // Every pending term, in a last phase of the last sweep.
+  // Every pending term, in a last phase of the last sweep, or where that has no
+  // room for it in a sweep of its own (whose program is well below the limit:
+  // a factor per tile qubit and a term per pair of qubits).
   void final_flush(PolyX& poly, std::vector<PSweep>& sweeps) {
     if (poly.empty() && !poly.has_cst) return;
     PSweep& last = sweeps.back();
     MPhase ph;
     fill(ph, last.local, nullptr);
-    // after an address change (of an empty last phase, or none) the state's order
-    const MPhase& before = last.micro.back();
-    memcpy(ph.vec, before.vec, sizeof(ph.vec));
-    ph.off = before.off;
     table(ph, poly);
     for (uint32_t q : ph.regs)
       if (poly.pending(q)) take_factor(ph.cross, poly, q);
@@ -975,6 +1019,21 @@ struct MicroPlanner {
     }
     if (!tile.terms.empty()) ph.fin.push_back(std::move(tile));
     poly.init(poly.n);
+    const size_t used = last.bytes;
+    count(last, ph);
+    if (last.bytes > (size_t)max_prog((int)pl.M) || last.slots > (uint32_t)kMaxSlots) {
+      PSweep own;
+      own.local = last.local;
+      own.bytes = frame_bytes() + last.bytes - used;
+      for (uint32_t k = 0; k < own.local.size(); ++k) ph.vec[k] = swz(1u << k);
+      own.micro.push_back(std::move(ph));
+      sweeps.push_back(std::move(own));
+      return;
+    }
+    // after an address change (of an empty last phase, or none) the state's order
+    const MPhase& before = last.micro.back();
+    memcpy(ph.vec, before.vec, sizeof(ph.vec));
+    ph.off = before.off;
     // an empty last phase is replaced
     if (before.t.empty() && !before.table && before.cross.empty() && before.flips.empty()) last.micro.pop_back();
     last.micro.push_back(std::move(ph));
@@ -2057,38 +2116,35 @@ int fused_run_segment(double2* amp, uint32_t n, std::vector<PGate>& G, Planner& 
     return DQ_OK;
   };
   // one pass of the planner with the given low qubits pinned
-  const bool micro = pl.micro_ok && poly.empty() && !poly.has_cst && micro_eligible(G);
-  uint32_t max_rot = 64;
+  bool micro = pl.micro_ok && poly.empty() && !poly.has_cst && micro_eligible(G);
   auto plan_with = [&](uint64_t pinned, Poly& p, std::vector<PSweep>& out) {
     pl.pinned = pinned;
     out.clear();
-    if (micro) {
-      MicroPlanner mp{pl};
-      mp.max_rot = max_rot;
-      mp.split(G);
-      PolyX px;  // a segment starts without pending terms
-      px.init(pl.n);
-      if (mp.ok) {
-        mp.plan(px, out);
-        if (!out.empty()) {
-          mp.final_flush(px, out);
-          return;
-        }
-      }
-      pl.plan(G, p, out);
-    } else {
-      pl.plan(G, p, out);
-    }
+    pl.plan(G, p, out);
     pl.final_flush(p, out);
   };
-  const Poly poly0 = poly;
   const uint64_t pin0 = pl.pinned;
-  for (;;) {
+  if (micro) {
+    // rotation phases are cheap enough that the two more tile qubits of
+    // 128-byte runs always save sweeps (28-qubit brickwork: 30 against 45)
+    if (pl.pin_auto) pl.pinned = 0x7ULL;
+    MicroPlanner mp{pl};
+    mp.split(G);
+    PolyX px;  // a segment starts without pending terms
+    px.init(pl.n);
+    if (mp.ok) mp.plan(px, sweeps);
+    micro = !sweeps.empty();  // no plan: not all gates are unitary, or none needs a sweep
     if (micro) {
-      // rotation phases are cheap enough that the two more tile qubits of
-      // 128-byte runs always save sweeps (28-qubit brickwork: 30 against 45)
-      plan_with(pl.pin_auto ? 0x7ULL : pin0, poly, sweeps);
-    } else if (pl.pin_auto && !pl.single_tile) {
+      mp.final_flush(px, sweeps);
+      if (encode() != DQ_OK) {  // planned as general ops instead
+        clear_error();
+        micro = false;
+      }
+    }
+    pl.pinned = pin0;
+  }
+  if (!micro) {
+    if (pl.pin_auto && !pl.single_tile) {
       // plan with qubits 0..4 pinned and with 0..2 pinned; the wider tile
       // choice wins only when it saves at least a tenth of the sweeps (its
       // 128-byte runs cost a little more per sweep)
@@ -2104,13 +2160,7 @@ int fused_run_segment(double2* amp, uint32_t n, std::vector<PGate>& G, Planner& 
       plan_with(pin0, poly, sweeps);
     }
     if (sweeps.empty()) return DQ_OK;
-    const int rc = encode();
-    if (rc == DQ_OK) break;
-    if (!micro || max_rot <= 8) return rc;
-    // a sweep's micro program outgrew its place in shared memory or its slots
-    clear_error();
-    max_rot /= 2;
-    poly = poly0;
+    DQ_TRY(encode());
   }
   blob.align16();
   if (fw.plan_out) {  // plan-only: hand the programs back instead of running them

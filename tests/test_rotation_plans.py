@@ -62,7 +62,22 @@ def smallest(n, _, rng):
     return [g("rx", 0, 0.7)] + [g("cx", a, b) for a, b in [(1, 2), (3, 2), (6, 2), (3, 10), (2, 10)]]
 
 
+def outside(n, cxs, rng, controls=1, targets=8):
+    """CX controlled from outside the tile: each phase takes four."""
+    return [u3(rng, 0)] + [g("cx", n - 1 - i % controls, i // controls % targets) for i in range(cxs)]
+
+
+def outside_pairs(n, cxs, rng):
+    """The same, then a phase for every pair of qubits: a last flush of every size."""
+    pairs = [g("cp", a, b, float(rng.uniform(0, 6))) for a in range(n) for b in range(a + 1, n)]
+    return outside(n, cxs, rng) + pairs
+
+
 FAMILIES = {
+    "outside": outside,
+    "outside_one": lambda n, k, rng: outside(n, k, rng, 1, 1),
+    "outside_many": lambda n, k, rng: outside(n, k, rng, 5),
+    "outside_pairs": outside_pairs,
     "smallest": smallest,
     "all_to_all": all_to_all,
     "pauli": pauli_evolution,
@@ -90,7 +105,10 @@ def oracle_case(kind, n, size, seed):
 
 SMALL = [("smallest", 11, 0), ("all_to_all", 11, 3), ("all_to_all", 13, 2), ("pauli", 11, 20), ("pauli", 14, 12),
          ("cx_half", 11, 400), ("cx_half", 12, 1000), ("cx_most", 11, 200), ("cx_most", 12, 1000), ("cx_most", 14, 400),
-         ("cx_nearly_all", 12, 400), ("cx_diagonal", 11, 300), ("cx_diagonal", 13, 500)]
+         ("cx_nearly_all", 12, 400), ("cx_diagonal", 11, 300), ("cx_diagonal", 13, 500),
+         # programs of more than one sweep's room
+         ("outside", 14, 200), ("outside", 13, 800), ("outside_one", 14, 800), ("outside_many", 16, 480),
+         ("outside_pairs", 13, 60), ("outside_pairs", 13, 80), ("outside_pairs", 13, 120), ("outside_pairs", 14, 160)]
 
 
 @pytest.mark.parametrize("kind,n,size", SMALL)
@@ -103,7 +121,9 @@ def test_plans_match_oracle(engine_lib, kind, n, size, seed):
 
 # sizes the oracle is slow for: every program has a plan
 @pytest.mark.parametrize("kind,size", [("all_to_all", 1), ("all_to_all", 5), ("pauli", 30), ("cx_half", 1000),
-                                       ("cx_most", 3000), ("cx_nearly_all", 1000), ("cx_diagonal", 3000)])
+                                       ("cx_most", 3000), ("cx_nearly_all", 1000), ("cx_diagonal", 3000),
+                                       ("outside", 3000), ("outside_one", 800), ("outside_many", 2000),
+                                       ("outside_pairs", 120)])
 @pytest.mark.parametrize("n", [17, 20, 24, 30])
 def test_every_program_has_a_plan(engine_lib, kind, size, n):
     for seed in range(8):
