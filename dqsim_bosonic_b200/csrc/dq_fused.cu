@@ -851,11 +851,13 @@ struct MicroPlanner {
       uint64_t seen = 0, blocked = 0;
       for (int gi : todo) {
         const MGate& g = G[gi];
-        if (!(g.touched & blocked) && !((seen >> g.t0) & 1ULL)) {
+        const bool now = g.kind != PG_DIAG && !(g.touched & blocked);
+        if (now && !((seen >> g.t0) & 1ULL)) {
           cand.push_back(g.t0);
           seen |= 1ULL << g.t0;
         }
-        blocked |= g.touched;
+        // (a control outside the tile is no one's target here)
+        blocked |= now && g.ctrl >= 0 && T.lidx[g.ctrl] < 0 ? 1ULL << g.t0 : g.touched;
       }
       // up to four of them, a target's quadratic partners with it; spare places
       // to partners that are not targets now (their terms then need no factor

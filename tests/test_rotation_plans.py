@@ -5,6 +5,7 @@ Tolerance: the fused path's 1e-12; a few thousand gates on unit-norm states roun
 1e-13.
 """
 import math
+import struct
 
 import numpy as np
 import pytest
@@ -108,7 +109,7 @@ SMALL = [("smallest", 11, 0), ("all_to_all", 11, 3), ("all_to_all", 13, 2), ("pa
          ("cx_nearly_all", 12, 400), ("cx_diagonal", 11, 300), ("cx_diagonal", 13, 500),
          # programs of more than one sweep's room
          ("outside", 14, 200), ("outside", 13, 800), ("outside_one", 14, 800), ("outside_many", 16, 480),
-         ("outside_pairs", 13, 60), ("outside_pairs", 13, 80), ("outside_pairs", 13, 120), ("outside_pairs", 14, 160)]
+         ("outside_pairs", 13, 60), ("outside_pairs", 13, 80), ("outside_pairs", 13, 120), ("outside_pairs", 14, 160), ("outside_pairs", 13, 280), ("outside_pairs", 13, 320)]
 
 
 @pytest.mark.parametrize("kind,n,size", SMALL)
@@ -119,7 +120,7 @@ def test_plans_match_oracle(engine_lib, kind, n, size, seed):
     assert np.max(np.abs(canonical(got, perm) - want)) < ATOL
 
 
-# sizes the oracle is slow for: every program has a plan
+# sizes the oracle is slow for: every program has a plan, of rotation phases
 @pytest.mark.parametrize("kind,size", [("all_to_all", 1), ("all_to_all", 5), ("pauli", 30), ("cx_half", 1000),
                                        ("cx_most", 3000), ("cx_nearly_all", 1000), ("cx_diagonal", 3000),
                                        ("outside", 3000), ("outside_one", 800), ("outside_many", 2000),
@@ -127,7 +128,15 @@ def test_plans_match_oracle(engine_lib, kind, n, size, seed):
 @pytest.mark.parametrize("n", [17, 20, 24, 30])
 def test_every_program_has_a_plan(engine_lib, kind, size, n):
     for seed in range(8):
-        assert plan(program(kind, n, size, seed))[0]
+        blobs = plan(program(kind, n, size, seed))[0]
+        assert blobs and all(struct.unpack_from("<I", b, 112)[0] for b in blobs)
+
+
+@pytest.mark.parametrize("n,kind,cxs", [(14, "outside", 200), (20, "outside", 480), (20, "outside_many", 480)])
+def test_cx_from_one_control_share_phases(engine_lib, n, kind, cxs):
+    # four CX a phase, whatever their controls outside the tile
+    blobs = plan(program(kind, n, cxs, 0))[0]
+    assert sum(struct.unpack_from("<4I", b, 0)[2] for b in blobs) <= cxs // 4 + 4 * len(blobs)
 
 
 @pytest.mark.gpu
