@@ -234,6 +234,7 @@ SIGNATURES = [
                                         _P, _P, ctypes.POINTER(AdjointBatchStats)]),
     ("dq_debug_plan", ctypes.c_int, [_U32, _P, _U64, ctypes.POINTER(RunOpts), _P, _U64,
                                      ctypes.POINTER(_U64)]),
+    ("dq_debug_alloc_limit", None, [_U64]),
     ("dq_block_merge", ctypes.c_int, [_P, _P, _U32, _P, _P, _U32, _P]),
     ("dq_mps_create", ctypes.c_int, [_U32, ctypes.c_int, _U32, ctypes.c_double, ctypes.POINTER(_P)]),
     ("dq_mps_destroy", ctypes.c_int, [_P]),

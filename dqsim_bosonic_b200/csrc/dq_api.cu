@@ -35,12 +35,16 @@ static thread_local std::string g_err;
 void set_error(const std::string& msg) { g_err = msg; }
 void clear_error() { g_err.clear(); }
 
+static thread_local uint64_t g_alloc_limit = 0;
+bool alloc_refused(size_t bytes) { return g_alloc_limit && bytes > g_alloc_limit; }
+
 // ---- stream-ordered scratch ----------------------------------------------------
 // Small per-call device buffers (observable terms, sweep programs of the
 // adjoint pass, reduction workspaces) come from one memory pool per device
 // that keeps up to 256 MiB when idle: the default pool returns its memory at
 // every synchronisation, so the next call would map it again.
 cudaError_t pool_malloc_async(void** p, size_t bytes, cudaStream_t st) {
+  if (alloc_refused(bytes)) return cudaErrorMemoryAllocation;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -78,6 +82,7 @@ constexpr size_t kMaxCachedPerKey = 2;
 }  // namespace
 
 int cache_alloc(int device, size_t bytes, void** out) {
+  if (alloc_refused(bytes)) return fail(DQ_ERR_OOM, "allocation limit");
   {
     std::lock_guard<std::mutex> lk(g_cache_mu);
     auto it = g_cache.find({device, bytes});
@@ -178,6 +183,10 @@ size_t pinned_class(size_t bytes) {
 
 int pinned_alloc(size_t bytes, void** out) {
   const size_t c = pinned_class(bytes);
+  if (alloc_refused(bytes)) {
+    *out = nullptr;
+    return fail(DQ_ERR_OOM, "allocation limit");
+  }
   {
     std::lock_guard<std::mutex> lk(g_pinned_mu);
     auto it = g_pinned.find(c);
@@ -1268,6 +1277,8 @@ int dq_norm_sqr(dq_state_t h, double* out) {
   DQ_TRY(launch_norm(h->amp, h->n, h->sc, d, h->stream, h->device));
   return read_scalars(h, d, 1, out);
 }
+
+void dq_debug_alloc_limit(uint64_t bytes) { g_alloc_limit = bytes; }
 
 int dq_debug_plan(uint32_t n, const dq_inst* prog, uint64_t ninst, const dq_run_opts* opts,
                   uint8_t* out, uint64_t cap, uint64_t* len) {

@@ -58,6 +58,8 @@ struct DeviceGuard {
 // Device buffers of state size are recycled through a per-(device, size) cache.
 int cache_alloc(int device, size_t bytes, void** out);
 void cache_free(int device, size_t bytes, void* p);
+// Whether the thread's limit (dq_debug_alloc_limit) refuses an allocation.
+bool alloc_refused(size_t bytes);
 // Device memory a call may try to allocate before it asks how much is free (a
 // sixteenth of the device's memory): cudaMemGetInfo takes 0.4 to 4 ms next to
 // live memory pools.  A call whose allocation fails asks after all.

@@ -1348,6 +1348,7 @@ uint32_t draws_of(const TOp* ops, size_t n) {
 // to `ndraws` draws each.  Saved states take at most 1 GiB (a split past that
 // runs its program again from the start, as every shot would without sharing),
 // the table of draws at most 64 MiB (draws past it are computed in place).
+// DQ_ERR_OOM without memory for them, with b and P as they were.
 // st: buffers from the engine's pool on that stream; null: they outlive a launch.
 int set_shared(LaunchBuffers& b, TrajParams& P, int device, uint32_t n, uint64_t shots, uint32_t ncbits,
                uint32_t ndraws, cudaStream_t st) {
@@ -1377,7 +1378,17 @@ int set_shared(LaunchBuffers& b, TrajParams& P, int device, uint32_t n, uint64_t
   }
   off[6] = at;  // ready flags
   void** mem = st ? &b.pooled_share : &b.share;
-  DQ_CUDA_TRY(st ? pool_malloc_async(mem, at + 4 * shots, st) : cudaMalloc(mem, at + 4 * shots));
+  const size_t need = at + 4 * shots;
+  const cudaError_t e = st ? pool_malloc_async(mem, need, st)
+                           : alloc_refused(need) ? cudaErrorMemoryAllocation : cudaMalloc(mem, need);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *mem = nullptr;
+    if (b.slots) cache_free(device, b.slot_bytes, b.slots);
+    b.slots = nullptr;
+    return fail(e == cudaErrorMemoryAllocation ? DQ_ERR_OOM : DQ_ERR_CUDA,
+                std::string("shared shots: ") + cudaGetErrorString(e));
+  }
   uint8_t* base = static_cast<uint8_t*>(*mem);
   P.order[0] = reinterpret_cast<uint32_t*>(base + off[0]);
   P.order[1] = reinterpret_cast<uint32_t*>(base + off[1]);
@@ -1388,6 +1399,19 @@ int set_shared(LaunchBuffers& b, TrajParams& P, int device, uint32_t n, uint64_t
   P.ready = reinterpret_cast<int*>(base + off[6]);
   P.slots = inline_slots ? reinterpret_cast<double2*>(base + off[5]) : static_cast<double2*>(b.slots);
   P.nslots = (uint32_t)slots;
+  return DQ_OK;
+}
+
+// set_shared, or without memory for it an item of its own for every shot.
+int share_or_split(LaunchSet& ls, LaunchBuffers& b, TrajParams& P, int device, cudaStream_t st) {
+  if (ls.items.size() != 1 || ls.items[0].count < 2) return DQ_OK;
+  const uint64_t shots = ls.items[0].count;
+  const int rc = set_shared(b, P, device, ls.progs[0].n, shots, ls.progs[0].ncbits,
+                            draws_of(ls.enc.ops.data(), ls.enc.ops.size()), st);
+  if (rc != DQ_ERR_OOM) return rc;
+  clear_error();
+  ls.items.resize(shots);
+  for (uint64_t s = 0; s < shots; ++s) ls.items[s] = TItem{0, 1, s};
   return DQ_OK;
 }
 
@@ -1411,6 +1435,10 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
   if (ls.enc.pool.empty()) ls.enc.pool.push_back(make_double2(0, 0));
   LaunchBuffers b;
   b.st = st;
+  // several shots of one program share states
+  TrajParams P{};
+  const uint64_t shots = ls.items.size() == 1 ? ls.items[0].count : 1;
+  DQ_TRY(share_or_split(ls, b, P, device, st));
   // one allocation and one copy from pinned memory; the sweep programs of HBM
   // items are already pinned and follow in a copy of their own
   const unsigned long long init[kCtrWords] = {0ULL, 0ULL, ls.items.size(), 0ULL, kNotFailed};
@@ -1439,7 +1467,6 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
   unsigned long long* d_ctr = reinterpret_cast<unsigned long long*>(dev + part[6].off);
   DQ_CUDA_TRY(cudaEventCreate(&b.e0));
   DQ_CUDA_TRY(cudaEventCreate(&b.e1));
-  TrajParams P{};
   P.ops = reinterpret_cast<const TOp*>(dev);
   P.pool = reinterpret_cast<const double2*>(dev + part[1].off);
   P.conds = reinterpret_cast<const dq_cond*>(dev + part[2].off);
@@ -1452,11 +1479,6 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
   P.boundary = d_ctr + 3;
   P.failed = reinterpret_cast<long long*>(d_ctr + 4);
   P.nitems = ls.items.size();
-  // several shots of one program share states
-  const uint64_t shots = ls.items.size() == 1 ? ls.items[0].count : 1;
-  const uint32_t ndraws = shots > 1 ? draws_of(ls.enc.ops.data(), ls.enc.ops.size()) : 0;
-  if (shots > 1)
-    DQ_TRY(set_shared(b, P, device, ls.progs[0].n, shots, ls.progs[0].ncbits, ndraws, st));
   TrajLaunch L;
   DQ_TRY(config_traj(threads, ls.C, stage_tables(ls, P, part[3].off), P.tasks ? shots : P.nitems, &L));
   const uint32_t clusters = L.clusters;
@@ -2047,6 +2069,7 @@ int dq_traj_plan_create(int device, uint32_t n, const dq_inst* prog, uint64_t ni
   if ((rc = upload(&p->buf.pool, ls.enc.pool, st)) != DQ_OK) return bail(rc);
   if ((rc = upload(&p->buf.conds, ls.conds, st)) != DQ_OK) return bail(rc);
   if ((rc = upload(&p->buf.progs, ls.progs, st)) != DQ_OK) return bail(rc);
+  if ((rc = share_or_split(ls, p->buf, p->P, device, nullptr)) != DQ_OK) return bail(rc);
   if ((rc = upload(&p->buf.items, ls.items, st)) != DQ_OK) return bail(rc);
   cu(cudaMalloc((void**)&p->buf.ctr, kCtrWords * sizeof(unsigned long long)), "cudaMalloc(counters)");
   cu(cudaMalloc((void**)&p->d_cbits, std::max<size_t>(out_bytes, 4)), "cudaMalloc(cbits)");
@@ -2073,10 +2096,6 @@ int dq_traj_plan_create(int device, uint32_t n, const dq_inst* prog, uint64_t ni
   P.boundary = p->buf.ctr + 3;
   P.failed = reinterpret_cast<long long*>(p->buf.ctr + 4);
   P.nitems = ls.items.size();
-  if (ls.items.size() == 1 &&
-      (rc = set_shared(p->buf, P, device, n, shots, (uint32_t)ncbits,
-                       draws_of(ls.enc.ops.data(), ls.enc.ops.size()), nullptr)) != DQ_OK)
-    return bail(rc);
   if ((rc = config_traj(threads, C, traj_smem(ls), P.tasks ? shots : P.nitems, &p->L)) != DQ_OK) return bail(rc);
   cu(cudaStreamSynchronize(st), "cudaStreamSynchronize");
   if (rc != DQ_OK) return bail(rc);

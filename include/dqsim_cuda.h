@@ -495,6 +495,12 @@ DQ_API int dq_mps_run_shots(int device, uint32_t n, uint32_t max_bond, double tr
 DQ_API int dq_debug_plan(uint32_t n, const dq_inst* prog, uint64_t ninst, const dq_run_opts* opts,
                          uint8_t* out, uint64_t cap, uint64_t* len);
 
+/* ---- memory refusal (tests) --------------------------------------------------
+ * Allocations of more than `bytes` by calls on this thread (device buffers of
+ * one call, cached buffers, pinned staging) fail as if memory had run out, so
+ * that what a call does then can be tested.  0, the default: no limit. */
+DQ_API void dq_debug_alloc_limit(uint64_t bytes);
+
 /* ---- RNG (host side; same stream the device uses) ------------------------
  * ChaCha8Rng::seed_from_u64(seed) (rand_chacha 0.3.1 / rand_core 0.6.4),
  * gen::<f64>() (rand 0.8.5): the draws at positions [skip, skip + count). */

@@ -1,3 +1,4 @@
+import contextlib
 import os
 import sys
 from pathlib import Path
@@ -34,6 +35,21 @@ def gpu(engine_lib):
     if _native.device_count() < 1:
         pytest.fail("a CUDA device is required for tests marked gpu")
     return 0
+
+
+@pytest.fixture
+def alloc_limit(engine_lib):
+    """``with alloc_limit(b):`` refuses larger allocations of this thread's engine calls."""
+
+    @contextlib.contextmanager
+    def limit(nbytes):
+        engine_lib.dq_debug_alloc_limit(nbytes)
+        try:
+            yield
+        finally:
+            engine_lib.dq_debug_alloc_limit(0)
+
+    return limit
 
 
 @pytest.fixture(autouse=True)

@@ -249,3 +249,25 @@ def test_shared_shots_match_oracle(gpu, n, rounds, shots, check):
     plan.release()
     tail, _ = trajectories_resident(prog, 77, 1, 0, shot0=shots - 1)
     assert np.array_equal(tail[0], got[-1])
+
+
+def test_shots_without_memory_to_share_states(gpu, alloc_limit):
+    # the lists of 60000 shared shots take more than 2 MB, every other buffer less
+    prog = prog_of(shot_circuit(5, 30, seed=3))
+    want, _ = run_trajectories(prog, 7, 60000, 0)
+    with alloc_limit(2 << 20):
+        got, _ = run_trajectories(prog, 7, 60000, 0)
+        plan = TrajectoryPlan(prog, 60000, 0)
+    assert np.array_equal(got, want)
+    assert np.array_equal(plan.run(7)[0], want)
+
+
+def test_shots_without_memory_to_share_states(gpu, alloc_limit):
+    # the lists of 60000 shared shots take more than 2 MB, every other buffer less
+    prog = prog_of(shot_circuit(5, 30, seed=3))
+    want, _, _ = run_trajectories(prog, 7, 60000, 0, tuner=False)
+    with alloc_limit(2 << 20):
+        got, _, _ = run_trajectories(prog, 7, 60000, 0, tuner=False)
+        plan = TrajectoryPlan(prog, 60000, 0)
+    assert np.array_equal(got, want)
+    assert np.array_equal(plan.run(7)[0], want)
