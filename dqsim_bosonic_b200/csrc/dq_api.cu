@@ -16,8 +16,8 @@
 #include <condition_variable>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -218,19 +218,24 @@ void pinned_free(size_t bytes, void* p) {
   }
 }
 
-// Pageable host memory takes a copy of its own either way; here it comes out of
-// pinned memory on several host threads (which also take the page faults of a
-// fresh array) while the next chunks cross PCIe.  64 MiB into a fresh array:
-// 13.7 ms as one pageable cudaMemcpy, 3.6 ms here.
-int copy_to_host(const void* src, size_t bytes, const std::vector<HostPiece>& pieces, cudaStream_t st) {
-  constexpr size_t kChunk = 1 << 20;
-  // The driver's own staging copies one small range as fast (4 MiB into memory
-  // already touched: 246 us, 607 us with threads; 16 MiB: 852 and 693 us).
-  if (bytes && bytes < (16u << 20) && pieces.size() == 1 && pieces[0].dst) {
-    DQ_CUDA_TRY(cudaMemcpyAsync(pieces[0].dst, src, bytes, cudaMemcpyDeviceToHost, st));
-    DQ_CUDA_TRY(cudaStreamSynchronize(st));
-    return DQ_OK;
+namespace {
+
+// Every piece in a copy of its own.
+int copy_pieces(const void* src, size_t bytes, const std::vector<HostPiece>& pieces, cudaStream_t st) {
+  for (size_t i = 0; i < pieces.size(); ++i) {
+    const size_t end = i + 1 < pieces.size() ? pieces[i + 1].off : bytes;
+    if (pieces[i].dst && end > pieces[i].off)
+      DQ_CUDA_TRY(cudaMemcpyAsync(pieces[i].dst, static_cast<const uint8_t*>(src) + pieces[i].off,
+                                  end - pieces[i].off, cudaMemcpyDeviceToHost, st));
   }
+  DQ_CUDA_TRY(cudaStreamSynchronize(st));
+  return DQ_OK;
+}
+
+// Through pinned chunks and host threads; DQ_ERR_OOM (or std::bad_alloc) with
+// nothing copied when there is no memory for that.
+int copy_staged(const void* src, size_t bytes, const std::vector<HostPiece>& pieces, cudaStream_t st) {
+  constexpr size_t kChunk = 1 << 20;
   const uint8_t* from = static_cast<const uint8_t*>(src);
   // calls f(piece, x, y) for the pieces with a destination that overlap bytes [a, b)
   auto overlaps = [&](size_t a, size_t b, auto f) {
@@ -252,7 +257,12 @@ int copy_to_host(const void* src, size_t bytes, const std::vector<HostPiece>& pi
   if (chunks.empty()) return DQ_OK;
   const size_t n = chunks.size(), slots = std::min<size_t>(n, 32);
   const size_t stage_bytes = n == 1 ? std::min(bytes - chunks[0], kChunk) : slots * kChunk;
-  void* stage = nullptr;
+  std::vector<char> busy(slots, 0);  // the slot holds a chunk not copied out yet
+  std::vector<cudaEvent_t> ev(slots, nullptr);
+  std::vector<std::thread> th;
+  const size_t want = std::min<size_t>(std::min(8u, std::max(1u, std::thread::hardware_concurrency())), n);
+  th.reserve(want);
+  void* stage = nullptr;  // (no exception from here on but those of starting a thread)
   DQ_TRY(pinned_alloc(stage_bytes, &stage));
   auto slot = [&](size_t c) { return static_cast<uint8_t*>(stage) + (c % slots) * kChunk; };
   auto issue = [&](size_t c) {
@@ -269,9 +279,6 @@ int copy_to_host(const void* src, size_t bytes, const std::vector<HostPiece>& pi
   std::mutex mu;
   std::condition_variable cv;
   size_t issued = 0, next = 0;
-  std::vector<char> busy(slots, 0);  // the slot holds a chunk not copied out yet
-  std::vector<cudaEvent_t> ev(slots, nullptr);
-  std::vector<std::thread> th;
   int dev = 0;
   cudaGetDevice(&dev);
   auto consume = [&] {
@@ -290,13 +297,12 @@ int copy_to_host(const void* src, size_t bytes, const std::vector<HostPiece>& pi
       cv.notify_all();
     }
   };
-  const size_t want = std::min<size_t>(std::min(8u, std::max(1u, std::thread::hardware_concurrency())), n);
   if (want > 1) {
     for (auto& x : ev)
       if (err == cudaSuccess) err = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
     try {
       for (size_t t = 1; t < want && err == cudaSuccess; ++t) th.emplace_back(consume);
-    } catch (const std::system_error&) {  // the threads there are do the work
+    } catch (...) {  // the threads there are do the work
     }
   }
   if (th.empty()) {
@@ -330,6 +336,25 @@ int copy_to_host(const void* src, size_t bytes, const std::vector<HostPiece>& pi
   pinned_free(stage_bytes, stage);
   if (err != cudaSuccess) return fail(DQ_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(err));
   return DQ_OK;
+}
+
+}  // namespace
+
+// Pageable host memory takes a copy of its own either way; here it comes out of
+// pinned memory on several host threads (which also take the page faults of a
+// fresh array) while the next chunks cross PCIe.  64 MiB into a fresh array:
+// 13.7 ms as one pageable cudaMemcpy, 3.6 ms here.
+int copy_to_host(const void* src, size_t bytes, const std::vector<HostPiece>& pieces, cudaStream_t st) {
+  // The driver's own staging copies one small range as fast (4 MiB into memory
+  // already touched: 246 us, 607 us with threads; 16 MiB: 852 and 693 us).
+  if (pieces.size() == 1 && bytes < (16u << 20)) return copy_pieces(src, bytes, pieces, st);
+  try {
+    const int rc = copy_staged(src, bytes, pieces, st);
+    if (rc != DQ_ERR_OOM) return rc;
+  } catch (const std::bad_alloc&) {
+  }
+  clear_error();
+  return copy_pieces(src, bytes, pieces, st);
 }
 
 }  // namespace dq

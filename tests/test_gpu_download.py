@@ -33,3 +33,24 @@ def test_batch_states_land_in_their_arrays(gpu, want):
             assert abs(np.vdot(s, s).real - 1.0) < 1e-12
         else:
             assert s is None
+
+
+# nothing, and less than the staging ring, for pinned memory
+@pytest.mark.parametrize("limit", [1, 4 << 20])
+def test_downloads_without_pinned_memory(gpu, alloc_limit, limit):
+    rng = np.random.default_rng(1)
+    v = rng.normal(size=1 << 21) + 1j * rng.normal(size=1 << 21)
+    st = nat.State(21, 0)
+    st.upload(v)
+    with alloc_limit(limit):
+        assert np.array_equal(st.download(), v)
+
+
+def test_batch_states_without_pinned_memory(gpu, alloc_limit):
+    # 17 states of 256 KiB: their device buffer is within the limit, five chunks are not
+    progs = [encode(decode_circuit_json(brickwork_u3_cx(14, 2, k).model_dump_json())) for k in range(17)]
+    _, want, _ = run_batch(progs, range(17), want_states=True)
+    with alloc_limit(17 << 18):
+        _, got, _ = run_batch(progs, range(17), want_states=True)
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
