@@ -232,10 +232,21 @@ int copy_pieces(const void* src, size_t bytes, const std::vector<HostPiece>& pie
   return DQ_OK;
 }
 
+bool page_locked(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost;
+}
+
+constexpr size_t kCopyChunk = 1 << 20;
+
 // Through pinned chunks and host threads; DQ_ERR_OOM (or std::bad_alloc) with
 // nothing copied when there is no memory for that.
 int copy_staged(const void* src, size_t bytes, const std::vector<HostPiece>& pieces, cudaStream_t st) {
-  constexpr size_t kChunk = 1 << 20;
+  constexpr size_t kChunk = kCopyChunk;
   const uint8_t* from = static_cast<const uint8_t*>(src);
   // calls f(piece, x, y) for the pieces with a destination that overlap bytes [a, b)
   auto overlaps = [&](size_t a, size_t b, auto f) {
@@ -349,8 +360,20 @@ int copy_to_host(const void* src, size_t bytes, const std::vector<HostPiece>& pi
   // already touched: 246 us, 607 us with threads; 16 MiB: 852 and 693 us).
   if (pieces.size() == 1 && bytes < (16u << 20)) return copy_pieces(src, bytes, pieces, st);
   try {
-    const int rc = copy_staged(src, bytes, pieces, st);
-    if (rc != DQ_ERR_OOM) return rc;
+    std::vector<HostPiece> rest = pieces;  // but for large pieces in page-locked memory
+    for (size_t i = 0; i < rest.size(); ++i) {
+      const size_t end = i + 1 < rest.size() ? rest[i + 1].off : bytes;
+      if (!rest[i].dst || end - rest[i].off < kCopyChunk || !page_locked(rest[i].dst)) continue;
+      DQ_CUDA_TRY(cudaMemcpyAsync(rest[i].dst, static_cast<const uint8_t*>(src) + rest[i].off, end - rest[i].off,
+                                  cudaMemcpyDeviceToHost, st));
+      rest[i].dst = nullptr;
+    }
+    const int rc = copy_staged(src, bytes, rest, st);
+    if (rc != DQ_OK && rc != DQ_ERR_OOM) return rc;
+    if (rc == DQ_OK) {
+      DQ_CUDA_TRY(cudaStreamSynchronize(st));
+      return DQ_OK;
+    }
   } catch (const std::bad_alloc&) {
   }
   clear_error();

@@ -54,3 +54,16 @@ def test_batch_states_without_pinned_memory(gpu, alloc_limit):
         _, got, _ = run_batch(progs, range(17), want_states=True)
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+def test_download_into_pinned_memory(gpu):
+    import torch
+
+    n = 21
+    rng = np.random.default_rng(2)
+    v = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    st = nat.State(n, 0)
+    st.upload(v)
+    out = torch.empty(1 << n, dtype=torch.complex128, pin_memory=True)
+    nat.check(nat.lib().dq_state_download(st.handle, out.data_ptr(), 1 << n))
+    assert np.array_equal(out.numpy(), v)
