@@ -477,7 +477,7 @@ int ensure_query_buffers(dq_state_t h, size_t dev_bytes, size_t host_bytes) {
     h->q_dev = nullptr;
     h->q_dev_cap = 0;
     const size_t cap = std::max<size_t>(dev_bytes, 64 * 1024);
-    cudaError_t e = cudaMalloc(&h->q_dev, cap);
+    cudaError_t e = alloc_refused(dev_bytes) ? cudaErrorMemoryAllocation : cudaMalloc(&h->q_dev, cap);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(DQ_ERR_OOM, std::string("cudaMalloc(query buffer): ") + cudaGetErrorString(e));
@@ -490,7 +490,7 @@ int ensure_query_buffers(dq_state_t h, size_t dev_bytes, size_t host_bytes) {
     h->q_host = nullptr;
     h->q_host_cap = 0;
     const size_t cap = std::max<size_t>(host_bytes, 64 * 1024);
-    cudaError_t e = cudaMallocHost(&h->q_host, cap);
+    cudaError_t e = alloc_refused(host_bytes) ? cudaErrorMemoryAllocation : cudaMallocHost(&h->q_host, cap);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(DQ_ERR_OOM, std::string("cudaMallocHost(query buffer): ") + cudaGetErrorString(e));
@@ -1096,10 +1096,19 @@ int dq_run(dq_state_t h, const dq_inst* prog, uint64_t ninst, const dq_cond* con
   for (uint64_t i = 0; i < ninst; ++i) meas += prog[i].kind == DQ_MEASURE || prog[i].kind == DQ_RESET;
   const bool small = !o.profile && h->n >= 1 && h->n <= kSmallQubits && ncbits <= kSmallCbits &&
                      (fused ? meas > 0 : ninst >= 8 || meas > 0);
+  bool done = false;
   if (small) {
     if (h->permuted) rc = canonicalize(h);
     if (rc == DQ_OK)
       rc = small_run(h, prog, ninst, conds, nconds, seed, cbits, ncbits, o.semantics, &c.prof);
+    done = rc != DQ_ERR_OOM;  // no memory for its tables: nothing was run
+    if (!done) {
+      clear_error();
+      rc = DQ_OK;
+    }
+  }
+  if (done) {
+    // the program has run, or failed for good
   } else if (fused) {
     FusedHooks hooks;
     hooks.measure = [&c, h](uint32_t q, int* out) {

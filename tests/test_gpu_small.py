@@ -141,3 +141,18 @@ def test_measurement_of_an_infinite_norm(gpu, n, mode):
     cb, _ = run_program(st, prog, 3, nat.SEM_SIMULATE, mode)
     assert cb.tolist() == wcb.tolist() == [1]
     assert np.array_equal(st.download(), want)
+
+
+@pytest.mark.parametrize("mode", [nat.EXEC_PER_GATE, nat.EXEC_FUSED])
+@pytest.mark.parametrize("n", [3, 10])
+def test_program_without_memory_for_its_tables(gpu, alloc_limit, n, mode):
+    # 3000 instructions take more than 64 KiB of tables; the measurements come back one by one
+    prog = prog_of(mixed(n, 3000, 3))
+    want, wcb, rc, _ = _oracle.run(prog, 5)
+    assert rc == 0
+    st = nat.State(n, 0)
+    with alloc_limit(1 << 16):
+        cb, prof = run_program(st, prog, 5, nat.SEM_SIMULATE, mode)
+        got = st.download()
+    assert prof.boundary_draws == 0 and cb.tolist() == wcb.tolist()
+    assert np.max(np.abs(got - want)) < 1e-12
