@@ -156,3 +156,26 @@ def test_program_without_memory_for_its_tables(gpu, alloc_limit, n, mode):
         got = st.download()
     assert prof.boundary_draws == 0 and cb.tolist() == wcb.tolist()
     assert np.max(np.abs(got - want)) < 1e-12
+
+
+# one launch where measurements are many for the gates, sweeps or grouped launches where they
+# are few, with the same results either way
+@pytest.mark.parametrize("mode,gates,meas,one_launch", [
+    (nat.EXEC_FUSED, 400, 1, False), (nat.EXEC_FUSED, 30, 6, True), (nat.EXEC_PER_GATE, 400, 1, True)])
+@pytest.mark.parametrize("n", [10, 12])
+def test_deep_programs_run_in_sweeps(gpu, mode, gates, meas, one_launch, n):
+    rng = np.random.default_rng(n)
+    insts = []
+    for k in range(gates):
+        if k % (gates // meas) == gates // meas - 1:
+            insts.append(g("measure", int(rng.integers(n)), 0))
+        a, b = rng.permutation(n)[:2].tolist()
+        insts.append([g("ry", a, 0.3), g("rz", a, 0.7), g("cp", a, b, 0.4), g("u3", a, 0.1, 0.2, 0.3)][k % 4])
+    prog = prog_of(JsonCircuit(n, insts, ncbits=1))
+    want, wcb, rc, _ = _oracle.run(prog, 9)
+    assert rc == 0
+    st = nat.State(n, 0)
+    cb, prof = run_program(st, prog, 9, nat.SEM_SIMULATE, mode)
+    assert prof.boundary_draws == 0 and cb.tolist() == wcb.tolist()
+    assert np.max(np.abs(st.download() - want)) < 1e-12
+    assert (prof.kernel_launches == 1 and prof.sweeps == 0) == one_launch
