@@ -1014,8 +1014,16 @@ int launch_sample(const double* cdf, uint64_t len, const uint32_t key[8], uint64
   return DQ_OK;
 }
 
+// One block takes 23 us and about 2 ns an amplitude and 8 ns a shot, the separate
+// launches 58 us (70 and 83 us for outcomes of 32 and 64 terms, which take one
+// thread there too), so amplitudes and shots are limited together.  11 qubits,
+// all sampled: 1000 shots 35 us (60 in separate launches), 4096 shots 58 (61),
+// 16384 shots 135 (65); 13 qubits, 9 of them: 45 (67), 63 (71), 136 (69); 14
+// qubits, 8 and 11 of them, 1000 shots: 58 (84) and 70 (63); 17 qubits, 11: 318 (96).
 bool sample_small_ok(uint32_t n, const uint32_t* qubits, uint32_t k, uint64_t shots, int device) {
-  return (1ULL << k) <= (uint64_t)kScanChunk && shots <= 16384 && plan_marginal(n, qubits, k, device).kind == 1;
+  if ((1ULL << k) > (uint64_t)kScanChunk || shots > 4864 || n > 14) return false;
+  const uint64_t most = n - k >= 6 ? 32768 : n - k == 5 ? 24576 : 20480;
+  return (1ULL << n) + 4 * shots <= most && (n <= 13 || k <= 10) && plan_marginal(n, qubits, k, device).kind == 1;
 }
 
 int launch_sample_small(const double2* s, uint32_t n, const uint32_t* qubits, uint32_t k, const uint32_t key[8],

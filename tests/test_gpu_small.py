@@ -179,3 +179,19 @@ def test_deep_programs_run_in_sweeps(gpu, mode, gates, meas, one_launch, n):
     assert prof.boundary_draws == 0 and cb.tolist() == wcb.tolist()
     assert np.max(np.abs(st.download() - want)) < 1e-12
     assert (prof.kernel_launches == 1 and prof.sweeps == 0) == one_launch
+
+
+# both sides of the line between one block and separate launches: the same indices
+@pytest.mark.parametrize("n,k,shots", [(11, 11, 4608), (11, 11, 4609), (13, 9, 3072), (13, 9, 3073), (14, 10, 1024),
+                                       (14, 11, 1024), (17, 11, 100)])
+def test_samples_beside_the_line(gpu, n, k, shots):
+    rng = np.random.default_rng(n * k)
+    v = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    v /= np.linalg.norm(v)
+    st = nat.State(n, 0)
+    st.upload(v)
+    qs = rng.permutation(n)[:k].tolist()
+    res = SimulationResult(st, n, {}, None)
+    got = res.sample_indices(shots, qs, seed=3)
+    assert res.last_boundary_draws == 0
+    assert got.tolist() == _oracle.sample(v, qs, 3, shots).tolist()
