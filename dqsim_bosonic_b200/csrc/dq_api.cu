@@ -1196,18 +1196,20 @@ int dq_run(dq_state_t h, const dq_inst* prog, uint64_t ninst, const dq_cond* con
       }
     }
   } else {
-    // runs of gates go through memory together (a profiled run times each gate)
+    // runs of gates go through memory together (a profiled run times each gate);
+    // a failing one is named by flush, also when a later instruction ends the run
     GateGroup group;
     std::vector<uint64_t> grouped;
     auto flush = [&]() -> int {
       int r = DQ_OK;
       if (group_worth(group, h->n)) {
         r = launch_group(h->amp, h->n, group, h->stream, &c.prof.kernel_launches);
+        if (r != DQ_OK) c.prof.failed_inst = (int64_t)grouped.front();
         for (uint64_t k : grouped) ++(gate_qubit_count(prog[k].kind) == 1 ? c.prof.apply_one_qubit_calls
                                                                            : c.prof.apply_n_qubit_calls);
       } else {
         for (uint64_t k : grouped)
-          if (r == DQ_OK) r = exec_inst(c, prog[k]);
+          if (r == DQ_OK && (r = exec_inst(c, prog[k])) != DQ_OK) c.prof.failed_inst = (int64_t)k;
       }
       group.clear();
       grouped.clear();
@@ -1231,8 +1233,7 @@ int dq_run(dq_state_t h, const dq_inst* prog, uint64_t ninst, const dq_cond* con
         rc = flush();
         if (!cond_holds(in, conds, cbits, ncbits)) continue;
       }
-      if (rc == DQ_OK) rc = exec_inst(c, in);
-      if (rc != DQ_OK) c.prof.failed_inst = (int64_t)i;
+      if (rc == DQ_OK && (rc = exec_inst(c, in)) != DQ_OK) c.prof.failed_inst = (int64_t)i;
     }
     if (rc == DQ_OK) rc = flush();
   }
