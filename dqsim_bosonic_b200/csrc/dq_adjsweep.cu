@@ -456,6 +456,7 @@ __device__ __forceinline__ void diag_grads(const double2 (&a)[8], const double2 
       if (c0 + (uint32_t)lane < cnt) accw[t.slot] += (neg & 1u) ? -t.w * v : t.w * v;
     }
     terms += cnt;
+    __syncwarp();  // another lane may add to the same slot in the next list
   }
 }
 
