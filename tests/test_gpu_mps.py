@@ -489,3 +489,14 @@ def test_shared_shots_match_oracle_per_shot(n, rounds, shots):
         assert bits[i].tolist() == rcb.tolist(), i
     again, st2 = run_mps_shots(prog, 9, shots, 0, None, 1e-12, batch=97)
     assert np.array_equal(again, bits) and st2.svd_calls == st.svd_calls
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_cluster_step_leaves_no_overlap(seed):
+    # overlaps of 4 eps at a truncation whose singular values differ by 1% cost 9e-14 a step,
+    # at random over some 30 truncated steps 5e-13 (overlaps at the convergence tolerance, 128
+    # eps, several times that)
+    c = brickwork_u3_cx(16, 20, seed)
+    sv, _, _, _ = device_run(c, SEED, max_bond=64)
+    ref, _, _, _ = _oracle.mps_run(prog_of(c), SEED, max_bond=64)
+    assert np.linalg.norm(sv - ref) < 5e-13
