@@ -183,7 +183,7 @@ size_t pinned_class(size_t bytes) {
 
 int pinned_alloc(size_t bytes, void** out) {
   const size_t c = pinned_class(bytes);
-  if (alloc_refused(bytes)) {
+  if (alloc_refused(c)) {
     *out = nullptr;
     return fail(DQ_ERR_OOM, "allocation limit");
   }

@@ -1305,7 +1305,7 @@ struct LaunchBuffers {
   cudaStream_t st = nullptr;
   bool own_st = false;  // destroy st with the buffers
   void* block = nullptr;      // one launch's buffers, from the engine's pool on st
-  void* stage = nullptr;      // their pinned image
+  void* stage = nullptr;      // their pinned image, if there is one
   size_t stage_bytes = 0;
   ~LaunchBuffers() {
     if (st) cudaStreamSynchronize(st);
@@ -1433,6 +1433,7 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
                dq_traj_stats* acc) {
   if (ls.items.empty()) return DQ_OK;
   if (ls.enc.pool.empty()) ls.enc.pool.push_back(make_double2(0, 0));
+  std::vector<uint8_t> pageable;  // the tables' image without pinned memory (outlives b's stream wait)
   LaunchBuffers b;
   b.st = st;
   // several shots of one program share states
@@ -1455,13 +1456,18 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
     x.off = image;
     image += (x.bytes + 15) / 16 * 16;
   }
-  DQ_TRY(pinned_alloc(image, &b.stage));
-  b.stage_bytes = image;
+  if (pinned_alloc(image, &b.stage) == DQ_OK) {
+    b.stage_bytes = image;
+  } else {
+    clear_error();
+    pageable.resize(image);
+  }
+  uint8_t* stage = b.stage ? static_cast<uint8_t*>(b.stage) : pageable.data();
   for (const auto& x : part)
-    if (x.bytes) memcpy(static_cast<uint8_t*>(b.stage) + x.off, x.p, x.bytes);
+    if (x.bytes) memcpy(stage + x.off, x.p, x.bytes);
   DQ_CUDA_TRY(pool_malloc_async(&b.block, image + ls.blob_host_bytes, st));
   uint8_t* dev = static_cast<uint8_t*>(b.block);
-  DQ_CUDA_TRY(cudaMemcpyAsync(dev, b.stage, image, cudaMemcpyHostToDevice, st));
+  DQ_CUDA_TRY(cudaMemcpyAsync(dev, stage, image, cudaMemcpyHostToDevice, st));
   if (ls.blob_host_bytes)
     DQ_CUDA_TRY(cudaMemcpyAsync(dev + image, ls.blob_host, ls.blob_host_bytes, cudaMemcpyHostToDevice, st));
   unsigned long long* d_ctr = reinterpret_cast<unsigned long long*>(dev + part[6].off);
@@ -1486,9 +1492,9 @@ int run_launch(LaunchSet& ls, int threads, int device, cudaStream_t st, int32_t*
   DQ_TRY(reset_shared(P, shots, st));
   DQ_TRY(launch_traj(L, P, st));
   DQ_CUDA_TRY(cudaEventRecord(b.e1, st));
-  // into the pinned image, whose copy has been consumed by then
-  const unsigned long long* ctr = static_cast<const unsigned long long*>(b.stage);
-  DQ_CUDA_TRY(cudaMemcpyAsync(b.stage, d_ctr, sizeof(init), cudaMemcpyDeviceToHost, st));
+  // into the staged image, whose copy has been consumed by then
+  const unsigned long long* ctr = reinterpret_cast<const unsigned long long*>(stage);
+  DQ_CUDA_TRY(cudaMemcpyAsync(stage, d_ctr, sizeof(init), cudaMemcpyDeviceToHost, st));
   DQ_CUDA_TRY(cudaStreamSynchronize(st));
   float ms = 0.f;
   DQ_CUDA_TRY(cudaEventElapsedTime(&ms, b.e0, b.e1));

@@ -271,3 +271,17 @@ def test_shots_without_memory_to_share_states(gpu, alloc_limit):
         plan = TrajectoryPlan(prog, 60000, 0)
     assert np.array_equal(got, want)
     assert np.array_equal(plan.run(7)[0], want)
+
+
+def test_tables_without_pinned_memory(gpu, alloc_limit):
+    # the smallest pinned buffer is 1 MiB; the tables of these batches take far less
+    prog = prog_of(shot_circuit(5, 30, seed=4))
+    progs = [prog, prog_of(_circuits.brickwork_u3_cx(12, 3, 1))]
+    want, _, _ = run_trajectories(prog, 7, 500, 0)
+    wbits, wstates, _ = run_batch(progs, [1, 2], want_states=True)
+    with alloc_limit((1 << 20) - 1):
+        got, _, _ = run_trajectories(prog, 7, 500, 0)
+        bits, states, _ = run_batch(progs, [1, 2], want_states=True)
+    assert np.array_equal(got, want)
+    for k in range(2):
+        assert np.array_equal(bits[k], wbits[k]) and np.array_equal(states[k], wstates[k])
