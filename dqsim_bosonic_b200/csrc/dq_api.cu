@@ -17,6 +17,7 @@
 #include <map>
 #include <mutex>
 #include <new>
+#include <set>
 #include <string>
 #include <thread>
 #include <utility>
@@ -34,6 +35,23 @@ namespace dq {
 static thread_local std::string g_err;
 void set_error(const std::string& msg) { g_err = msg; }
 void clear_error() { g_err.clear(); }
+
+int allow_shared(const void* kernel) {
+  int dev = 0;
+  DQ_CUDA_TRY(cudaGetDevice(&dev));
+  static std::mutex mu;
+  static std::set<std::pair<int, const void*>> done;
+  std::lock_guard<std::mutex> lk(mu);
+  if (done.count({dev, kernel})) return DQ_OK;
+  int most = 0;
+  cudaFuncAttributes fa{};
+  DQ_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  DQ_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
+  DQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   most - (int)fa.sharedSizeBytes));
+  done.insert({dev, kernel});
+  return DQ_OK;
+}
 
 static thread_local uint64_t g_alloc_limit = 0;
 bool alloc_refused(size_t bytes) { return g_alloc_limit && bytes > g_alloc_limit; }

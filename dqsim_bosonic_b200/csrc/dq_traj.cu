@@ -1231,8 +1231,7 @@ struct TrajLaunch {
 
 template <int THREADS>
 int config_traj_t(uint32_t C, size_t smem, uint64_t nitems, TrajLaunch* L) {
-  DQ_CUDA_TRY(cudaFuncSetAttribute(k_traj<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
+  DQ_TRY(allow_shared((const void*)k_traj<THREADS>));
   L->attr[0].id = cudaLaunchAttributeClusterDimension;
   L->attr[0].val.clusterDim.x = C;
   L->attr[0].val.clusterDim.y = 1;
@@ -1545,11 +1544,11 @@ int geometry(uint32_t n, uint32_t max_span, uint32_t force_lb, uint32_t* lb, uin
 // the latency of one op after another; launching every gate and reading every
 // p1 back costs about 3 us a gate and 20 us a measurement instead.
 template <int THREADS>
-cudaError_t launch_small(size_t smem, const TrajParams& P, cudaStream_t st) {
-  const cudaError_t e = cudaFuncSetAttribute(k_traj<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+int launch_small(size_t smem, const TrajParams& P, cudaStream_t st) {
+  DQ_TRY(allow_shared((const void*)k_traj<THREADS>));
   k_traj<THREADS><<<1, THREADS, smem, st>>>(P);
-  return cudaGetLastError();
+  DQ_CUDA_TRY(cudaGetLastError());
+  return DQ_OK;
 }
 
 double ms_since(std::chrono::steady_clock::time_point t0) {
@@ -1627,7 +1626,7 @@ int small_run(dq_state_t h, const dq_inst* prog, uint64_t ninst, const dq_cond* 
   ls.max_lb = h->n;
   ls.max_ncbits = (uint32_t)ncbits;
   const size_t smem = stage_tables(ls, P, off[3]);
-  DQ_CUDA_TRY(h->n <= 8 ? launch_small<128>(smem, P, h->stream) : launch_small<256>(smem, P, h->stream));
+  DQ_TRY(h->n <= 8 ? launch_small<128>(smem, P, h->stream) : launch_small<256>(smem, P, h->stream));
   h->lazy_basis = -1;  // the kernel writes the state, also up to a failing gate
   DQ_CUDA_TRY(cudaMemcpyAsync(up + off[6], dev + off[6], back, cudaMemcpyDeviceToHost, h->stream));
   DQ_CUDA_TRY(cudaStreamSynchronize(h->stream));

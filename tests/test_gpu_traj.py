@@ -285,3 +285,31 @@ def test_tables_without_pinned_memory(gpu, alloc_limit):
     assert np.array_equal(got, want)
     for k in range(2):
         assert np.array_equal(bits[k], wbits[k]) and np.array_equal(states[k], wstates[k])
+
+
+def test_threads_with_launches_of_different_sizes(gpu):
+    # trajectories of 16 qubits (128 KiB of state a block) beside small programs and batches
+    # of other sizes: the kernel's shared-memory limit is not one launch's own
+    from concurrent.futures import ThreadPoolExecutor
+
+    from dqsim_bosonic_b200.statevector import run_program
+
+    big, small = prog_of(shot_circuit(16, 12, seed=1)), prog_of(shot_circuit(9, 12, seed=2))
+    want_big, _, _ = run_trajectories(big, 3, 8, 0, tuner=False)
+    want_small, _, _ = run_trajectories(small, 3, 8, 0, tuner=False)
+
+    def trajectories(prog, want, rounds):
+        return all(np.array_equal(run_trajectories(prog, 3, 8, 0, tuner=False)[0], want) for _ in range(rounds))
+
+    def programs(rounds):
+        st = nat.State(9, 0)
+        bits = set()
+        for _ in range(rounds):
+            st.reset()
+            bits.add(tuple(run_program(st, small, 5, nat.SEM_SIMULATE, nat.EXEC_FUSED)[0].tolist()))
+        return len(bits) == 1
+
+    with ThreadPoolExecutor(4) as ex:
+        jobs = [ex.submit(trajectories, big, want_big, 150), ex.submit(trajectories, small, want_small, 150),
+                ex.submit(programs, 300), ex.submit(trajectories, big, want_big, 150)]
+        assert all(j.result() for j in jobs)
