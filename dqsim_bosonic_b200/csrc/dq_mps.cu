@@ -1560,18 +1560,9 @@ int alloc_buffers(dq_mps_s* h, uint32_t batch, uint32_t cap, uint32_t ncb) {
   DQ_TRY(mps_take(h, 5, sizeof(int) * 4));
   DQ_TRY(mps_take(h, 6, sizeof(unsigned long long)));
   DQ_TRY(mps_take(h, 7, sizeof(double2) * h->scratch_elems * h->slots * batch));
-  if (cap <= kWarpCap)
-    DQ_CUDA_TRY(cudaFuncSetAttribute(k_mps_measure_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(kRepsPer2q * warp_measure_bytes(cap))));
-  if (cap <= kWarpCap)
-    DQ_CUDA_TRY(cudaFuncSetAttribute(k_mps_2q_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(kRepsPer2q * warp_work_bytes(cap))));
-  if (h->smem) {
-    DQ_CUDA_TRY(cudaFuncSetAttribute(k_mps_2q, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)work_bytes));
-    DQ_CUDA_TRY(cudaFuncSetAttribute(k_mps_measure, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)work_bytes));
-  }
+  for (const void* k : {(const void*)k_mps_measure_warp, (const void*)k_mps_2q_warp, (const void*)k_mps_2q,
+                        (const void*)k_mps_measure, (const void*)k_mps_2q_cl})
+    DQ_TRY(allow_shared(k));
   return DQ_OK;
 }
 
@@ -1713,7 +1704,6 @@ uint32_t cluster_ctas(uint32_t cap, uint64_t steps) {
 int launch_cluster(dq_mps_s* h, const MpsView& v, uint32_t first, uint32_t count) {
   const uint32_t c = cluster_ctas(h->cap, (uint64_t)h->nrep * count);
   const size_t smem = cl_smem_bytes(h->cap, c);
-  DQ_CUDA_TRY(cudaFuncSetAttribute(k_mps_2q_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(h->nrep * c, count);
   cfg.blockDim = dim3(kClThreads);

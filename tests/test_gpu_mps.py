@@ -500,3 +500,17 @@ def test_cluster_step_leaves_no_overlap(seed):
     sv, _, _, _ = device_run(c, SEED, max_bond=64)
     ref, _, _, _ = _oracle.mps_run(prog_of(c), SEED, max_bond=64)
     assert np.linalg.norm(sv - ref) < 5e-13
+
+
+def test_a_handle_beside_a_smaller_one():
+    # a live handle of capacity 32 measures after one of capacity 16 was made
+    c = trajectory_circuit(12, 9, seed=3)
+    prog = prog_of(c)
+    h = MpsHandle(prog.num_qubits, 0, 32, 1e-12)
+    first, _ = h.run(prog, SEED)
+    h.reserve(32)
+    other = MpsHandle(prog.num_qubits, 0, 16, 1e-12)
+    cbits, _ = h.run(prog, SEED)
+    assert cbits.tolist() == first.tolist()
+    other.release()
+    h.release()
