@@ -148,3 +148,17 @@ def test_kernel(gpu, kind, n, size, seed):
     st.upload(v)
     run_program(st, prog, 0, nat.SEM_SIMULATE, nat.EXEC_FUSED)
     assert np.max(np.abs(st.download() - want)) < ATOL
+
+
+@pytest.mark.gpu
+def test_batch_items(gpu):
+    # tiles of 2^12 amplitudes and 8 thread bits, as a batch's larger items run
+    from dqsim_bosonic_b200.batch import run_batch
+
+    cases = [("all_to_all", 17, 1), ("cx_most", 17, 500), ("cx_diagonal", 17, 400), ("pauli", 18, 15),
+             ("outside", 17, 900), ("outside_pairs", 17, 200)]
+    progs = [program(k, n, s, 3) for k, n, s in cases]
+    _, states, st = run_batch(progs, range(len(progs)), want_states=True)
+    for (k, n, s), prog, got in zip(cases, progs, states):
+        assert np.max(np.abs(got - _oracle.run(prog, 0)[0])) < ATOL, (k, n, s)
+    assert st.engine_items == 0
