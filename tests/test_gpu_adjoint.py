@@ -532,3 +532,30 @@ def test_batched_sets_with_plans_of_different_kinds(gpu, n, kind):
             e1, g1 = adjoint_gradient(c, thetas[b], H, exec=mode)
             assert abs(es[b] - e1) < 1e-11
             assert np.max(np.abs(gs[b] - g1)) < 1e-11
+
+
+# single diagonal gates and single rotations between other ops, with and without derivatives
+# outside the register passes
+@pytest.mark.parametrize("ring", ["cx", "crx", "rzz"])
+@pytest.mark.parametrize("n", [4, 9, 11, 13])
+def test_alternating_gates_match_per_gate(gpu, n, ring):
+    # rounding of at most 160 gates on both vectors, observable of norm below 20: as above
+    c, k = ParamCircuit(n), 0
+    for layer in range(3):
+        for q in range(n):
+            c.rx(q, Param(k))
+            c.rz(q, Param(k + 1))
+            c.ry(q, Param(k + 2))
+            k += 3
+        for q in range(n):
+            if ring == "cx":
+                c.cx(q, (q + 1) % n)
+            else:
+                getattr(c, ring)(q, (q + 1) % n, Param(k))
+                k += 1
+    theta = np.random.default_rng(n).uniform(-np.pi, np.pi, size=k)
+    H = random_observable(n, 8, seed=n)
+    e1, g1 = adjoint_gradient(c, theta, H, exec="fused")
+    e2, g2 = adjoint_gradient(c, theta, H, exec="per_gate")
+    assert abs(e1 - e2) < 1e-12
+    assert np.max(np.abs(g1 - g2)) < 1e-11
