@@ -653,14 +653,14 @@ __device__ __forceinline__ void pass_tan(double2 (&a)[8], double2 (&b)[8], const
   if (lane < N && ps[lane].np) accw[ps[lane].slot] += ps[lane].v[0].y * v;
 }
 
-// The op data of one register phase: threads < cnt fill ps[0 .. cnt).
+// The op data of one register phase: threads th < cnt fill ps[0 .. cnt).
 __device__ __forceinline__ void stage_phase(const AOp& hdr, const AOp* sub, const double2* pool,
-                                            PSub* ps) {
+                                            PSub* ps, uint32_t th) {
   const uint32_t cnt = hdr.cnt;
   const uint32_t pbits[3] = {hdr.lt, hdr.lt2, (uint32_t)hdr.dq[0]};
-  if (threadIdx.x < cnt) {
-    const AOp op = sub[threadIdx.x];
-    PSub& P = ps[threadIdx.x];
+  if (th < cnt) {
+    const AOp op = sub[th];
+    PSub& P = ps[th];
     const double2* mt = pool + op.mat;
     P.np = op.np;
     P.slot = op.slot;
@@ -828,10 +828,13 @@ __device__ __forceinline__ void adj_sweep_body(double2* __restrict__ psi, double
     hi_tab[hv] = g;
   }
   __syncthreads();
-  for (uint32_t i = 0; i < H.nops; ++i) {
+  // a pass per warp: their loads from memory side by side (u3 on 14 qubits: 11 sweeps
+  // in 0.46 ms, 0.47 with one pass after the other)
+  for (uint32_t i = 0, k = 0; i < H.nops; ++i) {
     const AOp op = sops[i];
     if (op.type != A_PASS && op.type != A_PHASE) continue;
-    if (H.phase_ops) stage_phase(op, sops + i + 1, pool, psall + op.lctrl);
+    if (H.phase_ops && (k++ & (kAWarps - 1)) == w)
+      stage_phase(op, sops + i + 1, pool, psall + op.lctrl, threadIdx.x & 31u);
     if (op.type == A_PASS && op.ndq) {
       const double2* B = blob + op.slot;
       const uint32_t tab = reinterpret_cast<const DMask*>(B + 5)->tab;
@@ -906,7 +909,7 @@ __device__ __forceinline__ void adj_sweep_body(double2* __restrict__ psi, double
         const uint32_t cnt = (w1.x >> 8) & 0xffu;
         const PSub* ps = psall + (H.phase_ops ? w1.y : 0u);
         if (!H.phase_ops && cnt) {
-          stage_phase(sops[i], sops + i + 1, pool, psall);
+          stage_phase(sops[i], sops + i + 1, pool, psall, threadIdx.x);
           __syncthreads();
         }
         if ((w0.x & 0xffu) == A_PHASE) {
