@@ -71,13 +71,20 @@ __device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 acc) {
 // 20 ZZ and 20 X terms on 128 states of 20 qubits: 4.6 ms (8.4 with an amplitude
 // a thread and every partner from memory, 5.5 with 8 a thread and half the
 // warps); 24 and 24 on 24 qubits: 0.80 ms (1.32).
-constexpr int kPauliThreads = 512, kPauliRegs = 4;
-constexpr uint32_t kPauliTile = 11;
+constexpr uint32_t kPauliTB = 9, kPauliRB = 2;            // thread and register bits of the index
+// Small states: an amplitude a thread in many small blocks.  What counts there is
+// the latency of one group after another, and a block of 512 threads makes its
+// warps wait for each other.  200 random terms on 4 qubits each, whole calls with
+// blocks of 64, 256 and 512 (a tile of 2^11) threads: 13 qubits 131, 137 and 180 us,
+// 16 qubits 205, 132 and 181, 18 qubits 562, 218 and 181; 1500 terms: 13 qubits 487,
+// 516 and 847, 17 qubits 1906, 616 and 921, 18 qubits 3257, 1103 and 936.
+constexpr uint32_t kPauliSmallTB = 6, kPauliSmallQubits = 15;
+constexpr uint32_t kPauliMidTB = 8, kPauliMidQubits = 17;
 
-__device__ __forceinline__ void pauli_add(double2 (&acc)[kPauliRegs], const double2 (&p)[kPauliRegs], const double (&c)[kPauliRegs],
-                                          bool imag) {
+template <int R>
+__device__ __forceinline__ void pauli_add(double2 (&acc)[R], const double2 (&p)[R], const double (&c)[R], bool imag) {
 #pragma unroll
-  for (int i = 0; i < kPauliRegs; ++i) {
+  for (int i = 0; i < R; ++i) {
     if (imag)
       acc[i] = make_double2(fma(-c[i], p[i].y, acc[i].x), fma(c[i], p[i].x, acc[i].y));
     else
@@ -85,11 +92,13 @@ __device__ __forceinline__ void pauli_add(double2 (&acc)[kPauliRegs], const doub
   }
 }
 
-template <bool STORE>
+template <bool STORE, uint32_t TB, uint32_t RB>
 __device__ __forceinline__ void pauli_body(const double2* __restrict__ psi, double2* __restrict__ lam,
                                            uint64_t len, const PauliGroup* __restrict__ groups,
                                            uint32_t ngroups, const PauliTerm* __restrict__ terms,
                                            double* partial, unsigned* counter, double* out) {
+  constexpr int kPauliThreads = 1 << TB, kPauliRegs = 1 << RB;
+  constexpr uint32_t kPauliTile = TB + RB;
   __shared__ double2 tile[1u << kPauliTile];
   const uint32_t L = (uint32_t)(len < (1u << kPauliTile) ? len : (1u << kPauliTile));
   const uint32_t tid = threadIdx.x;
@@ -123,7 +132,7 @@ __device__ __forceinline__ void pauli_body(const double2* __restrict__ psi, doub
         if (count == 1) {
           const double v = part ? __ldg(&terms[f].cim) : __ldg(&terms[f].cre);
           const uint64_t z = __ldg(&terms[f].z);
-          const uint32_t neg = (uint32_t)__popcll(src & z), zr = (uint32_t)(z >> 9) & 3u;
+          const uint32_t neg = (uint32_t)__popcll(src & z), zr = (uint32_t)(z >> TB) & (kPauliRegs - 1u);
 #pragma unroll
           for (uint32_t i = 0; i < kPauliRegs; ++i) w[i] = ((neg + __popc(i & zr)) & 1u) ? -v : v;
         } else {
@@ -133,7 +142,7 @@ __device__ __forceinline__ void pauli_body(const double2* __restrict__ psi, doub
             double v = part ? __ldg(&terms[t].cim) : __ldg(&terms[t].cre);
             const uint64_t z = __ldg(&terms[t].z);
             if (__popcll(src & z) & 1) v = -v;
-            const uint32_t zr = (uint32_t)(z >> 9) & 3u;
+            const uint32_t zr = (uint32_t)(z >> TB) & (kPauliRegs - 1u);
 #pragma unroll
             for (uint32_t k = 0; k < kPauliRegs; ++k)
               if (zr == k) w[k] += v;
@@ -148,7 +157,7 @@ __device__ __forceinline__ void pauli_body(const double2* __restrict__ psi, doub
                 w[i | st] = u - v;
               }
         }
-        pauli_add(acc, p, w, part != 0);
+        pauli_add<kPauliRegs>(acc, p, w, part != 0);
       }
     }
 #pragma unroll
@@ -165,23 +174,23 @@ __device__ __forceinline__ void pauli_body(const double2* __restrict__ psi, doub
   finish_partials<1>(v, partial, counter, out);
 }
 
-template <bool STORE>
-__global__ void __launch_bounds__(kPauliThreads, 2) k_pauli(const double2* __restrict__ psi, double2* __restrict__ lam, uint64_t len,
+template <bool STORE, uint32_t TB, uint32_t RB>
+__global__ void __launch_bounds__(1 << TB, 1024 >> TB) k_pauli(const double2* __restrict__ psi, double2* __restrict__ lam, uint64_t len,
                         const PauliGroup* __restrict__ groups, uint32_t ngroups,
                         const PauliTerm* __restrict__ terms, double* partial, unsigned* counter,
                         double* out) {
-  pauli_body<STORE>(psi, lam, len, groups, ngroups, terms, partial, counter, out);
+  pauli_body<STORE, TB, RB>(psi, lam, len, groups, ngroups, terms, partial, counter, out);
 }
 
 // The same for B states in one launch: state b (blockIdx.y) at psi + b len,
 // its lambda at lam + b len, its reduction scratch at partial + b gridDim.x
 // and counter + b, its expectation value at out[b * out_stride].
-__global__ void __launch_bounds__(kPauliThreads, 2) k_pauli_multi(const double2* __restrict__ psi, double2* __restrict__ lam,
+__global__ void __launch_bounds__(1 << kPauliTB, 2) k_pauli_multi(const double2* __restrict__ psi, double2* __restrict__ lam,
                               uint64_t len, const PauliGroup* __restrict__ groups, uint32_t ngroups,
                               const PauliTerm* __restrict__ terms, double* partial,
                               unsigned* counter, double* out, uint64_t out_stride) {
   const uint64_t b = blockIdx.y;
-  pauli_body<true>(psi + b * len, lam + b * len, len, groups, ngroups, terms,
+  pauli_body<true, kPauliTB, kPauliRB>(psi + b * len, lam + b * len, len, groups, ngroups, terms,
                    partial + b * gridDim.x, counter + b, out + b * out_stride);
 }
 
@@ -518,25 +527,31 @@ void free_terms(DeviceTerms& t, cudaStream_t st) {
   t.terms = nullptr;
 }
 
-// Blocks of a Pauli kernel: a tile each, two a multiprocessor at most (or `most`).
-unsigned pauli_blocks(uint64_t len, int device, unsigned most = 0) {
+// Blocks of a Pauli kernel: a tile of 2^bits amplitudes each, `most` at most.
+unsigned pauli_blocks(uint64_t len, uint32_t bits, unsigned most) {
+  return (unsigned)std::min<uint64_t>((len + (1ULL << bits) - 1) >> bits, most);
+}
+
+template <bool STORE, uint32_t TB, uint32_t RB>
+void launch_pauli_t(dq_state_t h, double2* lam, const DeviceTerms& t, double* d_out) {
   int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  const uint64_t tiles = (len + (1u << kPauliTile) - 1) >> kPauliTile;
-  return (unsigned)std::min<uint64_t>(tiles, most ? most : 2u * (unsigned)sms);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  const unsigned blocks = pauli_blocks(h->len, TB + RB, (TB < 9 ? 4u : 2u) * (unsigned)sms);
+  k_pauli<STORE, TB, RB><<<blocks, 1 << TB, 0, h->stream>>>(h->amp, lam, h->len, t.groups, t.ngroups, t.terms,
+                                                            h->sc.d_partial, h->sc.d_counter, d_out);
+}
+
+template <bool STORE>
+int launch_pauli_s(dq_state_t h, double2* lam, const DeviceTerms& t, double* d_out) {
+  if (h->n <= kPauliSmallQubits) launch_pauli_t<STORE, kPauliSmallTB, 0>(h, lam, t, d_out);
+  else if (h->n <= kPauliMidQubits) launch_pauli_t<STORE, kPauliMidTB, 0>(h, lam, t, d_out);
+  else launch_pauli_t<STORE, kPauliTB, kPauliRB>(h, lam, t, d_out);
+  DQ_CUDA_TRY(cudaGetLastError());
+  return DQ_OK;
 }
 
 int launch_pauli(dq_state_t h, double2* lam, const DeviceTerms& t, double* d_out) {
-  const unsigned blocks = pauli_blocks(h->len, h->device);
-  if (lam)
-    k_pauli<true><<<blocks, kPauliThreads, 0, h->stream>>>(h->amp, lam, h->len, t.groups, t.ngroups,
-                                                         t.terms, h->sc.d_partial,
-                                                         h->sc.d_counter, d_out);
-  else
-    k_pauli<false><<<blocks, kPauliThreads, 0, h->stream>>>(h->amp, nullptr, h->len, t.groups,
-                                                          t.ngroups, t.terms, h->sc.d_partial,
-                                                          h->sc.d_counter, d_out);
-  DQ_CUDA_TRY(cudaGetLastError());
+  DQ_TRY(lam ? launch_pauli_s<true>(h, lam, t, d_out) : launch_pauli_s<false>(h, lam, t, d_out));
   return DQ_OK;
 }
 
@@ -903,7 +918,7 @@ int dq_adjoint_batch(int device, uint32_t n, const dq_inst* prog, uint64_t ninst
   unsigned* ctr = nullptr;
   uint8_t* fblob = nullptr;
   SweepJob* d_jobs = nullptr;
-  const unsigned pblocks = pauli_blocks(len, device, 64);
+  const unsigned pblocks = pauli_blocks(len, kPauliTB + kPauliRB, 64);
   const uint64_t sl = nslots + 1;  // per set: gradient slots, then E
   // all forward programs in one device buffer, staged in pinned host memory
   // (recycled across calls) by host threads
@@ -1007,7 +1022,7 @@ int dq_adjoint_batch(int device, uint32_t n, const dq_inst* prog, uint64_t ninst
     mark("forward enqueue");
     // lambda = H psi and E for every set of the group
     if (rc == DQ_OK) {
-      k_pauli_multi<<<dim3(pblocks, (unsigned)ng), kPauliThreads, 0, st>>>(
+      k_pauli_multi<<<dim3(pblocks, (unsigned)ng), 1 << kPauliTB, 0, st>>>(
           psi, lam, len, t.groups, t.ngroups, t.terms, part, ctr, slots + nslots, sl);
       cu(cudaGetLastError(), "k_pauli_multi");
       ++acc.launches;

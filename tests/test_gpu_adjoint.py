@@ -559,3 +559,26 @@ def test_alternating_gates_match_per_gate(gpu, n, ring):
     e2, g2 = adjoint_gradient(c, theta, H, exec="per_gate")
     assert abs(e1 - e2) < 1e-12
     assert np.max(np.abs(g1 - g2)) < 1e-11
+
+
+# the last and first sizes of each block size, and states of about one small block
+@pytest.mark.parametrize("n", [5, 6, 7, 15, 16, 17, 18])
+def test_pauli_block_sizes(gpu, n):
+    # 200 terms on unit-norm states: 1e-12 as above, and the same through the adjoint pass
+    rng = np.random.default_rng(n)
+    v = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    v /= np.linalg.norm(v)
+    H = random_observable(n, 200, seed=n)
+    terms = H.array()
+    st = nat.State(n, 0)
+    st.upload(v)
+    out = ctypes.c_double()
+    nat.check(nat.lib().dq_expval_pauli(st.handle, nat.ptr(terms), len(terms), ctypes.byref(out)))
+    assert abs(out.value - orc.expval_pauli(v, terms)) < 1e-12 * np.sum(np.abs(terms["coeff"]))
+    c = ParamCircuit(n)
+    for q in range(n):
+        c.ry(q, Param(q))
+    theta = rng.uniform(-3, 3, size=n)
+    e, g = adjoint_gradient(c, theta, H)
+    ps = orc.param_shift(c, theta, terms, occurrences=[0, n - 1])
+    assert np.max(np.abs(g[[0, n - 1]] - ps[[0, n - 1]])) < 1e-11 * np.sum(np.abs(terms["coeff"]))
