@@ -185,12 +185,13 @@ __global__ void __launch_bounds__(1 << TB, 1024 >> TB) k_pauli(const double2* __
 // The same for B states in one launch: state b (blockIdx.y) at psi + b len,
 // its lambda at lam + b len, its reduction scratch at partial + b gridDim.x
 // and counter + b, its expectation value at out[b * out_stride].
-__global__ void __launch_bounds__(1 << kPauliTB, 2) k_pauli_multi(const double2* __restrict__ psi, double2* __restrict__ lam,
+template <uint32_t TB, uint32_t RB>
+__global__ void __launch_bounds__(1 << TB, 1024 >> TB) k_pauli_multi(const double2* __restrict__ psi, double2* __restrict__ lam,
                               uint64_t len, const PauliGroup* __restrict__ groups, uint32_t ngroups,
                               const PauliTerm* __restrict__ terms, double* partial,
                               unsigned* counter, double* out, uint64_t out_stride) {
   const uint64_t b = blockIdx.y;
-  pauli_body<true, kPauliTB, kPauliRB>(psi + b * len, lam + b * len, len, groups, ngroups, terms,
+  pauli_body<true, TB, RB>(psi + b * len, lam + b * len, len, groups, ngroups, terms,
                    partial + b * gridDim.x, counter + b, out + b * out_stride);
 }
 
@@ -918,7 +919,12 @@ int dq_adjoint_batch(int device, uint32_t n, const dq_inst* prog, uint64_t ninst
   unsigned* ctr = nullptr;
   uint8_t* fblob = nullptr;
   SweepJob* d_jobs = nullptr;
-  const unsigned pblocks = pauli_blocks(len, kPauliTB + kPauliRB, 64);
+  // small blocks where the sets' tiles leave most of the device idle (whole calls, 2
+  // sets of 12 qubits and 1500 terms: 1.49 ms, 1.76 in tiles of 2^11; 8 sets 1.64 and
+  // 1.96; 32 sets of 14 qubits fill it)
+  const bool few_tiles = n <= 14 && pauli_blocks(len, kPauliTB + kPauliRB, 64) * G < 74;
+  const uint32_t ptb = !few_tiles ? kPauliTB : n <= 12 ? kPauliSmallTB : kPauliMidTB;
+  const unsigned pblocks = pauli_blocks(len, few_tiles ? ptb : kPauliTB + kPauliRB, 64);
   const uint64_t sl = nslots + 1;  // per set: gradient slots, then E
   // all forward programs in one device buffer, staged in pinned host memory
   // (recycled across calls) by host threads
@@ -1022,7 +1028,9 @@ int dq_adjoint_batch(int device, uint32_t n, const dq_inst* prog, uint64_t ninst
     mark("forward enqueue");
     // lambda = H psi and E for every set of the group
     if (rc == DQ_OK) {
-      k_pauli_multi<<<dim3(pblocks, (unsigned)ng), 1 << kPauliTB, 0, st>>>(
+      const auto kernel = ptb == kPauliTB ? k_pauli_multi<kPauliTB, kPauliRB>
+                          : ptb == kPauliMidTB ? k_pauli_multi<kPauliMidTB, 0> : k_pauli_multi<kPauliSmallTB, 0>;
+      kernel<<<dim3(pblocks, (unsigned)ng), 1 << ptb, 0, st>>>(
           psi, lam, len, t.groups, t.ngroups, t.terms, part, ctr, slots + nslots, sl);
       cu(cudaGetLastError(), "k_pauli_multi");
       ++acc.launches;

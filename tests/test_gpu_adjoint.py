@@ -582,3 +582,24 @@ def test_pauli_block_sizes(gpu, n):
     e, g = adjoint_gradient(c, theta, H)
     ps = orc.param_shift(c, theta, terms, occurrences=[0, n - 1])
     assert np.max(np.abs(g[[0, n - 1]] - ps[[0, n - 1]])) < 1e-11 * np.sum(np.abs(terms["coeff"]))
+
+
+# each block size of the batched observable, and both sides of its line
+@pytest.mark.parametrize("n,sets", [(10, 3), (12, 36), (12, 37), (13, 5), (14, 9), (14, 10), (15, 2)])
+def test_batched_observable_block_sizes(gpu, n, sets):
+    # the same sums in another order as set by set: as above
+    from dqsim_bosonic_b200.adjoint import adjoint_gradient_batch
+
+    rng = np.random.default_rng(n)
+    c = ParamCircuit(n)
+    for q in range(n):
+        c.ry(q, Param(q))
+    for q in range(n - 1):
+        c.cx(q, q + 1)
+    H = random_observable(n, 60, seed=n)
+    thetas = rng.uniform(-3, 3, size=(sets, n))
+    es, gs = adjoint_gradient_batch(c, thetas, H)
+    for b in sorted({0, sets // 2, sets - 1}):
+        e1, g1 = adjoint_gradient(c, thetas[b], H)
+        assert abs(es[b] - e1) < 1e-11
+        assert np.max(np.abs(gs[b] - g1)) < 1e-11
