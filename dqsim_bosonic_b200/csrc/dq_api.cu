@@ -17,7 +17,6 @@
 #include <map>
 #include <mutex>
 #include <new>
-#include <set>
 #include <string>
 #include <thread>
 #include <utility>
@@ -36,20 +35,16 @@ static thread_local std::string g_err;
 void set_error(const std::string& msg) { g_err = msg; }
 void clear_error() { g_err.clear(); }
 
-int allow_shared(const void* kernel) {
+int allow_shared(const void* kernel, size_t bytes) {
   int dev = 0;
   DQ_CUDA_TRY(cudaGetDevice(&dev));
   static std::mutex mu;
-  static std::set<std::pair<int, const void*>> done;
+  static std::map<std::pair<int, const void*>, size_t> limit;
   std::lock_guard<std::mutex> lk(mu);
-  if (done.count({dev, kernel})) return DQ_OK;
-  int most = 0;
-  cudaFuncAttributes fa{};
-  DQ_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  DQ_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
-  DQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   most - (int)fa.sharedSizeBytes));
-  done.insert({dev, kernel});
+  size_t& have = limit[{dev, kernel}];
+  if (bytes <= have) return DQ_OK;
+  DQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  have = bytes;
   return DQ_OK;
 }
 

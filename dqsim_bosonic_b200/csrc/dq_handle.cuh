@@ -58,10 +58,10 @@ struct DeviceGuard {
 // Device buffers of state size are recycled through a per-(device, size) cache.
 int cache_alloc(int device, size_t bytes, void** out);
 void cache_free(int device, size_t bytes, void* p);
-// Lets a kernel use all of a block's shared memory on the current device.  Set
-// once: the limit belongs to the kernel, and launches of other threads and
-// handles with other sizes share it.
-int allow_shared(const void* kernel);
+// Lets a kernel's launches on the current device use `bytes` of dynamic shared
+// memory.  The limit belongs to the kernel and is only ever raised: launches of
+// other threads and handles with other sizes share it.
+int allow_shared(const void* kernel, size_t bytes);
 // Whether the thread's limit (dq_debug_alloc_limit) refuses an allocation.
 bool alloc_refused(size_t bytes);
 // Device memory a call may try to allocate before it asks how much is free (a

@@ -1560,9 +1560,15 @@ int alloc_buffers(dq_mps_s* h, uint32_t batch, uint32_t cap, uint32_t ncb) {
   DQ_TRY(mps_take(h, 5, sizeof(int) * 4));
   DQ_TRY(mps_take(h, 6, sizeof(unsigned long long)));
   DQ_TRY(mps_take(h, 7, sizeof(double2) * h->scratch_elems * h->slots * batch));
-  for (const void* k : {(const void*)k_mps_measure_warp, (const void*)k_mps_2q_warp, (const void*)k_mps_2q,
-                        (const void*)k_mps_measure, (const void*)k_mps_2q_cl})
-    DQ_TRY(allow_shared(k));
+  if (cap <= kWarpCap) {
+    DQ_TRY(allow_shared((const void*)k_mps_measure_warp, kRepsPer2q * warp_measure_bytes(cap)));
+    DQ_TRY(allow_shared((const void*)k_mps_2q_warp, kRepsPer2q * warp_work_bytes(cap)));
+  }
+  if (h->smem) {
+    DQ_TRY(allow_shared((const void*)k_mps_2q, work_bytes));
+    DQ_TRY(allow_shared((const void*)k_mps_measure, work_bytes));
+  }
+  DQ_TRY(allow_shared((const void*)k_mps_2q_cl, kMaxSmem));
   return DQ_OK;
 }
 

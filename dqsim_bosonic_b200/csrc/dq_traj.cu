@@ -1231,7 +1231,7 @@ struct TrajLaunch {
 
 template <int THREADS>
 int config_traj_t(uint32_t C, size_t smem, uint64_t nitems, TrajLaunch* L) {
-  DQ_TRY(allow_shared((const void*)k_traj<THREADS>));
+  DQ_TRY(allow_shared((const void*)k_traj<THREADS>, smem));
   L->attr[0].id = cudaLaunchAttributeClusterDimension;
   L->attr[0].val.clusterDim.x = C;
   L->attr[0].val.clusterDim.y = 1;
@@ -1545,7 +1545,7 @@ int geometry(uint32_t n, uint32_t max_span, uint32_t force_lb, uint32_t* lb, uin
 // p1 back costs about 3 us a gate and 20 us a measurement instead.
 template <int THREADS>
 int launch_small(size_t smem, const TrajParams& P, cudaStream_t st) {
-  DQ_TRY(allow_shared((const void*)k_traj<THREADS>));
+  DQ_TRY(allow_shared((const void*)k_traj<THREADS>, smem));
   k_traj<THREADS><<<1, THREADS, smem, st>>>(P);
   DQ_CUDA_TRY(cudaGetLastError());
   return DQ_OK;
